@@ -1,0 +1,469 @@
+// The kernels around the grouped expert GEMMs: x rows packed for the tensor cores, the dense router, top-k with the
+// grouping of the (token, expert) pairs, activation rows of the wide-range mode, and the per-token reduction.
+#pragma once
+
+#include "batch_path.h"
+#include "decode_kernels.cuh"
+#include "tcgen05.cuh"
+
+namespace nvmai {
+
+constexpr uint32_t kBpNotLocal = 0xFFFFFFFFu;
+
+// ---- x rows ---------------------------------------------------------------------------------
+// One block per row, 8 values per thread: the row in the weights' K order, the sums of its 64-value groups as fp16
+// hi + lo behind it ([hi | lo | hi | 0], see expert_gemm.cuh), and the scalar gate of the row (the row is in registers
+// anyway; as a launch of its own the gate took 17-31 us).
+__global__ void __launch_bounds__(256) pack_x_kernel(PackXParams p) {
+    __shared__ float wsum[8];
+    pdl_wait();
+    pdl_launch_dependents();
+    const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    const size_t row = blockIdx.x;
+    const uint32_t extra = bp_extra_cols(p.n, 1), G = p.n / 64u;
+    const size_t stride = (size_t)p.n + extra;
+    __half *dst = p.dst + row * stride, *dst2 = p.dst2 != nullptr ? p.dst2 + row * stride : nullptr;
+    float gate = 0.0f;
+    for (uint32_t base = 0; base < p.n; base += 2048u) {
+        const uint32_t i8 = base + tid * 8u;
+        float part = 0.0f;
+        if (i8 < p.n) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(p.x + row * p.n + i8);
+            // natural (0,1)(2,3)(4,5)(6,7) -> (0,4)(1,5)(2,6)(3,7), the order of bp_k_order
+            const uint4 perm = make_uint4(__byte_perm(q.x, q.z, 0x5410), __byte_perm(q.x, q.z, 0x7632),
+                                          __byte_perm(q.y, q.w, 0x5410), __byte_perm(q.y, q.w, 0x7632));
+            *reinterpret_cast<uint4 *>(dst + i8) = p.permute ? perm : q;
+            if (dst2 != nullptr) *reinterpret_cast<uint4 *>(dst2 + i8) = p.permute ? q : perm;
+            const __half2 *h = reinterpret_cast<const __half2 *>(&q);
+            float f[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { const float2 t = __half22float2(h[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) part += f[i];
+            if (p.gate_row != nullptr) {
+                const uint4 w = __ldg(reinterpret_cast<const uint4 *>(p.gate_row + i8));
+                const __half2 *wh = reinterpret_cast<const __half2 *>(&w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 t = __half22float2(wh[i]);
+                    gate = fmaf(t.x, f[2 * i], gate);
+                    gate = fmaf(t.y, f[2 * i + 1], gate);
+                }
+            }
+        }
+        part += __shfl_xor_sync(0xffffffffu, part, 1);       // a group = 8 neighbouring lanes
+        part += __shfl_xor_sync(0xffffffffu, part, 2);
+        part += __shfl_xor_sync(0xffffffffu, part, 4);
+        if (i8 < p.n && (lane & 7u) == 0u) {
+            const float sum = part * kBpSumScale;
+            const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
+            const uint32_t g = i8 / 64u;
+            dst[p.n + g] = hi; dst[p.n + G + g] = lo; dst[p.n + 2u * G + g] = hi;
+            if (dst2 != nullptr) { dst2[p.n + g] = hi; dst2[p.n + G + g] = lo; dst2[p.n + 2u * G + g] = hi; }
+        }
+    }
+    for (uint32_t i = 3u * G + tid; i < extra; i += 256u) {
+        dst[p.n + i] = __float2half_rn(0.0f);
+        if (dst2 != nullptr) dst2[p.n + i] = __float2half_rn(0.0f);
+    }
+    if (p.gate_row != nullptr) {
+        gate = warp_sum(gate);
+        if (lane == 0) wsum[tid >> 5] = gate;
+        __syncthreads();
+        if (tid == 0) {
+            float tot = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) tot += wsum[i];
+            p.gate_val[row] = p.out_half ? round_f16(tot) : round11(tot);
+        }
+    }
+}
+
+// ---- dense router ---------------------------------------------------------------------------
+// logits[split][token][expert]: 128 router rows x 64 token rows per block, K split over blockIdx.z so that a small
+// batch still spreads over the chip (one block per 256 tokens took 20-29 us at any batch size).  Products of two fp16
+// values are exact in fp32: only the order of the additions differs from the decode router's.
+constexpr uint32_t kRouterStages = 4;
+constexpr uint32_t kRouterStageBytes = 128 * 128 + kRouterTileTokens * 128;
+constexpr size_t kRouterSmem = 2048 + kRouterStages * kRouterStageBytes;
+struct RouterBarriers { uint64_t full[kRouterStages], empty[kRouterStages], done; uint32_t tmem_slot; };
+
+__global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant__ RouterArgs args) {
+    extern __shared__ unsigned char rt_smem_raw[];
+    const RouterParams &p = args.p;
+    const uint32_t raw = smem_addr(rt_smem_raw), base = (raw + 1023u) & ~1023u;
+    RouterBarriers *bars = reinterpret_cast<RouterBarriers *>(rt_smem_raw + (base - raw));
+    const uint32_t ring = base + 1024u;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < kRouterStages; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 1); }
+        mbar_init(&bars->done, 1);
+        mbar_fence_init();
+    }
+    if (warp == 1) { tmem_alloc(&bars->tmem_slot, kRouterTileTokens); tmem_relinquish(); }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&bars->tmem_slot);
+    // x was complete before the kernel in front of this one (which packs it) could pass its own wait
+    const uint32_t n_kb = p.kdim / 64u / p.splits, kb0 = blockIdx.z * n_kb;
+    const uint32_t e0 = blockIdx.x * 128u, t0 = blockIdx.y * kRouterTileTokens;
+    bool ok = *reinterpret_cast<volatile unsigned int *>(p.status) == 0u;
+    ok = __syncthreads_and(ok);
+    if (warp == 0) {
+        if (elect_one()) {
+            for (uint32_t k = 0; k < n_kb && ok; ++k) {
+                const uint32_t s = k % kRouterStages, st = ring + s * kRouterStageBytes;
+                ok = mbar_wait(&bars->empty[s], ((k / kRouterStages) & 1u) ^ 1u, p.status);
+                if (!ok) break;
+                mbar_expect_tx(&bars->full[s], kRouterStageBytes);
+                tma_load_2d(st, &args.w, (kb0 + k) * 64u, e0, &bars->full[s]);
+                tma_load_2d(st + 128u * 128u, &args.x, (kb0 + k) * 64u, t0, &bars->full[s]);
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (elect_one()) {
+            const uint32_t idesc = umma_idesc_f16(128u, kRouterTileTokens);
+            for (uint32_t k = 0; k < n_kb && ok; ++k) {
+                const uint32_t s = k % kRouterStages, st = ring + s * kRouterStageBytes;
+                ok = mbar_wait(&bars->full[s], (k / kRouterStages) & 1u, p.status);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint64_t da = umma_desc_sw128(st), db = umma_desc_sw128(st + 128u * 128u);
+#pragma unroll
+                for (uint32_t j = 0; j < 4u; ++j) umma_f16_ss(tmem, da + 2u * j, db + 2u * j, idesc, (k | j) != 0u);
+                umma_commit(&bars->empty[s]);
+            }
+            if (ok) umma_commit(&bars->done);
+        }
+        __syncwarp();
+    }
+    if (ok) ok = mbar_wait(&bars->done, 0, p.status);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+        tc_fence_after_sync();
+        float *out = p.logits + ((size_t)blockIdx.z * p.tokens + t0) * p.experts + e0 + warp * 32u + lane;
+        for (uint32_t cb = 0; cb < kRouterTileTokens && t0 + cb < p.tokens; cb += 8u) {
+            uint32_t r[8];
+            tmem_ld8(tmem + ((warp * 32u) << 16) + cb, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; ++i)
+                if (t0 + cb + i < p.tokens) out[(size_t)(cb + i) * p.experts] = __uint_as_float(r[i]);
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, kRouterTileTokens);
+    pdl_wait();                     // the kernel after this one relies on the one before it being complete
+    pdl_launch_dependents();
+}
+
+// ---- top-k and grouping -----------------------------------------------------------------------
+// Tokens per block: 8 up to 1024 tokens (a warp per token), 32 above, so that the last block scans at most 128
+// histograms for a chunk of 4096.
+__host__ __device__ constexpr uint32_t bp_tokens_per_block(uint32_t tokens) { return tokens <= 1024u ? 8u : 32u; }
+
+// Router semantics of router_topk_select_k8 (moe.metal:233-285); the pairs end up in (expert, token, rank) order, as
+// PrefillMoEGrouping.groupTokenExpertPairs has them (PrefillMoEGrouping.swift:90-192).
+__global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
+    __shared__ uint32_t hist[kMaxExperts];
+    __shared__ uint32_t warp_tot[3][kMaxExperts / 32];
+    __shared__ bool last;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    hist[tid] = 0;
+    pdl_wait();
+    pdl_launch_dependents();
+    __syncthreads();
+    const uint32_t tpb = bp_tokens_per_block(p.tokens);
+    for (uint32_t t = warp; t < tpb; t += 8u) {
+        const uint32_t tok = blockIdx.x * tpb + t;
+        if (tok >= p.tokens) break;
+        if (p.logits != nullptr) {
+            float v[kMaxExperts / 32];
+#pragma unroll
+            for (int i = 0; i < kMaxExperts / 32; ++i) v[i] = lane + 32u * i < p.E ? 0.0f : -INFINITY;
+            for (uint32_t sp = 0; sp < p.splits; sp += 2u) {          // 16 loads in flight
+                const float *l0 = p.logits + ((size_t)sp * p.tokens + tok) * p.E;
+                const bool two = sp + 1u < p.splits;
+                float a[2][kMaxExperts / 32];
+#pragma unroll
+                for (int i = 0; i < kMaxExperts / 32; ++i) {
+                    const uint32_t e = lane + 32u * i;
+                    a[0][i] = e < p.E ? __ldcg(l0 + e) : 0.0f;
+                    a[1][i] = e < p.E && two ? __ldcg(l0 + (size_t)p.tokens * p.E + e) : 0.0f;
+                }
+#pragma unroll
+                for (int i = 0; i < kMaxExperts / 32; ++i) { v[i] += a[0][i]; if (two) v[i] += a[1][i]; }
+            }
+            topk_softmax_warp_vals(v, (int)p.E, (int)p.K, p.pes, p.idx + (size_t)tok * p.K, p.w + (size_t)tok * p.K);
+        }
+        if ((uint32_t)lane < p.K) {
+            const uint32_t g = min(p.idx[(size_t)tok * p.K + lane], p.E - 1u);
+            const uint32_t e = p.expert_map != nullptr ? p.expert_map[g] : g;
+            if (e != kBpNotLocal) atomicAdd(&hist[e], 1u);
+        }
+    }
+    __syncthreads();
+    p.block_hist[(size_t)blockIdx.x * kMaxExperts + tid] = hist[tid];
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(p.counter, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!last) return;
+    // thread e owns expert e: total, exclusive scans of the pairs and of both launches' work items
+    __threadfence();
+    if (tid == 0) *p.counter = 0u;
+    uint32_t total = 0;
+#pragma unroll 8
+    for (uint32_t b = 0; b < gridDim.x; ++b) total += __ldcg(p.block_hist + (size_t)b * kMaxExperts + tid);
+    uint32_t mine[3] = {total, (total + p.cap[0] - 1u) / p.cap[0], (total + p.cap[1] - 1u) / p.cap[1]}, pre[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        pre[j] = mine[j];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, pre[j], o);
+            if (lane >= o) pre[j] += v;
+        }
+        if (lane == 31) warp_tot[j][warp] = pre[j];
+    }
+    __syncthreads();
+    uint32_t all[3] = {0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        pre[j] -= mine[j];
+        for (int w = 0; w < kMaxExperts / 32; ++w) {
+            if (w < warp) pre[j] += warp_tot[j][w];
+            all[j] += warp_tot[j][w];
+        }
+    }
+    // an expert's rows are split evenly over its items (two items of 70 instead of 128 + 12)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const uint32_t items = mine[1 + j], even = items ? total / items : 0u, extra = items ? total % items : 0u;
+        for (uint32_t i = 0; i < items; ++i)
+            p.work[j][pre[1 + j] + i] = WorkItem{(uint32_t)tid, pre[0] + i * even + min(i, extra), even + (i < extra ? 1u : 0u), 0u};
+        if (tid == 0) p.n_work[j][0] = all[1 + j];
+    }
+    uint32_t run = pre[0];
+#pragma unroll 8
+    for (uint32_t b = 0; b < gridDim.x; ++b) {
+        const uint32_t c = __ldcg(p.block_hist + (size_t)b * kMaxExperts + tid);
+        p.block_hist[(size_t)b * kMaxExperts + tid] = run;
+        run += c;
+    }
+}
+
+// stable scatter of a block's pairs
+__global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
+    __shared__ uint16_t cnt[8][kMaxExperts];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) cnt[w][tid] = 0;
+    pdl_wait();
+    pdl_launch_dependents();
+    const uint32_t tpb = bp_tokens_per_block(p.tokens), pairs = tpb * p.K, first = blockIdx.x * pairs;     // <= 256 pairs
+    const uint32_t i = first + tid, P = p.tokens * p.K;
+    uint32_t e = kBpNotLocal;
+    const bool mine = (uint32_t)tid < pairs && i < P;
+    if (mine) {
+        const uint32_t g = min(p.idx[i], p.E - 1u);
+        e = p.expert_map != nullptr ? p.expert_map[g] : g;
+    }
+    const bool live = e != kBpNotLocal;
+    if (mine && !live) p.inv[i] = kBpNotLocal;
+    const uint32_t peers = __match_any_sync(0xffffffffu, e);
+    const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+    __syncthreads();
+    if (live && rank == 0u) cnt[warp][e] = (uint16_t)__popc(peers);
+    __syncthreads();
+    if (live) {
+        uint32_t pos = p.block_hist[(size_t)blockIdx.x * kMaxExperts + e] + rank;
+        for (int w = 0; w < warp; ++w) pos += cnt[w][e];
+        p.sorted_pair[pos] = i;
+        p.inv[i] = pos;
+    }
+}
+
+// ---- wide-range activation rows ------------------------------------------------------------------
+// One warp per row: fp32 rows scaled by a power of two that brings the row's largest magnitude to [2^14, 2^15), so
+// that the fp16 copy neither overflows nor loses its small entries to subnormals (the down GEMM's epilogue multiplies
+// the factor back), in the down weights' K order, with half-group sums.
+__global__ void __launch_bounds__(256) pack_acts_kernel(PackActsParams p) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const uint32_t row = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    const bool second = row >= p.rows;
+    const uint32_t r = second ? row - p.rows : row;
+    if (second && r >= p.rows2) return;
+    const uint32_t n = second ? p.n2 : p.n, permute = second ? p.permute2 : p.permute;
+    const float *src = (second ? p.src2 : p.src) + (size_t)r * n;
+    const uint32_t extra = bp_extra_cols(n, 2), slots = n / 32u;
+    __half *dst = (second ? p.dst2 : p.dst) + (size_t)r * (n + extra);
+    constexpr int kKeep = 4;                 // 256 values per pass; up to 1024 stay in registers between the two passes
+    float4 keep[kKeep][2];
+    float m = 0.0f;
+    auto load = [&](uint32_t i8, float4 (&v)[2]) {
+        const float4 *s4 = reinterpret_cast<const float4 *>(src + i8);
+        v[0] = s4[0]; v[1] = s4[1];
+    };
+    auto peak = [&](const float4 (&v)[2]) {
+        const float *f = reinterpret_cast<const float *>(v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { const float a = fabsf(f[i]); m = (a <= 3.0e38f && a > m) ? a : m; }   // not inf, not NaN
+    };
+#pragma unroll
+    for (int k = 0; k < kKeep; ++k) {
+        const uint32_t i8 = k * 256u + lane * 8u;
+        if (i8 < n) { load(i8, keep[k]); peak(keep[k]); }
+    }
+    for (uint32_t i8 = kKeep * 256u + lane * 8u; i8 < n; i8 += 256u) { float4 v[2]; load(i8, v); peak(v); }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    int e = 0;
+    if (m > 0.0f) frexpf(m, &e);                          // m = f * 2^e, f in [0.5, 1)
+    const int shift = m > 0.0f ? 15 - e : 0;
+    const float mul = ldexpf(1.0f, shift);
+    if (lane == 0) (second ? p.row_scale2 : p.row_scale)[r] = ldexpf(1.0f, -shift);
+    auto put = [&](uint32_t base, const float4 (&v)[2]) {
+        const uint32_t i8 = base + lane * 8u;
+        float part = 0.0f;
+        if (i8 < n) {
+            const float *f = reinterpret_cast<const float *>(v);
+            __half h[8], o[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { h[i] = __float2half_rn(f[i] * mul); part += __half2float(h[i]); }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = permute ? h[bp_k_order(i)] : h[i];
+            *reinterpret_cast<uint4 *>(dst + i8) = *reinterpret_cast<const uint4 *>(o);
+        }
+        part += __shfl_xor_sync(0xffffffffu, part, 1);     // half a group = 4 neighbouring lanes
+        part += __shfl_xor_sync(0xffffffffu, part, 2);
+        if (i8 < n && (lane & 3u) == 0u) {
+            const float sum = part * kBpSumScale;
+            const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
+            const uint32_t s = i8 / 32u;
+            dst[n + s] = hi; dst[n + slots + s] = lo; dst[n + 2u * slots + s] = hi;
+        }
+    };
+#pragma unroll
+    for (int k = 0; k < kKeep; ++k)
+        if (k * 256u < n) put(k * 256u, keep[k]);
+    for (uint32_t base = kKeep * 256u; base < n; base += 256u) {
+        float4 v[2] = {};
+        if (base + lane * 8u < n) load(base + lane * 8u, v);
+        put(base, v);
+    }
+}
+
+// ---- per-token reduction ----------------------------------------------------------------------
+// aligned: the caller's pointer is 16-byte aligned (i always is a multiple of 8)
+template <int OUT> __device__ __forceinline__ void load_out8(const void *p, size_t i, float (&v)[8], bool aligned = true) {
+    if (!aligned) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = load_out<OUT>(p, i + k);
+    } else if (OUT == OUT_F16) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(static_cast<const __half *>(p) + i);
+        const __half2 *h = reinterpret_cast<const __half2 *>(&q);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { const float2 t = __half22float2(h[k]); v[2 * k] = t.x; v[2 * k + 1] = t.y; }
+    } else {
+        const float4 *f = reinterpret_cast<const float4 *>(static_cast<const float *>(p) + i);
+        const float4 a = f[0], b = f[1];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+}
+template <int OUT> __device__ __forceinline__ void store_out8(void *p, size_t i, const float (&v)[8], bool aligned = true) {
+    if (!aligned) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) store_out<OUT>(p, i + k, v[k]);
+    } else if (OUT == OUT_F16) {
+        uint4 q;
+        uint32_t *w = reinterpret_cast<uint32_t *>(&q);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { const __half2 h = __floats2half2_rn(v[2 * k], v[2 * k + 1]); w[k] = *reinterpret_cast<const uint32_t *>(&h); }
+        *reinterpret_cast<uint4 *>(static_cast<__half *>(p) + i) = q;
+    } else {
+        float4 *f = reinterpret_cast<float4 *>(static_cast<float *>(p) + i);
+        f[0] = make_float4(v[0], v[1], v[2], v[3]);
+        f[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
+
+// One block per token, 8 values per thread; every slot's partial row is requested before any is used (the version that
+// walked the slots value by value took 19-23 us for any batch).  Slot order, so the result does not depend on the
+// grouping.  PART: type of the partial rows.  Prefill rounding (prefill.metal:437-458, RealForwardRunner.swift:3560-3569):
+// every partial is rounded to the output type, h2 = out(sum_r fma(w, partial)) on its own, and the residual takes two
+// steps: hidden = out(out(hidden + h1) + h2).  Decode order: one rounding of h1 + sum, one residual add.
+template <int OUT, int PART>
+__global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) {
+    __shared__ uint32_t pos[kMaxTopK];
+    __shared__ float wk[kMaxTopK];
+    pdl_wait();
+    pdl_launch_dependents();
+    const uint32_t tok = blockIdx.x;
+    if (threadIdx.x < p.K) {
+        pos[threadIdx.x] = p.inv[tok * p.K + threadIdx.x];
+        wk[threadIdx.x] = __half2float(p.routing_w[tok * p.K + threadIdx.x]);
+    }
+    __syncthreads();
+    const float gate = p.gate_val != nullptr ? p.gate_val[tok] : 0.0f;
+    for (uint32_t d = threadIdx.x * 8u; d < p.D; d += 2048u) {
+        const size_t i = (size_t)tok * p.D + d;
+        float v[kMaxTopK][8];
+#pragma unroll
+        for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
+            if (r < p.K && pos[r] != kBpNotLocal) load_out8<PART>(p.partial, (size_t)pos[r] * p.D + d, v[r]);
+        if (p.partial_y != nullptr) {          // expert parallelism: this rank's share of the sum
+            float acc[8] = {};
+#pragma unroll
+            for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
+                if (r < p.K && pos[r] != kBpNotLocal)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[k] += wk[r] * v[r][k];
+            store_out8<OUT_F32>(p.partial_y, i, acc, p.aligned);
+            continue;
+        }
+        float h1[8] = {};
+        if (p.shared_partial != nullptr) {
+            if (p.shared_half) load_out8<OUT_F16>(p.shared_partial, i, h1); else load_out8<OUT_F32>(p.shared_partial, i, h1);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                h1[k] = round_out<OUT>(h1[k]);
+                if (p.gate_val != nullptr) h1[k] = round_out<OUT>(sigmoid_div(h1[k], gate));
+            }
+        }
+        float y[8], hid[8] = {}, delta[8] = {};
+        if (p.hidden != nullptr) load_out8<OUT>(p.hidden, i, hid, p.aligned);
+        if (p.prefill) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                float h2 = 0.0f;
+#pragma unroll
+                for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
+                    if (r < p.K) h2 = fmaf(wk[r], round_out<OUT>(v[r][k]), h2);
+                h2 = round_out<OUT>(h2);
+                y[k] = h1[k] + h2;
+                hid[k] = round_out<OUT>(hid[k] + h1[k]) + h2;
+            }
+        } else {
+            if (p.hidden_delta != nullptr) load_out8<OUT_F16>(p.hidden_delta, i, delta, p.aligned);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                float acc = h1[k];
+#pragma unroll
+                for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
+                    if (r < p.K) acc += wk[r] * v[r][k];
+                y[k] = round_out<OUT>(acc);
+                if (p.hidden_delta != nullptr) hid[k] = round_out<OUT>(hid[k] + delta[k]);
+                hid[k] += y[k];
+            }
+        }
+        if (p.y != nullptr) store_out8<OUT>(p.y, i, y, p.aligned);
+        if (p.hidden != nullptr) store_out8<OUT>(p.hidden, i, hid, p.aligned);
+    }
+}
+
+}  // namespace nvmai

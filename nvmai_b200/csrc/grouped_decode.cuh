@@ -5,14 +5,13 @@
 // weighted sum over a token's 8 experts is taken afterwards in rank order, so the
 // result does not depend on how pairs were grouped.
 #pragma once
+#include "batch_path.h"
 #include "staged_decode.cuh"
 
 namespace nvmai {
 
 constexpr int kPairsPerItem = 8;
 constexpr uint32_t kSharedExpertId = 0xFFFFFFFFu;
-
-struct WorkItem { uint32_t expert, start, count, pad; };
 
 // PrefillTokenExpertPair (PrefillRouter.swift:4-28): 16 bytes, fields at 0/4/8/12.
 struct TokenExpertPair { uint32_t token, expert, rank, weight_bits; };

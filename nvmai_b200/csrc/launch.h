@@ -1,0 +1,51 @@
+// Kernel launches of the library's translation units.
+#pragma once
+#include <cuda_runtime.h>
+#include <map>
+#include <mutex>
+#include <utility>
+
+namespace nvmai {
+
+// Kernels here use more than the default 48 KB of dynamic shared memory; the
+// opt-in is per function and sticky, so it is raised once per (function, size).
+template <typename Kern>
+inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
+    // the attribute is per device and handles may be driven from several host threads
+    static std::map<std::pair<int, const void *>, size_t> granted;
+    static std::mutex guard;
+    int dev = 0;
+    cudaError_t de = cudaGetDevice(&dev);
+    if (de != cudaSuccess) return de;
+    std::lock_guard<std::mutex> lock(guard);
+    const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kern));
+    auto it = granted.find(key);
+    if (it != granted.end() && it->second >= bytes) return cudaSuccess;
+    if (bytes > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+    }
+    granted[key] = bytes;
+    return cudaSuccess;
+}
+
+// pdl: launch with programmatic stream serialization, so that the kernel's
+// prologue (its weight copies) may overlap the previous kernel's tail.
+template <typename Kern, typename... Params>
+inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
+    cudaError_t e = ensure_smem(kern, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, p...);
+}
+
+}  // namespace nvmai

@@ -9,6 +9,7 @@
 #include <fcntl.h>
 #include <unistd.h>
 #include <cerrno>
+#include <cmath>
 #include <chrono>
 
 #include <algorithm>
@@ -23,12 +24,14 @@
 #include <tuple>
 #include <vector>
 
+#include "batch_path.h"
 #include "ep_comm.cuh"
 #include "grouped_decode.cuh"
+#include "launch.h"
 #include "misc_kernels.cuh"
 #include "persistent_batch.cuh"
 #include "persistent_decode.cuh"
-#include "prefill_gemm.cuh"
+#include "tcgen05.cuh"
 
 using namespace nvmai;
 
@@ -38,6 +41,9 @@ struct LayerViews {
     bool registered = false;
     nvmai_cuda_moe_layer w{};
     std::vector<void *> owned;      // aligned copies of resident tensors whose base was not 16-byte aligned
+    // the packed codes (and a dense router) as tensor maps, made by the first call that runs the expert GEMMs
+    bool tc_maps = false;
+    CUtensorMap gate, up, down, sgate, sup, sdown, router;
 };
 
 struct StackGraphKey {
@@ -93,12 +99,17 @@ struct nvmai_cuda_moe {
     // prefill chunks on the tensor cores (default); NVMAI_CUDA_PREFILL_TC=0 sends them through the exact grouped
     // kernels of the batched decode path instead
     bool prefill_tc = true;
-    // prefill GEMMs: fp16 operand copies (allocated by the first prefill call)
-    __half *pf_x = nullptr;          // [T*K][D] x rows gathered into sorted pair order, in the weights' K order
-    __half *pf_xn = nullptr;         // [T][D] x rows in token order (shared expert), in its weights' K order
-    __half *pf_acts16 = nullptr;     // [T*K][F] routed activations as the down GEMM reads them
-    __half *pf_sacts16 = nullptr;    // [T][Fs] the shared expert's
+    // expert GEMMs: operand rows and routing scratch (allocated by the first call that takes them)
+    __half *pf_x = nullptr;          // [T][D + extra] x rows in the routed weights' K order, with their group sums
+    __half *pf_xs = nullptr;         // the same in the shared expert's K order, when that differs
+    __half *pf_acts16 = nullptr;     // [T*K][F + extra] routed activations as the down GEMM reads them
+    __half *pf_sacts16 = nullptr;    // [T][Fs + extra] the shared expert's
     float *pf_rowscale = nullptr, *pf_srowscale = nullptr;   // per row: power of two taken out of a wide-range row
+    float *pf_logits = nullptr;      // [splits][T][E]
+    uint32_t *pf_hist = nullptr;     // [routing blocks][256]
+    WorkItem *pf_work2 = nullptr;    // the down GEMM's work list (h->work is the gate/up GEMM's)
+    unsigned int *pf_counter = nullptr;
+    CUtensorMap map_acts, map_sacts;
     // expert parallelism over NCCL: communicator and exchange buffers
     NcclComm ep_comm = nullptr;
     uint32_t ep_rank = 0, ep_world = 0, ep_rows_own = 0;
@@ -236,47 +247,16 @@ int dispatch_bits_meta(uint32_t bits, uint32_t meta, F &&f) {
 
 // ---- stage launchers ---------------------------------------------------------
 
-// Kernels here use more than the default 48 KB of dynamic shared memory; the
-// opt-in is per function and sticky, so it is raised once per (function, size).
-template <typename Kern>
-cudaError_t ensure_smem(Kern kern, size_t bytes) {
-    // the attribute is per device and handles may be driven from several host threads
-    static std::map<std::pair<int, const void *>, size_t> granted;
-    static std::mutex guard;
-    int dev = 0;
-    cudaError_t de = cudaGetDevice(&dev);
-    if (de != cudaSuccess) return de;
-    std::lock_guard<std::mutex> lock(guard);
-    const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kern));
-    auto it = granted.find(key);
-    if (it != granted.end() && it->second >= bytes) return cudaSuccess;
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-    }
-    granted[key] = bytes;
-    return cudaSuccess;
-}
-
-// pdl: launch with programmatic stream serialization, so that the kernel's
-// prologue (its weight copies) may overlap the previous kernel's tail.
 template <typename Kern, typename... Params>
 int launch_kernel(nvmai_cuda_moe *h, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
                   const Params &...p) {
-    cudaError_t e = ensure_smem(kern, smem);
-    if (e != cudaSuccess) return record(h, e);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, kern, p...);
+    cudaError_t e = launch_pdl(kern, grid, block, smem, st, pdl, p...);
     g_launches.fetch_add(1, std::memory_order_relaxed);
+    return record(h, e);
+}
+// a launch made by batch_path.cu
+int launched(nvmai_cuda_moe *h, cudaError_t e, uint64_t launches = 1) {
+    g_launches.fetch_add(launches, std::memory_order_relaxed);
     return record(h, e);
 }
 
@@ -582,26 +562,13 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
 }
 
 // ---- prefill: grouped GEMMs on the tensor cores ----------------------------------
-int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
-    if (h->pf_acts16) return NVMAI_CUDA_OK;
-    // the first prefill call allocates; a stream under capture forbids that: make one eager call first
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (st != nullptr && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
-        cudaGetLastError();
-        return NVMAI_CUDA_EINVAL;
-    }
+// Splits of the router's K over blocks: as many as still fill the chip once.
+uint32_t router_splits(const nvmai_cuda_moe *h, uint32_t tokens) {
     const auto &c = h->cfg;
-    const size_t T = c.max_tokens, P = T * c.top_k;
-    auto alloc = [&](auto **ptr, size_t bytes) { return cudaMalloc(reinterpret_cast<void **>(ptr), bytes ? bytes : 16) == cudaSuccess; };
-    const size_t dx = c.d + pf_extra_cols(c.d), fx = c.f + pf_extra_cols(c.f), sfx = c.shared_f + pf_extra_cols(c.shared_f);
-    if (alloc(&h->pf_x, P * dx * 2) && alloc(&h->pf_xn, T * dx * 2) && alloc(&h->pf_acts16, P * fx * 2) &&
-        alloc(&h->pf_sacts16, T * sfx * 2) && alloc(&h->pf_rowscale, P * 4) && alloc(&h->pf_srowscale, T * 4))
-        return NVMAI_CUDA_OK;
-    cudaGetLastError();
-    cudaFree(h->pf_x); cudaFree(h->pf_xn); cudaFree(h->pf_acts16); cudaFree(h->pf_sacts16); cudaFree(h->pf_rowscale);
-    cudaFree(h->pf_srowscale);
-    h->pf_x = h->pf_xn = h->pf_acts16 = h->pf_sacts16 = nullptr; h->pf_rowscale = h->pf_srowscale = nullptr;
-    return NVMAI_CUDA_ENOMEM;
+    const uint32_t tiles = (c.num_experts / 128) * ((tokens + kRouterTileTokens - 1) / kRouterTileTokens);
+    uint32_t s = 1;
+    while (s < 16 && 2 * s * tiles <= (uint32_t)h->sm_count && (c.d / 64) % (2 * s) == 0) s *= 2;
+    return s;
 }
 
 // cuTensorMapEncodeTiled, looked up through the runtime (the library does not link libcuda)
@@ -620,16 +587,15 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Tensor map over fp16 rows [rows][cols] (row stride in elements), box = 64 values x box_rows rows, 128-byte
-// swizzle, zero fill outside.  Base and row stride must be 16-byte multiples.
-int make_rows_tmap(nvmai_cuda_moe *h, CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint64_t stride_elems,
-                   uint32_t box_rows) {
+// Tensor map over fp16 rows [rows][cols], box = 64 values x box_rows rows, 128-byte swizzle, zero fill outside.  Base
+// and row stride must be 16-byte multiples.
+int make_rows_tmap(nvmai_cuda_moe *h, CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return NVMAI_CUDA_ECUDA;
-    if (!aligned16(base) || (stride_elems * 2) % 16 != 0 || cols % kPfKBlock != 0) return NVMAI_CUDA_EINVAL;
+    if (!aligned16(base) || cols % 64 != 0) return NVMAI_CUDA_EINVAL;
     const cuuint64_t gdim[2] = {cols, rows};
-    const cuuint64_t gstride[1] = {stride_elems * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kPfKBlock, box_rows};
+    const cuuint64_t gstride[1] = {cols * 2};
+    const cuuint32_t box[2] = {64, box_rows};
     const cuuint32_t estride[2] = {1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), gdim, gstride, box, estride,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -637,46 +603,100 @@ int make_rows_tmap(nvmai_cuda_moe *h, CUtensorMap *map, const void *base, uint64
     if (r != CUDA_SUCCESS) { h->last_cuda_error = (int)r; return NVMAI_CUDA_ECUDA; }
     return NVMAI_CUDA_OK;
 }
-
-// b_rows: fp16 [b_count][kdim] in work-item order; b2_rows: the direct items' rows (token order), or nullptr
-template <int PHASE>
-int launch_prefill_gemm(nvmai_cuda_moe *h, uint32_t bits, const PrefillGemmParams &p, const void *b_rows, uint64_t b_count,
-                        const void *b2_rows, uint64_t b2_count, dim3 grid, cudaStream_t st) {
+// Tensor map over packed codes [experts][rows][row_bytes], box = 128 bytes x 128 rows of one expert.
+int make_codes_tmap(nvmai_cuda_moe *h, CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint64_t experts,
+                    uint64_t expert_stride) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return NVMAI_CUDA_ECUDA;
+    const cuuint64_t gdim[3] = {row_bytes, rows, experts};
+    const cuuint64_t gstride[2] = {row_bytes, expert_stride};
+    const cuuint32_t box[3] = {128, 128, 1};
+    const cuuint32_t estride[3] = {1, 1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), gdim, gstride, box, estride,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { h->last_cuda_error = (int)r; return NVMAI_CUDA_ECUDA; }
+    return NVMAI_CUDA_OK;
+}
+int ensure_layer_maps(nvmai_cuda_moe *h, LayerViews &lv) {
+    if (lv.tc_maps) return NVMAI_CUDA_OK;
     const auto &c = h->cfg;
-    PrefillGemmArgs args{};
-    args.p = p;
-    if (PHASE == 0 && h->pf_debug_drop) { args.p.debug_drop_b = 1; h->pf_debug_drop = false; }     // one launch only
-    const uint64_t cols = p.kdim + pf_extra_cols(p.kdim);        // the rows carry their correction columns
-    int rc = make_rows_tmap(h, &args.tmap_b, b_rows, b_count, cols, cols, kPfBoxRows);
-    if (rc) return rc;
-    if (b2_rows != nullptr) {
-        if ((rc = make_rows_tmap(h, &args.tmap_a, b2_rows, b2_count, cols, cols, kPfBoxRows))) return rc;
+    const uint8_t *blobs = static_cast<const uint8_t *>(lv.w.experts);
+    const uint64_t n = h->expert_map ? h->n_local : c.num_experts, st = lv.w.expert_stride;
+    const uint64_t dx = (uint64_t)c.d * c.routed_bits / 8, fx = (uint64_t)c.f * c.routed_bits / 8;
+    int rc;
+    if ((rc = make_codes_tmap(h, &lv.gate, blobs + lv.w.offsets.gate_w, dx, c.f, n, st)) ||
+        (rc = make_codes_tmap(h, &lv.up, blobs + lv.w.offsets.up_w, dx, c.f, n, st)) ||
+        (rc = make_codes_tmap(h, &lv.down, blobs + lv.w.offsets.down_w, fx, c.d, n, st)))
+        return rc;
+    if (c.shared_f != 0 && c.shared_f % 128 == 0) {
+        const uint64_t sdx = (uint64_t)c.d * c.shared_bits / 8, sfx = (uint64_t)c.shared_f * c.shared_bits / 8;
+        if ((rc = make_codes_tmap(h, &lv.sgate, lv.w.shared_gate_proj.w, sdx, c.shared_f, 1, sdx * c.shared_f)) ||
+            (rc = make_codes_tmap(h, &lv.sup, lv.w.shared_up_proj.w, sdx, c.shared_f, 1, sdx * c.shared_f)) ||
+            (rc = make_codes_tmap(h, &lv.sdown, lv.w.shared_down_proj.w, sfx, c.d, 1, sfx * c.d)))
+            return rc;
     } else {
-        args.tmap_a = args.tmap_b;
+        lv.sgate = lv.gate; lv.sup = lv.up; lv.sdown = lv.down;
     }
-    return dispatch_bits_meta(bits, c.meta_dtype, [&](auto B, auto M) {
-        return dispatch_out(c.out_dtype, [&](auto O) {
-            return launch_kernel(h, prefill_gemm_kernel<decltype(B)::value, decltype(M)::value, decltype(O)::value, PHASE>,
-                                 grid, dim3(kPfThreads), kPfSmemBytes, st, true, args);
-        });
-    });
+    if (c.router_kind == NVMAI_ROUTER_DENSE_F16 && c.num_experts % 128 == 0 &&
+        (rc = make_rows_tmap(h, &lv.router, lv.w.router.w, c.num_experts, c.d, 128)))
+        return rc;
+    lv.tc_maps = true;
+    return NVMAI_CUDA_OK;
 }
 
-// rows of src (out_dtype for intermediates, fp16 for x) -> fp16 rows in the K order the weights of `bits` unpack
-// in; gather != nullptr: output row r comes from source row gather[r] / gather_div
-int launch_pack_rows(nvmai_cuda_moe *h, const void *src, bool src_f32, __half *dst, float *row_scale, uint32_t rows,
-                     uint32_t n, uint32_t bits, cudaStream_t st, const uint32_t *gather = nullptr, uint32_t gather_div = 1,
-                     uint32_t src_rows = 1) {
-    PackRowsParams p{src, dst, src_f32 ? row_scale : nullptr, rows, n, bits == 4 ? 1u : 0u, gather, gather_div, src_rows, pf_extra_cols(n)};
-    const dim3 grid((rows + 7) / 8), block(256);
-    if (src_f32) return launch_kernel(h, pack_rows_kernel<1>, grid, block, 0, st, true, p);
-    return launch_kernel(h, pack_rows_kernel<0>, grid, block, 0, st, true, p);
+void free_prefill_scratch(nvmai_cuda_moe *h) {
+    cudaFree(h->pf_x); cudaFree(h->pf_xs); cudaFree(h->pf_acts16); cudaFree(h->pf_sacts16); cudaFree(h->pf_rowscale);
+    cudaFree(h->pf_srowscale); cudaFree(h->pf_logits); cudaFree(h->pf_hist); cudaFree(h->pf_work2); cudaFree(h->pf_counter);
+    h->pf_x = h->pf_xs = h->pf_acts16 = h->pf_sacts16 = nullptr;
+    h->pf_rowscale = h->pf_srowscale = h->pf_logits = nullptr;
+    h->pf_hist = nullptr; h->pf_work2 = nullptr; h->pf_counter = nullptr;
+}
+
+int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
+    if (h->pf_counter) return NVMAI_CUDA_OK;
+    // the first such call allocates; a stream under capture forbids that: make one eager call first
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (st != nullptr && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
+        cudaGetLastError();
+        return NVMAI_CUDA_EINVAL;
+    }
+    const auto &c = h->cfg;
+    const size_t T = c.max_tokens, P = T * c.top_k;
+    auto alloc = [&](auto **ptr, size_t bytes) { return cudaMalloc(reinterpret_cast<void **>(ptr), bytes ? bytes : 16) == cudaSuccess; };
+    const size_t dx = c.d + bp_extra_cols(c.d, 1), fx = c.f + bp_extra_cols(c.f, 2), sfx = c.shared_f + bp_extra_cols(c.shared_f, 2);
+    const bool two_orders = c.shared_f != 0 && c.shared_bits != c.routed_bits;
+    const size_t logit_rows = std::min<size_t>(16 * T, std::max<size_t>(T, (size_t)h->sm_count * kRouterTileTokens));
+    const size_t blocks = std::max(bp_route_blocks(c.max_tokens), bp_route_blocks(std::min(c.max_tokens, 1024u)));
+    // (the columns behind the sums are never written: they stay the zeros put there now)
+    const bool ok = alloc(&h->pf_x, T * dx * 2) && (!two_orders || alloc(&h->pf_xs, T * dx * 2)) && alloc(&h->pf_acts16, P * fx * 2) &&
+                    alloc(&h->pf_sacts16, T * sfx * 2) && alloc(&h->pf_rowscale, P * 4) && alloc(&h->pf_srowscale, T * 4) &&
+                    alloc(&h->pf_logits, logit_rows * c.num_experts * 4) && alloc(&h->pf_hist, blocks * kMaxExperts * 4) &&
+                    alloc(&h->pf_work2, (size_t)h->max_work * sizeof(WorkItem)) && alloc(&h->pf_counter, 16) &&
+                    cudaMemsetAsync(h->pf_acts16, 0, P * fx * 2, st) == cudaSuccess &&
+                    cudaMemsetAsync(h->pf_sacts16, 0, std::max<size_t>(T * sfx * 2, 16), st) == cudaSuccess &&
+                    cudaMemsetAsync(h->pf_counter, 0, 16, st) == cudaSuccess;
+    int rc = ok ? NVMAI_CUDA_OK : NVMAI_CUDA_ENOMEM;
+    if (!rc) rc = make_rows_tmap(h, &h->map_acts, h->pf_acts16, P, fx, 16);
+    if (!rc) rc = c.shared_f ? make_rows_tmap(h, &h->map_sacts, h->pf_sacts16, T, sfx, 16) : (h->map_sacts = h->map_acts, NVMAI_CUDA_OK);
+    if (rc) { cudaGetLastError(); free_prefill_scratch(h); }
+    return rc;
+}
+
+// Shapes the expert GEMMs cover: 128-row weight tiles, whole K blocks of the two-tile phases, and rings that fit.
+bool tc_shape_ok(const nvmai_cuda_moe *h, bool with_shared) {
+    const auto &c = h->cfg;
+    if (c.f % 128 != 0 || c.d % 256 != 0 || encode_tiled_fn() == nullptr) return false;
+    EgParams p{};
+    auto fits = [&](int phase, uint32_t kdim) { p.kdim = kdim; return eg_plan(p, phase, 16).cap != 0; };
+    if (!fits(0, c.d) || !fits(1, c.f)) return false;
+    return !with_shared || c.shared_f == 0 || (c.shared_f % 128 == 0 && fits(1, c.shared_f));
 }
 
 // The whole block for `tokens` rows: router, grouping, gate/up GEMMs + activation,
 // down GEMMs, rank-ordered weighted sum with the shared expert and the two-step
 // residual of the prefill path (RealForwardRunner.swift:3244-3591).
-// The same launches serve the batched decode entry points from a few dozen rows on, where the tensor-core tiles
+// The same launches serve the batched decode entry points from a few rows on, where the tensor-core tiles
 // beat the per-row tiles of the decode kernels:
 //   decode_order  the block's result takes the decode path's rounding (one rounding of h1 + sum, one residual add)
 //   routed_only   routing given by the caller (out_idx / out_w are inputs), no router, no shared expert
@@ -690,132 +710,172 @@ struct PrefillMode {
 
 int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32_t tokens, void *hidden, void *y,
                        uint32_t *out_idx, __half *out_w, cudaStream_t st, const PrefillMode mode = PrefillMode{}) {
-    const LayerViews &lv = h->layers[layer];
+    LayerViews &lv = h->layers[layer];
     int rc = ensure_prefill_scratch(h, st);
-    if (rc) return rc;
+    if (rc || (rc = ensure_layer_maps(h, lv))) return rc;
     nvmai_cuda_moe_config c = h->cfg;
     if (mode.routed_only) c.shared_f = 0;
     uint32_t *idx = out_idx ? out_idx : h->idx;
     __half *w = out_w ? out_w : h->w;
     const bool wide = c.out_dtype == NVMAI_OUT_FP32;
-    const XSource xsrc{x, c.d, nullptr, nullptr};
+    const uint32_t P = tokens * c.top_k;
+    const bool gated = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE;
+    const bool dense_gate = gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;
+    // The shared expert rides in the routed launches when bit width and shapes agree; otherwise it gets launches of
+    // its own.
+    const bool merged = c.shared_f != 0 && c.shared_bits == c.routed_bits && c.shared_f == c.f;
+    const bool two_orders = c.shared_f != 0 && c.shared_bits != c.routed_bits;
+    // with an expert map (this rank holds a part of the experts) the pairs of the other ranks' experts are left out
+    // of the grouping: the items and the partial rows then cover this rank's pairs only
+    const bool use_map = h->expert_map != nullptr;
+    const uint32_t experts = use_map ? h->n_local : c.num_experts;
+
+    // Longest work item: the accumulators are double-buffered up to 96 rows, one set of up to 192 rows pays above
+    // that; short items leave room for a deeper ring of rows.  rows: per expert, evenly routed.
+    const uint32_t rows = (P + c.num_experts - 1) / c.num_experts;
+    const uint32_t want = rows <= 12 ? 48 : rows <= 64 ? 96 : 192;
+    EgParams g0{}, g1{};
+    g0.kdim = c.d; g1.kdim = c.f;
+    const EgPlan plan0 = eg_plan(g0, 0, want), plan1 = eg_plan(g1, 1, std::min(want, 128u));
+
+    PackXParams px{};
+    px.x = x; px.dst = h->pf_x; px.dst2 = two_orders ? h->pf_xs : nullptr; px.rows = tokens; px.n = c.d;
+    px.permute = c.routed_bits == 4 ? 1 : 0;
+    px.gate_row = dense_gate ? static_cast<const __half *>(lv.w.shared_gate.w) : nullptr;
+    px.gate_val = h->gate_val; px.out_half = wide ? 0 : 1;
+    if ((rc = launched(h, bp_pack_x(px, st)))) return rc;
+
+    RouteParams r{};
+    r.pes = static_cast<const uint16_t *>(lv.w.per_expert_scale);
+    r.idx = idx; r.w = w; r.tokens = tokens; r.E = c.num_experts; r.K = c.top_k;
+    r.expert_map = use_map ? h->expert_map : nullptr; r.n_local = experts;
+    r.block_hist = h->pf_hist; r.counter = h->pf_counter; r.sorted_pair = h->sorted_pair; r.inv = h->inv;
+    r.work[0] = h->work; r.work[1] = h->pf_work2; r.n_work[0] = h->n_work; r.n_work[1] = h->n_work + 2;
+    r.cap[0] = plan0.cap; r.cap[1] = plan1.cap;
     // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
     // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
     // affine routers keep the exact code-times-activation kernel.
-    const bool gemm_router = c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr &&
-                             c.num_experts % (2 * kPfTileM) == 0;
-    if (mode.routed_only) {
-        // nothing to route
-    } else if (gemm_router) {
-        PrefillGemmArgs ra{};
-        PrefillGemmParams &r = ra.p;
-        r.shared_from = 0;
-        r.tokens = tokens; r.top_k = c.top_k; r.kdim = c.d;
-        r.out2 = h->logits; r.out_stride2 = c.num_experts; r.status = h->status;
-        if ((rc = make_rows_tmap(h, &ra.tmap_b, x, tokens, c.d, c.d, kPfBoxRows))) return rc;
-        if ((rc = make_rows_tmap(h, &ra.tmap_a, lv.w.router.w, c.num_experts, c.d, c.d, kPfTileM))) return rc;
-        const dim3 grid(c.num_experts / (2 * kPfTileM), (tokens + kPfTileN - 1) / kPfTileN);
-        if ((rc = launch_kernel(h, prefill_gemm_kernel<16, 0, 0, 2>, grid, dim3(kPfThreads), kPfSmemBytes, st, false, ra)))
-            return rc;
-        TopkRowsParams tk{h->logits, static_cast<const uint16_t *>(lv.w.per_expert_scale), idx, w, c.num_experts, c.top_k, tokens};
-        if ((rc = launch_kernel(h, topk_rows_kernel, dim3((tokens + 7) / 8), dim3(256), 0, st, true, tk))) return rc;
-        if (c.shared_f && (rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, false, false, true, false, st))) return rc;
-    } else if ((rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, false, c.shared_f != 0, false, st))) {
-        return rc;
+    const XSource xsrc{x, c.d, nullptr, nullptr};
+    if (!mode.routed_only && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0) {
+        RouterArgs ra{};
+        ra.w = lv.router;
+        if ((rc = make_rows_tmap(h, &ra.x, x, tokens, c.d, kRouterTileTokens))) return rc;
+        r.splits = router_splits(h, tokens);
+        r.logits = h->pf_logits;
+        ra.p = RouterParams{h->pf_logits, tokens, c.num_experts, c.d, r.splits, h->status};
+        if ((rc = launched(h, bp_router(ra, st)))) return rc;
+        if (gated && !dense_gate && (rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, false, false, true, false, st))) return rc;
+    } else if (!mode.routed_only) {
+        if ((rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, false, gated && !dense_gate, false, st))) return rc;
     }
-    // with an expert map (this rank holds a part of the experts) the pairs of the other ranks' experts are left out
-    // of the grouping: the items, the packed rows and the partial rows then cover this rank's pairs only
-    const bool use_map = h->expert_map != nullptr;
-    if ((rc = launch_group_pairs(h, idx, w, tokens, nullptr, nullptr, nullptr, true, true, st, false, use_map, kPfTileN, true)))
-        return rc;
-    const uint32_t P = tokens * c.top_k;
-    const uint32_t max_items = std::min(P, c.num_experts + P / kPfTileN);
-    const uint32_t shared_items = (tokens + kPfTileN - 1) / kPfTileN;
-    // x rows as the GEMMs read them: gathered into sorted pair order for the routed items (an item's rows are then
-    // one row range of the tensor map), token order for the shared expert; each in its weights' K order
-    if ((rc = launch_pack_rows(h, x, false, h->pf_x, nullptr, P, c.d, c.routed_bits, st, h->sorted_pair, c.top_k, tokens))) return rc;
-    if (c.shared_f && (rc = launch_pack_rows(h, x, false, h->pf_xn, nullptr, tokens, c.d, c.shared_bits, st))) return rc;
+    if ((rc = launched(h, bp_route(r, st), 2))) return rc;
 
-    PrefillGemmParams g{};
-    g.experts = static_cast<const uint8_t *>(lv.w.experts); g.stride = lv.w.expert_stride;
-    g.num_experts = use_map ? h->n_local : c.num_experts;
-    g.off = to_offsets(lv.w.offsets);
-    g.work = h->work; g.n_work = h->n_work; g.sorted_pair = h->sorted_pair;
-    g.tokens = tokens; g.top_k = c.top_k; g.act = c.activation; g.status = h->status;
-    // The shared expert rides in the routed launches (its token tiles after the routed items) when bit width and
-    // shapes agree; otherwise it gets launches of its own.
-    const bool merged = c.shared_f != 0 && c.shared_bits == c.routed_bits && c.shared_f == c.f;
-    const uint32_t none = 0xFFFFFFFFu;
+    const uint32_t shared_rows = merged ? tokens : 0;
+    auto set_common = [&](EgParams &g, const EgPlan &plan) {
+        g.experts = static_cast<const uint8_t *>(lv.w.experts); g.stride = lv.w.expert_stride; g.num_experts = experts;
+        g.sorted_pair = h->sorted_pair; g.tokens = tokens; g.top_k = c.top_k; g.act = c.activation; g.status = h->status;
+        g.shared_items = (shared_rows + plan.cap - 1) / plan.cap;
+        g.permute = c.routed_bits == 4 ? 1 : 0; g.shared_permute = c.shared_bits == 4 ? 1 : 0;
+    };
+    auto u8 = [](const void *p) { return static_cast<const uint8_t *>(p); };
+    auto set_shared = [&](EgParams &g, int phase) {
+        if (phase == 0) {
+            g.shared_s[0] = u8(lv.w.shared_gate_proj.scales); g.shared_b[0] = u8(lv.w.shared_gate_proj.biases);
+            g.shared_s[1] = u8(lv.w.shared_up_proj.scales); g.shared_b[1] = u8(lv.w.shared_up_proj.biases);
+        } else {
+            g.shared_s[0] = u8(lv.w.shared_down_proj.scales); g.shared_b[0] = u8(lv.w.shared_down_proj.biases);
+        }
+    };
+    auto units = [&](const EgParams &g, uint32_t cap) { return (g.shared_items + std::min(P, experts + P / cap)) * g.units_per_item; };
+    auto grid = [&](uint32_t n) { return std::max(1u, std::min(n, (uint32_t)h->sm_count)); };
+    // Down tiles per unit: a unit reads its rows once, so long runs save row traffic, while enough units must be left
+    // to spread over the chip (five rounds).
+    auto tiles_per_unit = [&](uint32_t items) {
+        uint32_t n = 8;
+        while (n > 1 && (c.d / 128 % n != 0 || (uint64_t)items * (c.d / 128 / n) < 5ull * h->sm_count)) n /= 2;
+        return n;
+    };
+    const bool split = mode.decode_order && c.meta_dtype == NVMAI_META_FP16;
+    EgArgs args{};
     // gate/up
-    g.kdim = c.d;
-    g.out = h->acts; g.out_stride = c.f; g.round_gate_up = 0;
-    g.s0 = to_mat(lv.w.shared_gate_proj); g.s1 = to_mat(lv.w.shared_up_proj);
-    g.out2 = h->shared_act; g.out_stride2 = c.shared_f; g.round_gate_up2 = 1; g.row_scale2 = nullptr;
-    g.trace = h->trace_on ? h->trace + ((size_t)layer * 3 + 0) * kTraceWords : nullptr;
-    g.shared_from = merged ? max_items : none;
-    if ((rc = launch_prefill_gemm<0>(h, c.routed_bits, g, h->pf_x, P, merged ? h->pf_xn : nullptr, tokens,
-                                     dim3(c.f / kPfTileM, max_items + (merged ? shared_items : 0)), st)))
-        return rc;
+    set_common(g0, plan0); set_shared(g0, 0);
+    g0.work = h->work; g0.n_work = h->n_work;
+    g0.off_s[0] = lv.w.offsets.gate_s; g0.off_b[0] = lv.w.offsets.gate_b; g0.off_s[1] = lv.w.offsets.up_s; g0.off_b[1] = lv.w.offsets.up_b;
+    g0.units_per_item = c.f / 128; g0.kfeat = c.f;
+    g0.out = wide ? h->acts : h->pf_acts16; g0.shared_out = wide ? h->shared_act : h->pf_sacts16;
+    g0.trace = h->trace_on ? h->trace + ((size_t)layer * 3 + 0) * kTraceWords : nullptr;
+    if (h->pf_debug_drop) { g0.debug_drop_rows = 1; h->pf_debug_drop = false; }     // one launch only
+    args.routed0 = lv.gate; args.routed1 = lv.up; args.shared0 = lv.sgate; args.shared1 = lv.sup;
+    g0.rows = h->pf_x; g0.shared_rows = h->pf_x;
+    args.p = g0;
+    if ((rc = launched(h, eg_launch(0, c.routed_bits, c.meta_dtype, c.out_dtype, split, args, grid(units(g0, plan0.cap)), plan0.smem, st)))) return rc;
     if (c.shared_f && !merged) {
-        PrefillGemmParams s = g;
-        s.shared_from = 0; s.trace = nullptr;
-        if ((rc = launch_prefill_gemm<0>(h, c.shared_bits, s, h->pf_xn, tokens, h->pf_xn, tokens,
-                                         dim3(c.shared_f / kPfTileM, shared_items), st)))
+        EgParams s = g0;
+        s.n_work = h->n_work + 3;            // a zero: no routed items
+        s.shared_items = (tokens + plan0.cap - 1) / plan0.cap;
+        s.units_per_item = c.shared_f / 128; s.kfeat = c.shared_f; s.trace = nullptr; s.debug_drop_rows = 0;
+        s.shared_rows = two_orders ? h->pf_xs : h->pf_x;
+        args.p = s;
+        if ((rc = launched(h, eg_launch(0, c.shared_bits, c.meta_dtype, c.out_dtype, split, args, grid(s.shared_items * s.units_per_item), plan0.smem, st))))
             return rc;
     }
-    // activation rows as the down GEMMs read them
-    const __half *acts16 = h->pf_acts16, *sacts16 = h->pf_sacts16;
-    if ((rc = launch_pack_rows(h, h->acts, wide, h->pf_acts16, h->pf_rowscale, P, c.f, c.routed_bits, st))) return rc;
-    if (c.shared_f &&
-        (rc = launch_pack_rows(h, h->shared_act, wide, h->pf_sacts16, h->pf_srowscale, tokens, c.shared_f, c.shared_bits, st)))
-        return rc;
-    // down
-    g.kdim = c.f; g.row_scale = wide ? h->pf_rowscale : nullptr;
-    g.out = h->partial; g.out_stride = c.d;
-    g.s0 = to_mat(lv.w.shared_down_proj); g.s1 = g.s0;
-    g.out2 = h->shared_partial; g.out_stride2 = c.d; g.row_scale2 = wide ? h->pf_srowscale : nullptr;
-    g.trace = h->trace_on ? h->trace + ((size_t)layer * 3 + 1) * kTraceWords : nullptr;
-    if ((rc = launch_prefill_gemm<1>(h, c.routed_bits, g, acts16, P, merged ? sacts16 : nullptr, tokens,
-                                     dim3(c.d / (2 * kPfTileM), max_items + (merged ? shared_items : 0)), st)))
-        return rc;
+    if (wide) {          // activation rows as the down GEMMs read them
+        PackActsParams pa{static_cast<const float *>(h->acts), h->pf_acts16, h->pf_rowscale, P, c.f, g0.permute,
+                          static_cast<const float *>(h->shared_act), h->pf_sacts16, h->pf_srowscale, c.shared_f ? tokens : 0, c.shared_f,
+                          g0.shared_permute};
+        if ((rc = launched(h, bp_pack_acts(pa, st)))) return rc;
+    }
+    // down; the prefill path rounds every partial to the output type, the decode path the sum
+    const bool part_half = !wide && !mode.decode_order && mode.partial_y == nullptr;
+    set_common(g1, plan1); set_shared(g1, 1);
+    g1.work = h->pf_work2; g1.n_work = h->n_work + 2;
+    g1.off_s[0] = lv.w.offsets.down_s; g1.off_b[0] = lv.w.offsets.down_b;
+    const double spread = 1.0 - std::pow(1.0 - (double)c.top_k / c.num_experts, (double)tokens);
+    g1.tiles_per_unit = tiles_per_unit((uint32_t)(experts * spread) + P / plan1.cap + g1.shared_items);
+    g1.units_per_item = c.d / 128 / g1.tiles_per_unit; g1.out_cols = c.d;
+    g1.out = h->partial; g1.shared_out = h->shared_partial; g1.out_half = part_half ? 1 : 0; g1.shared_out_half = wide ? 0 : 1;
+    g1.row_scale = wide ? h->pf_rowscale : nullptr; g1.shared_row_scale = wide ? h->pf_srowscale : nullptr;
+    g1.trace = h->trace_on ? h->trace + ((size_t)layer * 3 + 1) * kTraceWords : nullptr;
+    args.routed0 = lv.down; args.routed1 = lv.down; args.shared0 = lv.sdown; args.shared1 = lv.sdown;
+    args.rows = h->map_acts; args.shared_rows = h->map_sacts;
+    args.p = g1;
+    if ((rc = launched(h, eg_launch(1, c.routed_bits, c.meta_dtype, c.out_dtype, split, args, grid(units(g1, plan1.cap)), plan1.smem, st)))) return rc;
     if (c.shared_f && !merged) {
-        PrefillGemmParams s = g;
-        s.shared_from = 0; s.kdim = c.shared_f; s.trace = nullptr;
-        if ((rc = launch_prefill_gemm<1>(h, c.shared_bits, s, sacts16, tokens, sacts16, tokens,
-                                         dim3(c.d / (2 * kPfTileM), shared_items), st)))
+        EgParams s = g1;
+        s.kdim = c.shared_f;
+        const EgPlan plan = eg_plan(s, 1, std::min(want, 128u));
+        s.n_work = h->n_work + 3; s.trace = nullptr;
+        s.shared_items = (tokens + plan.cap - 1) / plan.cap;
+        s.tiles_per_unit = tiles_per_unit(s.shared_items); s.units_per_item = c.d / 128 / s.tiles_per_unit;
+        args.p = s;
+        if ((rc = launched(h, eg_launch(1, c.shared_bits, c.meta_dtype, c.out_dtype, split, args, grid(s.shared_items * s.units_per_item), plan.smem, st))))
             return rc;
     }
-    CombineParams pc{};
-    pc.partial = h->partial; pc.shared_partial = c.shared_f ? h->shared_partial : nullptr;
-    pc.inv = h->inv; pc.routing_w = w;
-    pc.gate_val = (c.shared_f && c.shared_gate_kind != NVMAI_GATE_NONE) ? h->gate_val : nullptr;
-    pc.residual = nullptr; pc.y = y; pc.hidden = hidden; pc.D = c.d; pc.K = c.top_k;
-    pc.partial_y = mode.partial_y; pc.prefill = mode.decode_order ? 0 : 1;
-    pc.hidden_delta = mode.hidden_delta;
-    if (mode.decode_order && mode.partial_y == nullptr) pc.next = h->next_norm;
-    return dispatch_out(c.out_dtype, [&](auto O) {
-        return launch_kernel(h, combine_kernel<decltype(O)::value>, dim3(tokens), dim3(256), 0, st, true, pc);
-    });
+    CombineRowsParams pc{};
+    pc.partial = h->partial; pc.partial_half = part_half ? 1 : 0;
+    pc.shared_partial = c.shared_f ? h->shared_partial : nullptr; pc.shared_half = wide ? 0 : 1;
+    pc.inv = h->inv; pc.routing_w = w; pc.gate_val = gated ? h->gate_val : nullptr;
+    pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y;
+    pc.tokens = tokens; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
+    return launched(h, bp_combine(pc, c.out_dtype, st));
 }
 
-// A batched decode call can take the tensor-core kernels when the fp16 operand holds the centred weight exactly
-// (bf16 scales; 8-bit codes go through as two nibbles) and the tile shapes divide the layer.
+// A batched decode call can take the tensor-core kernels when the tile shapes divide the layer (the fp16 operands hold
+// the centred weights exactly: 8-bit codes as two nibbles, fp16 scales as two parts).
 bool tc_batch_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared, cudaStream_t st) {
     const auto &c = h->cfg;
     if (tokens < h->tc_min_tokens) return false;
     // with an expert map only the routed-only form is taken (a rank's share of the routed sum); the whole block on
     // a part of the experts is the per-row kernels' business
     if (h->expert_map != nullptr && with_shared) return false;
-    if (h->pf_acts16 == nullptr && st != nullptr) {
+    if (h->pf_counter == nullptr && st != nullptr) {
         // the first such call allocates the packed-row scratch, which a stream under capture does not allow:
         // a call that is being captured before any eager one stays on the per-row kernels
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
     }
-    if (c.meta_dtype != NVMAI_META_BF16 || c.top_k > (uint32_t)kMaxTopK) return false;
-    if (c.f % kPfTileM != 0 || c.d % (2 * kPfTileM) != 0) return false;
-    if (with_shared && c.shared_f != 0 && c.shared_f % kPfTileM != 0) return false;
-    return true;
+    if (c.top_k > (uint32_t)kMaxTopK) return false;
+    return tc_shape_ok(h, with_shared);
 }
 
 
@@ -1186,7 +1246,7 @@ nvmai_cuda_moe *nvmai_cuda_moe_create(const nvmai_cuda_moe_config *config, int *
         h->max_work = (uint32_t)(std::min(P, c.num_experts + P / kPairsPerItem) + (T + kPairsPerItem - 1) / kPairsPerItem);
         if (ok) ok = alloc(&h->sorted_pair, P * 4) && alloc(&h->inv, P * 4) && alloc(&h->expert_offsets, kMaxExperts * 4) &&
                      alloc(&h->expert_counts, kMaxExperts * 4) && alloc(&h->work, (size_t)h->max_work * sizeof(WorkItem)) &&
-                     alloc(&h->n_work, 16) && alloc(&h->group_hist, ((P + kGroupThreads - 1) / kGroupThreads) * kMaxExperts * 4) && alloc(&h->trace, (size_t)c.num_layers * 3 * kTraceWords * sizeof(unsigned long long));
+                     alloc(&h->n_work, 16) && cudaMemset(h->n_work, 0, 16) == cudaSuccess && alloc(&h->group_hist, ((P + kGroupThreads - 1) / kGroupThreads) * kMaxExperts * 4) && alloc(&h->trace, (size_t)c.num_layers * 3 * kTraceWords * sizeof(unsigned long long));
         // per-pair partial rows are only needed by the batched path
         if (ok)
             ok = alloc(&h->partial, P * c.d * sizeof(float)) && alloc(&h->shared_partial, T * c.d * sizeof(float));
@@ -1223,7 +1283,7 @@ void nvmai_cuda_moe_destroy(nvmai_cuda_moe *h) {
     cudaFree(h->pd_trace);
     cudaFree(h->pb_xchg);
     cudaFree(h->pd_layers); cudaFree(h->pd_xchg); cudaFree(h->pd_epoch); cudaFree(h->pd_route_log);
-    cudaFree(h->pf_x); cudaFree(h->pf_xn); cudaFree(h->pf_acts16); cudaFree(h->pf_sacts16); cudaFree(h->pf_rowscale); cudaFree(h->pf_srowscale);
+    free_prefill_scratch(h);
     for (auto &lv : h->layers)
         for (void *p : lv.owned) cudaFree(p);
     cudaFree(h->logits); cudaFree(h->idx); cudaFree(h->w); cudaFree(h->acts); cudaFree(h->shared_act);
@@ -1285,6 +1345,7 @@ int nvmai_cuda_moe_register_layer(nvmai_cuda_moe *h, uint32_t layer, const nvmai
     h->layers[layer].owned = std::move(owned);
     h->layers[layer].w = *wts;
     h->layers[layer].registered = true;
+    h->layers[layer].tc_maps = false;
     h->graphs_stale = h->ep_graphs_stale = true;
     h->pd_layers_stale = true;
     return NVMAI_CUDA_OK;
@@ -1450,12 +1511,11 @@ int nvmai_cuda_moe_layer_prefill(nvmai_cuda_moe *h, uint32_t layer, const void *
     if (tokens == 0 || tokens > c.max_tokens) return NVMAI_CUDA_ERANGE;
     if (c.top_k > (uint32_t)kMaxTopK) return NVMAI_CUDA_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // The tensor-core kernels tile the weights by 128 rows per accumulator, two accumulators per block.  Shapes
+    // The tensor-core kernels tile the weights by 128 rows per accumulator.  Shapes
     // they do not cover (the reference's own prefill test runs d = f = 64, top-2), a rank that holds a subset of
     // the experts, and NVMAI_CUDA_PREFILL_TC=0 take the exact grouped kernels of the batched decode path with the
     // prefill shaders' rounding points: router, grouping, gate/up and down per (tile, work item), ordered combine.
-    const bool tiles_fit = c.f % kPfTileM == 0 && c.d % (2 * kPfTileM) == 0 && c.shared_f % kPfTileM == 0;
-    if (!tiles_fit || !h->prefill_tc) {
+    if (!tc_shape_ok(h, true) || !h->prefill_tc) {
         if (h->expert_map) return NVMAI_CUDA_EINVAL;      // prefill runs on one GPU's full expert set
         uint32_t *idx = out_idx ? out_idx : h->idx;
         __half *w = out_w_f16 ? static_cast<__half *>(out_w_f16) : h->w;
@@ -1482,6 +1542,7 @@ int nvmai_cuda_moe_set_expert_map(nvmai_cuda_moe *h, const uint32_t *map_host, u
     if (!h) return NVMAI_CUDA_EINVAL;
     const auto &c = h->cfg;
     h->pd_layers_stale = true;              // the tensor maps span the blobs this rank holds
+    for (auto &lv : h->layers) lv.tc_maps = false;
     if (map_host == nullptr) {              // back to "every expert is local"
         cudaFree(h->expert_map);
         h->expert_map = nullptr;
@@ -2148,6 +2209,7 @@ int nvmai_cuda_moe_debug_mute_block(nvmai_cuda_moe *h, uint32_t block) {
 
 int nvmai_cuda_moe_debug_set_wait_limit(uint64_t nanoseconds) {
     const unsigned long long v = nanoseconds ? nanoseconds : 1000000000ull;
+    if (bp_set_wait_limit(v) != cudaSuccess) return NVMAI_CUDA_ECUDA;
     return cudaMemcpyToSymbol(g_wait_limit_ns, &v, sizeof(v)) == cudaSuccess ? NVMAI_CUDA_OK : NVMAI_CUDA_ECUDA;
 }
 

@@ -1,0 +1,64 @@
+"""Edges of the grouped expert GEMMs (accumulator switches, ragged items, odd K-block counts, scale types) through the
+C ABI against the oracle."""
+import sys
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+for p_ in (ROOT, ROOT / "tests"):
+    if str(p_) not in sys.path:
+        sys.path.insert(0, str(p_))
+
+pytestmark = pytest.mark.gpu
+
+from nvmai_b200 import MoE, MoEConfig, synthetic      # noqa: E402
+from nvmai_b200 import format as fmt                  # noqa: E402
+from oracle import oracle as orc                      # noqa: E402
+import gpu_util as gu                                 # noqa: E402
+
+BF16, FP16 = fmt.META_BF16, fmt.META_FP16
+
+
+# 8 experts: every expert gets every row, so `tokens` is the experts' row count.  96 / 97 and 192 / 193 rows: where an
+# item is split; 16 / 17: one and two 16-row pieces; 1: the smallest item.  f = 384: an odd number of chunks of codes
+# per down tile (4-bit), an odd number of A slots per tile; d = 768: 12 K blocks, scales that do not come eight at a time.
+@pytest.mark.parametrize("bits,meta,out,tokens,d,f", [
+    (4, BF16, fmt.OUT_FP16, 1, 256, 128), (4, BF16, fmt.OUT_FP16, 17, 768, 384), (4, BF16, fmt.OUT_FP32, 96, 256, 384),
+    (4, BF16, fmt.OUT_FP16, 97, 512, 128), (4, BF16, fmt.OUT_FP16, 193, 256, 128), (8, BF16, fmt.OUT_FP16, 16, 768, 128),
+    (8, BF16, fmt.OUT_FP32, 130, 256, 384), (4, FP16, fmt.OUT_FP16, 33, 768, 384), (8, FP16, fmt.OUT_FP32, 40, 256, 128),
+    (8, FP16, fmt.OUT_FP16, 65, 512, 384)])
+@pytest.mark.parametrize("entry", ["decode", "prefill"])
+def test_rows_of_every_item_match_the_oracle(bits, meta, out, tokens, d, f, entry, monkeypatch):
+    monkeypatch.setenv("NVMAI_CUDA_TC_MIN", "1")
+    host = synthetic.layer(700 + tokens, d=d, f=f, shared_f=f, num_experts=8, routed_bits=bits, meta=meta)
+    if bits == 8:       # zero-mean weights: the one-sided ones leave fp16's range at 8 bits
+        rng = np.random.default_rng(tokens)
+        off = host["offsets"]
+        for name, n in (("gate", f * d), ("up", f * d), ("down", d * f)):
+            s = rng.uniform(0.0003, 0.0012, size=(8, n // 64)).astype(np.float32)
+            for key, v in (("_s", s), ("_b", -127.5 * s)):
+                raw = np.ascontiguousarray(fmt.f32_to_meta_bits(v, meta)).view(np.uint8)
+                host["experts"][:, off[name + key]:off[name + key] + raw.shape[1]] = raw
+        host["shared"] = [(w, fmt.f32_to_meta_bits(np.full(s.shape, 0.0007), meta), fmt.f32_to_meta_bits(np.full(s.shape, -0.0892), meta))
+                          for w, s, _ in host["shared"]]
+    cfg = MoEConfig(d=d, f=f, shared_f=f, num_experts=8, top_k=8, routed_bits=bits, shared_bits=bits, meta_dtype=meta,
+                    out_dtype=out, max_tokens=tokens)
+    moe = MoE(cfg)
+    dl = gu.DeviceLayer(host)
+    dl.register(moe, 0)
+    x = synthetic.hidden_rows(701, tokens, d)
+    f16 = out == fmt.OUT_FP16
+    y = gu.dev_empty(tokens * d, "f16" if f16 else "f32")
+    if entry == "decode":
+        moe.layer_decode(0, gu.to_dev(x), tokens, h2_out=y)
+    else:
+        moe.layer_prefill(0, gu.to_dev(x), tokens, y_out=y)
+    moe.synchronize()
+    got = (orc.f16_bits_to_f32(gu.from_dev(y, np.uint16)) if f16 else y.cpu().numpy()).reshape(tokens, d)
+    L, keep = gu.oracle_layer(host, cfg)
+    for t in sorted({0, tokens // 2, tokens - 1, min(tokens - 1, 15), min(tokens - 1, 95), min(tokens - 1, 96)}):
+        xr = np.ascontiguousarray(x[t])
+        want = gu.oracle_decode(L, cfg, xr)[2] if entry == "decode" else gu.oracle_prefill_row(L, cfg, xr, None)[2]
+        assert orc.rel_error(got[t], want) < (3e-3 if f16 else 1.5e-3), f"row {t}"
