@@ -7,6 +7,7 @@
 #include "batch_rows.cuh"
 #include "expert_gemm.cuh"
 #include "launch.h"
+#include "stream_gemm.cuh"
 
 namespace nvmai {
 
@@ -71,6 +72,61 @@ cudaError_t eg_launch(int phase, uint32_t bits, uint32_t meta, uint32_t out_dtyp
     return with_out(integral_constant<int, 8>{});
 }
 
+static bool sg_fast(int phase, uint32_t kdim) { return kdim == (phase == 0 ? 2048u : 512u); }
+
+size_t sg_plan(SgParams &p, int phase, uint32_t nb, bool wide) {
+    const uint32_t groups = p.kdim / 64, cols = 8 * nb;
+    const uint32_t rows = phase == 1 ? 256 : sg_fast(0, p.kdim) ? 64 : 128;        // features or down rows of a unit
+    if (p.out_cols % rows != 0) return 0;
+    p.units_per_item = p.out_cols / rows;
+    p.cap = cols;
+    p.meta_bytes = rows * groups * 2 * (phase == 0 ? 4 : 2);
+    auto up = [](size_t v) { return (v + 127) & ~(size_t)127; };
+    size_t fixed = 2 * p.meta_bytes + up((size_t)cols * (p.kdim * 2 + 16)) + (phase == 1 && wide ? up((size_t)cols * p.kdim * 4) : 0) +
+                   up((size_t)cols * (groups + 4) * 4) + up(cols * 4 + (phase == 0 ? 2 * 8 * 4 * nb * 32 * 4 : 0));
+    if (fixed + 2048 + 2 * kSgStageBytes > kMaxBlockSmem) return 0;
+    p.stages = (uint32_t)std::min<size_t>(kSgMaxStages, (kMaxBlockSmem - 2048 - fixed) / kSgStageBytes);
+    size_t o = 1024 + (size_t)p.stages * kSgStageBytes;
+    p.meta_off = (uint32_t)o; o += 2 * p.meta_bytes;
+    p.x_off = (uint32_t)o; o += up((size_t)cols * (p.kdim * 2 + 16));
+    p.raw_off = (uint32_t)o; o += phase == 1 && wide ? up((size_t)cols * p.kdim * 4) : 0;
+    p.sum_off = (uint32_t)o; o += up((size_t)cols * (groups + 4) * 4);
+    p.scale_off = (uint32_t)o; o += up(cols * 4 + (phase == 0 ? 2 * 8 * 4 * nb * 32 * 4 : 0));
+    return o + 1024;
+}
+
+cudaError_t sg_launch(int phase, uint32_t bits, uint32_t meta, uint32_t out_dtype, uint32_t nb, const SgArgs &args, uint32_t blocks,
+                      size_t smem, cudaStream_t st) {
+    using std::integral_constant;
+    const bool fast = sg_fast(phase, args.p.kdim);
+    auto go = [&](auto B, auto M, auto O, auto P, auto N, auto F) {
+        return launch_pdl(stream_gemm_kernel<decltype(B)::value, decltype(M)::value, decltype(O)::value, decltype(P)::value, decltype(N)::value,
+                                             decltype(F)::value>, dim3(blocks), dim3(kSgThreads + 32), smem, st, true, args);
+    };
+    auto with_fast = [&](auto B, auto M, auto O, auto P, auto N) {
+        if (fast) return go(B, M, O, P, N, integral_constant<bool, true>{});
+        return go(B, M, O, P, N, integral_constant<bool, false>{});
+    };
+    auto with_n = [&](auto B, auto M, auto O, auto P) {
+        if (nb == 1) return with_fast(B, M, O, P, integral_constant<int, 1>{});
+        return with_fast(B, M, O, P, integral_constant<int, 2>{});
+    };
+    auto with_p = [&](auto B, auto M, auto O) {
+        if (phase == 0) return with_n(B, M, O, integral_constant<int, 0>{});
+        return with_n(B, M, O, integral_constant<int, 1>{});
+    };
+    auto with_o = [&](auto B, auto M) {
+        if (out_dtype == OUT_F16) return with_p(B, M, integral_constant<int, OUT_F16>{});
+        return with_p(B, M, integral_constant<int, OUT_F32>{});
+    };
+    auto with_m = [&](auto B) {
+        if (meta == META_BF16) return with_o(B, integral_constant<int, META_BF16>{});
+        return with_o(B, integral_constant<int, META_FP16>{});
+    };
+    if (bits == 4) return with_m(integral_constant<int, 4>{});
+    return with_m(integral_constant<int, 8>{});
+}
+
 cudaError_t bp_pack_x(const PackXParams &p, cudaStream_t st) {
     return launch_pdl(pack_x_kernel, dim3(p.rows), dim3(256), 0, st, true, p);
 }
@@ -87,6 +143,7 @@ uint32_t bp_route_blocks(uint32_t tokens) {
 }
 
 cudaError_t bp_route(const RouteParams &p, cudaStream_t st) {
+    if (p.tokens <= kSmallRoute) return launch_pdl(route_small_kernel, dim3(1), dim3(1024), 0, st, true, p);
     const dim3 grid(bp_route_blocks(p.tokens));
     cudaError_t e = launch_pdl(route_kernel, grid, dim3(256), 0, st, true, p);
     if (e != cudaSuccess) return e;

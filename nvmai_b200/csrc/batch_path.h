@@ -60,6 +60,27 @@ EgPlan eg_plan(EgParams &p, int phase, uint32_t want_cap);
 cudaError_t eg_launch(int phase, uint32_t bits, uint32_t meta, uint32_t out_dtype, bool split, const EgArgs &args, uint32_t blocks,
                       size_t smem, cudaStream_t st);
 
+// ---- few rows per expert: codes streamed through mma.sync (stream_gemm.cuh) -----------------
+struct SgParams {
+    const uint8_t *experts; unsigned long long stride; uint32_t num_experts;
+    uint32_t off_s[2], off_b[2];
+    const uint8_t *shared_s[2], *shared_b[2];
+    const void *rows, *shared_rows;           // phase 0: fp16 x rows [token][kdim]; phase 1: activation rows (fp16 / fp32)
+    const WorkItem *work; const uint32_t *n_work; const uint32_t *sorted_pair;
+    uint32_t shared_items, units_per_item, tokens, top_k, cap, kdim, out_cols, act;
+    void *out, *shared_out;                   // phase 0: activations [row][F]; phase 1: fp32 partial rows [row][D]
+    uint32_t stages, meta_off, meta_bytes, x_off, raw_off, sum_off, scale_off;
+    unsigned int *status;
+};
+struct alignas(64) SgArgs {
+    CUtensorMap routed0, routed1, shared0, shared1;     // codes, boxes of 64 rows x 128 bytes
+    SgParams p;
+};
+// Fills the shared-memory geometry of p (kdim and out_cols set) for items of up to 8 * nb rows; 0: does not fit.
+size_t sg_plan(SgParams &p, int phase, uint32_t nb, bool wide);
+cudaError_t sg_launch(int phase, uint32_t bits, uint32_t meta, uint32_t out_dtype, uint32_t nb, const SgArgs &args, uint32_t blocks,
+                      size_t smem, cudaStream_t st);
+
 // ---- rows, routing and reduction around them (batch_rows.cuh) --------------------------------
 // x rows -> fp16 rows in the weights' K order with their group sums; optionally the scalar gate of every row
 struct PackXParams {
@@ -89,7 +110,9 @@ struct RouteParams {
     WorkItem *work[2]; uint32_t *n_work[2]; uint32_t cap[2];
 };
 uint32_t bp_route_blocks(uint32_t tokens);
-cudaError_t bp_route(const RouteParams &p, cudaStream_t st);      // two launches
+constexpr uint32_t kSmallRoute = 32;          // up to this many tokens one block does it all
+cudaError_t bp_route(const RouteParams &p, cudaStream_t st);
+inline uint64_t bp_route_launches(uint32_t tokens) { return tokens <= kSmallRoute ? 1 : 2; }
 
 // wide-range activations: fp32 rows -> scaled fp16 rows in the down weights' K order with half-group sums
 // (routed rows, then the shared expert's)

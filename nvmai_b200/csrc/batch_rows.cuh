@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(PackXParams p) {
             // natural (0,1)(2,3)(4,5)(6,7) -> (0,4)(1,5)(2,6)(3,7), the order of bp_k_order
             const uint4 perm = make_uint4(__byte_perm(q.x, q.z, 0x5410), __byte_perm(q.x, q.z, 0x7632),
                                           __byte_perm(q.y, q.w, 0x5410), __byte_perm(q.y, q.w, 0x7632));
-            *reinterpret_cast<uint4 *>(dst + i8) = p.permute ? perm : q;
+            if (p.dst != nullptr) *reinterpret_cast<uint4 *>(dst + i8) = p.permute ? perm : q;
             if (dst2 != nullptr) *reinterpret_cast<uint4 *>(dst2 + i8) = p.permute ? q : perm;
             const __half2 *h = reinterpret_cast<const __half2 *>(&q);
             float f[8];
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(PackXParams p) {
         part += __shfl_xor_sync(0xffffffffu, part, 1);       // a group = 8 neighbouring lanes
         part += __shfl_xor_sync(0xffffffffu, part, 2);
         part += __shfl_xor_sync(0xffffffffu, part, 4);
-        if (i8 < p.n && (lane & 7u) == 0u) {
+        if (p.dst != nullptr && i8 < p.n && (lane & 7u) == 0u) {
             const float sum = part * kBpSumScale;
             const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
             const uint32_t g = i8 / 64u;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256) pack_x_kernel(PackXParams p) {
             if (dst2 != nullptr) { dst2[p.n + g] = hi; dst2[p.n + G + g] = lo; dst2[p.n + 2u * G + g] = hi; }
         }
     }
-    for (uint32_t i = 3u * G + tid; i < extra; i += 256u) {
+    for (uint32_t i = 3u * G + tid; p.dst != nullptr && i < extra; i += 256u) {
         dst[p.n + i] = __float2half_rn(0.0f);
         if (dst2 != nullptr) dst2[p.n + i] = __float2half_rn(0.0f);
     }
@@ -165,6 +165,33 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
 // histograms for a chunk of 4096.
 __host__ __device__ constexpr uint32_t bp_tokens_per_block(uint32_t tokens) { return tokens <= 1024u ? 8u : 32u; }
 
+// Expert e's work items in list j: its rows split evenly over them (two items of 70 instead of 128 + 12).
+__device__ __forceinline__ void write_items(const RouteParams &p, int j, uint32_t e, uint32_t rows, uint32_t items, uint32_t first_row,
+                                            uint32_t first_item) {
+    const uint32_t even = items ? rows / items : 0u, extra = items ? rows % items : 0u;
+    for (uint32_t i = 0; i < items; ++i)
+        p.work[j][first_item + i] = WorkItem{e, first_row + i * even + min(i, extra), even + (i < extra ? 1u : 0u), 0u};
+}
+
+// v[i] = logit of expert lane + 32 i: the splits added in order, up to 32 loads in flight
+__device__ __forceinline__ void add_splits(float (&v)[kMaxExperts / 32], const RouteParams &p, uint32_t tok, uint32_t lane) {
+    for (uint32_t sp = 0; sp < p.splits; sp += 4u) {
+        float a[4][kMaxExperts / 32];
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k)
+#pragma unroll
+            for (int i = 0; i < kMaxExperts / 32; ++i) {
+                const uint32_t e = lane + 32u * i;
+                a[k][i] = e < p.E && sp + k < p.splits ? __ldcg(p.logits + ((size_t)(sp + k) * p.tokens + tok) * p.E + e) : 0.0f;
+            }
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k)
+#pragma unroll
+            for (int i = 0; i < kMaxExperts / 32; ++i)
+                if (sp + k < p.splits) v[i] += a[k][i];
+    }
+}
+
 // Router semantics of router_topk_select_k8 (moe.metal:233-285); the pairs end up in (expert, token, rank) order, as
 // PrefillMoEGrouping.groupTokenExpertPairs has them (PrefillMoEGrouping.swift:90-192).
 __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
@@ -184,19 +211,7 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
             float v[kMaxExperts / 32];
 #pragma unroll
             for (int i = 0; i < kMaxExperts / 32; ++i) v[i] = lane + 32u * i < p.E ? 0.0f : -INFINITY;
-            for (uint32_t sp = 0; sp < p.splits; sp += 2u) {          // 16 loads in flight
-                const float *l0 = p.logits + ((size_t)sp * p.tokens + tok) * p.E;
-                const bool two = sp + 1u < p.splits;
-                float a[2][kMaxExperts / 32];
-#pragma unroll
-                for (int i = 0; i < kMaxExperts / 32; ++i) {
-                    const uint32_t e = lane + 32u * i;
-                    a[0][i] = e < p.E ? __ldcg(l0 + e) : 0.0f;
-                    a[1][i] = e < p.E && two ? __ldcg(l0 + (size_t)p.tokens * p.E + e) : 0.0f;
-                }
-#pragma unroll
-                for (int i = 0; i < kMaxExperts / 32; ++i) { v[i] += a[0][i]; if (two) v[i] += a[1][i]; }
-            }
+            add_splits(v, p, tok, lane);
             topk_softmax_warp_vals(v, (int)p.E, (int)p.K, p.pes, p.idx + (size_t)tok * p.K, p.w + (size_t)tok * p.K);
         }
         if ((uint32_t)lane < p.K) {
@@ -239,12 +254,9 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
             all[j] += warp_tot[j][w];
         }
     }
-    // an expert's rows are split evenly over its items (two items of 70 instead of 128 + 12)
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        const uint32_t items = mine[1 + j], even = items ? total / items : 0u, extra = items ? total % items : 0u;
-        for (uint32_t i = 0; i < items; ++i)
-            p.work[j][pre[1 + j] + i] = WorkItem{(uint32_t)tid, pre[0] + i * even + min(i, extra), even + (i < extra ? 1u : 0u), 0u};
+        write_items(p, j, tid, total, mine[1 + j], pre[0], pre[1 + j]);
         if (tid == 0) p.n_work[j][0] = all[1 + j];
     }
     uint32_t run = pre[0];
@@ -284,6 +296,88 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
         for (int w = 0; w < warp; ++w) pos += cnt[w][e];
         p.sorted_pair[pos] = i;
         p.inv[i] = pos;
+    }
+}
+
+// The same in one block for up to kSmallRoute tokens: histogram, scan and scatter stay in shared memory (two launches
+// and two trips through global memory less: 13 rows 12.4 + 3.2 us as two launches).
+__global__ void __launch_bounds__(1024) route_small_kernel(RouteParams p) {
+    __shared__ uint32_t hist[kMaxExperts], first[kMaxExperts];
+    __shared__ uint16_t cnt[8][kMaxExperts];                  // per warp of pairs, at most 256 pairs
+    __shared__ uint16_t pair_expert[kSmallRoute * kMaxTopK];
+    __shared__ uint32_t warp_tot[3][kMaxExperts / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid < kMaxExperts) {
+        hist[tid] = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) cnt[w][tid] = 0;
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    __syncthreads();
+    for (uint32_t tok = warp; tok < p.tokens; tok += 32u) {
+        if (p.logits != nullptr) {
+            float v[kMaxExperts / 32];
+#pragma unroll
+            for (int i = 0; i < kMaxExperts / 32; ++i) v[i] = lane + 32u * i < p.E ? 0.0f : -INFINITY;
+            add_splits(v, p, tok, lane);
+            topk_softmax_warp_vals(v, (int)p.E, (int)p.K, p.pes, p.idx + (size_t)tok * p.K, p.w + (size_t)tok * p.K);
+        }
+        if ((uint32_t)lane < p.K) {
+            const uint32_t g = min(p.idx[(size_t)tok * p.K + lane], p.E - 1u);
+            const uint32_t e = p.expert_map != nullptr ? p.expert_map[g] : g;
+            pair_expert[tok * p.K + lane] = (uint16_t)(e == kBpNotLocal ? 0xFFFFu : e);
+            if (e != kBpNotLocal) atomicAdd(&hist[e], 1u);
+        }
+    }
+    __syncthreads();
+    const uint32_t P = p.tokens * p.K;
+    const uint32_t e = (uint32_t)tid < P ? pair_expert[tid] : 0xFFFFu;
+    const bool live = e != 0xFFFFu;
+    const uint32_t peers = __match_any_sync(0xffffffffu, e);
+    const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+    if (live && rank == 0u) cnt[warp][e] = (uint16_t)__popc(peers);
+    uint32_t total = 0, mine[3] = {}, pre[3] = {};
+    if (tid < kMaxExperts) {
+        total = hist[tid];
+        mine[0] = total; mine[1] = (total + p.cap[0] - 1u) / p.cap[0]; mine[2] = (total + p.cap[1] - 1u) / p.cap[1];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            pre[j] = mine[j];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, pre[j], o);
+                if (lane >= o) pre[j] += v;
+            }
+            if (lane == 31) warp_tot[j][warp] = pre[j];
+        }
+    }
+    __syncthreads();
+    if (tid < kMaxExperts) {
+        uint32_t all[3] = {0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            pre[j] -= mine[j];
+            for (int w = 0; w < kMaxExperts / 32; ++w) {
+                if (w < warp) pre[j] += warp_tot[j][w];
+                all[j] += warp_tot[j][w];
+            }
+        }
+        first[tid] = pre[0];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            write_items(p, j, tid, total, mine[1 + j], pre[0], pre[1 + j]);
+            if (tid == 0) p.n_work[j][0] = all[1 + j];
+        }
+    }
+    __syncthreads();
+    if (live) {
+        uint32_t pos = first[e] + rank;
+        for (int w = 0; w < warp; ++w) pos += cnt[w][e];
+        p.sorted_pair[pos] = tid;
+        p.inv[tid] = pos;
+    } else if ((uint32_t)tid < P) {
+        p.inv[tid] = kBpNotLocal;
     }
 }
 

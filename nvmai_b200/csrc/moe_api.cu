@@ -44,6 +44,7 @@ struct LayerViews {
     // the packed codes (and a dense router) as tensor maps, made by the first call that runs the expert GEMMs
     bool tc_maps = false;
     CUtensorMap gate, up, down, sgate, sup, sdown, router;
+    CUtensorMap gate64, up64, down64, sgate64, sup64, sdown64;     // the same codes in boxes of 64 rows (stream_gemm.cuh)
 };
 
 struct StackGraphKey {
@@ -95,7 +96,11 @@ struct nvmai_cuda_moe {
     // B200 (8-bit layer): 4 rows 60 us separate / 102 us grouped, 16 rows 190 / 265, 64 rows 697 / 570.
     // NVMAI_CUDA_GROUPED_MIN overrides it.
     uint32_t grouped_min_tokens = 24;
-    uint32_t tc_min_tokens = 32;     // batched decode calls from this many rows on run the tensor-core (prefill) kernels
+    // Batched decode calls from this many rows on run the batched experts' kernels (stream_gemm.cuh, expert_gemm.cuh).
+    // Measured per layer, separate rows / batched: 3 rows 36 / 39 us, 4 rows 46 / 41, 13 rows 132 / 63, 40 rows 4-bit
+    // 420 / 105.  NVMAI_CUDA_TC_MIN overrides it (32 when only NVMAI_CUDA_GROUPED_MIN is given).
+    uint32_t tc_min_tokens = 4;
+    uint32_t stream_max_rows = ~0u;  // NVMAI_CUDA_STREAM_ROWS: rows per expert up to which stream_gemm.cuh serves a call
     // prefill chunks on the tensor cores (default); NVMAI_CUDA_PREFILL_TC=0 sends them through the exact grouped
     // kernels of the batched decode path instead
     bool prefill_tc = true;
@@ -562,12 +567,13 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
 }
 
 // ---- prefill: grouped GEMMs on the tensor cores ----------------------------------
-// Splits of the router's K over blocks: as many as still fill the chip once.
+// Splits of the router's K over blocks: up to four, while they fill the chip once (the top-k reads every split: with
+// sixteen it took 10 us for 13 rows, most of it one SM reading partial logits).
 uint32_t router_splits(const nvmai_cuda_moe *h, uint32_t tokens) {
     const auto &c = h->cfg;
     const uint32_t tiles = (c.num_experts / 128) * ((tokens + kRouterTileTokens - 1) / kRouterTileTokens);
     uint32_t s = 1;
-    while (s < 16 && 2 * s * tiles <= (uint32_t)h->sm_count && (c.d / 64) % (2 * s) == 0) s *= 2;
+    while (s < 4 && 2 * s * tiles <= (uint32_t)h->sm_count && (c.d / 64) % (2 * s) == 0) s *= 2;
     return s;
 }
 
@@ -603,14 +609,14 @@ int make_rows_tmap(nvmai_cuda_moe *h, CUtensorMap *map, const void *base, uint64
     if (r != CUDA_SUCCESS) { h->last_cuda_error = (int)r; return NVMAI_CUDA_ECUDA; }
     return NVMAI_CUDA_OK;
 }
-// Tensor map over packed codes [experts][rows][row_bytes], box = 128 bytes x 128 rows of one expert.
+// Tensor map over packed codes [experts][rows][row_bytes], box = 128 bytes x box_rows rows of one expert.
 int make_codes_tmap(nvmai_cuda_moe *h, CUtensorMap *map, const void *base, uint64_t row_bytes, uint64_t rows, uint64_t experts,
-                    uint64_t expert_stride) {
+                    uint64_t expert_stride, uint32_t box_rows) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return NVMAI_CUDA_ECUDA;
     const cuuint64_t gdim[3] = {row_bytes, rows, experts};
     const cuuint64_t gstride[2] = {row_bytes, expert_stride};
-    const cuuint32_t box[3] = {128, 128, 1};
+    const cuuint32_t box[3] = {128, box_rows, 1};
     const cuuint32_t estride[3] = {1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), gdim, gstride, box, estride,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -625,18 +631,22 @@ int ensure_layer_maps(nvmai_cuda_moe *h, LayerViews &lv) {
     const uint64_t n = h->expert_map ? h->n_local : c.num_experts, st = lv.w.expert_stride;
     const uint64_t dx = (uint64_t)c.d * c.routed_bits / 8, fx = (uint64_t)c.f * c.routed_bits / 8;
     int rc;
-    if ((rc = make_codes_tmap(h, &lv.gate, blobs + lv.w.offsets.gate_w, dx, c.f, n, st)) ||
-        (rc = make_codes_tmap(h, &lv.up, blobs + lv.w.offsets.up_w, dx, c.f, n, st)) ||
-        (rc = make_codes_tmap(h, &lv.down, blobs + lv.w.offsets.down_w, fx, c.d, n, st)))
-        return rc;
-    if (c.shared_f != 0 && c.shared_f % 128 == 0) {
-        const uint64_t sdx = (uint64_t)c.d * c.shared_bits / 8, sfx = (uint64_t)c.shared_f * c.shared_bits / 8;
-        if ((rc = make_codes_tmap(h, &lv.sgate, lv.w.shared_gate_proj.w, sdx, c.shared_f, 1, sdx * c.shared_f)) ||
-            (rc = make_codes_tmap(h, &lv.sup, lv.w.shared_up_proj.w, sdx, c.shared_f, 1, sdx * c.shared_f)) ||
-            (rc = make_codes_tmap(h, &lv.sdown, lv.w.shared_down_proj.w, sfx, c.d, 1, sfx * c.d)))
+    const bool shared = c.shared_f != 0 && c.shared_f % 128 == 0;
+    const uint64_t sdx = (uint64_t)c.d * c.shared_bits / 8, sfx = (uint64_t)c.shared_f * c.shared_bits / 8;
+    for (const uint32_t box : {128u, 64u}) {
+        const bool tall = box == 128;
+        if ((rc = make_codes_tmap(h, tall ? &lv.gate : &lv.gate64, blobs + lv.w.offsets.gate_w, dx, c.f, n, st, box)) ||
+            (rc = make_codes_tmap(h, tall ? &lv.up : &lv.up64, blobs + lv.w.offsets.up_w, dx, c.f, n, st, box)) ||
+            (rc = make_codes_tmap(h, tall ? &lv.down : &lv.down64, blobs + lv.w.offsets.down_w, fx, c.d, n, st, box)))
             return rc;
-    } else {
+        if (shared && ((rc = make_codes_tmap(h, tall ? &lv.sgate : &lv.sgate64, lv.w.shared_gate_proj.w, sdx, c.shared_f, 1, sdx * c.shared_f, box)) ||
+                       (rc = make_codes_tmap(h, tall ? &lv.sup : &lv.sup64, lv.w.shared_up_proj.w, sdx, c.shared_f, 1, sdx * c.shared_f, box)) ||
+                       (rc = make_codes_tmap(h, tall ? &lv.sdown : &lv.sdown64, lv.w.shared_down_proj.w, sfx, c.d, 1, sfx * c.d, box))))
+            return rc;
+    }
+    if (!shared) {
         lv.sgate = lv.gate; lv.sup = lv.up; lv.sdown = lv.down;
+        lv.sgate64 = lv.gate64; lv.sup64 = lv.up64; lv.sdown64 = lv.down64;
     }
     if (c.router_kind == NVMAI_ROUTER_DENSE_F16 && c.num_experts % 128 == 0 &&
         (rc = make_rows_tmap(h, &lv.router, lv.w.router.w, c.num_experts, c.d, 128)))
@@ -666,7 +676,7 @@ int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
     auto alloc = [&](auto **ptr, size_t bytes) { return cudaMalloc(reinterpret_cast<void **>(ptr), bytes ? bytes : 16) == cudaSuccess; };
     const size_t dx = c.d + bp_extra_cols(c.d, 1), fx = c.f + bp_extra_cols(c.f, 2), sfx = c.shared_f + bp_extra_cols(c.shared_f, 2);
     const bool two_orders = c.shared_f != 0 && c.shared_bits != c.routed_bits;
-    const size_t logit_rows = std::min<size_t>(16 * T, std::max<size_t>(T, (size_t)h->sm_count * kRouterTileTokens));
+    const size_t logit_rows = std::min<size_t>(4 * T, std::max<size_t>(T, (size_t)h->sm_count * kRouterTileTokens));
     const size_t blocks = std::max(bp_route_blocks(c.max_tokens), bp_route_blocks(std::min(c.max_tokens, 1024u)));
     // (the columns behind the sums are never written: they stay the zeros put there now)
     const bool ok = alloc(&h->pf_x, T * dx * 2) && (!two_orders || alloc(&h->pf_xs, T * dx * 2)) && alloc(&h->pf_acts16, P * fx * 2) &&
@@ -708,8 +718,133 @@ struct PrefillMode {
     const __half *hidden_delta = nullptr;
 };
 
+// What comes before the experts' GEMMs: the rows packed (px says how; without dst only the scalar gate is taken), the
+// router, top-k and the pairs grouped by expert.  c: the handle's configuration, shared_f = 0 for routed rows only.
+int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c, const __half *x, uint32_t tokens, uint32_t *idx, __half *w,
+               PackXParams px, const uint32_t (&caps)[2], bool routed_only, cudaStream_t st) {
+    int rc;
+    const bool gated = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE;
+    const bool dense_gate = gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;
+    px.x = x; px.rows = tokens; px.n = c.d;
+    px.gate_row = dense_gate ? static_cast<const __half *>(lv.w.shared_gate.w) : nullptr;
+    px.gate_val = h->gate_val; px.out_half = c.out_dtype == NVMAI_OUT_FP32 ? 0 : 1;
+    if ((px.dst != nullptr || dense_gate || !routed_only) && (rc = launched(h, bp_pack_x(px, st)))) return rc;
+
+    RouteParams r{};
+    r.pes = static_cast<const uint16_t *>(lv.w.per_expert_scale);
+    r.idx = idx; r.w = w; r.tokens = tokens; r.E = c.num_experts; r.K = c.top_k;
+    r.expert_map = h->expert_map; r.n_local = h->expert_map ? h->n_local : c.num_experts;
+    r.block_hist = h->pf_hist; r.counter = h->pf_counter; r.sorted_pair = h->sorted_pair; r.inv = h->inv;
+    r.work[0] = h->work; r.work[1] = h->pf_work2; r.n_work[0] = h->n_work; r.n_work[1] = h->n_work + 2;
+    r.cap[0] = caps[0]; r.cap[1] = caps[1];
+    // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
+    // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
+    // affine routers keep the exact code-times-activation kernel.
+    const XSource xsrc{x, c.d, nullptr, nullptr};
+    if (!routed_only && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0) {
+        RouterArgs ra{};
+        ra.w = lv.router;
+        if ((rc = make_rows_tmap(h, &ra.x, x, tokens, c.d, kRouterTileTokens))) return rc;
+        r.splits = router_splits(h, tokens);
+        r.logits = h->pf_logits;
+        ra.p = RouterParams{h->pf_logits, tokens, c.num_experts, c.d, r.splits, h->status};
+        if ((rc = launched(h, bp_router(ra, st)))) return rc;
+        if (gated && !dense_gate && (rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, false, false, true, false, st))) return rc;
+    } else if (!routed_only) {
+        if ((rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, false, gated && !dense_gate, false, st))) return rc;
+    }
+    return launched(h, bp_route(r, st), bp_route_launches(tokens));
+}
+
+// Batches that bring few rows per expert (stream_gemm.cuh); the modes as in layer_prefill_impl.  Column blocks of an
+// item: 8 rows up to 9 per expert (evenly routed), else 16.  Measured, 8-bit layer: 256 rows 238 us in blocks of 8,
+// 251 us in blocks of 16; 400 rows 332 / 289 us.
+uint32_t stream_blocks(const nvmai_cuda_moe *h, uint32_t tokens) { return tokens * h->cfg.top_k <= 9 * h->cfg.num_experts ? 1 : 2; }
+
+// Up to here the streaming kernel is ahead of the tcgen05 kernel, whose cost at few rows is the conversion of the
+// codes, one pass per 4 bits of a code and per part of a scale.  Measured per layer, streaming / tcgen05: one pass
+// 320 rows 215 / 234 us, 512 rows 285 / 241; two passes (8-bit) 512 rows 353 / 410, 700 rows 459 / 421; four passes
+// (8-bit, fp16 scales kept exact) 700 rows 453 / 657.
+uint32_t stream_limit(const nvmai_cuda_moe *h, bool decode_order) {
+    if (h->stream_max_rows != ~0u) return h->stream_max_rows;
+    const auto &c = h->cfg;
+    return 10 * (c.routed_bits / 4) * (decode_order && c.meta_dtype == NVMAI_META_FP16 ? 2 : 1);
+}
+
+bool stream_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared) {
+    const auto &c = h->cfg;
+    if (!tc_shape_ok(h, with_shared) || c.top_k > (uint32_t)kMaxTopK) return false;
+    const bool wide = c.out_dtype == NVMAI_OUT_FP32;
+    const uint32_t nb = stream_blocks(h, tokens);
+    auto fits = [&](int phase, uint32_t kdim, uint32_t cols) {
+        SgParams p{};
+        p.kdim = kdim; p.out_cols = cols;
+        return sg_plan(p, phase, nb, wide) != 0;
+    };
+    return fits(0, c.d, c.f) && fits(1, c.f, c.d) && (!with_shared || c.shared_f == 0 || (fits(0, c.d, c.shared_f) && fits(1, c.shared_f, c.d)));
+}
+
+int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32_t tokens, void *hidden, void *y, uint32_t *out_idx,
+                      __half *out_w, cudaStream_t st, const PrefillMode mode) {
+    LayerViews &lv = h->layers[layer];
+    int rc = ensure_prefill_scratch(h, st);
+    if (rc || (rc = ensure_layer_maps(h, lv))) return rc;
+    nvmai_cuda_moe_config c = h->cfg;
+    if (mode.routed_only) c.shared_f = 0;
+    uint32_t *idx = out_idx ? out_idx : h->idx;
+    __half *w = out_w ? out_w : h->w;
+    const bool wide = c.out_dtype == NVMAI_OUT_FP32;
+    const uint32_t P = tokens * c.top_k, experts = h->expert_map ? h->n_local : c.num_experts, nb = stream_blocks(h, tokens);
+    const bool merged = c.shared_f != 0 && c.shared_bits == c.routed_bits && c.shared_f == c.f;
+    const uint32_t caps[2] = {8 * nb, 8 * nb};
+    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, PackXParams{}, caps, mode.routed_only, st))) return rc;
+    auto u8 = [](const void *p) { return static_cast<const uint8_t *>(p); };
+    for (int phase = 0; phase < 2; ++phase) {
+        SgArgs a{};
+        SgParams &p = a.p;
+        p.kdim = phase == 0 ? c.d : c.f; p.out_cols = phase == 0 ? c.f : c.d;
+        p.experts = u8(lv.w.experts); p.stride = lv.w.expert_stride; p.num_experts = experts;
+        p.work = h->work; p.n_work = h->n_work; p.sorted_pair = h->sorted_pair;
+        p.tokens = tokens; p.top_k = c.top_k; p.act = c.activation; p.status = h->status;
+        if (phase == 0) {
+            p.off_s[0] = lv.w.offsets.gate_s; p.off_b[0] = lv.w.offsets.gate_b; p.off_s[1] = lv.w.offsets.up_s; p.off_b[1] = lv.w.offsets.up_b;
+            p.shared_s[0] = u8(lv.w.shared_gate_proj.scales); p.shared_b[0] = u8(lv.w.shared_gate_proj.biases);
+            p.shared_s[1] = u8(lv.w.shared_up_proj.scales); p.shared_b[1] = u8(lv.w.shared_up_proj.biases);
+            p.rows = p.shared_rows = x; p.out = h->acts; p.shared_out = h->shared_act;
+            a.routed0 = lv.gate64; a.routed1 = lv.up64; a.shared0 = lv.sgate64; a.shared1 = lv.sup64;
+        } else {
+            p.off_s[0] = lv.w.offsets.down_s; p.off_b[0] = lv.w.offsets.down_b;
+            p.shared_s[0] = u8(lv.w.shared_down_proj.scales); p.shared_b[0] = u8(lv.w.shared_down_proj.biases);
+            p.rows = h->acts; p.shared_rows = h->shared_act; p.out = h->partial; p.shared_out = h->shared_partial;
+            a.routed0 = a.routed1 = lv.down64; a.shared0 = a.shared1 = lv.sdown64;
+        }
+        const size_t smem = sg_plan(p, phase, nb, wide);
+        p.shared_items = merged ? (tokens + p.cap - 1) / p.cap : 0;
+        const uint32_t units = (p.shared_items + std::min(P, experts + P / p.cap)) * p.units_per_item;
+        if ((rc = launched(h, sg_launch(phase, c.routed_bits, c.meta_dtype, c.out_dtype, nb, a, std::max(1u, std::min(units, (uint32_t)h->sm_count)), smem, st))))
+            return rc;
+        if (c.shared_f && !merged) {         // the shared expert's own bit width or size: a launch of its own
+            p.n_work = h->n_work + 3;        // a zero: no routed items
+            p.kdim = phase == 0 ? c.d : c.shared_f; p.out_cols = phase == 0 ? c.shared_f : c.d;
+            const size_t own = sg_plan(p, phase, nb, wide);
+            p.shared_items = (tokens + p.cap - 1) / p.cap;
+            if ((rc = launched(h, sg_launch(phase, c.shared_bits, c.meta_dtype, c.out_dtype, nb, a,
+                                            std::min(p.shared_items * p.units_per_item, (uint32_t)h->sm_count), own, st))))
+                return rc;
+        }
+    }
+    CombineRowsParams pc{};
+    pc.partial = h->partial; pc.shared_partial = c.shared_f ? h->shared_partial : nullptr;
+    pc.inv = h->inv; pc.routing_w = w; pc.gate_val = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE ? h->gate_val : nullptr;
+    pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y;
+    pc.tokens = tokens; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
+    return launched(h, bp_combine(pc, c.out_dtype, st));
+}
+
 int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32_t tokens, void *hidden, void *y,
                        uint32_t *out_idx, __half *out_w, cudaStream_t st, const PrefillMode mode = PrefillMode{}) {
+    if ((uint64_t)tokens * h->cfg.top_k <= (uint64_t)stream_limit(h, mode.decode_order) * h->cfg.num_experts && stream_ok(h, tokens, !mode.routed_only))
+        return layer_stream_impl(h, layer, x, tokens, hidden, y, out_idx, out_w, st, mode);
     LayerViews &lv = h->layers[layer];
     int rc = ensure_prefill_scratch(h, st);
     if (rc || (rc = ensure_layer_maps(h, lv))) return rc;
@@ -720,7 +855,6 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     const bool wide = c.out_dtype == NVMAI_OUT_FP32;
     const uint32_t P = tokens * c.top_k;
     const bool gated = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE;
-    const bool dense_gate = gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;
     // The shared expert rides in the routed launches when bit width and shapes agree; otherwise it gets launches of
     // its own.
     const bool merged = c.shared_f != 0 && c.shared_bits == c.routed_bits && c.shared_f == c.f;
@@ -739,36 +873,9 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     const EgPlan plan0 = eg_plan(g0, 0, want), plan1 = eg_plan(g1, 1, std::min(want, 128u));
 
     PackXParams px{};
-    px.x = x; px.dst = h->pf_x; px.dst2 = two_orders ? h->pf_xs : nullptr; px.rows = tokens; px.n = c.d;
-    px.permute = c.routed_bits == 4 ? 1 : 0;
-    px.gate_row = dense_gate ? static_cast<const __half *>(lv.w.shared_gate.w) : nullptr;
-    px.gate_val = h->gate_val; px.out_half = wide ? 0 : 1;
-    if ((rc = launched(h, bp_pack_x(px, st)))) return rc;
-
-    RouteParams r{};
-    r.pes = static_cast<const uint16_t *>(lv.w.per_expert_scale);
-    r.idx = idx; r.w = w; r.tokens = tokens; r.E = c.num_experts; r.K = c.top_k;
-    r.expert_map = use_map ? h->expert_map : nullptr; r.n_local = experts;
-    r.block_hist = h->pf_hist; r.counter = h->pf_counter; r.sorted_pair = h->sorted_pair; r.inv = h->inv;
-    r.work[0] = h->work; r.work[1] = h->pf_work2; r.n_work[0] = h->n_work; r.n_work[1] = h->n_work + 2;
-    r.cap[0] = plan0.cap; r.cap[1] = plan1.cap;
-    // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
-    // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
-    // affine routers keep the exact code-times-activation kernel.
-    const XSource xsrc{x, c.d, nullptr, nullptr};
-    if (!mode.routed_only && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0) {
-        RouterArgs ra{};
-        ra.w = lv.router;
-        if ((rc = make_rows_tmap(h, &ra.x, x, tokens, c.d, kRouterTileTokens))) return rc;
-        r.splits = router_splits(h, tokens);
-        r.logits = h->pf_logits;
-        ra.p = RouterParams{h->pf_logits, tokens, c.num_experts, c.d, r.splits, h->status};
-        if ((rc = launched(h, bp_router(ra, st)))) return rc;
-        if (gated && !dense_gate && (rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, false, false, true, false, st))) return rc;
-    } else if (!mode.routed_only) {
-        if ((rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, false, gated && !dense_gate, false, st))) return rc;
-    }
-    if ((rc = launched(h, bp_route(r, st), 2))) return rc;
+    px.dst = h->pf_x; px.dst2 = two_orders ? h->pf_xs : nullptr; px.permute = c.routed_bits == 4 ? 1 : 0;
+    const uint32_t caps[2] = {plan0.cap, plan1.cap};
+    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, px, caps, mode.routed_only, st))) return rc;
 
     const uint32_t shared_rows = merged ? tokens : 0;
     auto set_common = [&](EgParams &g, const EgPlan &plan) {
@@ -1224,7 +1331,8 @@ nvmai_cuda_moe *nvmai_cuda_moe_create(const nvmai_cuda_moe_config *config, int *
     h->layers.resize(c.num_layers);
     if (const char *env = std::getenv("NVMAI_CUDA_L2_PREFETCH")) h->l2_prefetch = env[0] == '1';
     if (const char *env = std::getenv("NVMAI_CUDA_PREFILL_TC")) h->prefill_tc = env[0] != '0';
-    if (const char *env = std::getenv("NVMAI_CUDA_GROUPED_MIN")) h->grouped_min_tokens = (uint32_t)std::max(1, std::atoi(env));
+    if (const char *env = std::getenv("NVMAI_CUDA_GROUPED_MIN")) { h->grouped_min_tokens = (uint32_t)std::max(1, std::atoi(env)); h->tc_min_tokens = 32; }
+    if (const char *env = std::getenv("NVMAI_CUDA_STREAM_ROWS")) h->stream_max_rows = (uint32_t)std::max(0, std::atoi(env));
     if (const char *env = std::getenv("NVMAI_CUDA_TC_MIN")) h->tc_min_tokens = (uint32_t)std::max(1, std::atoi(env));
     const size_t T = c.max_tokens;
     auto alloc = [&](auto **ptr, size_t bytes) -> bool {

@@ -1,5 +1,5 @@
-"""Edges of the grouped expert GEMMs (accumulator switches, ragged items, odd K-block counts, scale types) through the
-C ABI against the oracle."""
+"""Edges of the batched experts' kernels (accumulator switches, ragged items, odd K-block counts, scale types) through
+the C ABI against the oracle."""
 import sys
 from pathlib import Path
 
@@ -28,10 +28,12 @@ BF16, FP16 = fmt.META_BF16, fmt.META_FP16
     (4, BF16, fmt.OUT_FP16, 1, 256, 128), (4, BF16, fmt.OUT_FP16, 17, 768, 384), (4, BF16, fmt.OUT_FP32, 96, 256, 384),
     (4, BF16, fmt.OUT_FP16, 97, 512, 128), (4, BF16, fmt.OUT_FP16, 193, 256, 128), (8, BF16, fmt.OUT_FP16, 16, 768, 128),
     (8, BF16, fmt.OUT_FP32, 130, 256, 384), (4, FP16, fmt.OUT_FP16, 33, 768, 384), (8, FP16, fmt.OUT_FP32, 40, 256, 128),
-    (8, FP16, fmt.OUT_FP16, 65, 512, 384)])
+    (8, FP16, fmt.OUT_FP16, 65, 512, 384), (4, BF16, fmt.OUT_FP32, 5, 2048, 512), (8, FP16, fmt.OUT_FP16, 3, 2048, 512)])
 @pytest.mark.parametrize("entry", ["decode", "prefill"])
-def test_rows_of_every_item_match_the_oracle(bits, meta, out, tokens, d, f, entry, monkeypatch):
+@pytest.mark.parametrize("stream_rows", [0, 1000])
+def test_rows_of_every_item_match_the_oracle(bits, meta, out, tokens, d, f, stream_rows, entry, monkeypatch):
     monkeypatch.setenv("NVMAI_CUDA_TC_MIN", "1")
+    monkeypatch.setenv("NVMAI_CUDA_STREAM_ROWS", str(stream_rows))     # the tcgen05 kernel, the streaming kernel
     host = synthetic.layer(700 + tokens, d=d, f=f, shared_f=f, num_experts=8, routed_bits=bits, meta=meta)
     if bits == 8:       # zero-mean weights: the one-sided ones leave fp16's range at 8 bits
         rng = np.random.default_rng(tokens)
