@@ -117,6 +117,7 @@ __device__ __forceinline__ float router_row_logit(uint32_t kind, const uint8_t *
     float acc = 0.0f;
     if (kind == 0) {   // dense fp16 [E][D]
         const __half *wr = reinterpret_cast<const __half *>(W) + (size_t)row * D;
+#pragma unroll 4
         for (int c = lane; c < D / 8; c += 32) {
             uint4 wv = load_row16<SMEM>(wr + c * 8);
             const __half2 *wh = reinterpret_cast<const __half2 *>(&wv);
@@ -290,19 +291,19 @@ __device__ __forceinline__ void topk_select_block_vals(float s_in, int E, int K,
         if (valid && rank < 8) { cand_score[warp * 8 + rank] = s; cand_idx[warp * 8 + rank] = (uint32_t)tid; }
     }
     __syncthreads();
-    if (tid < 64) {
-        const float s = cand_score[tid];
-        const uint32_t e = cand_idx[tid];
-        if (e != 0xFFFFFFFFu) {
-            int rank = 0;
-#pragma unroll 16
-            for (int j = 0; j < 64; ++j) {
-                const float os = cand_score[j];
-                const uint32_t oe = cand_idx[j];      // empty slots: -inf score, index 0xFFFFFFFF: they lose every comparison
-                rank += (int)((os > s) | ((os == s) & (oe < e)));
-            }
-            if (rank < K) { sel_idx[rank] = e; sel_score[rank] = s; }
+    if (tid < kMaxExperts) {      // four threads per candidate, each against every fourth one
+        const float s = cand_score[tid >> 2];
+        const uint32_t e = cand_idx[tid >> 2];
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float os = cand_score[4 * j + (tid & 3)];
+            const uint32_t oe = cand_idx[4 * j + (tid & 3)];      // empty slots: -inf score, index 0xFFFFFFFF: they lose every comparison
+            rank += (int)((os > s) | ((os == s) & (oe < e)));
         }
+        rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+        rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+        if ((tid & 3) == 0 && e != 0xFFFFFFFFu && rank < K) { sel_idx[rank] = e; sel_score[rank] = s; }
     }
     __syncthreads();
 }
@@ -427,12 +428,32 @@ struct NextNorm {
 
 template <int OUT>
 __device__ __forceinline__ void next_norm_row(const NextNorm &nn, const void *hidden, uint32_t tok, int D, float *wsum) {
+    // the first 2048 values stay in registers between the two passes, and they and their weights are requested in one
+    // batch: this runs in one block while the chip waits for it
+    constexpr int kKeep = 8;
     const size_t base = (size_t)tok * D;
+    auto load = [&](int i) {
+        return OUT == OUT_F16 ? __half2float(__ldcg(reinterpret_cast<const __half *>(hidden) + base + i))
+                              : __ldcg(reinterpret_cast<const float *>(hidden) + base + i);
+    };
+    float keep[kKeep];
+    uint16_t w[kKeep];
     float ss = 0.0f;
     if (threadIdx.x < 256) {
-        for (int i = threadIdx.x; i < D; i += 256) {
-            const float v = OUT == OUT_F16 ? __half2float(__ldcg(reinterpret_cast<const __half *>(hidden) + base + i))
-                                           : __ldcg(reinterpret_cast<const float *>(hidden) + base + i);
+#pragma unroll
+        for (int j = 0; j < kKeep; ++j) {
+            const int i = threadIdx.x + j * 256;
+            keep[j] = i < D ? load(i) : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < kKeep; ++j) {
+            const int i = threadIdx.x + j * 256;
+            w[j] = i < D ? ldg_u16(nn.w + i) : (uint16_t)0;
+        }
+#pragma unroll
+        for (int j = 0; j < kKeep; ++j) ss = fmaf(keep[j], keep[j], ss);
+        for (int i = threadIdx.x + kKeep * 256; i < D; i += 256) {
+            const float v = load(i);
             ss = fmaf(v, v, ss);
         }
         ss = warp_sum(ss);
@@ -444,11 +465,13 @@ __device__ __forceinline__ void next_norm_row(const NextNorm &nn, const void *hi
 #pragma unroll
         for (int i = 0; i < 8; ++i) tot += wsum[i];
         const float sc = rsqrtf(tot / (float)D + nn.eps);
-        for (int i = threadIdx.x; i < D; i += 256) {
-            const float v = OUT == OUT_F16 ? __half2float(__ldcg(reinterpret_cast<const __half *>(hidden) + base + i))
-                                           : __ldcg(reinterpret_cast<const float *>(hidden) + base + i);
-            nn.x_next[base + i] = __float2half_rn(v * sc * meta_to_float<META_BF16>(ldg_u16(nn.w + i)));
+#pragma unroll
+        for (int j = 0; j < kKeep; ++j) {
+            const int i = threadIdx.x + j * 256;
+            if (i < D) nn.x_next[base + i] = __float2half_rn(keep[j] * sc * meta_to_float<META_BF16>(w[j]));
         }
+        for (int i = threadIdx.x + kKeep * 256; i < D; i += 256)
+            nn.x_next[base + i] = __float2half_rn(load(i) * sc * meta_to_float<META_BF16>(ldg_u16(nn.w + i)));
     }
 }
 

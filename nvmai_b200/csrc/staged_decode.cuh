@@ -96,6 +96,67 @@ __device__ __forceinline__ float norm_input(const XSource &src, size_t i) {
 __device__ __forceinline__ __half norm_output(const XSource &src, float scaled, int col) {
     return __float2half_rn(src.norm_w != nullptr ? scaled * meta_to_float<META_BF16>(ldg_u16(src.norm_w + col)) : scaled);
 }
+// One trip to memory: the row (KEEP values per thread; longer rows are re-read) stays in registers between the sum of
+// squares and the scaling, and the row, the delta and the norm weights are each requested as one batch before any of
+// them is used.  (With the delta's branch inside the loop the requests of a thread went out one after the other: 5.4
+// of a layer's 30 us.)
+template <int OUT, int KEEP>
+__device__ __forceinline__ void stage_normed_x(const XSource &src, uint32_t tok, int D, __half *xs, float *wsum, bool write_back) {
+    const size_t base = (size_t)tok * D;
+    const int n = blockDim.x;
+    float keep[KEEP];
+    uint16_t nw[KEEP];
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+        const int i = threadIdx.x + j * n;
+        keep[j] = i < D ? load_out<OUT>(src.y_prev, base + i) : 0.0f;
+    }
+    if (src.norm_w != nullptr) {
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            const int i = threadIdx.x + j * n;
+            nw[j] = i < D ? ldg_u16(src.norm_w + i) : (uint16_t)0;
+        }
+    }
+    if (src.delta != nullptr) {
+        __half d[KEEP];
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            const int i = threadIdx.x + j * n;
+            d[j] = i < D ? src.delta[base + i] : __float2half_rn(0.0f);
+        }
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) keep[j] = round_out<OUT>(keep[j] + __half2float(d[j]));
+    }
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) ss = fmaf(keep[j], keep[j], ss);
+    for (int i = threadIdx.x + KEEP * n; i < D; i += n) {
+        const float v = norm_input<OUT>(src, base + i);
+        ss = fmaf(v, v, ss);
+    }
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float tot = 0.0f;
+    for (int i = 0; i < (n >> 5); ++i) tot += wsum[i];
+    const float sc = rsqrtf(tot / (float)D + src.eps);
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+        const int i = threadIdx.x + j * n;
+        if (i < D) {
+            const float v = keep[j] * sc;
+            const __half h = __float2half_rn(src.norm_w != nullptr ? v * meta_to_float<META_BF16>(nw[j]) : v);
+            xs[i] = h;
+            if (write_back) src.x_out[base + i] = h;
+        }
+    }
+    for (int i = threadIdx.x + KEEP * n; i < D; i += n) {
+        const __half h = norm_output(src, norm_input<OUT>(src, base + i) * sc, i);
+        xs[i] = h;
+        if (write_back) src.x_out[base + i] = h;
+    }
+}
 template <int OUT>
 __device__ __forceinline__ void stage_x(const XSource &src, uint32_t tok, int D, __half *xs, float *wsum,
                                         bool write_back) {
@@ -103,46 +164,22 @@ __device__ __forceinline__ void stage_x(const XSource &src, uint32_t tok, int D,
         const __half *xrow = src.x + (size_t)tok * src.x_stride;
         for (int i = threadIdx.x * 8; i < D; i += blockDim.x * 8)
             *reinterpret_cast<uint4 *>(xs + i) = *reinterpret_cast<const uint4 *>(xrow + i);
+    } else if (D <= 8 * (int)blockDim.x) {
+        stage_normed_x<OUT, 8>(src, tok, D, xs, wsum, write_back);
     } else {
-        // one trip to memory: the row stays in registers between the sum of squares
-        // and the scaling (up to 16 values per thread; longer rows are re-read)
-        constexpr int kKeep = 16;
-        const size_t base = (size_t)tok * D;
-        float keep[kKeep];
-        float ss = 0.0f;
-#pragma unroll
-        for (int j = 0; j < kKeep; ++j) {
-            const int i = threadIdx.x + j * blockDim.x;
-            keep[j] = i < D ? norm_input<OUT>(src, base + i) : 0.0f;
-        }
-#pragma unroll
-        for (int j = 0; j < kKeep; ++j) ss = fmaf(keep[j], keep[j], ss);
-        for (int i = threadIdx.x + kKeep * blockDim.x; i < D; i += blockDim.x) {
-            const float v = norm_input<OUT>(src, base + i);
-            ss = fmaf(v, v, ss);
-        }
-        ss = warp_sum(ss);
-        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = ss;
-        __syncthreads();
-        float tot = 0.0f;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tot += wsum[i];
-        const float sc = rsqrtf(tot / (float)D + src.eps);
-#pragma unroll
-        for (int j = 0; j < kKeep; ++j) {
-            const int i = threadIdx.x + j * blockDim.x;
-            if (i < D) {
-                const __half h = norm_output(src, keep[j] * sc, i);
-                xs[i] = h;
-                if (write_back) src.x_out[base + i] = h;
-            }
-        }
-        for (int i = threadIdx.x + kKeep * blockDim.x; i < D; i += blockDim.x) {
-            const __half h = norm_output(src, norm_input<OUT>(src, base + i) * sc, i);
-            xs[i] = h;
-            if (write_back) src.x_out[base + i] = h;
-        }
+        stage_normed_x<OUT, 16>(src, tok, D, xs, wsum, write_back);
     }
     __syncthreads();
+}
+// Asks the L2 for what the norm reads and no kernel before this one brought in: the norm weights and the delta rows.
+// A hint only, so it may run before the wait for the kernels that write them.
+__device__ __forceinline__ void prefetch_norm_input(const XSource &src, uint32_t tok_begin, uint32_t tok_end, int D) {
+    if (src.y_prev == nullptr) return;
+    if (src.norm_w != nullptr)
+        for (int i = threadIdx.x * 64; i < D; i += blockDim.x * 64) l2_prefetch_line(src.norm_w + i);
+    if (src.delta != nullptr)
+        for (size_t i = (size_t)tok_begin * D + threadIdx.x * 64; i < (size_t)tok_end * D; i += blockDim.x * 64)
+            l2_prefetch_line(src.delta + i);
 }
 
 // ---------------------------------------------------------------------------
@@ -340,6 +377,7 @@ __device__ __forceinline__ void rows_block(unsigned char *smem, uint32_t kind, c
             }
         }
     }
+    prefetch_norm_input(p.xsrc, tok_begin, tok_end, p.D);
     pdl_wait();
     pdl_launch_dependents();
     trace_mark(p.trace, 0);
@@ -497,6 +535,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) stage2_kernel(Stage2Params 
     }
     // once this block's own tile is in: warm the L2 with its share of the expert's down projection (stage 3 reads it next)
     auto late = [&]() {
+        trace_mark(p.trace, 2);
         if (pf_blob == nullptr) return;
         l2_prefetch_slice(pf_blob + p.off.o[6], (size_t)p.D * p.F * BITS / 8, blockIdx.x, gridDim.x, lane);
         l2_prefetch_slice(pf_blob + p.off.o[7], (size_t)p.D * (p.F / kGroup) * 2, blockIdx.x, gridDim.x, lane);
@@ -701,6 +740,7 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32) stage3_kerne
         for (int i = 0; i < 6; ++i)
             if (p.next_ptr[i] != nullptr) l2_prefetch_slice(p.next_ptr[i], p.next_bytes[i], blockIdx.x, gridDim.x, lane);
     }
+    if (p.next.w != nullptr && p.hidden != nullptr && blockIdx.x < p.D / 64 && threadIdx.x == 0) l2_prefetch_line(p.next.w + blockIdx.x * 64);
     __syncthreads();        // the barrier of each unit is initialised before its second warp waits on it
     pdl_wait();
     pdl_launch_dependents();
@@ -709,6 +749,13 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32) stage3_kerne
     float *wk_s = part + (kMaxTopK + 1) * kDownSplit * 16;
     if (threadIdx.x < p.top_k) wk_s[threadIdx.x] = __half2float(p.routing_w[(size_t)tok * p.top_k + threadIdx.x]);
     const float gate_v = (p.gate_val != nullptr && threadIdx.x < 16) ? p.gate_val[tok] : 0.0f;
+    // likewise the hidden state and the delta this thread adds to (no other thread writes them)
+    float hidden_v = 0.0f, delta_v = 0.0f;
+    if (p.hidden != nullptr && threadIdx.x < 16) {
+        const size_t i = (size_t)tok * p.D + row0 + threadIdx.x;
+        hidden_v = load_out<OUT>(p.hidden, i);
+        if (p.hidden_delta != nullptr) delta_v = __half2float(p.hidden_delta[i]);
+    }
     bool ok = true;
     float v[2] = {0.0f, 0.0f};
     if (routed && local) {
@@ -776,23 +823,27 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32) stage3_kerne
         const float yv = round_out<OUT>(acc);
         if (p.y != nullptr) store_out<OUT>(p.y, i, yv);
         if (p.hidden != nullptr) {                                                              // utility.metal:94-103
-            float hv = load_out<OUT>(p.hidden, i);
-            if (p.hidden_delta != nullptr) hv = round_out<OUT>(hv + __half2float(p.hidden_delta[i]));
+            const float hv = p.hidden_delta != nullptr ? round_out<OUT>(hidden_v + delta_v) : hidden_v;
             store_out<OUT>(p.hidden, i, hv + yv);
         }
     }
+    trace_mark(p.trace, 3);
     if (p.next.w != nullptr && p.hidden != nullptr) {
         // the row's blocks count themselves; the one that finds the row complete normalises it for the next block
         __shared__ bool row_done;
         __shared__ float wsum_next[8];
-        if (threadIdx.x < 16) __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const unsigned int prev = atomicAdd(p.next.row_counter + tok, 1u);
-            row_done = prev == gridDim.x - 1;
-            if (row_done) { p.next.row_counter[tok] = 0; __threadfence(); }
+        if (warp == 0) {          // the warp that stored the block's 16 values
+            __syncwarp();
+            if (lane == 0) {
+                __threadfence();
+                const unsigned int prev = atomicAdd(p.next.row_counter + tok, 1u);
+                row_done = prev == gridDim.x - 1;
+                if (row_done) { p.next.row_counter[tok] = 0; __threadfence(); }
+            }
         }
         __syncthreads();
+        trace_mark(p.trace, 4);
+        if (p.trace != nullptr && row_done && threadIdx.x == 0) p.trace[2 + 5] = global_timer_ns();
         if (row_done) next_norm_row<OUT>(p.next, p.hidden, tok, p.D, wsum_next);
     }
     trace_end(p.trace);

@@ -41,6 +41,7 @@ __device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 // this block's share of a contiguous range, cut into pieces one lane issues each
+__device__ __forceinline__ void l2_prefetch_line(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void l2_prefetch_slice(const void *base, size_t total_bytes, uint32_t part, uint32_t parts,
                                                   int lane) {
     const size_t per = ((total_bytes + parts - 1) / parts + 15) & ~(size_t)15;
