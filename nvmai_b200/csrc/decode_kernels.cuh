@@ -65,6 +65,11 @@ __device__ __forceinline__ const uint8_t *expert_blob(const RoutedSource &src, u
     return src.base + (size_t)e * src.stride;
 }
 
+// the same as an index into the layer's blobs (no expert map): `sel` = the block's own selection, used when logits are given
+__device__ __forceinline__ uint32_t routed_expert(const RoutedSource &src, const uint32_t *sel, uint32_t token, uint32_t slot, uint32_t top_k) {
+    return min(src.logits != nullptr ? sel[slot] : src.idx[(size_t)token * top_k + slot], src.num_experts - 1u);
+}
+
 // ---------------------------------------------------------------------------
 // Router logits (moe.metal:174-231): one warp per expert row.
 // ---------------------------------------------------------------------------

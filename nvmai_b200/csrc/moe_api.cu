@@ -44,6 +44,8 @@ struct LayerViews {
     // the packed codes (and a dense router) as tensor maps, made by the first call that runs the expert GEMMs
     bool tc_maps = false;
     CUtensorMap gate, up, down, sgate, sup, sdown, router;
+    TileMaps tiles;                 // the decode stages' boxes
+    int tile_maps = 0;              // 0 not looked at yet, 1 made, -1 the layout has none
     CUtensorMap gate64, up64, down64, sgate64, sup64, sdown64;     // the same codes in boxes of 64 rows (stream_gemm.cuh)
 };
 
@@ -321,9 +323,102 @@ int launch_stage1(nvmai_cuda_moe *h, const LayerViews &lv, const XSource &xsrc, 
     });
 }
 
+// cuTensorMapEncodeTiled, looked up through the runtime (the library does not link libcuda)
+using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled_fn() {
+    static EncodeTiledFn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
+// One tensor map: `rank` dimensions, dim 0 contiguous; strides in bytes for dims 1.. .
+int encode_map(nvmai_cuda_moe *h, CUtensorMap *map, CUtensorMapDataType dt, uint32_t rank, const void *base,
+              const cuuint64_t *gdim, const cuuint64_t *gstride, const cuuint32_t *box, bool swizzle) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return NVMAI_CUDA_ECUDA;
+    const cuuint32_t estride[5] = {1, 1, 1, 1, 1};
+    const CUresult r = enc(map, dt, rank, const_cast<void *>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { h->last_cuda_error = (int)r; return NVMAI_CUDA_ECUDA; }
+    return NVMAI_CUDA_OK;
+}
+
+// Tensor maps of a layer's expert weights (the expert is a coordinate).  NVMAI_CUDA_EINVAL when the layer's blob layout
+// is not the regular one the maps describe.
+int encode_tile_maps(nvmai_cuda_moe *h, const nvmai_cuda_moe_layer &w, TileMaps &m) {
+    const auto &c = h->cfg;
+    const auto &o = w.offsets;
+    const uint64_t rbd = (uint64_t)c.d * c.routed_bits / 8, rbf = (uint64_t)c.f * c.routed_bits / 8, gd = c.d / 64, gf = c.f / 64;
+    const uint64_t n_blobs = h->expert_map ? h->n_local : c.num_experts;      // blobs this rank holds, in local-index order
+    const uint8_t *base = static_cast<const uint8_t *>(w.experts);
+    // gate and up must be laid out alike, scales before biases (the repacker's order, RepackPlanner.swift:365-426)
+    if (w.expert_stride == 0 || o.up_w <= o.gate_w || o.up_s <= o.gate_s || o.gate_b <= o.gate_s || o.down_b <= o.down_s ||
+        o.up_s - o.gate_s != o.up_b - o.gate_b)
+        return NVMAI_CUDA_EINVAL;
+    int rc;
+    {   // routed gate + up codes: {128 B, row, chunk, gate|up, expert}
+        const cuuint64_t gdim[5] = {128, c.f, rbd / 128, 2, n_blobs};
+        const cuuint64_t gstr[4] = {rbd, 128, (cuuint64_t)(o.up_w - o.gate_w), w.expert_stride};
+        const cuuint32_t box[5] = {128, (cuuint32_t)kTileFeatures, (cuuint32_t)(rbd / 128), 2, 1};
+        if ((rc = encode_map(h, &m.gu_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base + o.gate_w, gdim, gstr, box, true))) return rc;
+    }
+    {   // their scales and biases: {value, gate|up, scale|bias, expert}
+        const cuuint64_t gdim[4] = {(cuuint64_t)c.f * gd, 2, 2, n_blobs};
+        const cuuint64_t gstr[3] = {(cuuint64_t)(o.up_s - o.gate_s), (cuuint64_t)(o.gate_b - o.gate_s), w.expert_stride};
+        const cuuint32_t box[4] = {(cuuint32_t)(kTileFeatures * gd), 2, 2, 1};
+        if ((rc = encode_map(h, &m.gu_meta, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, base + o.gate_s, gdim, gstr, box, false))) return rc;
+    }
+    {   // routed down codes: {128 B, row, chunk, expert}
+        const cuuint64_t gdim[4] = {128, c.d, rbf / 128, n_blobs};
+        const cuuint64_t gstr[3] = {rbf, 128, w.expert_stride};
+        const cuuint32_t box[4] = {128, (cuuint32_t)kTileRows, (cuuint32_t)(rbf / 128), 1};
+        if ((rc = encode_map(h, &m.dn_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base + o.down_w, gdim, gstr, box, true))) return rc;
+    }
+    {   // and meta: {value, scale|bias, expert}
+        const cuuint64_t gdim[3] = {(cuuint64_t)c.d * gf, 2, n_blobs};
+        const cuuint64_t gstr[2] = {(cuuint64_t)(o.down_b - o.down_s), w.expert_stride};
+        const cuuint32_t box[3] = {(cuuint32_t)(kTileRows * gf), 2, 1};
+        if ((rc = encode_map(h, &m.dn_meta, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, base + o.down_s, gdim, gstr, box, false))) return rc;
+    }
+    if (c.shared_f && c.shared_bits == c.routed_bits) {   // the shared expert's gate and up codes: {128 B, row, chunk}
+        const cuuint64_t gdim[3] = {128, c.shared_f, rbd / 128};
+        const cuuint64_t gstr[2] = {rbd, 128};
+        const cuuint32_t box[3] = {128, (cuuint32_t)kTileFeatures, (cuuint32_t)(rbd / 128)};
+        if ((rc = encode_map(h, &m.sg_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.shared_gate_proj.w, gdim, gstr, box, true))) return rc;
+        if ((rc = encode_map(h, &m.su_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.shared_up_proj.w, gdim, gstr, box, true))) return rc;
+    }
+    return NVMAI_CUDA_OK;
+}
+
+// A layer's maps for the decode stages, made once per registration; nullptr where the shape or the layout has none: whole
+// 128-byte lines per row, boxes of at most 256 lines and values, every expert on this rank.
+const TileMaps *ensure_tile_maps(nvmai_cuda_moe *h, LayerViews &lv) {
+    if (lv.tile_maps == 0) {
+        const auto &c = h->cfg;
+        const uint32_t rbd = c.d * c.routed_bits / 8, rbf = c.f * c.routed_bits / 8;
+        const bool fits = h->expert_map == nullptr && rbd % 128 == 0 && rbf % 128 == 0 && kTileFeatures * (c.d / 64) <= 256 &&
+                          kTileRows * (c.f / 64) <= 256 && rbd / 128 <= 256 && c.f % kTileFeatures == 0 && encode_tiled_fn() != nullptr;
+        const int cuda_error = h->last_cuda_error;
+        lv.tile_maps = fits && encode_tile_maps(h, lv.w, lv.tiles) == NVMAI_CUDA_OK ? 1 : -1;
+        h->last_cuda_error = cuda_error;
+    }
+    return lv.tile_maps > 0 ? &lv.tiles : nullptr;
+}
+
+// maps: the layer's tensor maps, or nullptr (blobs that no map describes): the tiles are then copied row by row.
+// shared: with maps, the layer whose shared expert's gate/up tiles run here as well.
 int launch_stage2(nvmai_cuda_moe *h, const RoutedSource &src, const ExpertOffsets &off, const __half *x,
                   uint32_t x_stride, uint32_t tokens, void *acts, const uint32_t *active_slots_dev,
-                  uint32_t n_slots, bool pdl, cudaStream_t st) {
+                  uint32_t n_slots, bool pdl, cudaStream_t st, const TileMaps *maps = nullptr, const LayerViews *shared = nullptr) {
     const auto &c = h->cfg;
     Stage2Params p{};
     p.src = src; p.off = off; p.x = x; p.x_stride = x_stride; p.acts = acts;
@@ -332,17 +427,24 @@ int launch_stage2(nvmai_cuda_moe *h, const RoutedSource &src, const ExpertOffset
     p.prefetch_down = (h->l2_prefetch && h->in_layer_chain) ? 1u : 0u;
     p.status = h->status;
     p.trace = h->cur_trace;
-    dim3 grid((c.f + kBlockFeatures - 1) / kBlockFeatures, n_slots, tokens);
-    const size_t smem = GateUpLayout(c.d, c.routed_bits).total;
+    p.n_slots = n_slots;
+    if (shared) {
+        p.sgate = to_mat(shared->w.shared_gate_proj); p.sup = to_mat(shared->w.shared_up_proj);
+        p.shared_f = c.shared_f; p.shared_act = h->shared_act;
+    }
+    const uint32_t f = shared ? std::max(c.f, c.shared_f) : c.f;
+    dim3 grid((f + kBlockFeatures - 1) / kBlockFeatures, n_slots + (shared ? 1 : 0), tokens);
+    const size_t smem = GateUpLayout(c.d, c.routed_bits, maps != nullptr).total;
     return dispatch_bits_meta(c.routed_bits, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
-            return launch_kernel(h, stage2_kernel<decltype(B)::value, decltype(M)::value, decltype(O)::value>, grid,
-                                 dim3(kDecodeThreads), smem, st, pdl, p);
+            constexpr int b = decltype(B)::value, m = decltype(M)::value, o = decltype(O)::value;
+            return maps ? launch_kernel(h, stage2_kernel<b, m, o, true>, grid, dim3(kDecodeThreads), smem, st, pdl, p, *maps)
+                        : launch_kernel(h, stage2_kernel<b, m, o, false>, grid, dim3(kDecodeThreads), smem, st, pdl, p, TileMaps{});
         });
     });
 }
 
-int launch_stage3(nvmai_cuda_moe *h, Stage3Params p, uint32_t tokens, bool pdl, cudaStream_t st) {
+int launch_stage3(nvmai_cuda_moe *h, Stage3Params p, uint32_t tokens, bool pdl, cudaStream_t st, const TileMaps *maps = nullptr) {
     const auto &c = h->cfg;
     p.D = c.d; p.F = c.f;
     p.status = h->status;
@@ -350,11 +452,12 @@ int launch_stage3(nvmai_cuda_moe *h, Stage3Params p, uint32_t tokens, bool pdl, 
     dim3 grid(c.d / kTileRows, tokens);
     const uint32_t units = p.top_k + (p.shared_f ? 1 : 0);
     const uint32_t threads = (units < 1 ? 1 : units) * kDownSplit * 32;
-    const size_t smem = DownLayout(c.f, p.shared_f, c.routed_bits, p.shared_bits, units).total;
+    const size_t smem = DownLayout(c.f, p.shared_f, c.routed_bits, p.shared_bits, units, maps != nullptr).total;
     return dispatch_bits_meta(c.routed_bits, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
-            return launch_kernel(h, stage3_kernel<decltype(B)::value, decltype(M)::value, decltype(O)::value>, grid,
-                                 dim3(threads), smem, st, pdl, p);
+            constexpr int b = decltype(B)::value, m = decltype(M)::value, o = decltype(O)::value;
+            return maps ? launch_kernel(h, stage3_kernel<b, m, o, true>, grid, dim3(threads), smem, st, pdl, p, *maps)
+                        : launch_kernel(h, stage3_kernel<b, m, o, false>, grid, dim3(threads), smem, st, pdl, p, TileMaps{});
         });
     });
 }
@@ -499,16 +602,19 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
                       void *hidden, void *h2_out, uint32_t *out_idx, __half *out_w, cudaStream_t st,
                       const LayerViews *next_layer = nullptr, const __half *hidden_delta = nullptr) {
     const auto &c = h->cfg;
-    const LayerViews &lv = h->layers[layer];
+    LayerViews &lv = h->layers[layer];
     uint32_t *idx = out_idx ? out_idx : h->idx;
     __half *w = out_w ? out_w : h->w;
     const bool grouped = tokens >= h->grouped_min_tokens;
+    const TileMaps *maps = grouped ? nullptr : ensure_tile_maps(h, lv);
+    // with boxes the shared expert's gate/up tiles ride in stage 2, which leaves stage 1 to the router (1 us less to wait for)
+    const bool shared_late = maps != nullptr && c.shared_f != 0 && c.shared_bits == c.routed_bits;
     auto slot = [&](int stage) { return (h->trace_on && !grouped) ? h->trace + ((size_t)layer * 3 + stage) * kTraceWords : nullptr; };
     h->cur_trace = slot(0);
     // single-token path: the expert stages select the experts themselves from the logits
     // (the block-wide selection wants one thread per expert in the down stage's block too)
     const bool defer = !grouped && (c.top_k + (c.shared_f ? 1 : 0)) * kDownSplit * 32 >= (uint32_t)kMaxExperts;
-    int rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, c.shared_f != 0 && !grouped, c.shared_f != 0, true, st,
+    int rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, c.shared_f != 0 && !grouped && !shared_late, c.shared_f != 0, true, st,
                            defer);
     if (rc) return rc;
     h->cur_trace = nullptr;
@@ -522,7 +628,8 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
         src.publish_w = w;
     }
     h->in_layer_chain = true;
-    rc = launch_stage2(h, src, to_offsets(lv.w.offsets), x_rows, c.d, tokens, h->acts, nullptr, c.top_k, true, st);
+    rc = launch_stage2(h, src, to_offsets(lv.w.offsets), x_rows, c.d, tokens, h->acts, nullptr, c.top_k, true, st, maps,
+                       shared_late ? &lv : nullptr);
     h->in_layer_chain = false;
     h->cur_trace = nullptr;
     if (rc) return rc;
@@ -561,7 +668,7 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
             add(nw.shared_gate_proj.scales, sm);   // the remaining meta arrays are small; the copies fetch them
         }
     }
-    rc = launch_stage3(h, p, tokens, true, st);
+    rc = launch_stage3(h, p, tokens, true, st, maps);
     h->cur_trace = nullptr;
     return rc;
 }
@@ -575,22 +682,6 @@ uint32_t router_splits(const nvmai_cuda_moe *h, uint32_t tokens) {
     uint32_t s = 1;
     while (s < 4 && 2 * s * tiles <= (uint32_t)h->sm_count && (c.d / 64) % (2 * s) == 0) s *= 2;
     return s;
-}
-
-// cuTensorMapEncodeTiled, looked up through the runtime (the library does not link libcuda)
-using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
 }
 
 // Tensor map over fp16 rows [rows][cols], box = 64 values x box_rows rows, 128-byte swizzle, zero fill outside.  Base
@@ -1040,72 +1131,25 @@ bool pd_plan(const nvmai_cuda_moe *h, PdPlan &plan) {
     return true;
 }
 
-// One tensor map: `rank` dimensions, dim 0 contiguous; strides in bytes for dims 1.. .
-int pd_encode(nvmai_cuda_moe *h, CUtensorMap *map, CUtensorMapDataType dt, uint32_t rank, const void *base,
-              const cuuint64_t *gdim, const cuuint64_t *gstride, const cuuint32_t *box, bool swizzle) {
-    EncodeTiledFn enc = encode_tiled_fn();
-    if (!enc) return NVMAI_CUDA_ECUDA;
-    const cuuint32_t estride[5] = {1, 1, 1, 1, 1};
-    const CUresult r = enc(map, dt, rank, const_cast<void *>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { h->last_cuda_error = (int)r; return NVMAI_CUDA_ECUDA; }
-    return NVMAI_CUDA_OK;
-}
-
 // The per-layer table of the resident kernel: tensor maps over the layer's expert array (the expert is a coordinate)
 // and the plain pointers.  NVMAI_CUDA_EINVAL when a layer's blob layout is not the regular one the maps describe.
 int pd_build_layers(nvmai_cuda_moe *h, std::vector<PdLayer> &host) {
     const auto &c = h->cfg;
-    const uint64_t bits = c.routed_bits;
-    const uint64_t rbd = (uint64_t)c.d * bits / 8, rbf = (uint64_t)c.f * bits / 8, rbs = (uint64_t)c.shared_f * bits / 8;
-    const uint64_t gd = c.d / 64, gf = c.f / 64;
+    const uint64_t rbs = (uint64_t)c.shared_f * c.routed_bits / 8;
     host.assign(c.num_layers, PdLayer{});
-    const uint64_t n_blobs = h->expert_map ? h->n_local : c.num_experts;      // blobs this rank holds, in local-index order
     for (uint32_t l = 0; l < c.num_layers; ++l) {
         const auto &w = h->layers[l].w;
-        const auto &o = w.offsets;
         PdLayer &d = host[l];
-        const uint8_t *base = static_cast<const uint8_t *>(w.experts);
-        // gate and up must be laid out alike, scales before biases (the repacker's order, RepackPlanner.swift:365-426)
-        if (w.expert_stride == 0 || o.up_w <= o.gate_w || o.up_s <= o.gate_s || o.gate_b <= o.gate_s || o.down_b <= o.down_s ||
-            o.up_s - o.gate_s != o.up_b - o.gate_b)
-            return NVMAI_CUDA_EINVAL;
+        TileMaps m;
         int rc;
-        {   // routed gate + up codes: {128 B, row, chunk, gate|up, expert}
-            const cuuint64_t gdim[5] = {128, c.f, rbd / 128, 2, n_blobs};
-            const cuuint64_t gstr[4] = {rbd, 128, (cuuint64_t)(o.up_w - o.gate_w), w.expert_stride};
-            const cuuint32_t box[5] = {128, (cuuint32_t)kTileFeatures, (cuuint32_t)(rbd / 128), 2, 1};
-            if ((rc = pd_encode(h, &d.gu_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base + o.gate_w, gdim, gstr, box, true))) return rc;
-        }
-        {   // their scales and biases: {value, gate|up, scale|bias, expert}
-            const cuuint64_t gdim[4] = {(cuuint64_t)c.f * gd, 2, 2, n_blobs};
-            const cuuint64_t gstr[3] = {(cuuint64_t)(o.up_s - o.gate_s), (cuuint64_t)(o.gate_b - o.gate_s), w.expert_stride};
-            const cuuint32_t box[4] = {(cuuint32_t)(kTileFeatures * gd), 2, 2, 1};
-            if ((rc = pd_encode(h, &d.gu_meta, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, base + o.gate_s, gdim, gstr, box, false))) return rc;
-        }
-        {   // routed down codes: {128 B, row, chunk, expert}
-            const cuuint64_t gdim[4] = {128, c.d, rbf / 128, n_blobs};
-            const cuuint64_t gstr[3] = {rbf, 128, w.expert_stride};
-            const cuuint32_t box[4] = {128, (cuuint32_t)kTileRows, (cuuint32_t)(rbf / 128), 1};
-            if ((rc = pd_encode(h, &d.dn_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base + o.down_w, gdim, gstr, box, true))) return rc;
-        }
-        {   // and meta: {value, scale|bias, expert}
-            const cuuint64_t gdim[3] = {(cuuint64_t)c.d * gf, 2, n_blobs};
-            const cuuint64_t gstr[2] = {(cuuint64_t)(o.down_b - o.down_s), w.expert_stride};
-            const cuuint32_t box[3] = {(cuuint32_t)(kTileRows * gf), 2, 1};
-            if ((rc = pd_encode(h, &d.dn_meta, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, base + o.down_s, gdim, gstr, box, false))) return rc;
-        }
-        if (c.shared_f) {   // the shared expert's three code matrices: {128 B, row, chunk}
-            const cuuint64_t gdim[3] = {128, c.shared_f, rbd / 128};
-            const cuuint64_t gstr[2] = {rbd, 128};
-            const cuuint32_t box[3] = {128, (cuuint32_t)kTileFeatures, (cuuint32_t)(rbd / 128)};
-            if ((rc = pd_encode(h, &d.sg_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.shared_gate_proj.w, gdim, gstr, box, true))) return rc;
-            if ((rc = pd_encode(h, &d.su_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.shared_up_proj.w, gdim, gstr, box, true))) return rc;
+        if ((rc = encode_tile_maps(h, w, m))) return rc;
+        d.gu_w = m.gu_w; d.gu_meta = m.gu_meta; d.dn_w = m.dn_w; d.dn_meta = m.dn_meta;
+        if (c.shared_f) { d.sg_w = m.sg_w; d.su_w = m.su_w; }
+        if (c.shared_f) {   // the shared expert's down codes: {128 B, row, chunk}
             const cuuint64_t ddim[3] = {128, c.d, rbs / 128};
             const cuuint64_t dstr[2] = {rbs, 128};
             const cuuint32_t dbox[3] = {128, (cuuint32_t)kTileRows, (cuuint32_t)(rbs / 128)};
-            if ((rc = pd_encode(h, &d.sd_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.shared_down_proj.w, ddim, dstr, dbox, true))) return rc;
+            if ((rc = encode_map(h, &d.sd_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, w.shared_down_proj.w, ddim, dstr, dbox, true))) return rc;
         }
         d.experts_stride = w.expert_stride;
         d.rW = static_cast<const uint8_t *>(w.router.w);
@@ -1454,6 +1498,7 @@ int nvmai_cuda_moe_register_layer(nvmai_cuda_moe *h, uint32_t layer, const nvmai
     h->layers[layer].w = *wts;
     h->layers[layer].registered = true;
     h->layers[layer].tc_maps = false;
+    h->layers[layer].tile_maps = 0;
     h->graphs_stale = h->ep_graphs_stale = true;
     h->pd_layers_stale = true;
     return NVMAI_CUDA_OK;
@@ -1650,7 +1695,7 @@ int nvmai_cuda_moe_set_expert_map(nvmai_cuda_moe *h, const uint32_t *map_host, u
     if (!h) return NVMAI_CUDA_EINVAL;
     const auto &c = h->cfg;
     h->pd_layers_stale = true;              // the tensor maps span the blobs this rank holds
-    for (auto &lv : h->layers) lv.tc_maps = false;
+    for (auto &lv : h->layers) { lv.tc_maps = false; lv.tile_maps = 0; }
     if (map_host == nullptr) {              // back to "every expert is local"
         cudaFree(h->expert_map);
         h->expert_map = nullptr;

@@ -217,23 +217,6 @@ struct PdParams {
 };
 
 // ---- copies ---------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_addr(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                 ::"r"(smem_addr(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
-                                            uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                 ::"r"(smem_addr(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
-
 // one lane: the gate/up tile of features f0..f0+7 of routed expert e (codes: one operation; scales + biases: one)
 __device__ __forceinline__ void pd_issue_routed_tile(unsigned char *tile, const PdLayout &L, uint64_t *bar, const PdLayer &ly,
                                                      int f0, uint32_t e, int D, int bits) {
@@ -307,101 +290,6 @@ __device__ __forceinline__ void pd_issue_shared_down(unsigned char *region, cons
     else if (lane < 3)
         bulk_g2s(region + L.dn_meta_s + (lane == 1 ? 0 : meta_bytes), (lane == 1 ? ly.sdS : ly.sdB) + (size_t)row0 * groups,
                  meta_bytes, bar);
-}
-
-// ---- swizzled tiles ----------------------------------------------------------------
-// A box of R rows x C chunks of 128 bytes lands as [chunk][row][128 B] with the 16-byte unit index XORed with
-// (line index mod 8) = row mod 8 (R is 8 or 16).  The codes of lane (g, t) for group G of row r:
-//   4-bit  8 bytes at row byte 32 G + 8 t      8-bit  16 bytes at row byte 64 G + 16 t
-template <int BITS>
-__device__ __forceinline__ uint32_t swz_offset(int G, int r, int t, int rows_per_chunk) {
-    if (BITS == 4) {
-        const int chunk = G >> 2, unit = ((G & 3) << 1) | (t >> 1);
-        return (uint32_t)(((chunk * rows_per_chunk + r) << 7) | (((unit ^ (r & 7)) << 4) | ((t & 1) << 3)));
-    }
-    const int chunk = G >> 1, unit = ((G & 1) << 2) | t;
-    return (uint32_t)(((chunk * rows_per_chunk + r) << 7) | ((unit ^ (r & 7)) << 4));
-}
-
-// acc += rows ra / rb (box rows; meta rows ma / mb) of a swizzled tile over groups [g_begin, g_begin + NG) against
-// prepared activation fragments.  The arithmetic of tile_accumulate_prepared.
-template <int BITS, int META, int NG>
-__device__ __forceinline__ void swz_accumulate_prepared(const unsigned char *box_a, const unsigned char *box_b, int rows_per_chunk,
-                                                        int ra, int rb, const uint16_t *s, const uint16_t *b, int ma, int mb,
-                                                        int groups_total, int g_begin, const uint32_t (&xb)[NG][8],
-                                                        const float (&xsum)[NG], float (&acc)[1][4]) {
-    using vec = typename GroupBytes<BITS>::vec;
-    using MW = typename MetaWord<NG>::type;
-    const int t = threadIdx.x & 3;
-    const MW sa = *reinterpret_cast<const MW *>(s + ma * groups_total + g_begin);
-    const MW sb = *reinterpret_cast<const MW *>(s + mb * groups_total + g_begin);
-    const MW ba = *reinterpret_cast<const MW *>(b + ma * groups_total + g_begin);
-    const MW bb = *reinterpret_cast<const MW *>(b + mb * groups_total + g_begin);
-    // g_begin is a multiple of NG (= 4) at every call: written as 4 * (g_begin / 4) + j, the group index shows the
-    // compiler which of its bits are the constant j, and the swizzle of the four groups folds to a few operations
-    const int g4 = (g_begin >> 2) << 2;
-#pragma unroll
-    for (int j = 0; j < NG; ++j) {
-        const vec wa[1] = {*reinterpret_cast<const vec *>(box_a + swz_offset<BITS>(g4 + j, ra, t, rows_per_chunk))};
-        const vec wb[1] = {*reinterpret_cast<const vec *>(box_b + swz_offset<BITS>(g4 + j, rb, t, rows_per_chunk))};
-        const uint16_t s0[1] = {meta_pick(sa, j)}, s1[1] = {meta_pick(sb, j)};
-        const uint16_t b0[1] = {meta_pick(ba, j)}, b1[1] = {meta_pick(bb, j)};
-        group_step<BITS, META, 1, true>(wa, wb, s0, s1, b0, b1, xb[j], xsum[j], 0.0f, acc);
-    }
-}
-
-// Two tiles against the same prepared fragments (two consecutive gate/up tiles of one pair): the two tiles' chains are
-// independent, so their loads and tensor-core steps overlap; each tile's own arithmetic is that of the function above.
-template <int BITS, int META, int NG>
-__device__ __forceinline__ void swz_accumulate_prepared2(const unsigned char *const (&box_a)[2], const unsigned char *const (&box_b)[2],
-                                                         int rows_per_chunk, int ra, int rb, const uint16_t *const (&s)[2],
-                                                         const uint16_t *const (&b)[2], int ma, int mb, int groups_total, int g_begin,
-                                                         const uint32_t (&xb)[NG][8], const float (&xsum)[NG], float (&acc)[2][4]) {
-    using vec = typename GroupBytes<BITS>::vec;
-    using MW = typename MetaWord<NG>::type;
-    const int t = threadIdx.x & 3;
-    MW sa[2], sb[2], ba[2], bb[2];
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        sa[m] = *reinterpret_cast<const MW *>(s[m] + ma * groups_total + g_begin);
-        sb[m] = *reinterpret_cast<const MW *>(s[m] + mb * groups_total + g_begin);
-        ba[m] = *reinterpret_cast<const MW *>(b[m] + ma * groups_total + g_begin);
-        bb[m] = *reinterpret_cast<const MW *>(b[m] + mb * groups_total + g_begin);
-    }
-    const int g4 = (g_begin >> 2) << 2;         // g_begin is a multiple of 4, see above
-#pragma unroll
-    for (int j = 0; j < NG; ++j) {
-        vec wa[2], wb[2];
-        uint16_t s0[2], s1[2], b0[2], b1[2];
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            wa[m] = *reinterpret_cast<const vec *>(box_a[m] + swz_offset<BITS>(g4 + j, ra, t, rows_per_chunk));
-            wb[m] = *reinterpret_cast<const vec *>(box_b[m] + swz_offset<BITS>(g4 + j, rb, t, rows_per_chunk));
-            s0[m] = meta_pick(sa[m], j); s1[m] = meta_pick(sb[m], j);
-            b0[m] = meta_pick(ba[m], j); b1[m] = meta_pick(bb[m], j);
-        }
-        group_step<BITS, META, 2, true>(wa, wb, s0, s1, b0, b1, xb[j], xsum[j], 0.0f, acc);
-    }
-}
-
-// the same over any group range, activation fragments read from the row in shared memory
-template <int BITS, int META>
-__device__ __forceinline__ void swz_accumulate_range(const unsigned char *box_a, const unsigned char *box_b, int rows_per_chunk,
-                                                     int ra, int rb, const uint16_t *s, const uint16_t *b, int ma, int mb,
-                                                     int groups_total, int g_begin, int g_end, const __half *xrow,
-                                                     const float *xsum, float (&acc)[1][4]) {
-    using vec = typename GroupBytes<BITS>::vec;
-    const int t = threadIdx.x & 3;
-    for (int G = g_begin; G < g_end; ++G) {
-        const vec wa[1] = {*reinterpret_cast<const vec *>(box_a + swz_offset<BITS>(G, ra, t, rows_per_chunk))};
-        const vec wb[1] = {*reinterpret_cast<const vec *>(box_b + swz_offset<BITS>(G, rb, t, rows_per_chunk))};
-        const uint16_t s0[1] = {s[ma * groups_total + G]}, s1[1] = {s[mb * groups_total + G]};
-        const uint16_t b0[1] = {b[ma * groups_total + G]}, b1[1] = {b[mb * groups_total + G]};
-        uint32_t xb[8];
-        const uint4 *xp = reinterpret_cast<const uint4 *>(xrow + (size_t)G * kGroup + t * 16);
-        permute_x<BITS>(xp[0], xp[1], xb);
-        group_step<BITS, META, 1, true>(wa, wb, s0, s1, b0, b1, xb, xsum[G], 0.0f, acc);
-    }
 }
 
 // ---- out-of-line copies of the larger helpers ------------------------------------------

@@ -14,59 +14,74 @@ constexpr size_t kTopkSmemBytes = 16 + (kMaxExperts + 64) * sizeof(float);
 // shared-memory layouts (one definition for the host's size computation and the
 // device's addressing); every offset is a multiple of 16 bytes
 // ---------------------------------------------------------------------------
+// boxed: the tiles come as tiled TMA boxes (128-byte swizzle, no padding; the base then is a multiple of 1 KB)
 struct GateUpLayout {     // kTilesPerBlock tiles of 8 gate rows + the matching 8 up rows, and the token's x row
-    size_t xs, xsum, w0, w_step, meta0, meta_step, red, wsum, total;
-    __host__ __device__ GateUpLayout(int D, int bits) {
-        const size_t stride = (size_t)D * bits / 8 + (bits == 4 ? 32 : 64);
-        size_t o = 16 * kTilesPerBlock;      // one transaction barrier per tile
-        xs = o; o += (size_t)D * 2;
-        xsum = o; o += ((size_t)(D / kGroup) * sizeof(float) + 15) & ~(size_t)15;
+    uint32_t xs, xsum, w0, w_step, meta0, meta_step, meta_tile, red, sel, wsum;
+    size_t total;
+    __host__ __device__ GateUpLayout(int D, int bits, bool boxed = false) {
+        const uint32_t stride = (uint32_t)D * bits / 8 + (boxed ? 0 : bits == 4 ? 32 : 64);
+        uint32_t o = 16 * kTilesPerBlock;      // one transaction barrier per tile
+        xs = o; o += (uint32_t)D * 2;
+        xsum = o; o += ((uint32_t)(D / kGroup) * 4u + 15) & ~15u;
         w_step = kTileRows * stride;         // tile rows 0-7 gate, 8-15 up
+        if (boxed) o = (o + 1023) & ~1023u;
         w0 = o; o += kTilesPerBlock * w_step;
-        meta_step = (((size_t)kTileRows * (D / kGroup) * 2) + 15) & ~(size_t)15;
-        meta0 = o; o += kTilesPerBlock * 2 * meta_step;   // per tile: scales[16][G], biases[16][G]
-        red = o; o += (size_t)kTilesPerBlock * kDecodeWarps * 16 * sizeof(float);
+        meta_step = (uint32_t)kTileRows * (D / kGroup) * 2;
+        meta_tile = boxed ? (2 * meta_step + 127) & ~127u : 2 * meta_step;
+        meta0 = o; o += kTilesPerBlock * meta_tile;       // per tile: scales[16][G], biases[16][G]
+        red = o; o += (uint32_t)kTilesPerBlock * kDecodeWarps * 16 * 4u;
+        sel = o; o += 768;                   // selection: idx[32], score[32], candidates 64 + 64
         wsum = o; o += 64;
-        total = o;
+        total = o + (boxed ? 1024 : 0);      // the kernel rounds its base up
     }
-    __host__ __device__ size_t w(int tile) const { return w0 + tile * w_step; }
-    __host__ __device__ size_t meta(int tile, int i) const { return meta0 + (tile * 2 + i) * meta_step; }
+    __host__ __device__ uint32_t w(int tile) const { return w0 + tile * w_step; }
+    __host__ __device__ uint32_t meta(int tile, int i) const { return meta0 + tile * meta_tile + i * meta_step; }
 };
 
 struct RowsLayout {       // up to 8 rows of the router (or the gate row) + x
-    size_t xs, rows, meta0, meta_step, wsum, total;
+    uint32_t xs, rows, meta0, meta_step, wsum;
+    size_t total;
     __host__ __device__ RowsLayout(int D, uint32_t kind) {
-        const size_t row_bytes = kind == 0 ? (size_t)D * 2 : (size_t)D * kind / 8;
-        const size_t meta_bytes = kind == 0 ? 0 : (size_t)kRowsPerRouterBlock * (D / kGroup) * 2;
-        size_t o = 16;
-        xs = o; o += (size_t)D * 2;
+        const uint32_t row_bytes = kind == 0 ? (uint32_t)D * 2 : (uint32_t)D * kind / 8;
+        const uint32_t meta_bytes = kind == 0 ? 0 : (uint32_t)kRowsPerRouterBlock * (D / kGroup) * 2;
+        uint32_t o = 16;
+        xs = o; o += (uint32_t)D * 2;
         rows = o; o += kRowsPerRouterBlock * row_bytes;
-        meta_step = (meta_bytes + 15) & ~(size_t)15;
+        meta_step = (meta_bytes + 15) & ~15u;
         meta0 = o; o += 2 * meta_step;
         wsum = o; o += 64;
         total = o;
     }
-    __host__ __device__ size_t meta(int i) const { return meta0 + i * meta_step; }
+    __host__ __device__ uint32_t meta(int i) const { return meta0 + i * meta_step; }
 };
 
-struct DownLayout {       // per warp: barrier, activation row, 16-row down tile, scales, biases
-    size_t act, xsum, w, meta0, meta_step, region, part, total;
-    __host__ __device__ DownLayout(int F, int Fs, int bits, int sbits, int warps) {
+struct DownLayout {       // per unit: 16-row down tile, scales, biases, barrier, activation row
+    uint32_t w, meta0, meta_step, bar, act, xsum, region, part;
+    size_t total;
+    __host__ __device__ DownLayout(int F, int Fs, int bits, int sbits, int units, bool boxed = false) {
         const int n = F > Fs ? F : Fs;
         const int b = (Fs != 0 && sbits > bits) ? sbits : bits;
-        const size_t stride = (size_t)n * b / 8 + 64;
-        const size_t meta_bytes = (size_t)kTileRows * (n / kGroup) * 2;
-        size_t o = 16;
-        act = o; o += (size_t)n * 2;
-        xsum = o; o += (((size_t)(n / kGroup) * sizeof(float)) + 15) & ~(size_t)15;
+        const uint32_t stride = (uint32_t)n * b / 8 + 64;
+        uint32_t o = 0;
         w = o; o += kTileRows * stride;
-        meta_step = (meta_bytes + 15) & ~(size_t)15;
+        if (boxed) o = (o + 127) & ~127u;
+        meta_step = (uint32_t)kTileRows * (n / kGroup) * 2;
         meta0 = o; o += 2 * meta_step;
-        region = (o + 127) & ~(size_t)127;
-        part = (size_t)warps * region;
-        total = part + ((kMaxTopK + 1) * 2 * 16 + 32) * sizeof(float);   // partial sums + routing weights
+        bar = o; o += 16;
+        act = o; o += (uint32_t)n * 2;
+        xsum = o; o += (((uint32_t)(n / kGroup) * 4u) + 15) & ~15u;
+        region = boxed ? (o + 1023) & ~1023u : (o + 127) & ~127u;
+        part = (uint32_t)units * region;
+        total = part + ((kMaxTopK + 1) * 2 * 16 + 32) * 4u + (boxed ? 1024 : 0);   // partial sums + routing weights
     }
-    __host__ __device__ size_t meta(int i) const { return meta0 + i * meta_step; }
+    __host__ __device__ uint32_t meta(int i) const { return meta0 + i * meta_step; }
+};
+
+// Tensor maps of a layer's expert weights for tiled TMA (see ensure_tile_maps); kernels that get none copy row by row.
+struct TileMaps {
+    CUtensorMap gu_w, gu_meta;     // routed gate|up codes {128 B, row, chunk, gate|up, expert}, meta {value, gate|up, scale|bias, expert}
+    CUtensorMap dn_w, dn_meta;     // routed down codes {128 B, row, chunk, expert}, meta {value, scale|bias, expert}
+    CUtensorMap sg_w, su_w;        // shared expert's gate and up codes {128 B, row, chunk}
 };
 
 // ---------------------------------------------------------------------------
@@ -211,6 +226,37 @@ __device__ __forceinline__ void issue_gate_up_copies(unsigned char *smem, const 
     }
 }
 
+// The same as two boxes (codes; scales and biases) of a tensor map, one lane: the row copies of a block's two tiles took
+// 2.4 us to issue, a tenth of a layer.
+template <int BITS>
+__device__ __forceinline__ void issue_gate_up_boxes(unsigned char *smem, const GateUpLayout &L, int tile, const TileMaps &m,
+                                                    int f0, uint32_t expert, int D, uint32_t extra_tx_bytes) {
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 16 * tile);
+    const uint32_t groups = D / kGroup;
+    mbar_expect_tx(bar, (uint32_t)(kTileRows * D * BITS / 8) + 4u * kTileFeatures * groups * 2u + extra_tx_bytes);
+    tma_load_5d(smem + L.w(tile), &m.gu_w, 0, f0, 0, 0, (int)expert, bar);
+    tma_load_4d(smem + L.meta(tile, 0), &m.gu_meta, f0 * (int)groups, 0, 0, (int)expert, bar);
+}
+// the shared expert's tile, one warp
+template <int BITS>
+__device__ __forceinline__ void issue_shared_boxes(unsigned char *smem, const GateUpLayout &L, int tile, const TileMaps &m,
+                                                   const AffineMat &gate, const AffineMat &up, int f0, int D, uint32_t extra_tx_bytes) {
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 16 * tile);
+    const int lane = threadIdx.x & 31;
+    const uint32_t groups = D / kGroup, half_w = (uint32_t)(kTileFeatures * D * BITS / 8);
+    const uint32_t meta_bytes = (uint32_t)kTileFeatures * groups * 2;
+    if (lane == 0) mbar_expect_tx(bar, 2 * half_w + 4 * meta_bytes + extra_tx_bytes);
+    __syncwarp();
+    if (lane == 0) tma_load_3d(smem + L.w(tile), &m.sg_w, 0, f0, 0, bar);
+    else if (lane == 1) tma_load_3d(smem + L.w(tile) + half_w, &m.su_w, 0, f0, 0, bar);
+    else if (lane < 6) {
+        const int i = lane - 2;                 // 0 gate scales, 1 up scales, 2 gate biases, 3 up biases
+        const AffineMat &mat = (i & 1) ? up : gate;
+        bulk_g2s(smem + L.meta(tile, i >> 1) + (size_t)(i & 1) * meta_bytes, ((i >> 1) ? mat.b : mat.s) + (size_t)f0 * groups,
+                 meta_bytes, bar);
+    }
+}
+
 __device__ __forceinline__ void init_tile_barriers(unsigned char *smem) {
     if (threadIdx.x == 0) {
 #pragma unroll
@@ -239,7 +285,7 @@ struct NoLateWork { __device__ __forceinline__ void operator()() const {} };
 
 // after_first_tile: called by every thread once the block's first tile has landed (the
 // place for requests that must not compete with the block's own copies).
-template <int BITS, int META, int OUT, typename Late = NoLateWork>
+template <int BITS, int META, int OUT, bool BOXED = false, typename Late = NoLateWork>
 __device__ __forceinline__ void gate_up_compute(unsigned char *smem, const GateUpLayout &L, int f0, int n_tiles,
                                                 int D, uint32_t act, bool round_gate_up, void *out_base,
                                                 size_t out_row_offset, unsigned int *status,
@@ -254,7 +300,35 @@ __device__ __forceinline__ void gate_up_compute(unsigned char *smem, const GateU
     bool ok = mbar_wait(reinterpret_cast<uint64_t *>(smem), 0, status);      // tile 0 (and x, when it was copied)
     after_first_tile();
     const bool fast = gpw == 4 && g_end - g_begin == 4 && (groups & 3) == 0;
-    if (fast) {
+    if (BOXED && fast) {
+        float v = sum8_halves(*reinterpret_cast<const uint4 *>(xs + (size_t)(g_begin + (lane >> 3)) * kGroup + (lane & 7) * 8));
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        float xsum[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xsum[j] = __shfl_sync(0xffffffffu, v, j * 8);
+        auto tiles = [&](auto N) {
+            constexpr int NT = decltype(N)::value;
+            float acc[NT][4] = {};
+            swz_accumulate_tiles<BITS, META, NT>(smem + L.w(0), L.w_step, (size_t)kTileFeatures * D * BITS / 8, kTileFeatures, g, g,
+                                                 reinterpret_cast<const uint16_t *>(smem + L.meta(0, 0)),
+                                                 reinterpret_cast<const uint16_t *>(smem + L.meta(0, 1)), L.meta_tile / 2, g, g + 8, groups,
+                                                 g_begin, xs, xsum, acc);
+#pragma unroll
+            for (int tile = 0; tile < NT; ++tile)
+                if (t == 0) {
+                    red[(tile * kDecodeWarps + warp) * 16 + g] = acc[tile][0];
+                    red[(tile * kDecodeWarps + warp) * 16 + g + 8] = acc[tile][2];
+                }
+        };
+        if (n_tiles == kTilesPerBlock) {
+            ok = mbar_wait(reinterpret_cast<uint64_t *>(smem + 16), 0, status) && ok;
+            tiles(std::integral_constant<int, kTilesPerBlock>{});
+        } else {
+            tiles(std::integral_constant<int, 1>{});
+        }
+    } else if (!BOXED && fast) {
         // x fragments and group sums once, reused by every tile
         uint32_t xb[4][8];
         float xsum[4];
@@ -296,7 +370,11 @@ __device__ __forceinline__ void gate_up_compute(unsigned char *smem, const GateU
             const SmemTile tiles[1] = {{smem + L.w(tile), reinterpret_cast<const uint16_t *>(smem + L.meta(tile, 0)),
                                         reinterpret_cast<const uint16_t *>(smem + L.meta(tile, 1))}};
             float acc[1][4] = {};
-            tile_accumulate_auto<BITS, META, 1, true>(tiles, D, g_begin, g_end - g_begin, xs, xsum, acc);
+            if constexpr (BOXED)
+                swz_accumulate_range<BITS, META>(tiles[0].w, tiles[0].w + (size_t)kTileFeatures * D * BITS / 8, kTileFeatures, g, g,
+                                                 tiles[0].s, tiles[0].b, g, g + 8, groups, g_begin, g_end, xs, xsum, acc);
+            else
+                tile_accumulate_auto<BITS, META, 1, true>(tiles, D, g_begin, g_end - g_begin, xs, xsum, acc);
             if (t == 0) {
                 red[(tile * kDecodeWarps + warp) * 16 + g] = acc[0][0];
                 red[(tile * kDecodeWarps + warp) * 16 + g + 8] = acc[0][2];
@@ -476,57 +554,81 @@ struct Stage2Params {
     const uint32_t *active_slots;       // device, or nullptr = identity
     uint32_t D, F, top_k, act;
     uint32_t prefetch_down;             // also ask the L2 for the experts' down projections
+    // the shared expert's gate/up tiles as slot n_slots (tiled TMA only; otherwise stage 1 has them): shared_f == 0 disables
+    AffineMat sgate, sup;
+    uint32_t n_slots, shared_f;
+    void *shared_act;                   // [tokens][shared_f]
     unsigned int *status;
     unsigned long long *trace;   // optional {start, end} timestamps of this launch
 };
 
-template <int BITS, int META, int OUT>
-__global__ void __launch_bounds__(kDecodeThreads, 2) stage2_kernel(Stage2Params p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    const GateUpLayout L(p.D, BITS);
+// 64 registers, so that the next stage's blocks (which request their tiles ahead of this stage's end) fit beside two of
+// these blocks: at 101 they started when these had left, 2 us late.
+template <int BITS, int META, int OUT, bool BOXED>
+__global__ void __launch_bounds__(kDecodeThreads, 4) stage2_kernel(const __grid_constant__ Stage2Params p, const __grid_constant__ TileMaps maps) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char *smem = BOXED ? smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u) : smem_raw;
+    const GateUpLayout L(p.D, BITS, BOXED);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t tok = blockIdx.z;
     const int f0 = blockIdx.x * kBlockFeatures;
-    const int n_tiles = min(kTilesPerBlock, (int)(p.F - f0) / kTileFeatures);
     trace_begin(p.trace);
     init_tile_barriers(smem);
+    if (BOXED && blockIdx.y == p.n_slots) {      // the shared expert's tiles (its weights are requested before the wait)
+        const int n_tiles = min(kTilesPerBlock, ((int)p.shared_f - f0) / kTileFeatures);
+        if (n_tiles > 0 && warp == 0)
+            for (int tile = 0; tile < n_tiles; ++tile)
+                issue_shared_boxes<BITS>(smem, L, tile, maps, p.sgate, p.sup, f0 + tile * kTileFeatures, p.D, tile == 0 ? p.D * 2 : 0);
+        pdl_wait();
+        pdl_launch_dependents();
+        if (n_tiles <= 0) return;
+        if (threadIdx.x == 0) bulk_g2s(smem + L.xs, p.x + (size_t)tok * p.x_stride, p.D * 2, reinterpret_cast<uint64_t *>(smem));
+        gate_up_compute<BITS, META, OUT, BOXED>(smem, L, f0, n_tiles, p.D, p.act, true, p.shared_act, (size_t)tok * p.shared_f, p.status);
+        trace_end(p.trace);
+        return;
+    }
+    const int n_tiles = min(kTilesPerBlock, ((int)p.F - f0) / kTileFeatures);
+    if (BOXED && threadIdx.x == 0) { tma_prefetch_map(&maps.gu_w); tma_prefetch_map(&maps.gu_meta); }
     pdl_wait();                 // the expert indices come from stage 1
     pdl_launch_dependents();
     trace_mark(p.trace, 0);
     uint32_t slot = blockIdx.y;
     if (p.active_slots != nullptr) slot = p.active_slots[slot];
-    if (slot >= p.top_k) return;        // moe.metal:720
-    // deferred selection (see RoutedSource); the scratch is the red area, unused until the reduction
-    uint32_t *sel_idx = reinterpret_cast<uint32_t *>(smem + L.red);
-    float *sel_score = reinterpret_cast<float *>(smem + L.red) + 32;
+    if (slot >= p.top_k || n_tiles <= 0) return;        // moe.metal:720
+    uint32_t *sel_idx = reinterpret_cast<uint32_t *>(smem + L.sel);      // deferred selection (see RoutedSource)
+    float *sel_score = reinterpret_cast<float *>(smem + L.sel) + 32;
     if (p.src.logits != nullptr) {
         topk_select_block(p.src.logits + (size_t)tok * p.src.num_experts, p.src.num_experts, p.top_k, sel_idx, sel_score,
-                          reinterpret_cast<float *>(smem + L.red) + 64);
+                          reinterpret_cast<float *>(smem + L.sel) + 64);
         trace_mark(p.trace, 1);
     }
     // an expert held by another rank (expert parallelism): nothing to do here beyond block (0, 0)'s publication
     const bool local = p.src.logits == nullptr || expert_blob(p.src, sel_idx[slot]) != nullptr;
     if (warp == 0) {
-        const uint8_t *blob;
-        if (p.src.logits != nullptr) {
-            blob = expert_blob(p.src, sel_idx[slot]);
-            if (blockIdx.x == 0 && blockIdx.y == 0)
-                routing_weights_warp(sel_idx, sel_score, p.top_k, p.src.pes, p.src.publish_idx + (size_t)tok * p.top_k,
-                                     p.src.publish_w + (size_t)tok * p.top_k);
-        } else {
-            blob = routed_blob(p.src, tok, slot, p.top_k);
+        if (BOXED) {
+            if (lane == 0) {
+                const uint32_t e = routed_expert(p.src, sel_idx, tok, slot, p.top_k);
+                for (int tile = 0; tile < n_tiles; ++tile) {
+                    issue_gate_up_boxes<BITS>(smem, L, tile, maps, f0 + tile * kTileFeatures, e, p.D, tile == 0 ? p.D * 2 : 0);
+                    if (tile == 0)
+                        bulk_g2s(smem + L.xs, p.x + (size_t)tok * p.x_stride, p.D * 2, reinterpret_cast<uint64_t *>(smem));
+                }
+            }
+        } else if (local) {
+            const uint8_t *blob = p.src.logits != nullptr ? expert_blob(p.src, sel_idx[slot]) : routed_blob(p.src, tok, slot, p.top_k);
+            const AffineMat gate = {blob + p.off.o[0], reinterpret_cast<const uint16_t *>(blob + p.off.o[1]),
+                                    reinterpret_cast<const uint16_t *>(blob + p.off.o[2])};
+            const AffineMat up = {blob + p.off.o[3], reinterpret_cast<const uint16_t *>(blob + p.off.o[4]),
+                                  reinterpret_cast<const uint16_t *>(blob + p.off.o[5])};
+            issue_gate_up_copies<BITS>(smem, L, 0, gate, up, f0, p.D, p.D * 2);
+            if (lane == 0) bulk_g2s(smem + L.xs, p.x + (size_t)tok * p.x_stride, p.D * 2, reinterpret_cast<uint64_t *>(smem));
+            for (int tile = 1; tile < n_tiles; ++tile)
+                issue_gate_up_copies<BITS>(smem, L, tile, gate, up, f0 + tile * kTileFeatures, p.D, 0);
         }
-        if (!local) blob = nullptr;
-        if (blob != nullptr) {
-        const AffineMat gate = {blob + p.off.o[0], reinterpret_cast<const uint16_t *>(blob + p.off.o[1]),
-                                reinterpret_cast<const uint16_t *>(blob + p.off.o[2])};
-        const AffineMat up = {blob + p.off.o[3], reinterpret_cast<const uint16_t *>(blob + p.off.o[4]),
-                              reinterpret_cast<const uint16_t *>(blob + p.off.o[5])};
-        issue_gate_up_copies<BITS>(smem, L, 0, gate, up, f0, p.D, p.D * 2);
-        if (lane == 0) bulk_g2s(smem + L.xs, p.x + (size_t)tok * p.x_stride, p.D * 2, reinterpret_cast<uint64_t *>(smem));
-        for (int tile = 1; tile < n_tiles; ++tile)
-            issue_gate_up_copies<BITS>(smem, L, tile, gate, up, f0 + tile * kTileFeatures, p.D, 0);
-        }
+        trace_mark(p.trace, 2);
+        if (p.src.logits != nullptr && blockIdx.x == 0 && blockIdx.y == 0)
+            routing_weights_warp(sel_idx, sel_score, p.top_k, p.src.pes, p.src.publish_idx + (size_t)tok * p.top_k,
+                                 p.src.publish_w + (size_t)tok * p.top_k);
     }
     if (!local) { trace_end(p.trace); return; }
     const uint8_t *pf_blob = nullptr;
@@ -535,14 +637,15 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) stage2_kernel(Stage2Params 
     }
     // once this block's own tile is in: warm the L2 with its share of the expert's down projection (stage 3 reads it next)
     auto late = [&]() {
-        trace_mark(p.trace, 2);
+        trace_mark(p.trace, 3);
         if (pf_blob == nullptr) return;
         l2_prefetch_slice(pf_blob + p.off.o[6], (size_t)p.D * p.F * BITS / 8, blockIdx.x, gridDim.x, lane);
         l2_prefetch_slice(pf_blob + p.off.o[7], (size_t)p.D * (p.F / kGroup) * 2, blockIdx.x, gridDim.x, lane);
         l2_prefetch_slice(pf_blob + p.off.o[8], (size_t)p.D * (p.F / kGroup) * 2, blockIdx.x, gridDim.x, lane);
     };
-    gate_up_compute<BITS, META, OUT>(smem, L, f0, n_tiles, p.D, p.act, false, p.acts,
-                                     ((size_t)tok * p.top_k + slot) * p.F, p.status, late);
+    gate_up_compute<BITS, META, OUT, BOXED>(smem, L, f0, n_tiles, p.D, p.act, false, p.acts,
+                                            ((size_t)tok * p.top_k + slot) * p.F, p.status, late);
+    trace_mark(p.trace, 4);
     trace_end(p.trace);
 }
 
@@ -584,7 +687,8 @@ struct Stage3Params {
 // one warp: bulk-copy a 16-row down tile (+ scales, biases) into its region
 template <int BITS>
 __device__ __forceinline__ void issue_down_copies(unsigned char *region, const DownLayout &L, const AffineMat &mat,
-                                                  int row0, int n, uint64_t *bar) {
+                                                  int row0, int n) {
+    uint64_t *bar = reinterpret_cast<uint64_t *>(region + L.bar);
     const int lane = threadIdx.x & 31;
     const uint32_t row_bytes = (uint32_t)n * BITS / 8;
     const uint32_t meta_bytes = (uint32_t)kTileRows * (n / kGroup) * 2;
@@ -598,6 +702,17 @@ __device__ __forceinline__ void issue_down_copies(unsigned char *region, const D
                  meta_bytes, bar);
 }
 
+// one lane: the same as two boxes of a tensor map
+template <int BITS>
+__device__ __forceinline__ void issue_down_boxes(unsigned char *region, const DownLayout &L, const TileMaps &m, int row0, uint32_t expert, int n) {
+    uint64_t *bar = reinterpret_cast<uint64_t *>(region + L.bar);
+    const int groups = n / kGroup;
+    mbar_init(bar, 1); mbar_fence_init();
+    mbar_expect_tx(bar, (uint32_t)(kTileRows * n * BITS / 8) + 2u * kTileRows * (uint32_t)groups * 2u);
+    tma_load_4d(region + L.w, &m.dn_w, 0, row0, 0, (int)expert, bar);
+    tma_load_3d(region + L.meta0, &m.dn_meta, row0 * groups, 0, (int)expert, bar);
+}
+
 constexpr int kDownSplit = 2;    // warps per (slot, tile): the down row's groups are split in halves
 
 // The part of the activation row this warp consumes -> shared memory as scaled
@@ -609,9 +724,9 @@ __device__ __forceinline__ const __half *stage_row_part(const void *rows, size_t
     if (OUT == OUT_F16) return reinterpret_cast<const __half *>(rows) + row_offset;
     const int lane = threadIdx.x & 31;
     const float *src = reinterpret_cast<const float *>(rows) + row_offset;
-    // one trip to memory: up to 1024 values stay in registers between the maximum
+    // one trip to memory: up to 512 values stay in registers between the maximum
     // (a property of the whole row) and the conversion; longer rows are re-read
-    constexpr int kKeep = 8;
+    constexpr int kKeep = 4;
     float4 keep[kKeep];
     float m = 0.0f;
 #pragma unroll
@@ -652,7 +767,7 @@ __device__ __forceinline__ const __half *stage_row_part(const void *rows, size_t
 }
 
 // one warp of the pair that owns (slot, tile): its half of the groups
-template <int BITS, int META, int OUT>
+template <int BITS, int META, int OUT, bool BOXED>
 __device__ __forceinline__ bool down_warp(unsigned char *region, const DownLayout &L, int n, int half,
                                           const void *act_rows, size_t act_offset, unsigned int *status,
                                           float (&out)[2]) {
@@ -660,7 +775,7 @@ __device__ __forceinline__ bool down_warp(unsigned char *region, const DownLayou
     const int groups = n / kGroup;
     const int gpw = (groups + kDownSplit - 1) / kDownSplit;
     const int g_begin = min(half * gpw, groups), g_end = min(g_begin + gpw, groups);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(region);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(region + L.bar);
     float scale_up;
     const __half *arow = stage_row_part<OUT>(act_rows, act_offset, n, g_begin * kGroup, (g_end - g_begin) * kGroup,
                                              reinterpret_cast<__half *>(region + L.act), scale_up);
@@ -681,14 +796,22 @@ __device__ __forceinline__ bool down_warp(unsigned char *region, const DownLayou
     }
     __syncwarp();
     if (!mbar_wait(bar, 0, status)) return false;
-    const SmemTile tiles[1] = {{region + L.w, reinterpret_cast<const uint16_t *>(region + L.meta(0)),
-                                reinterpret_cast<const uint16_t *>(region + L.meta(1))}};
+    const uint16_t *ms = reinterpret_cast<const uint16_t *>(region + L.meta0);
+    const uint16_t *mb = BOXED ? ms + kTileRows * groups : reinterpret_cast<const uint16_t *>(region + L.meta(1));
+    const SmemTile tiles[1] = {{region + L.w, ms, mb}};
+    const int g = lane >> 2;
     float acc[1][4] = {};
     if (g_end - g_begin == 4 && (g_begin & 3) == 0 && (groups & 3) == 0) {
-        uint32_t xb[4][8];
         const float xs4[4] = {xsum[g_begin], xsum[g_begin + 1], xsum[g_begin + 2], xsum[g_begin + 3]};
-        load_x_fragments<BITS, 4>(arow, g_begin, xb);
-        tile_accumulate_prepared<BITS, META, 4>(tiles[0], n, g_begin, xb, xs4, acc);
+        if constexpr (BOXED) {
+            swz_accumulate_tiles<BITS, META, 1>(region + L.w, 0, 0, kTileRows, g, g + 8, ms, mb, 0, g, g + 8, groups, g_begin, arow, xs4, acc);
+        } else {
+            uint32_t xb[4][8];
+            load_x_fragments<BITS, 4>(arow, g_begin, xb);
+            tile_accumulate_prepared<BITS, META, 4>(tiles[0], n, g_begin, xb, xs4, acc);
+        }
+    } else if constexpr (BOXED) {
+        swz_accumulate_range<BITS, META>(tiles[0].w, tiles[0].w, kTileRows, g, g + 8, ms, mb, g, g + 8, groups, g_begin, g_end, arow, xsum, acc);
     } else {
         tile_accumulate_auto<BITS, META, 1, true>(tiles, n, g_begin, g_end - g_begin, arow, xsum, acc);
     }
@@ -697,19 +820,19 @@ __device__ __forceinline__ bool down_warp(unsigned char *region, const DownLayou
     return true;
 }
 
-template <int BITS, int META, int OUT>
-__global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32) stage3_kernel(Stage3Params p) {
-    extern __shared__ __align__(128) unsigned char smem[];
+template <int BITS, int META, int OUT, bool BOXED>
+__global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32, 2) stage3_kernel(const __grid_constant__ Stage3Params p, const __grid_constant__ TileMaps maps) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char *smem = BOXED ? smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u) : smem_raw;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int unit = warp / kDownSplit, half = warp % kDownSplit;   // unit k < top_k: slot k; unit top_k: shared expert
     const uint32_t tok = blockIdx.y;
     const int row0 = blockIdx.x * kTileRows;
     const int units = p.top_k + (p.shared_f ? 1 : 0);
-    const DownLayout L(p.F, p.shared_f, BITS, p.shared_bits, units);
+    const DownLayout L(p.F, p.shared_f, BITS, p.shared_bits, units, BOXED);
     float *part = reinterpret_cast<float *>(smem + L.part);      // [unit][half][16]
     unsigned char *region = smem + (size_t)unit * L.region;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(region);
     const bool routed = unit < (int)p.top_k;
     const bool shared = unit == (int)p.top_k && p.shared_f != 0;
     trace_begin(p.trace);
@@ -724,15 +847,18 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32) stage3_kerne
     bool local = true;
     if (routed && p.src.logits != nullptr) local = expert_blob(p.src, reinterpret_cast<uint32_t *>(part)[unit]) != nullptr;
     if (half == 0) {
-        if (routed && local) {
+        if (routed && BOXED) {
+            if (lane == 0)
+                issue_down_boxes<BITS>(region, L, maps, row0, routed_expert(p.src, reinterpret_cast<uint32_t *>(part), tok, unit, p.top_k), p.F);
+        } else if (routed && local) {
             const uint8_t *blob = p.src.logits != nullptr ? expert_blob(p.src, reinterpret_cast<uint32_t *>(part)[unit])
                                                           : routed_blob(p.src, tok, unit, p.top_k);
             const AffineMat mat{blob + p.off.o[6], reinterpret_cast<const uint16_t *>(blob + p.off.o[7]),
                                 reinterpret_cast<const uint16_t *>(blob + p.off.o[8])};
-            issue_down_copies<BITS>(region, L, mat, row0, p.F, bar);
+            issue_down_copies<BITS>(region, L, mat, row0, p.F);
         } else if (shared) {
-            if (p.shared_bits == 4) issue_down_copies<4>(region, L, p.sdown, row0, p.shared_f, bar);
-            else issue_down_copies<8>(region, L, p.sdown, row0, p.shared_f, bar);
+            if (p.shared_bits == 4) issue_down_copies<4>(region, L, p.sdown, row0, p.shared_f);
+            else issue_down_copies<8>(region, L, p.sdown, row0, p.shared_f);
         }
     }
     if (warp == (int)(blockDim.x >> 5) - 1) {
@@ -759,12 +885,12 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32) stage3_kerne
     bool ok = true;
     float v[2] = {0.0f, 0.0f};
     if (routed && local) {
-        ok = down_warp<BITS, META, OUT>(region, L, p.F, half, p.acts, ((size_t)tok * p.top_k + unit) * p.F, p.status, v);
+        ok = down_warp<BITS, META, OUT, BOXED>(region, L, p.F, half, p.acts, ((size_t)tok * p.top_k + unit) * p.F, p.status, v);
     } else if (shared) {
         if (p.shared_bits == 4)
-            ok = down_warp<4, META, OUT>(region, L, p.shared_f, half, p.shared_act, (size_t)tok * p.shared_f, p.status, v);
+            ok = down_warp<4, META, OUT, false>(region, L, p.shared_f, half, p.shared_act, (size_t)tok * p.shared_f, p.status, v);
         else
-            ok = down_warp<8, META, OUT>(region, L, p.shared_f, half, p.shared_act, (size_t)tok * p.shared_f, p.status, v);
+            ok = down_warp<8, META, OUT, false>(region, L, p.shared_f, half, p.shared_act, (size_t)tok * p.shared_f, p.status, v);
     }
     if (t == 0 && (routed || shared)) {
         part[(unit * kDownSplit + half) * 16 + g] = v[0];

@@ -294,4 +294,135 @@ __device__ __forceinline__ void tile_accumulate_auto(const SmemTile (&tiles)[NMA
         tile_accumulate_smem<BITS, META, NMAT, 0, ONE_COL>(tiles, n, g_begin, g_begin + count, xrow, xsum, acc, xsum_stride);
 }
 
+// ---- swizzled tiles ----------------------------------------------------------------
+// A box of R rows x C chunks of 128 bytes lands as [chunk][row][128 B] with the 16-byte unit index XORed with
+// (line index mod 8) = row mod 8 (R is 8 or 16).  The codes of lane (g, t) for group G of row r:
+//   4-bit  8 bytes at row byte 32 G + 8 t      8-bit  16 bytes at row byte 64 G + 16 t
+template <int BITS>
+__device__ __forceinline__ uint32_t swz_offset(int G, int r, int t, int rows_per_chunk) {
+    if (BITS == 4) {
+        const int chunk = G >> 2, unit = ((G & 3) << 1) | (t >> 1);
+        return (uint32_t)(((chunk * rows_per_chunk + r) << 7) | (((unit ^ (r & 7)) << 4) | ((t & 1) << 3)));
+    }
+    const int chunk = G >> 1, unit = ((G & 1) << 2) | t;
+    return (uint32_t)(((chunk * rows_per_chunk + r) << 7) | ((unit ^ (r & 7)) << 4));
+}
+
+// acc += rows ra / rb (box rows; meta rows ma / mb) of a swizzled tile over groups [g_begin, g_begin + NG) against
+// prepared activation fragments.  The arithmetic of tile_accumulate_prepared.
+template <int BITS, int META, int NG>
+__device__ __forceinline__ void swz_accumulate_prepared(const unsigned char *box_a, const unsigned char *box_b, int rows_per_chunk,
+                                                        int ra, int rb, const uint16_t *s, const uint16_t *b, int ma, int mb,
+                                                        int groups_total, int g_begin, const uint32_t (&xb)[NG][8],
+                                                        const float (&xsum)[NG], float (&acc)[1][4]) {
+    using vec = typename GroupBytes<BITS>::vec;
+    using MW = typename MetaWord<NG>::type;
+    const int t = threadIdx.x & 3;
+    const MW sa = *reinterpret_cast<const MW *>(s + ma * groups_total + g_begin);
+    const MW sb = *reinterpret_cast<const MW *>(s + mb * groups_total + g_begin);
+    const MW ba = *reinterpret_cast<const MW *>(b + ma * groups_total + g_begin);
+    const MW bb = *reinterpret_cast<const MW *>(b + mb * groups_total + g_begin);
+    // g_begin is a multiple of NG (= 4) at every call: written as 4 * (g_begin / 4) + j, the group index shows the
+    // compiler which of its bits are the constant j, and the swizzle of the four groups folds to a few operations
+    const int g4 = (g_begin >> 2) << 2;
+#pragma unroll
+    for (int j = 0; j < NG; ++j) {
+        const vec wa[1] = {*reinterpret_cast<const vec *>(box_a + swz_offset<BITS>(g4 + j, ra, t, rows_per_chunk))};
+        const vec wb[1] = {*reinterpret_cast<const vec *>(box_b + swz_offset<BITS>(g4 + j, rb, t, rows_per_chunk))};
+        const uint16_t s0[1] = {meta_pick(sa, j)}, s1[1] = {meta_pick(sb, j)};
+        const uint16_t b0[1] = {meta_pick(ba, j)}, b1[1] = {meta_pick(bb, j)};
+        group_step<BITS, META, 1, true>(wa, wb, s0, s1, b0, b1, xb[j], xsum[j], 0.0f, acc);
+    }
+}
+
+// NT consecutive tiles (`step` bytes of codes, `meta_step` values of scales and biases apart) against one activation row
+// in shared memory, four groups from g_begin (a multiple of 4) on: the fragments of a group are loaded where they are used,
+// for all tiles, so that a block of 64 registers a thread holds them.  Each tile's arithmetic is that of the function above.
+template <int BITS, int META, int NT>
+__device__ __forceinline__ void swz_accumulate_tiles(const unsigned char *box, size_t step, size_t b_off, int rows_per_chunk, int ra, int rb,
+                                                     const uint16_t *s, const uint16_t *b, size_t meta_step, int ma, int mb, int groups_total,
+                                                     int g_begin, const __half *xrow, const float (&xsum)[4], float (&acc)[NT][4]) {
+    using vec = typename GroupBytes<BITS>::vec;
+    const int t = threadIdx.x & 3;
+    const int g4 = (g_begin >> 2) << 2;
+    uint2 sa[NT], sb[NT], ba[NT], bb[NT];
+#pragma unroll
+    for (int m = 0; m < NT; ++m) {
+        sa[m] = *reinterpret_cast<const uint2 *>(s + m * meta_step + ma * groups_total + g_begin);
+        sb[m] = *reinterpret_cast<const uint2 *>(s + m * meta_step + mb * groups_total + g_begin);
+        ba[m] = *reinterpret_cast<const uint2 *>(b + m * meta_step + ma * groups_total + g_begin);
+        bb[m] = *reinterpret_cast<const uint2 *>(b + m * meta_step + mb * groups_total + g_begin);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        vec wa[NT], wb[NT];
+        uint16_t s0[NT], s1[NT], b0[NT], b1[NT];
+#pragma unroll
+        for (int m = 0; m < NT; ++m) {
+            wa[m] = *reinterpret_cast<const vec *>(box + m * step + swz_offset<BITS>(g4 + j, ra, t, rows_per_chunk));
+            wb[m] = *reinterpret_cast<const vec *>(box + m * step + b_off + swz_offset<BITS>(g4 + j, rb, t, rows_per_chunk));
+            s0[m] = meta_pick(sa[m], j); s1[m] = meta_pick(sb[m], j);
+            b0[m] = meta_pick(ba[m], j); b1[m] = meta_pick(bb[m], j);
+        }
+        uint32_t xb[8];
+        const uint4 *xp = reinterpret_cast<const uint4 *>(xrow + (size_t)(g4 + j) * kGroup + t * 16);
+        permute_x<BITS>(xp[0], xp[1], xb);
+        group_step<BITS, META, NT, true>(wa, wb, s0, s1, b0, b1, xb, xsum[j], 0.0f, acc);
+    }
+}
+
+// Two tiles against the same prepared fragments (two consecutive gate/up tiles of one pair): the two tiles' chains are
+// independent, so their loads and tensor-core steps overlap; each tile's own arithmetic is that of the function above.
+template <int BITS, int META, int NG>
+__device__ __forceinline__ void swz_accumulate_prepared2(const unsigned char *const (&box_a)[2], const unsigned char *const (&box_b)[2],
+                                                         int rows_per_chunk, int ra, int rb, const uint16_t *const (&s)[2],
+                                                         const uint16_t *const (&b)[2], int ma, int mb, int groups_total, int g_begin,
+                                                         const uint32_t (&xb)[NG][8], const float (&xsum)[NG], float (&acc)[2][4]) {
+    using vec = typename GroupBytes<BITS>::vec;
+    using MW = typename MetaWord<NG>::type;
+    const int t = threadIdx.x & 3;
+    MW sa[2], sb[2], ba[2], bb[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        sa[m] = *reinterpret_cast<const MW *>(s[m] + ma * groups_total + g_begin);
+        sb[m] = *reinterpret_cast<const MW *>(s[m] + mb * groups_total + g_begin);
+        ba[m] = *reinterpret_cast<const MW *>(b[m] + ma * groups_total + g_begin);
+        bb[m] = *reinterpret_cast<const MW *>(b[m] + mb * groups_total + g_begin);
+    }
+    const int g4 = (g_begin >> 2) << 2;         // g_begin is a multiple of 4, see above
+#pragma unroll
+    for (int j = 0; j < NG; ++j) {
+        vec wa[2], wb[2];
+        uint16_t s0[2], s1[2], b0[2], b1[2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            wa[m] = *reinterpret_cast<const vec *>(box_a[m] + swz_offset<BITS>(g4 + j, ra, t, rows_per_chunk));
+            wb[m] = *reinterpret_cast<const vec *>(box_b[m] + swz_offset<BITS>(g4 + j, rb, t, rows_per_chunk));
+            s0[m] = meta_pick(sa[m], j); s1[m] = meta_pick(sb[m], j);
+            b0[m] = meta_pick(ba[m], j); b1[m] = meta_pick(bb[m], j);
+        }
+        group_step<BITS, META, 2, true>(wa, wb, s0, s1, b0, b1, xb[j], xsum[j], 0.0f, acc);
+    }
+}
+
+// the same over any group range, activation fragments read from the row in shared memory
+template <int BITS, int META>
+__device__ __forceinline__ void swz_accumulate_range(const unsigned char *box_a, const unsigned char *box_b, int rows_per_chunk,
+                                                     int ra, int rb, const uint16_t *s, const uint16_t *b, int ma, int mb,
+                                                     int groups_total, int g_begin, int g_end, const __half *xrow,
+                                                     const float *xsum, float (&acc)[1][4]) {
+    using vec = typename GroupBytes<BITS>::vec;
+    const int t = threadIdx.x & 3;
+    for (int G = g_begin; G < g_end; ++G) {
+        const vec wa[1] = {*reinterpret_cast<const vec *>(box_a + swz_offset<BITS>(G, ra, t, rows_per_chunk))};
+        const vec wb[1] = {*reinterpret_cast<const vec *>(box_b + swz_offset<BITS>(G, rb, t, rows_per_chunk))};
+        const uint16_t s0[1] = {s[ma * groups_total + G]}, s1[1] = {s[mb * groups_total + G]};
+        const uint16_t b0[1] = {b[ma * groups_total + G]}, b1[1] = {b[mb * groups_total + G]};
+        uint32_t xb[8];
+        const uint4 *xp = reinterpret_cast<const uint4 *>(xrow + (size_t)G * kGroup + t * 16);
+        permute_x<BITS>(xp[0], xp[1], xb);
+        group_step<BITS, META, 1, true>(wa, wb, s0, s1, b0, b1, xb, xsum[G], 0.0f, acc);
+    }
+}
+
 }  // namespace nvmai
