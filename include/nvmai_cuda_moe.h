@@ -353,11 +353,12 @@ NVMAI_API int nvmai_cuda_moe_ep_stack_decode(nvmai_cuda_moe *h, const void *x_ow
 NVMAI_API int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16, uint32_t tokens, void *y_last,
                                 void *stream);
 
-/* How a single-token nvmai_cuda_moe_stack_decode step runs (no counterpart in the
- * reference, whose command buffers are its only launch unit):
- *   0  (default) one resident kernel for the whole step when the shape allows it
+/* How an nvmai_cuda_moe_stack_decode step runs (no counterpart in the reference, whose
+ * command buffers are its only launch unit):
+ *   0  (default) one row: one resident kernel for the whole step when the shape allows it
  *      (top_k <= 8, shared_bits == routed_bits, d <= 16 * SM count, f and shared_f <= 1024,
- *      no expert map, stream not under capture), the staged kernels otherwise;
+ *      no expert map, stream not under capture), the staged kernels otherwise; several rows:
+ *      the kernels nvmai_cuda_moe_layer_decode runs for that many rows, as a CUDA graph;
  *   1  always the staged kernels (three launches per layer, replayed as a CUDA graph);
  *   2  the resident kernel, or NVMAI_CUDA_EINVAL when the shape does not allow it.
  * Both paths give bit-identical results.  NVMAI_CUDA_DECODE_MODE in the environment sets
@@ -369,7 +370,7 @@ NVMAI_API int nvmai_cuda_moe_set_decode_mode(nvmai_cuda_moe *h, int mode);
  * (RealForwardRunner.swift:1208-1237).  Synchronises the device. */
 NVMAI_API int nvmai_cuda_moe_read_route_log(nvmai_cuda_moe *h, uint32_t *out_host, uint32_t layers);
 
-/* The same after a step of several rows (2..8 rows through the resident kernel, or an
+/* The same after a step of several rows (2..8 rows in modes 0 and 2, or an
  * expert-parallel step, where the rows are those of all ranks): u32 [layers][rows][top_k].
  * `rows` must be the row count of that step. */
 NVMAI_API int nvmai_cuda_moe_read_route_log_rows(nvmai_cuda_moe *h, uint32_t *out_host, uint32_t layers, uint32_t rows);

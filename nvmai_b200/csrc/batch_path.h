@@ -122,6 +122,7 @@ struct PackActsParams {
 };
 cudaError_t bp_pack_acts(const PackActsParams &p, cudaStream_t st);
 
+constexpr uint32_t kBpNormRow = 2048;     // longest row that the reduction normalises itself
 struct CombineRowsParams {
     const void *partial; uint32_t partial_half;
     const void *shared_partial; uint32_t shared_half;     // nullptr: no shared expert
@@ -129,6 +130,7 @@ struct CombineRowsParams {
     void *y, *hidden;
     const __half *hidden_delta;   // decode order only
     float *partial_y;             // this rank's share only
+    __half *x_next;               // or nullptr: the next block's input, half(y * rsqrt(mean(y^2) + 1e-6)); D <= kBpNormRow, decode order
     uint32_t tokens, D, K, prefill;
     uint32_t aligned;             // set by bp_combine
 };

@@ -495,6 +495,8 @@ template <int OUT, int PART>
 __global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) {
     __shared__ uint32_t pos[kMaxTopK];
     __shared__ float wk[kMaxTopK];
+    __shared__ float row[kBpNormRow];
+    __shared__ float wsum[8];
     pdl_wait();
     pdl_launch_dependents();
     const uint32_t tok = blockIdx.x;
@@ -557,6 +559,32 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) 
         }
         if (p.y != nullptr) store_out8<OUT>(p.y, i, y, p.aligned);
         if (p.hidden != nullptr) store_out8<OUT>(p.hidden, i, hid, p.aligned);
+        if (p.x_next != nullptr)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) row[d + k] = y[k];
+    }
+    if (p.x_next == nullptr) return;
+    // the reduction tree of stage_x (staged_decode.cuh), so that a stack's rows have the bits of its layers run one by one
+    __syncthreads();
+    float keep[kBpNormRow / 256], ss = 0.0f;
+#pragma unroll
+    for (uint32_t j = 0; j < kBpNormRow / 256; ++j) {
+        const uint32_t i = threadIdx.x + j * 256u;
+        keep[j] = i < p.D ? row[i] : 0.0f;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kBpNormRow / 256; ++j) ss = fmaf(keep[j], keep[j], ss);
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31u) == 0) wsum[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float tot = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tot += wsum[i];
+    const float sc = rsqrtf(tot / (float)p.D + 1e-6f);
+#pragma unroll
+    for (uint32_t j = 0; j < kBpNormRow / 256; ++j) {
+        const uint32_t i = threadIdx.x + j * 256u;
+        if (i < p.D) p.x_next[(size_t)tok * p.D + i] = __float2half_rn(keep[j] * sc);
     }
 }
 

@@ -50,9 +50,9 @@ struct LayerViews {
 };
 
 struct StackGraphKey {
-    const void *x0; void *y; uint32_t tokens; cudaStream_t stream;
+    const void *x0; void *y; uint32_t tokens; cudaStream_t stream; bool batched, logged;
     bool operator<(const StackGraphKey &o) const {
-        return std::tie(x0, y, tokens, stream) < std::tie(o.x0, o.y, o.tokens, o.stream);
+        return std::tie(x0, y, tokens, stream, batched, logged) < std::tie(o.x0, o.y, o.tokens, o.stream, o.batched, o.logged);
     }
 };
 
@@ -88,7 +88,7 @@ struct nvmai_cuda_moe {
     const void **blob_table = nullptr;   // unused on device; kept for symmetry
     void *stage_x = nullptr;        // host-call staging: [T][D] fp16
     void *stage_y = nullptr;        // host-call staging: [T][D] out_dtype
-    std::map<StackGraphKey, cudaGraphExec_t> stack_graphs;
+    std::map<StackGraphKey, std::pair<cudaGraphExec_t, uint64_t>> stack_graphs;      // graph, kernels in it
     bool graphs_stale = false, ep_graphs_stale = false;
     // L2 prefetch of the next stage's weights in the fused layer chain: off unless
     // NVMAI_CUDA_L2_PREFETCH=1 (measured slower on B200: the prefetch competes with the
@@ -807,6 +807,7 @@ struct PrefillMode {
     bool routed_only = false;
     float *partial_y = nullptr;
     const __half *hidden_delta = nullptr;
+    __half *x_next = nullptr;       // the reduction also writes the next block's input (see CombineRowsParams)
 };
 
 // What comes before the experts' GEMMs: the rows packed (px says how; without dst only the scalar gate is taken), the
@@ -927,7 +928,7 @@ int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32
     CombineRowsParams pc{};
     pc.partial = h->partial; pc.shared_partial = c.shared_f ? h->shared_partial : nullptr;
     pc.inv = h->inv; pc.routing_w = w; pc.gate_val = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE ? h->gate_val : nullptr;
-    pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y;
+    pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y; pc.x_next = mode.x_next;
     pc.tokens = tokens; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
     return launched(h, bp_combine(pc, c.out_dtype, st));
 }
@@ -1053,7 +1054,7 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     pc.partial = h->partial; pc.partial_half = part_half ? 1 : 0;
     pc.shared_partial = c.shared_f ? h->shared_partial : nullptr; pc.shared_half = wide ? 0 : 1;
     pc.inv = h->inv; pc.routing_w = w; pc.gate_val = gated ? h->gate_val : nullptr;
-    pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y;
+    pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y; pc.x_next = mode.x_next;
     pc.tokens = tokens; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
     return launched(h, bp_combine(pc, c.out_dtype, st));
 }
@@ -1430,7 +1431,7 @@ nvmai_cuda_moe *nvmai_cuda_moe_create(const nvmai_cuda_moe_config *config, int *
 
 void nvmai_cuda_moe_destroy(nvmai_cuda_moe *h) {
     if (!h) return;
-    for (auto &kv : h->stack_graphs) cudaGraphExecDestroy(kv.second);
+    for (auto &kv : h->stack_graphs) cudaGraphExecDestroy(kv.second.first);
     ep_release(h);
     cudaFree(h->pd_trace);
     cudaFree(h->pb_xchg);
@@ -1766,8 +1767,22 @@ int nvmai_cuda_moe_rms_renorm(nvmai_cuda_moe *h, const void *y, uint32_t tokens,
 // Layer l > 0 reads the previous layer's block output and renormalises it inside
 // its own stage 1 (every block derives the same rows; block 0 stores them for
 // stage 2), so a layer is exactly three launches.
-static int stack_enqueue(nvmai_cuda_moe *h, const __half *x0, uint32_t tokens, void *y_last, cudaStream_t st) {
+// batched: through the batched experts' kernels, whose reduction normalises the rows for the next layer.
+// route_log: where the selected experts go, [num_layers][tokens][top_k], or nullptr.
+static int stack_enqueue(nvmai_cuda_moe *h, const __half *x0, uint32_t tokens, void *y_last, cudaStream_t st, bool batched, uint32_t *route_log) {
     const auto &c = h->cfg;
+    auto log = [&](uint32_t l) { return route_log ? route_log + (size_t)l * tokens * c.top_k : nullptr; };
+    if (batched) {
+        for (uint32_t l = 0; l < c.num_layers; ++l) {
+            const bool last = l + 1 == c.num_layers;
+            PrefillMode mode;
+            mode.decode_order = true;
+            mode.x_next = last ? nullptr : h->xnorm;
+            int rc = layer_prefill_impl(h, l, l == 0 ? x0 : h->xnorm, tokens, nullptr, last ? y_last : nullptr, log(l), nullptr, st, mode);
+            if (rc) return rc;
+        }
+        return NVMAI_CUDA_OK;
+    }
     for (uint32_t l = 0; l < c.num_layers; ++l) {
         const bool last = l + 1 == c.num_layers;
         void *y = last ? y_last : h->y;
@@ -1775,7 +1790,7 @@ static int stack_enqueue(nvmai_cuda_moe *h, const __half *x0, uint32_t tokens, v
         const __half *x_rows;
         if (l == 0) { xsrc.x = x0; xsrc.x_stride = c.d; x_rows = x0; }
         else { xsrc.y_prev = h->y; xsrc.x_out = h->xnorm; x_rows = h->xnorm; }
-        int rc = layer_decode_impl(h, l, xsrc, x_rows, tokens, nullptr, y, nullptr, nullptr, st,
+        int rc = layer_decode_impl(h, l, xsrc, x_rows, tokens, nullptr, y, log(l), nullptr, st,
                                    last ? nullptr : &h->layers[l + 1]);
         if (rc) return rc;
     }
@@ -1803,26 +1818,41 @@ int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16, uint32_t 
         if (pd_plan(h, plan) && pd_prepare(h, st) == NVMAI_CUDA_OK)
             return pd_launch(h, plan, static_cast<const __half *>(x0_f16), y_last, st);
     }
-    if (h->decode_mode != 1 && tokens >= 2 && tokens <= (uint32_t)kPbMaxRows && cs == cudaStreamCaptureStatusNone) {
-        PbPlan bplan;      // a few rows: the resident kernel with the rows as the tensor-core step's columns
+    // A few rows through the resident kernel: only on request, the kernels of the single layer are ahead.  Four
+    // layers on B200, resident / these: 2 rows 4-bit 134 / 101 us, 3 rows 8-bit 211 / 189, 5 rows 4-bit 230 / 187, 8 rows
+    // 8-bit 430 / 264.
+    if (h->decode_mode == 2 && tokens >= 2 && tokens <= (uint32_t)kPbMaxRows && cs == cudaStreamCaptureStatusNone) {
+        PbPlan bplan;      // the rows as the tensor-core step's columns
         if (pb_plan(h, tokens, bplan) && pd_prepare(h, st) == NVMAI_CUDA_OK)
             return pb_launch(h, bplan, static_cast<const __half *>(x0_f16), tokens, y_last, 0, 1, nullptr, st);
     }
     if (h->decode_mode == 2) return NVMAI_CUDA_EINVAL;
+    const bool batched = h->decode_mode == 0 && tokens >= 2 && c.d <= kBpNormRow && cs == cudaStreamCaptureStatusNone &&
+                         tc_batch_ok(h, tokens, true, st);
+    uint32_t *route_log = nullptr;
+    if (h->decode_mode == 0 && tokens >= 2 && tokens <= (uint32_t)kPbMaxRows && cs == cudaStreamCaptureStatusNone && h->pd_route_log != nullptr) {
+        route_log = h->pd_route_log;
+        h->pd_route_rows = tokens;
+    }
     if (st == nullptr || cs != cudaStreamCaptureStatusNone)
-        return stack_enqueue(h, static_cast<const __half *>(x0_f16), tokens, y_last, st);
+        return stack_enqueue(h, static_cast<const __half *>(x0_f16), tokens, y_last, st, batched, route_log);
+    if (batched) {       // what a capture may not do: scratch
+        int rc = ensure_prefill_scratch(h, st);
+        if (rc) return rc;
+    }
     if (h->graphs_stale) {
-        for (auto &kv : h->stack_graphs) cudaGraphExecDestroy(kv.second);
+        for (auto &kv : h->stack_graphs) cudaGraphExecDestroy(kv.second.first);
         h->stack_graphs.clear();
         h->graphs_stale = false;
     }
-    StackGraphKey key{x0_f16, y_last, tokens, st};
+    StackGraphKey key{x0_f16, y_last, tokens, st, batched, route_log != nullptr};
     auto it = h->stack_graphs.find(key);
     if (it == h->stack_graphs.end()) {
         int rc = record(h, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         if (rc) return rc;
         const uint64_t launches_before = g_launches.load();
-        rc = stack_enqueue(h, static_cast<const __half *>(x0_f16), tokens, y_last, st);
+        rc = stack_enqueue(h, static_cast<const __half *>(x0_f16), tokens, y_last, st, batched, route_log);
+        const uint64_t captured = g_launches.load() - launches_before;
         g_launches.store(launches_before);        // captured, not launched
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(st, &graph);
@@ -1832,10 +1862,10 @@ int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16, uint32_t 
         e = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         if ((rc = record(h, e))) return rc;
-        it = h->stack_graphs.emplace(key, exec).first;
+        it = h->stack_graphs.emplace(key, std::make_pair(exec, captured)).first;
     }
-    int rc = record(h, cudaGraphLaunch(it->second, st));
-    if (rc == NVMAI_CUDA_OK) g_launches.fetch_add((uint64_t)c.num_layers * 3, std::memory_order_relaxed);
+    int rc = record(h, cudaGraphLaunch(it->second.first, st));
+    if (rc == NVMAI_CUDA_OK) g_launches.fetch_add(it->second.second, std::memory_order_relaxed);
     return rc;
 }
 

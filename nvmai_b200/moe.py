@@ -264,7 +264,7 @@ class MoE:
     DECODE_AUTO, DECODE_STAGED, DECODE_RESIDENT = 0, 1, 2
 
     def set_decode_mode(self, mode: int) -> None:
-        """How a single-token stack step runs: one resident kernel (auto / forced) or the staged launches."""
+        """How a stack step runs: auto (one row: one resident kernel), the staged launches, or the resident kernel forced."""
         check(self._lib.nvmai_cuda_moe_set_decode_mode(self._h, int(mode)), "set_decode_mode")
 
     def debug_mute_block(self, block: int = 0xFFFFFFFF) -> None:
@@ -280,7 +280,7 @@ class MoE:
         return out
 
     def read_route_log_rows(self, rows: int, layers: int | None = None):
-        """-> uint32 [layers, rows, top_k] after a resident-kernel step of `rows` rows (2..8, or all ranks' rows)."""
+        """-> uint32 [layers, rows, top_k] after a step of `rows` rows (2..8, or all ranks' rows)."""
         import numpy as np
         n = self.config.num_layers if layers is None else layers
         out = np.zeros((n, rows, self.config.top_k), dtype=np.uint32)
