@@ -159,11 +159,14 @@ cudaError_t bp_combine(const CombineRowsParams &in, uint32_t out_dtype, cudaStre
     p.aligned = ((reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.hidden) | reinterpret_cast<uintptr_t>(p.hidden_delta) |
                   reinterpret_cast<uintptr_t>(p.partial_y)) & 15u) == 0 ? 1u : 0u;
     const dim3 grid(p.tokens), block(256);
+    if (p.x_next != nullptr)
+        return out_dtype == OUT_F16 ? launch_pdl(combine_rows_kernel<OUT_F16, OUT_F32, true>, grid, block, 0, st, true, p)
+                                    : launch_pdl(combine_rows_kernel<OUT_F32, OUT_F32, true>, grid, block, 0, st, true, p);
     if (out_dtype == OUT_F16) {
-        if (p.partial_half) return launch_pdl(combine_rows_kernel<OUT_F16, OUT_F16>, grid, block, 0, st, true, p);
-        return launch_pdl(combine_rows_kernel<OUT_F16, OUT_F32>, grid, block, 0, st, true, p);
+        if (p.partial_half) return launch_pdl(combine_rows_kernel<OUT_F16, OUT_F16, false>, grid, block, 0, st, true, p);
+        return launch_pdl(combine_rows_kernel<OUT_F16, OUT_F32, false>, grid, block, 0, st, true, p);
     }
-    return launch_pdl(combine_rows_kernel<OUT_F32, OUT_F32>, grid, block, 0, st, true, p);
+    return launch_pdl(combine_rows_kernel<OUT_F32, OUT_F32, false>, grid, block, 0, st, true, p);
 }
 
 cudaError_t bp_set_wait_limit(unsigned long long ns) { return cudaMemcpyToSymbol(g_wait_limit_ns, &ns, sizeof(ns)); }

@@ -230,9 +230,20 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
     // thread e owns expert e: total, exclusive scans of the pairs and of both launches' work items
     __threadfence();
     if (tid == 0) *p.counter = 0u;
-    uint32_t total = 0;
-#pragma unroll 8
-    for (uint32_t b = 0; b < gridDim.x; ++b) total += __ldcg(p.block_hist + (size_t)b * kMaxExperts + tid);
+    // (the blocks' counts come 32 at a time: this runs in one block while the chip waits; eight at a time the
+    // kernel took 24 us at 4096 rows, now 20.7)
+    constexpr uint32_t kBatch = 32;
+    uint32_t total = 0, counts[kBatch];
+    auto fetch = [&](uint32_t b0) {
+#pragma unroll
+        for (uint32_t k = 0; k < kBatch; ++k)
+            counts[k] = b0 + k < gridDim.x ? __ldcg(p.block_hist + (size_t)(b0 + k) * kMaxExperts + tid) : 0u;
+    };
+    for (uint32_t b0 = 0; b0 < gridDim.x; b0 += kBatch) {
+        fetch(b0);
+#pragma unroll
+        for (uint32_t k = 0; k < kBatch; ++k) total += counts[k];
+    }
     uint32_t mine[3] = {total, (total + p.cap[0] - 1u) / p.cap[0], (total + p.cap[1] - 1u) / p.cap[1]}, pre[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -260,11 +271,14 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
         if (tid == 0) p.n_work[j][0] = all[1 + j];
     }
     uint32_t run = pre[0];
-#pragma unroll 8
-    for (uint32_t b = 0; b < gridDim.x; ++b) {
-        const uint32_t c = __ldcg(p.block_hist + (size_t)b * kMaxExperts + tid);
-        p.block_hist[(size_t)b * kMaxExperts + tid] = run;
-        run += c;
+    for (uint32_t b0 = 0; b0 < gridDim.x; b0 += kBatch) {
+        if (gridDim.x > kBatch) fetch(b0);         // else they are still there
+#pragma unroll
+        for (uint32_t k = 0; k < kBatch; ++k)
+            if (b0 + k < gridDim.x) {
+                p.block_hist[(size_t)(b0 + k) * kMaxExperts + tid] = run;
+                run += counts[k];
+            }
     }
 }
 
@@ -486,16 +500,36 @@ template <int OUT> __device__ __forceinline__ void store_out8(void *p, size_t i,
     }
 }
 
+// 8 values of a partial row as they were loaded
+template <int PART> struct Part8 {
+    uint4 q[PART == OUT_F16 ? 1 : 2];
+    __device__ __forceinline__ void load(const void *p, size_t i) {
+        const uint4 *s = PART == OUT_F16 ? reinterpret_cast<const uint4 *>(static_cast<const __half *>(p) + i)
+                                         : reinterpret_cast<const uint4 *>(static_cast<const float *>(p) + i);
+#pragma unroll
+        for (int k = 0; k < (PART == OUT_F16 ? 1 : 2); ++k) q[k] = s[k];
+    }
+    __device__ __forceinline__ float at(int k) const {      // k: a constant
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(q);
+        if (PART == OUT_F32) return __uint_as_float(w[k]);
+        const __half2 h = *reinterpret_cast<const __half2 *>(&w[k >> 1]);
+        return (k & 1) ? __high2float(h) : __low2float(h);
+    }
+};
+
 // One block per token, 8 values per thread; every slot's partial row is requested before any is used (the version that
 // walked the slots value by value took 19-23 us for any batch).  Slot order, so the result does not depend on the
 // grouping.  PART: type of the partial rows.  Prefill rounding (prefill.metal:437-458, RealForwardRunner.swift:3560-3569):
 // every partial is rounded to the output type, h2 = out(sum_r fma(w, partial)) on its own, and the residual takes two
 // steps: hidden = out(out(hidden + h1) + h2).  Decode order: one rounding of h1 + sum, one residual add.
-template <int OUT, int PART>
-__global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) {
+// NORM: the row's RMS-normalised form is stored as the next block's input.  Its own variant: with the norm's code in it the
+// plain reduction of 1531 rows took 47 us instead of 26; with the partial rows kept as loaded (80 registers, three blocks
+// per SM, for half rows) it takes 20, 46 at 4096 rows.
+template <int OUT, int PART, bool NORM>
+__global__ void __launch_bounds__(256, PART == OUT_F16 ? 3 : 2) combine_rows_kernel(CombineRowsParams p) {
     __shared__ uint32_t pos[kMaxTopK];
     __shared__ float wk[kMaxTopK];
-    __shared__ float row[kBpNormRow];
+    __shared__ float row[NORM ? kBpNormRow : 1];
     __shared__ float wsum[8];
     pdl_wait();
     pdl_launch_dependents();
@@ -508,17 +542,17 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) 
     const float gate = p.gate_val != nullptr ? p.gate_val[tok] : 0.0f;
     for (uint32_t d = threadIdx.x * 8u; d < p.D; d += 2048u) {
         const size_t i = (size_t)tok * p.D + d;
-        float v[kMaxTopK][8];
+        Part8<PART> v[kMaxTopK];
 #pragma unroll
         for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
-            if (r < p.K && pos[r] != kBpNotLocal) load_out8<PART>(p.partial, (size_t)pos[r] * p.D + d, v[r]);
+            if (r < p.K && pos[r] != kBpNotLocal) v[r].load(p.partial, (size_t)pos[r] * p.D + d);
         if (p.partial_y != nullptr) {          // expert parallelism: this rank's share of the sum
             float acc[8] = {};
 #pragma unroll
             for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
                 if (r < p.K && pos[r] != kBpNotLocal)
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) acc[k] += wk[r] * v[r][k];
+                    for (int k = 0; k < 8; ++k) acc[k] += wk[r] * v[r].at(k);
             store_out8<OUT_F32>(p.partial_y, i, acc, p.aligned);
             continue;
         }
@@ -539,7 +573,7 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) 
                 float h2 = 0.0f;
 #pragma unroll
                 for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
-                    if (r < p.K) h2 = fmaf(wk[r], round_out<OUT>(v[r][k]), h2);
+                    if (r < p.K) h2 = fmaf(wk[r], round_out<OUT>(v[r].at(k)), h2);
                 h2 = round_out<OUT>(h2);
                 y[k] = h1[k] + h2;
                 hid[k] = round_out<OUT>(hid[k] + h1[k]) + h2;
@@ -551,7 +585,7 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) 
                 float acc = h1[k];
 #pragma unroll
                 for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
-                    if (r < p.K) acc += wk[r] * v[r][k];
+                    if (r < p.K) acc += wk[r] * v[r].at(k);
                 y[k] = round_out<OUT>(acc);
                 if (p.hidden_delta != nullptr) hid[k] = round_out<OUT>(hid[k] + delta[k]);
                 hid[k] += y[k];
@@ -559,11 +593,11 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) 
         }
         if (p.y != nullptr) store_out8<OUT>(p.y, i, y, p.aligned);
         if (p.hidden != nullptr) store_out8<OUT>(p.hidden, i, hid, p.aligned);
-        if (p.x_next != nullptr)
+        if constexpr (NORM)
 #pragma unroll
             for (int k = 0; k < 8; ++k) row[d + k] = y[k];
     }
-    if (p.x_next == nullptr) return;
+    if constexpr (!NORM) return;
     // the reduction tree of stage_x (staged_decode.cuh), so that a stack's rows have the bits of its layers run one by one
     __syncthreads();
     float keep[kBpNormRow / 256], ss = 0.0f;
@@ -584,7 +618,7 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(CombineRowsParams p) 
 #pragma unroll
     for (uint32_t j = 0; j < kBpNormRow / 256; ++j) {
         const uint32_t i = threadIdx.x + j * 256u;
-        if (i < p.D) p.x_next[(size_t)tok * p.D + i] = __float2half_rn(keep[j] * sc);
+        if (NORM && i < p.D) p.x_next[(size_t)tok * p.D + i] = __float2half_rn(keep[j] * sc);
     }
 }
 
