@@ -31,6 +31,7 @@ struct EgParams {
     const WorkItem *work; const uint32_t *n_work; const uint32_t *sorted_pair;
     const __half *rows, *shared_rows;         // phase 0: x rows with their correction columns (phase 1: the tensor maps)
     uint32_t shared_items;                    // items 0 .. shared_items - 1 are even runs of token rows (shared expert)
+    const uint32_t *shared_on;                // none of them if this word is 0
     uint32_t units_per_item, tiles_per_unit;  // phase 0: F / 128, -; phase 1: D / 128 / tiles_per_unit, tiles_per_unit
     uint32_t tokens, top_k, cap;              // cap: most rows of an item
     uint32_t kdim;                            // D (phase 0) / F (phase 1)
@@ -67,9 +68,11 @@ struct SgParams {
     const uint8_t *shared_s[2], *shared_b[2];
     const void *rows, *shared_rows;           // phase 0: fp16 x rows [token][kdim]; phase 1: activation rows (fp16 / fp32)
     const WorkItem *work; const uint32_t *n_work; const uint32_t *sorted_pair;
+    const uint32_t *shared_on;                // 0 there: no shared items
     uint32_t shared_items, units_per_item, tokens, top_k, cap, kdim, out_cols, act;
     void *out, *shared_out;                   // phase 0: activations [row][F]; phase 1: fp32 partial rows [row][D]
     uint32_t stages, meta_off, meta_bytes, x_off, raw_off, sum_off, scale_off;
+    uint32_t beside;                          // 1: runs beside the kernel in front of it, needs only what that one waited for
     unsigned int *status;
 };
 struct alignas(64) SgArgs {
@@ -98,7 +101,7 @@ constexpr uint32_t kRouterTileTokens = 64;
 cudaError_t bp_router(const RouterArgs &args, cudaStream_t st);
 
 // top-k of every row (or the given experts), histograms per block, and in the last block the scan: offsets per expert,
-// first positions per block, both GEMMs' work lists
+// first positions per block, the GEMMs' work lists
 struct RouteParams {
     const float *logits; uint32_t splits;     // nullptr: idx is given
     const uint16_t *pes;
@@ -107,7 +110,11 @@ struct RouteParams {
     const uint32_t *expert_map; uint32_t n_local;
     uint32_t *block_hist; unsigned int *counter;
     uint32_t *sorted_pair, *inv;
-    WorkItem *work[2]; uint32_t *n_work[2]; uint32_t cap[2];
+    // work lists: 0, 1 the grouped GEMMs' (gate/up, down) of the experts with more than `heavy` rows, 2 the streaming
+    // kernel's of the others (both phases).  `heavy` is taken as "none" where those experts hold less than a quarter of
+    // the pairs; shared_on[0] / [1]: 1 if the grouped GEMMs / the streaming kernel have the shared expert.
+    uint32_t *shared_on;
+    WorkItem *work[3]; uint32_t *n_work[3]; uint32_t cap[3]; uint32_t heavy;
 };
 uint32_t bp_route_blocks(uint32_t tokens);
 constexpr uint32_t kSmallRoute = 32;          // up to this many tokens one block does it all

@@ -173,6 +173,25 @@ __device__ __forceinline__ void write_items(const RouteParams &p, int j, uint32_
         p.work[j][first_item + i] = WorkItem{e, first_row + i * even + min(i, extra), even + (i < extra ? 1u : 0u), 0u};
 }
 
+__device__ __forceinline__ uint32_t item_count(const RouteParams &p, int j, uint32_t rows, uint32_t heavy) {
+    return (rows > heavy) == (j < 2) ? (rows + p.cap[j] - 1u) / p.cap[j] : 0u;
+}
+// whole block, `rows` = the rows of expert threadIdx.x: the limit that applies (see RouteParams); ends in sync
+__device__ __forceinline__ uint32_t heavy_limit(const RouteParams &p, uint32_t rows) {
+    __shared__ uint32_t heavy_pairs;
+    if (p.heavy == 0u || p.heavy == ~0u) {
+        if (threadIdx.x == 0) { p.shared_on[0] = p.heavy == 0u; p.shared_on[1] = p.heavy != 0u; }
+        return p.heavy;
+    }
+    if (threadIdx.x == 0) heavy_pairs = 0u;
+    __syncthreads();
+    if (rows > p.heavy) atomicAdd(&heavy_pairs, rows);
+    __syncthreads();
+    const bool many = 4u * heavy_pairs >= p.tokens * p.K;
+    if (threadIdx.x == 0) { p.shared_on[0] = many; p.shared_on[1] = !many; }
+    return many ? p.heavy : ~0u;
+}
+
 // v[i] = logit of expert lane + 32 i: the splits added in order, up to 32 loads in flight
 __device__ __forceinline__ void add_splits(float (&v)[kMaxExperts / 32], const RouteParams &p, uint32_t tok, uint32_t lane) {
     for (uint32_t sp = 0; sp < p.splits; sp += 4u) {
@@ -196,7 +215,7 @@ __device__ __forceinline__ void add_splits(float (&v)[kMaxExperts / 32], const R
 // PrefillMoEGrouping.groupTokenExpertPairs has them (PrefillMoEGrouping.swift:90-192).
 __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
     __shared__ uint32_t hist[kMaxExperts];
-    __shared__ uint32_t warp_tot[3][kMaxExperts / 32];
+    __shared__ uint32_t warp_tot[4][kMaxExperts / 32];
     __shared__ bool last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     hist[tid] = 0;
@@ -244,9 +263,10 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
 #pragma unroll
         for (uint32_t k = 0; k < kBatch; ++k) total += counts[k];
     }
-    uint32_t mine[3] = {total, (total + p.cap[0] - 1u) / p.cap[0], (total + p.cap[1] - 1u) / p.cap[1]}, pre[3];
+    const uint32_t heavy = heavy_limit(p, total);
+    uint32_t mine[4] = {total, item_count(p, 0, total, heavy), item_count(p, 1, total, heavy), item_count(p, 2, total, heavy)}, pre[4];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+    for (int j = 0; j < 4; ++j) {
         pre[j] = mine[j];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -256,9 +276,9 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
         if (lane == 31) warp_tot[j][warp] = pre[j];
     }
     __syncthreads();
-    uint32_t all[3] = {0, 0, 0};
+    uint32_t all[4] = {};
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+    for (int j = 0; j < 4; ++j) {
         pre[j] -= mine[j];
         for (int w = 0; w < kMaxExperts / 32; ++w) {
             if (w < warp) pre[j] += warp_tot[j][w];
@@ -266,7 +286,7 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
         }
     }
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < 3; ++j) {
         write_items(p, j, tid, total, mine[1 + j], pre[0], pre[1 + j]);
         if (tid == 0) p.n_work[j][0] = all[1 + j];
     }
@@ -319,7 +339,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(RouteParams p) {
     __shared__ uint32_t hist[kMaxExperts], first[kMaxExperts];
     __shared__ uint16_t cnt[8][kMaxExperts];                  // per warp of pairs, at most 256 pairs
     __shared__ uint16_t pair_expert[kSmallRoute * kMaxTopK];
-    __shared__ uint32_t warp_tot[3][kMaxExperts / 32];
+    __shared__ uint32_t warp_tot[4][kMaxExperts / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid < kMaxExperts) {
         hist[tid] = 0;
@@ -351,12 +371,15 @@ __global__ void __launch_bounds__(1024) route_small_kernel(RouteParams p) {
     const uint32_t peers = __match_any_sync(0xffffffffu, e);
     const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
     if (live && rank == 0u) cnt[warp][e] = (uint16_t)__popc(peers);
-    uint32_t total = 0, mine[3] = {}, pre[3] = {};
+    const uint32_t heavy = heavy_limit(p, tid < kMaxExperts ? hist[tid] : 0u);
+    uint32_t total = 0, mine[4] = {}, pre[4] = {};
     if (tid < kMaxExperts) {
         total = hist[tid];
-        mine[0] = total; mine[1] = (total + p.cap[0] - 1u) / p.cap[0]; mine[2] = (total + p.cap[1] - 1u) / p.cap[1];
+        mine[0] = total;
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
+        for (int j = 0; j < 3; ++j) mine[1 + j] = item_count(p, j, total, heavy);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
             pre[j] = mine[j];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -368,9 +391,9 @@ __global__ void __launch_bounds__(1024) route_small_kernel(RouteParams p) {
     }
     __syncthreads();
     if (tid < kMaxExperts) {
-        uint32_t all[3] = {0, 0, 0};
+        uint32_t all[4] = {};
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
+        for (int j = 0; j < 4; ++j) {
             pre[j] -= mine[j];
             for (int w = 0; w < kMaxExperts / 32; ++w) {
                 if (w < warp) pre[j] += warp_tot[j][w];
@@ -379,7 +402,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(RouteParams p) {
         }
         first[tid] = pre[0];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < 3; ++j) {
             write_items(p, j, tid, total, mine[1 + j], pre[0], pre[1 + j]);
             if (tid == 0) p.n_work[j][0] = all[1 + j];
         }

@@ -102,7 +102,7 @@ struct nvmai_cuda_moe {
     // Measured per layer, separate rows / batched: 3 rows 36 / 39 us, 4 rows 46 / 41, 13 rows 132 / 63, 40 rows 4-bit
     // 420 / 105.  NVMAI_CUDA_TC_MIN overrides it (32 when only NVMAI_CUDA_GROUPED_MIN is given).
     uint32_t tc_min_tokens = 4;
-    uint32_t stream_max_rows = ~0u;  // NVMAI_CUDA_STREAM_ROWS: rows per expert up to which stream_gemm.cuh serves a call
+    uint32_t stream_max_rows = ~0u;  // NVMAI_CUDA_STREAM_ROWS: rows up to which an expert is stream_gemm.cuh's
     // prefill chunks on the tensor cores (default); NVMAI_CUDA_PREFILL_TC=0 sends them through the exact grouped
     // kernels of the batched decode path instead
     bool prefill_tc = true;
@@ -115,6 +115,7 @@ struct nvmai_cuda_moe {
     float *pf_logits = nullptr;      // [splits][T][E]
     uint32_t *pf_hist = nullptr;     // [routing blocks][256]
     WorkItem *pf_work2 = nullptr;    // the down GEMM's work list (h->work is the gate/up GEMM's)
+    WorkItem *pf_work3 = nullptr;    // the streaming kernel's
     unsigned int *pf_counter = nullptr;
     CUtensorMap map_acts, map_sacts;
     // expert parallelism over NCCL: communicator and exchange buffers
@@ -748,10 +749,10 @@ int ensure_layer_maps(nvmai_cuda_moe *h, LayerViews &lv) {
 
 void free_prefill_scratch(nvmai_cuda_moe *h) {
     cudaFree(h->pf_x); cudaFree(h->pf_xs); cudaFree(h->pf_acts16); cudaFree(h->pf_sacts16); cudaFree(h->pf_rowscale);
-    cudaFree(h->pf_srowscale); cudaFree(h->pf_logits); cudaFree(h->pf_hist); cudaFree(h->pf_work2); cudaFree(h->pf_counter);
+    cudaFree(h->pf_srowscale); cudaFree(h->pf_logits); cudaFree(h->pf_hist); cudaFree(h->pf_work2); cudaFree(h->pf_work3); cudaFree(h->pf_counter);
     h->pf_x = h->pf_xs = h->pf_acts16 = h->pf_sacts16 = nullptr;
     h->pf_rowscale = h->pf_srowscale = h->pf_logits = nullptr;
-    h->pf_hist = nullptr; h->pf_work2 = nullptr; h->pf_counter = nullptr;
+    h->pf_hist = nullptr; h->pf_work2 = h->pf_work3 = nullptr; h->pf_counter = nullptr;
 }
 
 int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
@@ -773,10 +774,11 @@ int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
     const bool ok = alloc(&h->pf_x, T * dx * 2) && (!two_orders || alloc(&h->pf_xs, T * dx * 2)) && alloc(&h->pf_acts16, P * fx * 2) &&
                     alloc(&h->pf_sacts16, T * sfx * 2) && alloc(&h->pf_rowscale, P * 4) && alloc(&h->pf_srowscale, T * 4) &&
                     alloc(&h->pf_logits, logit_rows * c.num_experts * 4) && alloc(&h->pf_hist, blocks * kMaxExperts * 4) &&
-                    alloc(&h->pf_work2, (size_t)h->max_work * sizeof(WorkItem)) && alloc(&h->pf_counter, 16) &&
+                    alloc(&h->pf_work2, (size_t)h->max_work * sizeof(WorkItem)) && alloc(&h->pf_work3, (size_t)h->max_work * sizeof(WorkItem)) && alloc(&h->pf_counter, 16) &&
                     cudaMemsetAsync(h->pf_acts16, 0, P * fx * 2, st) == cudaSuccess &&
                     cudaMemsetAsync(h->pf_sacts16, 0, std::max<size_t>(T * sfx * 2, 16), st) == cudaSuccess &&
-                    cudaMemsetAsync(h->pf_counter, 0, 16, st) == cudaSuccess;
+                    cudaMemsetAsync(h->pf_counter, 1, 16, st) == cudaSuccess &&          // word 3 stays non-zero (EgParams::shared_on)
+                    cudaMemsetAsync(h->pf_counter, 0, 4, st) == cudaSuccess;
     int rc = ok ? NVMAI_CUDA_OK : NVMAI_CUDA_ENOMEM;
     if (!rc) rc = make_rows_tmap(h, &h->map_acts, h->pf_acts16, P, fx, 16);
     if (!rc) rc = c.shared_f ? make_rows_tmap(h, &h->map_sacts, h->pf_sacts16, T, sfx, 16) : (h->map_sacts = h->map_acts, NVMAI_CUDA_OK);
@@ -813,7 +815,7 @@ struct PrefillMode {
 // What comes before the experts' GEMMs: the rows packed (px says how; without dst only the scalar gate is taken), the
 // router, top-k and the pairs grouped by expert.  c: the handle's configuration, shared_f = 0 for routed rows only.
 int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c, const __half *x, uint32_t tokens, uint32_t *idx, __half *w,
-               PackXParams px, const uint32_t (&caps)[2], bool routed_only, cudaStream_t st) {
+               PackXParams px, const uint32_t (&caps)[3], uint32_t heavy, bool routed_only, cudaStream_t st) {
     int rc;
     const bool gated = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE;
     const bool dense_gate = gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;
@@ -827,8 +829,10 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
     r.idx = idx; r.w = w; r.tokens = tokens; r.E = c.num_experts; r.K = c.top_k;
     r.expert_map = h->expert_map; r.n_local = h->expert_map ? h->n_local : c.num_experts;
     r.block_hist = h->pf_hist; r.counter = h->pf_counter; r.sorted_pair = h->sorted_pair; r.inv = h->inv;
-    r.work[0] = h->work; r.work[1] = h->pf_work2; r.n_work[0] = h->n_work; r.n_work[1] = h->n_work + 2;
-    r.cap[0] = caps[0]; r.cap[1] = caps[1];
+    r.work[0] = h->work; r.work[1] = h->pf_work2; r.work[2] = h->pf_work3;
+    r.n_work[0] = h->n_work; r.n_work[1] = h->n_work + 2; r.n_work[2] = h->n_work + 1;      // n_work[3] stays 0
+    for (int j = 0; j < 3; ++j) r.cap[j] = caps[j];
+    r.heavy = heavy; r.shared_on = h->pf_counter + 1;
     // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
     // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
     // affine routers keep the exact code-times-activation kernel.
@@ -853,16 +857,6 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
 // 251 us in blocks of 16; 400 rows 332 / 289 us.
 uint32_t stream_blocks(const nvmai_cuda_moe *h, uint32_t tokens) { return tokens * h->cfg.top_k <= 9 * h->cfg.num_experts ? 1 : 2; }
 
-// Up to here the streaming kernel is ahead of the tcgen05 kernel, whose cost at few rows is the conversion of the
-// codes, one pass per 4 bits of a code and per part of a scale.  Measured per layer, streaming / tcgen05: one pass
-// 320 rows 215 / 234 us, 512 rows 285 / 241; two passes (8-bit) 512 rows 353 / 410, 700 rows 459 / 421; four passes
-// (8-bit, fp16 scales kept exact) 700 rows 453 / 657.
-uint32_t stream_limit(const nvmai_cuda_moe *h, bool decode_order) {
-    if (h->stream_max_rows != ~0u) return h->stream_max_rows;
-    const auto &c = h->cfg;
-    return 10 * (c.routed_bits / 4) * (decode_order && c.meta_dtype == NVMAI_META_FP16 ? 2 : 1);
-}
-
 bool stream_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared) {
     const auto &c = h->cfg;
     if (!tc_shape_ok(h, with_shared) || c.top_k > (uint32_t)kMaxTopK) return false;
@@ -876,6 +870,61 @@ bool stream_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared) {
     return fits(0, c.d, c.f) && fits(1, c.f, c.d) && (!with_shared || c.shared_f == 0 || (fits(0, c.d, c.shared_f) && fits(1, c.shared_f, c.d)));
 }
 
+// Which experts of a batched call the streaming kernel has: those with up to `heavy` rows (>= the call's rows: all, 0: none).
+// tcgen05 pays for converting an expert's codes once per pass (4 bits of a code, parts of a scale), mma.sync for every 8
+// rows; they are level at 16 rows.  Below 6 rows per expert, evenly routed, few experts can have more and the grouped
+// launches (10 us, empty) are not worth it; above 12 per pass few have less.  Measured per layer, streaming / mixed /
+// tcgen05, 4-bit: 256 rows even 182 / 191 / 231; skewed (popularity 1 / rank^0.6) 183 / 156 / 189, 1 / rank^1.1 159 / 117 / 130;
+// 450 rows even 257 / 239 / 240; 8-bit 256 rows (1.1) 186 / 140 / 183, 700 rows (0.4) 456 / 352 / 421.
+struct ExpertSplit { uint32_t heavy; };
+ExpertSplit expert_split(const nvmai_cuda_moe *h, uint32_t tokens, const PrefillMode &mode) {
+    if (!stream_ok(h, tokens, !mode.routed_only)) return {0};
+    if (h->stream_max_rows != ~0u) return {h->stream_max_rows};
+    const auto &c = h->cfg;
+    const uint64_t passes = (c.routed_bits / 4) * (mode.decode_order && c.meta_dtype == NVMAI_META_FP16 ? 2 : 1);
+    const uint64_t P = (uint64_t)tokens * c.top_k, E = c.num_experts;
+    return {P < 6 * E ? ~0u : P <= 12 * passes * E ? 16u : 0u};
+}
+
+// One phase (0 gate/up, 1 down) of the streaming kernel over its work list and the shared expert; c as in route_rows.
+// beside: next to the grouped GEMM that was launched just before.
+int stream_phase(nvmai_cuda_moe *h, const LayerViews &lv, const nvmai_cuda_moe_config &c, int phase, const __half *x, uint32_t tokens, bool beside,
+                 cudaStream_t st) {
+    const bool wide = c.out_dtype == NVMAI_OUT_FP32;
+    const uint32_t P = tokens * c.top_k, experts = h->expert_map ? h->n_local : c.num_experts, nb = stream_blocks(h, tokens);
+    const bool merged = c.shared_f != 0 && c.shared_bits == c.routed_bits && c.shared_f == c.f, shared = c.shared_f != 0 && (merged || !beside);
+    auto u8 = [](const void *p) { return static_cast<const uint8_t *>(p); };
+    SgArgs a{};
+    SgParams &p = a.p;
+    p.kdim = phase == 0 ? c.d : c.f; p.out_cols = phase == 0 ? c.f : c.d;
+    p.experts = u8(lv.w.experts); p.stride = lv.w.expert_stride; p.num_experts = experts;
+    p.work = h->pf_work3; p.n_work = h->n_work + 1; p.sorted_pair = h->sorted_pair;
+    p.tokens = tokens; p.top_k = c.top_k; p.act = c.activation; p.status = h->status; p.beside = beside ? 1 : 0;
+    p.shared_on = h->pf_counter + 2;
+    if (phase == 0) {
+        p.off_s[0] = lv.w.offsets.gate_s; p.off_b[0] = lv.w.offsets.gate_b; p.off_s[1] = lv.w.offsets.up_s; p.off_b[1] = lv.w.offsets.up_b;
+        p.shared_s[0] = u8(lv.w.shared_gate_proj.scales); p.shared_b[0] = u8(lv.w.shared_gate_proj.biases);
+        p.shared_s[1] = u8(lv.w.shared_up_proj.scales); p.shared_b[1] = u8(lv.w.shared_up_proj.biases);
+        p.rows = p.shared_rows = x; p.out = h->acts; p.shared_out = h->shared_act;
+        a.routed0 = lv.gate64; a.routed1 = lv.up64; a.shared0 = lv.sgate64; a.shared1 = lv.sup64;
+    } else {
+        p.off_s[0] = lv.w.offsets.down_s; p.off_b[0] = lv.w.offsets.down_b;
+        p.shared_s[0] = u8(lv.w.shared_down_proj.scales); p.shared_b[0] = u8(lv.w.shared_down_proj.biases);
+        p.rows = h->acts; p.shared_rows = h->shared_act; p.out = h->partial; p.shared_out = h->shared_partial;
+        a.routed0 = a.routed1 = lv.down64; a.shared0 = a.shared1 = lv.sdown64;
+    }
+    const size_t smem = sg_plan(p, phase, nb, wide);
+    p.shared_items = merged ? (tokens + p.cap - 1) / p.cap : 0;
+    const uint32_t units = (p.shared_items + std::min(P, experts + P / p.cap)) * p.units_per_item;
+    int rc = launched(h, sg_launch(phase, c.routed_bits, c.meta_dtype, c.out_dtype, nb, a, std::max(1u, std::min(units, (uint32_t)h->sm_count)), smem, st));
+    if (rc || !shared || merged) return rc;
+    p.n_work = h->n_work + 3;        // the shared expert's own bit width or size: a launch of its own, no routed items
+    p.kdim = phase == 0 ? c.d : c.shared_f; p.out_cols = phase == 0 ? c.shared_f : c.d;
+    const size_t own = sg_plan(p, phase, nb, wide);
+    p.shared_items = (tokens + p.cap - 1) / p.cap;
+    return launched(h, sg_launch(phase, c.shared_bits, c.meta_dtype, c.out_dtype, nb, a, std::min(p.shared_items * p.units_per_item, (uint32_t)h->sm_count), own, st));
+}
+
 int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32_t tokens, void *hidden, void *y, uint32_t *out_idx,
                       __half *out_w, cudaStream_t st, const PrefillMode mode) {
     LayerViews &lv = h->layers[layer];
@@ -885,46 +934,10 @@ int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32
     if (mode.routed_only) c.shared_f = 0;
     uint32_t *idx = out_idx ? out_idx : h->idx;
     __half *w = out_w ? out_w : h->w;
-    const bool wide = c.out_dtype == NVMAI_OUT_FP32;
-    const uint32_t P = tokens * c.top_k, experts = h->expert_map ? h->n_local : c.num_experts, nb = stream_blocks(h, tokens);
-    const bool merged = c.shared_f != 0 && c.shared_bits == c.routed_bits && c.shared_f == c.f;
-    const uint32_t caps[2] = {8 * nb, 8 * nb};
-    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, PackXParams{}, caps, mode.routed_only, st))) return rc;
-    auto u8 = [](const void *p) { return static_cast<const uint8_t *>(p); };
-    for (int phase = 0; phase < 2; ++phase) {
-        SgArgs a{};
-        SgParams &p = a.p;
-        p.kdim = phase == 0 ? c.d : c.f; p.out_cols = phase == 0 ? c.f : c.d;
-        p.experts = u8(lv.w.experts); p.stride = lv.w.expert_stride; p.num_experts = experts;
-        p.work = h->work; p.n_work = h->n_work; p.sorted_pair = h->sorted_pair;
-        p.tokens = tokens; p.top_k = c.top_k; p.act = c.activation; p.status = h->status;
-        if (phase == 0) {
-            p.off_s[0] = lv.w.offsets.gate_s; p.off_b[0] = lv.w.offsets.gate_b; p.off_s[1] = lv.w.offsets.up_s; p.off_b[1] = lv.w.offsets.up_b;
-            p.shared_s[0] = u8(lv.w.shared_gate_proj.scales); p.shared_b[0] = u8(lv.w.shared_gate_proj.biases);
-            p.shared_s[1] = u8(lv.w.shared_up_proj.scales); p.shared_b[1] = u8(lv.w.shared_up_proj.biases);
-            p.rows = p.shared_rows = x; p.out = h->acts; p.shared_out = h->shared_act;
-            a.routed0 = lv.gate64; a.routed1 = lv.up64; a.shared0 = lv.sgate64; a.shared1 = lv.sup64;
-        } else {
-            p.off_s[0] = lv.w.offsets.down_s; p.off_b[0] = lv.w.offsets.down_b;
-            p.shared_s[0] = u8(lv.w.shared_down_proj.scales); p.shared_b[0] = u8(lv.w.shared_down_proj.biases);
-            p.rows = h->acts; p.shared_rows = h->shared_act; p.out = h->partial; p.shared_out = h->shared_partial;
-            a.routed0 = a.routed1 = lv.down64; a.shared0 = a.shared1 = lv.sdown64;
-        }
-        const size_t smem = sg_plan(p, phase, nb, wide);
-        p.shared_items = merged ? (tokens + p.cap - 1) / p.cap : 0;
-        const uint32_t units = (p.shared_items + std::min(P, experts + P / p.cap)) * p.units_per_item;
-        if ((rc = launched(h, sg_launch(phase, c.routed_bits, c.meta_dtype, c.out_dtype, nb, a, std::max(1u, std::min(units, (uint32_t)h->sm_count)), smem, st))))
-            return rc;
-        if (c.shared_f && !merged) {         // the shared expert's own bit width or size: a launch of its own
-            p.n_work = h->n_work + 3;        // a zero: no routed items
-            p.kdim = phase == 0 ? c.d : c.shared_f; p.out_cols = phase == 0 ? c.shared_f : c.d;
-            const size_t own = sg_plan(p, phase, nb, wide);
-            p.shared_items = (tokens + p.cap - 1) / p.cap;
-            if ((rc = launched(h, sg_launch(phase, c.shared_bits, c.meta_dtype, c.out_dtype, nb, a,
-                                            std::min(p.shared_items * p.units_per_item, (uint32_t)h->sm_count), own, st))))
-                return rc;
-        }
-    }
+    const uint32_t cap = 8 * stream_blocks(h, tokens), caps[3] = {cap, cap, cap};
+    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, PackXParams{}, caps, ~0u, mode.routed_only, st))) return rc;
+    for (int phase = 0; phase < 2; ++phase)
+        if ((rc = stream_phase(h, lv, c, phase, x, tokens, false, st))) return rc;
     CombineRowsParams pc{};
     pc.partial = h->partial; pc.shared_partial = c.shared_f ? h->shared_partial : nullptr;
     pc.inv = h->inv; pc.routing_w = w; pc.gate_val = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE ? h->gate_val : nullptr;
@@ -935,8 +948,11 @@ int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32
 
 int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32_t tokens, void *hidden, void *y,
                        uint32_t *out_idx, __half *out_w, cudaStream_t st, const PrefillMode mode = PrefillMode{}) {
-    if ((uint64_t)tokens * h->cfg.top_k <= (uint64_t)stream_limit(h, mode.decode_order) * h->cfg.num_experts && stream_ok(h, tokens, !mode.routed_only))
-        return layer_stream_impl(h, layer, x, tokens, hidden, y, out_idx, out_w, st, mode);
+    const ExpertSplit split_at = expert_split(h, tokens, mode);
+    if (split_at.heavy >= tokens) return layer_stream_impl(h, layer, x, tokens, hidden, y, out_idx, out_w, st, mode);
+    // experts with up to `heavy` rows through the streaming kernel, beside the grouped GEMMs of the others
+    const uint32_t heavy = split_at.heavy;
+    const bool mixed = heavy != 0;
     LayerViews &lv = h->layers[layer];
     int rc = ensure_prefill_scratch(h, st);
     if (rc || (rc = ensure_layer_maps(h, lv))) return rc;
@@ -959,21 +975,21 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     // Longest work item: the accumulators are double-buffered up to 96 rows, one set of up to 192 rows pays above
     // that; short items leave room for a deeper ring of rows.  rows: per expert, evenly routed.
     const uint32_t rows = (P + c.num_experts - 1) / c.num_experts;
-    const uint32_t want = rows <= 12 ? 48 : rows <= 64 ? 96 : 192;
+    const uint32_t want = mixed ? 96 : rows <= 12 ? 48 : rows <= 64 ? 96 : 192;
     EgParams g0{}, g1{};
     g0.kdim = c.d; g1.kdim = c.f;
     const EgPlan plan0 = eg_plan(g0, 0, want), plan1 = eg_plan(g1, 1, std::min(want, 128u));
 
     PackXParams px{};
     px.dst = h->pf_x; px.dst2 = two_orders ? h->pf_xs : nullptr; px.permute = c.routed_bits == 4 ? 1 : 0;
-    const uint32_t caps[2] = {plan0.cap, plan1.cap};
-    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, px, caps, mode.routed_only, st))) return rc;
+    const uint32_t caps[3] = {plan0.cap, plan1.cap, 8 * stream_blocks(h, tokens)};
+    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, px, caps, mixed ? heavy : 0, mode.routed_only, st))) return rc;
 
     const uint32_t shared_rows = merged ? tokens : 0;
     auto set_common = [&](EgParams &g, const EgPlan &plan) {
         g.experts = static_cast<const uint8_t *>(lv.w.experts); g.stride = lv.w.expert_stride; g.num_experts = experts;
         g.sorted_pair = h->sorted_pair; g.tokens = tokens; g.top_k = c.top_k; g.act = c.activation; g.status = h->status;
-        g.shared_items = (shared_rows + plan.cap - 1) / plan.cap;
+        g.shared_items = (shared_rows + plan.cap - 1) / plan.cap; g.shared_on = h->pf_counter + 1;
         g.permute = c.routed_bits == 4 ? 1 : 0; g.shared_permute = c.shared_bits == 4 ? 1 : 0;
     };
     auto u8 = [](const void *p) { return static_cast<const uint8_t *>(p); };
@@ -1010,7 +1026,7 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     if ((rc = launched(h, eg_launch(0, c.routed_bits, c.meta_dtype, c.out_dtype, split, args, grid(units(g0, plan0.cap)), plan0.smem, st)))) return rc;
     if (c.shared_f && !merged) {
         EgParams s = g0;
-        s.n_work = h->n_work + 3;            // a zero: no routed items
+        s.shared_on = h->pf_counter + 3; s.n_work = h->n_work + 3;            // a zero: no routed items
         s.shared_items = (tokens + plan0.cap - 1) / plan0.cap;
         s.units_per_item = c.shared_f / 128; s.kfeat = c.shared_f; s.trace = nullptr; s.debug_drop_rows = 0;
         s.shared_rows = two_orders ? h->pf_xs : h->pf_x;
@@ -1018,6 +1034,7 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
         if ((rc = launched(h, eg_launch(0, c.shared_bits, c.meta_dtype, c.out_dtype, split, args, grid(s.shared_items * s.units_per_item), plan0.smem, st))))
             return rc;
     }
+    if (mixed && (rc = stream_phase(h, lv, c, 0, x, tokens, true, st))) return rc;
     if (wide) {          // activation rows as the down GEMMs read them
         PackActsParams pa{static_cast<const float *>(h->acts), h->pf_acts16, h->pf_rowscale, P, c.f, g0.permute,
                           static_cast<const float *>(h->shared_act), h->pf_sacts16, h->pf_srowscale, c.shared_f ? tokens : 0, c.shared_f,
@@ -1025,14 +1042,14 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
         if ((rc = launched(h, bp_pack_acts(pa, st)))) return rc;
     }
     // down; the prefill path rounds every partial to the output type, the decode path the sum
-    const bool part_half = !wide && !mode.decode_order && mode.partial_y == nullptr;
+    const bool part_half = !wide && !mode.decode_order && mode.partial_y == nullptr && !mixed;
     set_common(g1, plan1); set_shared(g1, 1);
     g1.work = h->pf_work2; g1.n_work = h->n_work + 2;
     g1.off_s[0] = lv.w.offsets.down_s; g1.off_b[0] = lv.w.offsets.down_b;
     const double spread = 1.0 - std::pow(1.0 - (double)c.top_k / c.num_experts, (double)tokens);
-    g1.tiles_per_unit = tiles_per_unit((uint32_t)(experts * spread) + P / plan1.cap + g1.shared_items);
+    g1.tiles_per_unit = tiles_per_unit((mixed ? P / (2 * heavy) : (uint32_t)(experts * spread) + P / plan1.cap) + g1.shared_items);
     g1.units_per_item = c.d / 128 / g1.tiles_per_unit; g1.out_cols = c.d;
-    g1.out = h->partial; g1.shared_out = h->shared_partial; g1.out_half = part_half ? 1 : 0; g1.shared_out_half = wide ? 0 : 1;
+    g1.out = h->partial; g1.shared_out = h->shared_partial; g1.out_half = part_half ? 1 : 0; g1.shared_out_half = wide || mixed ? 0 : 1;
     g1.row_scale = wide ? h->pf_rowscale : nullptr; g1.shared_row_scale = wide ? h->pf_srowscale : nullptr;
     g1.trace = h->trace_on ? h->trace + ((size_t)layer * 3 + 1) * kTraceWords : nullptr;
     args.routed0 = lv.down; args.routed1 = lv.down; args.shared0 = lv.sdown; args.shared1 = lv.sdown;
@@ -1043,16 +1060,17 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
         EgParams s = g1;
         s.kdim = c.shared_f;
         const EgPlan plan = eg_plan(s, 1, std::min(want, 128u));
-        s.n_work = h->n_work + 3; s.trace = nullptr;
+        s.shared_on = h->pf_counter + 3; s.n_work = h->n_work + 3; s.trace = nullptr;
         s.shared_items = (tokens + plan.cap - 1) / plan.cap;
         s.tiles_per_unit = tiles_per_unit(s.shared_items); s.units_per_item = c.d / 128 / s.tiles_per_unit;
         args.p = s;
         if ((rc = launched(h, eg_launch(1, c.shared_bits, c.meta_dtype, c.out_dtype, split, args, grid(s.shared_items * s.units_per_item), plan.smem, st))))
             return rc;
     }
+    if (mixed && (rc = stream_phase(h, lv, c, 1, x, tokens, true, st))) return rc;
     CombineRowsParams pc{};
     pc.partial = h->partial; pc.partial_half = part_half ? 1 : 0;
-    pc.shared_partial = c.shared_f ? h->shared_partial : nullptr; pc.shared_half = wide ? 0 : 1;
+    pc.shared_partial = c.shared_f ? h->shared_partial : nullptr; pc.shared_half = wide || mixed ? 0 : 1;
     pc.inv = h->inv; pc.routing_w = w; pc.gate_val = gated ? h->gate_val : nullptr;
     pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y; pc.x_next = mode.x_next;
     pc.tokens = tokens; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;

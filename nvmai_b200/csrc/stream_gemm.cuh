@@ -138,12 +138,14 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
         for (uint32_t i = 0; i < 16; ++i) mbar_init(&bars->h_full[i >> 3][i & 7], 1);
         mbar_fence_init();
     }
-    pdl_wait();
+    if (!p.beside) pdl_wait();
     pdl_launch_dependents();
     bool ok = __syncthreads_and(*reinterpret_cast<volatile unsigned int *>(p.status) == 0u);
-    const uint32_t total = ok ? (p.shared_items + p.n_work[0]) * p.units_per_item : 0u;
-    const uint32_t u0 = (uint32_t)((unsigned long long)total * blockIdx.x / gridDim.x);
-    const uint32_t u1 = (uint32_t)((unsigned long long)total * (blockIdx.x + 1) / gridDim.x);
+    // the units of the launch: those of the shared items come first and are skipped where another kernel has them
+    const uint32_t skip = *p.shared_on != 0u ? 0u : p.shared_items * p.units_per_item;
+    const uint32_t total = ok ? (p.shared_items + p.n_work[0]) * p.units_per_item - skip : 0u;
+    const uint32_t u0 = skip + (uint32_t)((unsigned long long)total * blockIdx.x / gridDim.x);
+    const uint32_t u1 = skip + (uint32_t)((unsigned long long)total * (blockIdx.x + 1) / gridDim.x);
     const uint32_t n_chunk = (p.kdim * BITS / 8u + 127u) / 128u / KS;          // stages of a unit
     constexpr uint32_t kMats = PHASE == 0 ? 2u : 1u;
 
@@ -428,6 +430,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
         const unsigned long long t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
+    if (p.beside) pdl_wait();              // the kernel after this one relies on the one before it being complete
 }
 
 }  // namespace nvmai

@@ -64,3 +64,42 @@ def test_rows_of_every_item_match_the_oracle(bits, meta, out, tokens, d, f, stre
         xr = np.ascontiguousarray(x[t])
         want = gu.oracle_decode(L, cfg, xr)[2] if entry == "decode" else gu.oracle_prefill_row(L, cfg, xr, None)[2]
         assert orc.rel_error(got[t], want) < (3e-3 if f16 else 1.5e-3), f"row {t}"
+
+
+# Mixed calls: experts with more rows than the limit through the grouped GEMMs, the others (and, where those are few, all
+# of them and the shared expert) through the streaming kernel.  40 rows on 32 experts: 10 rows each on average; a limit
+# of 8: many above it; 16: few, so none is taken as heavy; 39: at most the call's rows minus one.
+@pytest.mark.parametrize("bits,meta,out,limit", [(4, BF16, fmt.OUT_FP16, 8), (8, BF16, fmt.OUT_FP32, 8), (8, FP16, fmt.OUT_FP16, 9),
+                                                 (4, BF16, fmt.OUT_FP32, 16), (4, FP16, fmt.OUT_FP16, 39)])
+@pytest.mark.parametrize("entry", ["decode", "prefill"])
+def test_calls_split_between_the_two_kernels_match_the_oracle(bits, meta, out, limit, entry, monkeypatch):
+    monkeypatch.setenv("NVMAI_CUDA_STREAM_ROWS", str(limit))
+    d, f, tokens = 512, 256, 40
+    host = synthetic.layer(811 + limit, d=d, f=f, shared_f=f, num_experts=32, routed_bits=bits, meta=meta)
+    if bits == 8:
+        rng = np.random.default_rng(limit)
+        off = host["offsets"]
+        for name, n in (("gate", f * d), ("up", f * d), ("down", d * f)):
+            s = rng.uniform(0.0003, 0.0012, size=(32, n // 64)).astype(np.float32)
+            for key, v in (("_s", s), ("_b", -127.5 * s)):
+                raw = np.ascontiguousarray(fmt.f32_to_meta_bits(v, meta)).view(np.uint8)
+                host["experts"][:, off[name + key]:off[name + key] + raw.shape[1]] = raw
+        host["shared"] = [(w, fmt.f32_to_meta_bits(np.full(s.shape, 0.0007), meta), fmt.f32_to_meta_bits(np.full(s.shape, -0.0892), meta))
+                          for w, s, _ in host["shared"]]
+    cfg = MoEConfig(d=d, f=f, shared_f=f, num_experts=32, top_k=8, routed_bits=bits, shared_bits=bits, meta_dtype=meta,
+                    out_dtype=out, max_tokens=tokens)
+    moe = MoE(cfg)
+    dl = gu.DeviceLayer(host)
+    dl.register(moe, 0)
+    x = synthetic.hidden_rows(812, tokens, d)
+    f16 = out == fmt.OUT_FP16
+    y = gu.dev_empty(tokens * d, "f16" if f16 else "f32")
+    call = moe.layer_decode if entry == "decode" else moe.layer_prefill
+    call(0, gu.to_dev(x), tokens, **{"h2_out" if entry == "decode" else "y_out": y})
+    moe.synchronize()
+    got = (orc.f16_bits_to_f32(gu.from_dev(y, np.uint16)) if f16 else y.cpu().numpy()).reshape(tokens, d)
+    L, keep = gu.oracle_layer(host, cfg)
+    for t in range(0, tokens, 3):
+        xr = np.ascontiguousarray(x[t])
+        want = gu.oracle_decode(L, cfg, xr)[2] if entry == "decode" else gu.oracle_prefill_row(L, cfg, xr, None)[2]
+        assert orc.rel_error(got[t], want) < (3e-3 if f16 else 1.5e-3), f"row {t}"
