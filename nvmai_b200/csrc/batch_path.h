@@ -111,10 +111,10 @@ struct RouteParams {
     uint32_t *block_hist; unsigned int *counter;
     uint32_t *sorted_pair, *inv;
     // work lists: 0, 1 the grouped GEMMs' (gate/up, down) of the experts with more than `heavy` rows, 2 the streaming
-    // kernel's of the others (both phases).  `heavy` is taken as "none" where those experts hold less than a quarter of
-    // the pairs; shared_on[0] / [1]: 1 if the grouped GEMMs / the streaming kernel have the shared expert.
+    // kernel's of the others (both phases).  `heavy` is taken as "none" where those experts hold fewer than
+    // `heavy_min` pairs; shared_on[0] / [1]: 1 if the grouped GEMMs / the streaming kernel have the shared expert.
     uint32_t *shared_on;
-    WorkItem *work[3]; uint32_t *n_work[3]; uint32_t cap[3]; uint32_t heavy;
+    WorkItem *work[3]; uint32_t *n_work[3]; uint32_t cap[3]; uint32_t heavy, heavy_min;
 };
 uint32_t bp_route_blocks(uint32_t tokens);
 constexpr uint32_t kSmallRoute = 32;          // up to this many tokens one block does it all

@@ -187,7 +187,7 @@ __device__ __forceinline__ uint32_t heavy_limit(const RouteParams &p, uint32_t r
     __syncthreads();
     if (rows > p.heavy) atomicAdd(&heavy_pairs, rows);
     __syncthreads();
-    const bool many = 4u * heavy_pairs >= p.tokens * p.K;
+    const bool many = heavy_pairs >= p.heavy_min;
     if (threadIdx.x == 0) { p.shared_on[0] = many; p.shared_on[1] = !many; }
     return many ? p.heavy : ~0u;
 }

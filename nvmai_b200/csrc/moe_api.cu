@@ -832,7 +832,9 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
     r.work[0] = h->work; r.work[1] = h->pf_work2; r.work[2] = h->pf_work3;
     r.n_work[0] = h->n_work; r.n_work[1] = h->n_work + 2; r.n_work[2] = h->n_work + 1;      // n_work[3] stays 0
     for (int j = 0; j < 3; ++j) r.cap[j] = caps[j];
-    r.heavy = heavy; r.shared_on = h->pf_counter + 1;
+    // A quarter of the pairs pays for the grouped launches.  A rank's share of the routed sum splits by the expert's rows
+    // alone: every rank, and a handle with all experts, then takes the same kernel for an expert.
+    r.heavy = heavy; r.heavy_min = routed_only ? 0 : tokens * c.top_k / 4; r.shared_on = h->pf_counter + 1;
     // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
     // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
     // affine routers keep the exact code-times-activation kernel.
