@@ -122,7 +122,6 @@ __device__ __forceinline__ float router_row_logit(uint32_t kind, const uint8_t *
     float acc = 0.0f;
     if (kind == 0) {   // dense fp16 [E][D]
         const __half *wr = reinterpret_cast<const __half *>(W) + (size_t)row * D;
-#pragma unroll 4
         for (int c = lane; c < D / 8; c += 32) {
             uint4 wv = load_row16<SMEM>(wr + c * 8);
             const __half2 *wh = reinterpret_cast<const __half2 *>(&wv);

@@ -49,6 +49,28 @@ struct LayerViews {
     CUtensorMap gate64, up64, down64, sgate64, sup64, sdown64;     // the same codes in boxes of 64 rows (stream_gemm.cuh)
 };
 
+// Device scratch carved out of one allocation (a cudaMalloc takes 0.1-0.2 ms on B200): the buffers are asked for first,
+// then made in one go, those that have to start as zeros together in front.
+struct Slab {
+    struct Want { void **ptr; size_t bytes; };
+    std::vector<Want> zeros, plain;
+    template <typename T> void want(T **ptr, size_t bytes, bool zero = false) {
+        (zero ? zeros : plain).push_back({reinterpret_cast<void **>(ptr), (bytes + 1023) & ~(size_t)1023});
+    }
+    cudaError_t make(void *&base, cudaStream_t st) {
+        size_t front = 0, total = 0;
+        for (auto &w : zeros) front += w.bytes;
+        total = front;
+        for (auto &w : plain) total += w.bytes;
+        cudaError_t e = cudaMalloc(&base, total ? total : 16);
+        if (e != cudaSuccess) { base = nullptr; return e; }
+        char *at = static_cast<char *>(base);
+        for (auto *list : {&zeros, &plain})
+            for (auto &w : *list) { *w.ptr = w.bytes ? at : nullptr; at += w.bytes; }
+        return front ? cudaMemsetAsync(base, 0, front, st) : cudaSuccess;
+    }
+};
+
 struct StackGraphKey {
     const void *x0; void *y; uint32_t tokens; cudaStream_t stream; bool batched, logged;
     bool operator<(const StackGraphKey &o) const {
@@ -107,6 +129,7 @@ struct nvmai_cuda_moe {
     // kernels of the batched decode path instead
     bool prefill_tc = true;
     // expert GEMMs: operand rows and routing scratch (allocated by the first call that takes them)
+    void *pf_slab = nullptr;         // all of these
     __half *pf_x = nullptr;          // [T][D + extra] x rows in the routed weights' K order, with their group sums
     __half *pf_xs = nullptr;         // the same in the shared expert's K order, when that differs
     __half *pf_acts16 = nullptr;     // [T*K][F + extra] routed activations as the down GEMM reads them
@@ -748,11 +771,9 @@ int ensure_layer_maps(nvmai_cuda_moe *h, LayerViews &lv) {
 }
 
 void free_prefill_scratch(nvmai_cuda_moe *h) {
-    cudaFree(h->pf_x); cudaFree(h->pf_xs); cudaFree(h->pf_acts16); cudaFree(h->pf_sacts16); cudaFree(h->pf_rowscale);
-    cudaFree(h->pf_srowscale); cudaFree(h->pf_logits); cudaFree(h->pf_hist); cudaFree(h->pf_work2); cudaFree(h->pf_work3); cudaFree(h->pf_counter);
-    h->pf_x = h->pf_xs = h->pf_acts16 = h->pf_sacts16 = nullptr;
-    h->pf_rowscale = h->pf_srowscale = h->pf_logits = nullptr;
-    h->pf_hist = nullptr; h->pf_work2 = h->pf_work3 = nullptr; h->pf_counter = nullptr;
+    cudaFree(h->pf_slab);
+    h->pf_slab = nullptr;
+    h->pf_counter = nullptr;        // "not there"
 }
 
 int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
@@ -765,20 +786,20 @@ int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
     }
     const auto &c = h->cfg;
     const size_t T = c.max_tokens, P = T * c.top_k;
-    auto alloc = [&](auto **ptr, size_t bytes) { return cudaMalloc(reinterpret_cast<void **>(ptr), bytes ? bytes : 16) == cudaSuccess; };
     const size_t dx = c.d + bp_extra_cols(c.d, 1), fx = c.f + bp_extra_cols(c.f, 2), sfx = c.shared_f + bp_extra_cols(c.shared_f, 2);
     const bool two_orders = c.shared_f != 0 && c.shared_bits != c.routed_bits;
     const size_t logit_rows = std::min<size_t>(4 * T, std::max<size_t>(T, (size_t)h->sm_count * kRouterTileTokens));
     const size_t blocks = std::max(bp_route_blocks(c.max_tokens), bp_route_blocks(std::min(c.max_tokens, 1024u)));
+    Slab slab;
+    slab.want(&h->pf_x, T * dx * 2); slab.want(&h->pf_xs, two_orders ? T * dx * 2 : 0);
     // (the columns behind the sums are never written: they stay the zeros put there now)
-    const bool ok = alloc(&h->pf_x, T * dx * 2) && (!two_orders || alloc(&h->pf_xs, T * dx * 2)) && alloc(&h->pf_acts16, P * fx * 2) &&
-                    alloc(&h->pf_sacts16, T * sfx * 2) && alloc(&h->pf_rowscale, P * 4) && alloc(&h->pf_srowscale, T * 4) &&
-                    alloc(&h->pf_logits, logit_rows * c.num_experts * 4) && alloc(&h->pf_hist, blocks * kMaxExperts * 4) &&
-                    alloc(&h->pf_work2, (size_t)h->max_work * sizeof(WorkItem)) && alloc(&h->pf_work3, (size_t)h->max_work * sizeof(WorkItem)) && alloc(&h->pf_counter, 16) &&
-                    cudaMemsetAsync(h->pf_acts16, 0, P * fx * 2, st) == cudaSuccess &&
-                    cudaMemsetAsync(h->pf_sacts16, 0, std::max<size_t>(T * sfx * 2, 16), st) == cudaSuccess &&
-                    cudaMemsetAsync(h->pf_counter, 1, 16, st) == cudaSuccess &&          // word 3 stays non-zero (EgParams::shared_on)
-                    cudaMemsetAsync(h->pf_counter, 0, 4, st) == cudaSuccess;
+    slab.want(&h->pf_acts16, P * fx * 2, true); slab.want(&h->pf_sacts16, std::max<size_t>(T * sfx * 2, 16), true);
+    slab.want(&h->pf_rowscale, P * 4); slab.want(&h->pf_srowscale, T * 4);
+    slab.want(&h->pf_logits, logit_rows * c.num_experts * 4); slab.want(&h->pf_hist, blocks * kMaxExperts * 4);
+    slab.want(&h->pf_work2, (size_t)h->max_work * sizeof(WorkItem)); slab.want(&h->pf_work3, (size_t)h->max_work * sizeof(WorkItem));
+    slab.want(&h->pf_counter, 16, true);
+    const bool ok = slab.make(h->pf_slab, st) == cudaSuccess &&
+                    cudaMemsetAsync(h->pf_counter + 3, 1, 4, st) == cudaSuccess;        // stays non-zero (EgParams::shared_on)
     int rc = ok ? NVMAI_CUDA_OK : NVMAI_CUDA_ENOMEM;
     if (!rc) rc = make_rows_tmap(h, &h->map_acts, h->pf_acts16, P, fx, 16);
     if (!rc) rc = c.shared_f ? make_rows_tmap(h, &h->map_sacts, h->pf_sacts16, T, sfx, 16) : (h->map_sacts = h->map_acts, NVMAI_CUDA_OK);
