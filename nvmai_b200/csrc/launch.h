@@ -21,7 +21,7 @@ inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
     const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kern));
     auto it = granted.find(key);
     if (it != granted.end() && it->second >= bytes) return cudaSuccess;
-    if (bytes > 48 * 1024) {
+    if (bytes > 40 * 1024) {        // the default limit counts the kernel's static shared memory too
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return e;
     }

@@ -103,3 +103,39 @@ def test_calls_split_between_the_two_kernels_match_the_oracle(bits, meta, out, l
         xr = np.ascontiguousarray(x[t])
         want = gu.oracle_decode(L, cfg, xr)[2] if entry == "decode" else gu.oracle_prefill_row(L, cfg, xr, None)[2]
         assert orc.rel_error(got[t], want) < (3e-3 if f16 else 1.5e-3), f"row {t}"
+
+
+# A stack of several rows as one graph: 3 rows the staged kernels, 4 and more the batched experts' with the norm of the
+# next layer's rows in the reduction; 2304: a row longer than that norm takes, 8: the most rows the route log keeps.
+@pytest.mark.parametrize("rows,bits,out,d,f,experts", [(3, 4, fmt.OUT_FP32, 512, 256, 64), (4, 8, fmt.OUT_FP32, 256, 128, 128),
+                                                       (8, 4, fmt.OUT_FP16, 2048, 512, 256), (9, 4, fmt.OUT_FP32, 2304, 128, 32)])
+def test_stack_of_rows_equals_its_layers_one_by_one(rows, bits, out, d, f, experts):
+    layers = 3
+    torch = gu.torch_cuda()
+    cfg = MoEConfig(d=d, f=f, shared_f=f, num_experts=experts, top_k=8, routed_bits=bits, shared_bits=bits, meta_dtype=BF16,
+                    out_dtype=out, max_tokens=rows, num_layers=layers)
+    moe = MoE(cfg)
+    keep = [synthetic.device_layer(90 + 3 * l + bits, d=d, f=f, shared_f=f, num_experts=experts, routed_bits=bits, shared_bits=bits,
+                                   meta=BF16) for l in range(layers)]
+    for l, dev in enumerate(keep):
+        synthetic.register_device_layer(moe, l, dev)
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        x0 = torch.randn((rows, d), device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).half()
+        kind = torch.float16 if out == fmt.OUT_FP16 else torch.float32
+        y, again, y1 = (torch.zeros((rows, d), dtype=kind, device="cuda") for _ in range(3))
+        idx = torch.empty((rows, 8), dtype=torch.int32, device="cuda")
+        moe.stack_decode(x0, rows, y, stream=st)
+        moe.stack_decode(x0, rows, again, stream=st)
+        moe.synchronize(st)
+        log = moe.read_route_log_rows(rows) if rows <= 8 else None
+        x = x0
+        for l in range(layers):
+            moe.layer_decode(l, x, rows, h2_out=y1, out_idx=idx, stream=st)
+            moe.synchronize(st)
+            if log is not None:
+                np.testing.assert_array_equal(log[l].astype(np.int64), idx.cpu().numpy())
+            v = y1.float()
+            x = (v * torch.rsqrt((v * v).mean(dim=1, keepdim=True) + 1e-6)).half()
+    assert torch.equal(y, again) and bool(torch.isfinite(y).all())
+    assert float((y.float() - y1.float()).norm() / y1.float().norm()) < 3e-3
