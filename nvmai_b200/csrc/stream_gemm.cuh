@@ -10,7 +10,7 @@
 // One block per SM, 16 compute warps and one that issues the copies.  A unit = an item (an expert, up to 8 * NB of its
 // rows as tensor-core columns) x 64 or 128 features (phase 0: gate and up rows of each) or 256 rows of the down
 // projection (phase 1); a block takes consecutive units, so the rows of an item are staged once for several of them.
-// The codes come as boxes of 64 rows x 128 bytes, 32 KB a stage, three to five stages in flight.  KS = 2: two warps
+// The codes come as boxes of 64 rows x 128 bytes, 32 KB a stage, as many stages (two to six) as the shared memory holds.  KS = 2: two warps
 // share a tile, each half of K, so that a unit is small enough to balance over the chip.
 #pragma once
 
@@ -360,14 +360,20 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
                 }
             }
             if (!ok) break;
-            // the unit's scales, and with its last unit the item's rows, are done with
+            // with its last unit the item's rows are done with
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&bars->m_empty[mb]);
-                if (u + 1u == u1 || next.item != item) mbar_arrive(&bars->x_empty);
-            }
-            if ((mb ^= 1u) == 0u) m_ph ^= 1u;
+            if (lane == 0 && (u + 1u == u1 || next.item != item)) mbar_arrive(&bars->x_empty);
+            // The unit's scales too, but with KS = 2 only once the hand-over below has been read: the scales of the unit
+            // after the next come when every warp has released these, and the first half's warp needs them before it
+            // writes this hand-over slot again.  (The ring of codes would hold that warp back as well, but only while its
+            // stages are fewer than two units'.)
+            auto scales_done = [&]() {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->m_empty[mb]);
+                if ((mb ^= 1u) == 0u) m_ph ^= 1u;
+            };
+            if (KS == 1u) scales_done();
             if (PHASE == 0) {
                 bool mine = true;
                 if (FAST) {
@@ -391,6 +397,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
                             for (int i = 0; i < 4; ++i)
                                 tot[n][i] = (((h[(n * 4 + i) * 32] + part[0][n][i]) + part[1][n][i]) + part[2][n][i]) + part[3][n][i];
                     }
+                    scales_done();
                     ++turn;
                 }
                 if (mine) {
