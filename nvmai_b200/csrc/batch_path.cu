@@ -72,11 +72,17 @@ cudaError_t eg_launch(int phase, uint32_t bits, uint32_t meta, uint32_t out_dtyp
     return with_out(integral_constant<int, 8>{});
 }
 
-static bool sg_fast(int phase, uint32_t kdim) { return kdim == (phase == 0 ? 2048u : 512u); }
+// Are the parts of a row (an eighth of its groups in gate/up, a half in down) one quad of groups each (1), several whole
+// quads (2) or neither (0)?  At 4096 inputs the unit of 128 features that 0 takes leaves no room for its scales: 5 rows of
+// 4096 / 1024, 8-bit, took 307 us through the tcgen05 kernel and 252 as separate rows; in units of 64 features 142.
+static int sg_quads(int phase, uint32_t kdim) {
+    const uint32_t part = kdim / 64 / (phase == 0 ? 8 : 2);
+    return kdim / 64 % (phase == 0 ? 32 : 8) != 0 ? 0 : part == 4 ? 1 : 2;
+}
 
 size_t sg_plan(SgParams &p, int phase, uint32_t nb, bool wide) {
     const uint32_t groups = p.kdim / 64, cols = 8 * nb;
-    const uint32_t rows = phase == 1 ? 256 : sg_fast(0, p.kdim) ? 64 : 128;        // features or down rows of a unit
+    const uint32_t rows = phase == 1 ? 256 : sg_quads(0, p.kdim) != 0 ? 64 : 128;        // features or down rows of a unit
     if (p.out_cols % rows != 0) return 0;
     p.units_per_item = p.out_cols / rows;
     p.cap = cols;
@@ -98,18 +104,20 @@ size_t sg_plan(SgParams &p, int phase, uint32_t nb, bool wide) {
 cudaError_t sg_launch(int phase, uint32_t bits, uint32_t meta, uint32_t out_dtype, uint32_t nb, const SgArgs &args, uint32_t blocks,
                       size_t smem, cudaStream_t st) {
     using std::integral_constant;
-    const bool fast = sg_fast(phase, args.p.kdim);
+    const int quads = sg_quads(phase, args.p.kdim);
     auto go = [&](auto B, auto M, auto O, auto P, auto N, auto F) {
         return launch_pdl(stream_gemm_kernel<decltype(B)::value, decltype(M)::value, decltype(O)::value, decltype(P)::value, decltype(N)::value,
                                              decltype(F)::value>, dim3(blocks), dim3(kSgThreads + 32), smem, st, true, args);
     };
-    auto with_fast = [&](auto B, auto M, auto O, auto P, auto N) {
-        if (fast) return go(B, M, O, P, N, integral_constant<bool, true>{});
-        return go(B, M, O, P, N, integral_constant<bool, false>{});
+    auto with_quads = [&](auto B, auto M, auto O, auto P, auto N) {
+        if (quads == 0) return go(B, M, O, P, N, integral_constant<int, 0>{});
+        if (quads == 1) return go(B, M, O, P, N, integral_constant<int, 1>{});
+        if constexpr (decltype(P)::value == 0 && decltype(N)::value == 2) return cudaErrorInvalidValue;   // no room for 16 rows (sg_plan)
+        else return go(B, M, O, P, N, integral_constant<int, 2>{});
     };
     auto with_n = [&](auto B, auto M, auto O, auto P) {
-        if (nb == 1) return with_fast(B, M, O, P, integral_constant<int, 1>{});
-        return with_fast(B, M, O, P, integral_constant<int, 2>{});
+        if (nb == 1) return with_quads(B, M, O, P, integral_constant<int, 1>{});
+        return with_quads(B, M, O, P, integral_constant<int, 2>{});
     };
     auto with_p = [&](auto B, auto M, auto O) {
         if (phase == 0) return with_n(B, M, O, integral_constant<int, 0>{});

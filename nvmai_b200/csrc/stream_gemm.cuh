@@ -110,11 +110,14 @@ __device__ __forceinline__ void sg_group(uint32_t code_a, uint32_t code_b, uint3
 }
 
 // BITS, META: codes and scales; OUT: type of the activations; PHASE 0 gate/up, 1 down; NB: column blocks of 8 rows.
-// FAST: the parts of a row are four groups each (2048 inputs in phase 0, where KS = 2 then; 512 in phase 1).
-template <int BITS, int META, int OUT, int PHASE, int NB, bool FAST>
+// QUADS 1, 2: the parts of a row are whole quads of groups (sg_quads: a multiple of 2048 inputs in phase 0, where KS = 2
+// then, of 512 in phase 1), so scales, biases and row sums are read four at a time; 1: a part is one quad, its code
+// without the loop (with it, 4 rows of 2048 / 512 took 49.2 us instead of 48.4, 13 rows 66.2 instead of 64.8); 2: any
+// number of quads; 0: other shapes.
+template <int BITS, int META, int OUT, int PHASE, int NB, int QUADS>
 __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const __grid_constant__ SgArgs args) {
     const SgParams &p = args.p;
-    constexpr uint32_t KS = PHASE == 0 && FAST ? 2u : 1u;
+    constexpr uint32_t KS = PHASE == 0 && QUADS != 0 ? 2u : 1u;
     constexpr uint32_t kChunkGroups = BITS == 4 ? 4u : 2u;        // groups in 128 bytes of a row
     constexpr uint32_t kRows = PHASE == 0 ? 128u / KS : 256u;     // features (phase 0) or down rows of a unit
     constexpr uint32_t kCols = 8u * NB;
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
             if (!ok) break;
             const uint32_t meta = meta0 + mb * p.meta_bytes;
             const uint32_t bias = meta + kMats * meta_bytes;
-            float tot[NB][4] = {}, part[FAST && PHASE == 0 ? 4 : 1][NB][4];
+            float tot[NB][4] = {}, part[QUADS != 0 && PHASE == 0 ? 4 : 1][NB][4];
             float su[NB][2];
 #pragma unroll
             for (int n = 0; n < NB; ++n) {
@@ -297,13 +300,10 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
                 if (lane == 0) mbar_arrive(&bars->empty[s]);
                 if (++s == p.stages) { s = 0; s_ph ^= 1u; }
             };
-            if (FAST) {
+            if (QUADS != 0) {
                 constexpr uint32_t kParts = PHASE == 0 ? 4u : 2u;
-#pragma unroll
-                for (uint32_t q = 0; q < kParts; ++q) {
-                    const uint32_t G0 = (ks * kParts + q) * 4u;
-                    float acc[NB][4] = {};
-                    uint2 sa, sb, ba, bb;                 // the part's scales and biases of both rows
+                auto quad = [&](uint32_t G0, float (&acc)[NB][4]) {
+                    uint2 sa, sb, ba, bb;                 // the quad's scales and biases of both rows
                     sg_lds(sa, meta + m_a + G0 * 2u); sg_lds(sb, meta + m_b + G0 * 2u);
                     sg_lds(ba, bias + m_a + G0 * 2u); sg_lds(bb, bias + m_b + G0 * 2u);
                     float xs[4][NB][2];
@@ -321,6 +321,17 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
                         sg_group<BITS, META, NB>((code_a + at) ^ jx, (code_b + at) ^ jx, x_at + (G0 + j) * 128u, x_block, meta_pick(sa, j),
                                                  meta_pick(sb, j), meta_pick(ba, j), meta_pick(bb, j), xs[j], acc);
                         if (j % kChunkGroups == kChunkGroups - 1u) stage_done();
+                    }
+                };
+                const uint32_t part_groups = groups / (PHASE == 0 ? 8u : 2u);
+#pragma unroll
+                for (uint32_t q = 0; q < kParts; ++q) {
+                    float acc[NB][4] = {};
+                    if constexpr (QUADS == 1) {
+                        quad((ks * kParts + q) * 4u, acc);
+                    } else {
+                        const uint32_t G1 = (ks * kParts + q + 1u) * part_groups;
+                        for (uint32_t G0 = G1 - part_groups; ok && G0 < G1; G0 += 4u) quad(G0, acc);
                     }
                     if (!ok) break;
 #pragma unroll
@@ -376,7 +387,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
             if (KS == 1u) scales_done();
             if (PHASE == 0) {
                 bool mine = true;
-                if (FAST) {
+                if (QUADS != 0) {
                     // the first half's running sum goes to the warp of the second half, which goes on from there
                     float *h = handover + (((turn & 1u) * 8u + tl) * (4u * NB)) * 32u + lane;
                     if (ks == 0u) {

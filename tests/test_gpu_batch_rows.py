@@ -1,0 +1,74 @@
+"""A row of a decode batch has the bits of a call of its own, on the kernels that a call takes by default."""
+import sys
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+for p_ in (ROOT, ROOT / "tests"):
+    if str(p_) not in sys.path:
+        sys.path.insert(0, str(p_))
+
+pytestmark = pytest.mark.gpu
+
+from nvmai_b200 import MoE, MoEConfig, synthetic      # noqa: E402
+from nvmai_b200 import format as fmt                  # noqa: E402
+import gpu_util as gu                                 # noqa: E402
+
+BF16, FP16 = fmt.META_BF16, fmt.META_FP16
+DENSE, AFF8 = fmt.ROUTER_DENSE_F16, fmt.ROUTER_AFFINE8
+
+
+def _layer(seed, cfg):
+    """zero-mean weights on the device; affine router and gate rows where the configuration asks for them"""
+    torch = gu.torch_cuda()
+    dev = synthetic.device_layer(seed, d=cfg.d, f=cfg.f, shared_f=cfg.shared_f, num_experts=cfg.num_experts,
+                                 routed_bits=cfg.routed_bits, shared_bits=cfg.shared_bits, meta=cfg.meta_dtype)
+    gen = torch.Generator(device="cuda").manual_seed(seed + 1)
+    if cfg.router_kind != DENSE:
+        dev["router"] = synthetic._device_affine(torch, gen, cfg.num_experts, cfg.d, cfg.router_kind, cfg.meta_dtype, "cuda")
+    if cfg.shared_f and cfg.shared_gate_kind not in (DENSE, fmt.GATE_NONE):
+        dev["gate"] = synthetic._device_affine(torch, gen, 1, cfg.d, cfg.shared_gate_kind, cfg.meta_dtype, "cuda")
+    return dev
+
+
+def _config(bits, meta, out, rows, d, f, experts, router, **other):
+    kw = dict(d=d, f=f, shared_f=f, num_experts=experts, top_k=8, routed_bits=bits, shared_bits=bits, router_kind=router,
+              shared_gate_kind=router, meta_dtype=meta, out_dtype=out, max_tokens=rows)
+    kw.update(other)
+    return MoEConfig(**kw)
+
+
+def _check_rows_alone(cfg, rows, seed):
+    torch = gu.torch_cuda()
+    moe = MoE(cfg)
+    dev = _layer(seed, cfg)
+    synthetic.register_device_layer(moe, 0, dev)
+    x = torch.randn((rows, cfg.d), device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed)).half()
+    kind = torch.float16 if cfg.out_dtype == fmt.OUT_FP16 else torch.float32
+
+    def call(first, n):
+        h2 = torch.zeros((n, cfg.d), dtype=kind, device="cuda")
+        hidden = torch.full((n, cfg.d), 0.75, dtype=kind, device="cuda")
+        idx = torch.zeros((n, 8), dtype=torch.int32, device="cuda")
+        w = torch.zeros((n, 8), dtype=torch.float16, device="cuda")
+        moe.layer_decode(0, x[first:first + n], n, hidden=hidden, h2_out=h2, out_idx=idx, out_w=w)
+        moe.synchronize()
+        return idx, w, h2, hidden
+
+    batch = call(0, rows)
+    assert bool(torch.isfinite(batch[2]).all())
+    for t in range(rows):
+        for name, all_rows, one in zip(("idx", "w", "h2", "hidden"), batch, call(t, 1)):
+            assert torch.equal(all_rows[t], one[0]), f"row {t}: {name}"
+
+
+# Rows of 4096 values: parts of two quads of groups in both phases of the streaming kernel; 1536: three quads in the down
+# projection.
+@pytest.mark.parametrize("bits,meta,out,rows,d,f", [
+    (4, BF16, fmt.OUT_FP16, 5, 4096, 1024), (8, BF16, fmt.OUT_FP32, 4, 4096, 1024), (8, FP16, fmt.OUT_FP16, 9, 4096, 512),
+    (4, BF16, fmt.OUT_FP32, 13, 2048, 1536), (4, FP16, fmt.OUT_FP32, 6, 2048, 1024)])
+def test_long_rows_equal_calls_of_their_own(bits, meta, out, rows, d, f):
+    cfg = _config(bits, meta, out, rows, d, f, 32, AFF8)
+    _check_rows_alone(cfg, rows, seed=100 + rows)
