@@ -295,10 +295,10 @@ constexpr size_t kMaxSmem = 227 * 1024;
 
 // with_shared: the shared expert's gate/up tiles run here (one block per token and
 // tile); with_gate: the scalar gate row.  The batched path runs the tiles in its
-// grouped stage instead and asks for the gate only.
+// grouped stage instead and asks for the router and the gate (spread_rows; its routing kernel selects: defer_topk).
 int launch_stage1(nvmai_cuda_moe *h, const LayerViews &lv, const XSource &xsrc, uint32_t tokens,
                   uint32_t *out_idx, __half *out_w, bool with_router, bool with_shared, bool with_gate, bool pdl,
-                  cudaStream_t st, bool defer_topk = false) {
+                  cudaStream_t st, bool defer_topk = false, bool spread_rows = false) {
     const auto &c = h->cfg;
     Stage1Params p{};
     p.rW = static_cast<const uint8_t *>(lv.w.router.w);
@@ -325,9 +325,13 @@ int launch_stage1(nvmai_cuda_moe *h, const LayerViews &lv, const XSource &xsrc, 
     p.trace = h->cur_trace;
     p.D = c.d; p.E = c.num_experts; p.K = c.top_k; p.act = c.activation;
     p.status = h->status;
-    p.tokens_per_chunk = tokens <= 8 ? tokens : 8;
-    const uint32_t chunks = (tokens + p.tokens_per_chunk - 1) / p.tokens_per_chunk;
     p.router_row_blocks = (c.num_experts + kRowsPerRouterBlock - 1) / kRowsPerRouterBlock;
+    p.tokens_per_chunk = tokens <= 8 ? tokens : 8;
+    if (spread_rows) {      // fewer rows a block where that still is one wave of blocks
+        const uint32_t wave = std::max(1u, (uint32_t)h->sm_count / p.router_row_blocks);
+        p.tokens_per_chunk = std::min(p.tokens_per_chunk, (tokens + wave - 1) / wave);
+    }
+    const uint32_t chunks = (tokens + p.tokens_per_chunk - 1) / p.tokens_per_chunk;
     p.n_router_blocks = with_router ? p.router_row_blocks * chunks : 0;
     p.n_shared_blocks = with_shared ? ((c.shared_f + kBlockFeatures - 1) / kBlockFeatures) * tokens : 0;
     const bool gated = with_gate && c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE;
@@ -839,11 +843,15 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
                PackXParams px, const uint32_t (&caps)[3], uint32_t heavy, bool routed_only, cudaStream_t st) {
     int rc;
     const bool gated = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE;
-    const bool dense_gate = gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;
+    // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
+    // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
+    // affine routers keep the exact code-times-activation kernel.
+    const bool gemm = !routed_only && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0;
+    const bool gate_here = gemm && gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;      // else stage 1 has the gate
     px.x = x; px.rows = tokens; px.n = c.d;
-    px.gate_row = dense_gate ? static_cast<const __half *>(lv.w.shared_gate.w) : nullptr;
+    px.gate_row = gate_here ? static_cast<const __half *>(lv.w.shared_gate.w) : nullptr;
     px.gate_val = h->gate_val; px.out_half = c.out_dtype == NVMAI_OUT_FP32 ? 0 : 1;
-    if ((px.dst != nullptr || dense_gate || !routed_only) && (rc = launched(h, bp_pack_x(px, st)))) return rc;
+    if ((px.dst != nullptr || gemm) && (rc = launched(h, bp_pack_x(px, st)))) return rc;       // (the GEMM starts beside this one)
 
     RouteParams r{};
     r.pes = static_cast<const uint16_t *>(lv.w.per_expert_scale);
@@ -856,11 +864,8 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
     // A quarter of the pairs pays for the grouped launches.  A rank's share of the routed sum splits by the expert's rows
     // alone: every rank, and a handle with all experts, then takes the same kernel for an expert.
     r.heavy = heavy; r.heavy_min = routed_only ? 0 : tokens * c.top_k / 4; r.shared_on = h->pf_counter + 1;
-    // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
-    // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
-    // affine routers keep the exact code-times-activation kernel.
     const XSource xsrc{x, c.d, nullptr, nullptr};
-    if (!routed_only && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0) {
+    if (gemm) {
         RouterArgs ra{};
         ra.w = lv.router;
         if ((rc = make_rows_tmap(h, &ra.x, x, tokens, c.d, kRouterTileTokens))) return rc;
@@ -868,9 +873,13 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
         r.logits = h->pf_logits;
         ra.p = RouterParams{h->pf_logits, tokens, c.num_experts, c.d, r.splits, h->status};
         if ((rc = launched(h, bp_router(ra, st)))) return rc;
-        if (gated && !dense_gate && (rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, false, false, true, false, st))) return rc;
+        if (gated && !gate_here && (rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, false, false, true, false, st))) return rc;
     } else if (!routed_only) {
-        if ((rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, false, gated && !dense_gate, false, st))) return rc;
+        // (top-k in the routing kernel: left to this one's last block of every eight rows, and after the packing instead of
+        // beside what came before, four rows of an 8-bit router took 57.7 us for the block, 47.1 as separate rows)
+        r.splits = 1;
+        r.logits = h->logits;
+        if ((rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, true, false, gated, true, st, true, true))) return rc;
     }
     return launched(h, bp_route(r, st), bp_route_launches(tokens));
 }

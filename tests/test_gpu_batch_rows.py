@@ -72,3 +72,13 @@ def _check_rows_alone(cfg, rows, seed):
 def test_long_rows_equal_calls_of_their_own(bits, meta, out, rows, d, f):
     cfg = _config(bits, meta, out, rows, d, f, 32, AFF8)
     _check_rows_alone(cfg, rows, seed=100 + rows)
+
+
+# Affine routers (what a repacked artifact has): the routing kernel selects from the logits of the rows' blocks.  4 rows: a
+# block's rows are spread over four; 9: an odd number a block; 31: the most rows.  1: no batched kernels at all.
+@pytest.mark.parametrize("bits,meta,out,rows,router", [
+    (4, BF16, fmt.OUT_FP16, 1, AFF8), (4, BF16, fmt.OUT_FP16, 4, AFF8), (8, FP16, fmt.OUT_FP32, 9, fmt.ROUTER_AFFINE4),
+    (4, FP16, fmt.OUT_FP16, 31, AFF8)])
+def test_rows_of_an_affine_router_equal_calls_of_their_own(bits, meta, out, rows, router):
+    cfg = _config(bits, meta, out, rows, 512, 256, 256, router)
+    _check_rows_alone(cfg, rows, seed=200 + rows)
