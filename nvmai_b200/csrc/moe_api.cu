@@ -338,10 +338,12 @@ int launch_stage1(nvmai_cuda_moe *h, const LayerViews &lv, const XSource &xsrc, 
     p.n_gate_blocks = gated ? chunks : 0;
     const uint32_t grid = p.n_router_blocks + p.n_shared_blocks + p.n_gate_blocks;
     if (grid == 0) return NVMAI_CUDA_OK;
+    p.x_rows = spread_rows ? p.tokens_per_chunk : 1;
+    if (std::max(RowsLayout(c.d, c.router_kind, p.x_rows).total, gated ? RowsLayout(c.d, c.shared_gate_kind, p.x_rows).total : 0) > kMaxSmem) p.x_rows = 1;
     size_t smem = 0;
-    if (with_router) smem = std::max(smem, RowsLayout(c.d, c.router_kind).total);
+    if (with_router) smem = std::max(smem, RowsLayout(c.d, c.router_kind, p.x_rows).total);
     if (with_router && !defer_topk) smem = std::max(smem, kTopkSmemBytes);      // the last router block selects in place
-    if (gated) smem = std::max(smem, RowsLayout(c.d, c.shared_gate_kind).total);
+    if (gated) smem = std::max(smem, RowsLayout(c.d, c.shared_gate_kind, p.x_rows).total);
     if (with_shared) smem = std::max(smem, GateUpLayout(c.d, c.shared_bits).total);
     return dispatch_bits_meta(c.shared_f ? c.shared_bits : 4, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
@@ -829,6 +831,7 @@ bool tc_shape_ok(const nvmai_cuda_moe *h, bool with_shared) {
 //   decode_order  the block's result takes the decode path's rounding (one rounding of h1 + sum, one residual add)
 //   routed_only   routing given by the caller (out_idx / out_w are inputs), no router, no shared expert
 //   partial_y     fp32 rows that receive sum_r w_r * down_r instead of y / hidden (expert-parallel share, replay)
+constexpr uint32_t kExactRows = 32;      // decode calls of fewer rows give every row the bits of a call of its own
 struct PrefillMode {
     bool decode_order = false;
     bool routed_only = false;
@@ -840,13 +843,15 @@ struct PrefillMode {
 // What comes before the experts' GEMMs: the rows packed (px says how; without dst only the scalar gate is taken), the
 // router, top-k and the pairs grouped by expert.  c: the handle's configuration, shared_f = 0 for routed rows only.
 int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c, const __half *x, uint32_t tokens, uint32_t *idx, __half *w,
-               PackXParams px, const uint32_t (&caps)[3], uint32_t heavy, bool routed_only, cudaStream_t st) {
+               PackXParams px, const uint32_t (&caps)[3], uint32_t heavy, const PrefillMode &mode, cudaStream_t st) {
+    const bool routed_only = mode.routed_only;
     int rc;
     const bool gated = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE;
     // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
     // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
-    // affine routers keep the exact code-times-activation kernel.
-    const bool gemm = !routed_only && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0;
+    // affine routers keep the exact code-times-activation kernel, and so do decode calls of a few rows (4-bit block with the
+    // GEMM / this kernel: 4 rows 41.3 / 38.6 us, 13 rows 64.4 / 65.4, 31 rows 94.7 / 97.7).
+    const bool gemm = !routed_only && !(mode.decode_order && tokens < kExactRows) && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0;
     const bool gate_here = gemm && gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;      // else stage 1 has the gate
     px.x = x; px.rows = tokens; px.n = c.d;
     px.gate_row = gate_here ? static_cast<const __half *>(lv.w.shared_gate.w) : nullptr;
@@ -887,19 +892,22 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
 // Batches that bring few rows per expert (stream_gemm.cuh); the modes as in layer_prefill_impl.  Column blocks of an
 // item: 8 rows up to 9 per expert (evenly routed), else 16.  Measured, 8-bit layer: 256 rows 238 us in blocks of 8,
 // 251 us in blocks of 16; 400 rows 332 / 289 us.
-uint32_t stream_blocks(const nvmai_cuda_moe *h, uint32_t tokens) { return tokens * h->cfg.top_k <= 9 * h->cfg.num_experts ? 1 : 2; }
-
-bool stream_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared) {
+// (16 rows of 4096 values leave no room for the codes: blocks of 8 then too.)
+bool stream_fits(const nvmai_cuda_moe *h, uint32_t nb, bool with_shared) {
     const auto &c = h->cfg;
-    if (!tc_shape_ok(h, with_shared) || c.top_k > (uint32_t)kMaxTopK) return false;
     const bool wide = c.out_dtype == NVMAI_OUT_FP32;
-    const uint32_t nb = stream_blocks(h, tokens);
     auto fits = [&](int phase, uint32_t kdim, uint32_t cols) {
         SgParams p{};
         p.kdim = kdim; p.out_cols = cols;
         return sg_plan(p, phase, nb, wide) != 0;
     };
     return fits(0, c.d, c.f) && fits(1, c.f, c.d) && (!with_shared || c.shared_f == 0 || (fits(0, c.d, c.shared_f) && fits(1, c.shared_f, c.d)));
+}
+uint32_t stream_blocks(const nvmai_cuda_moe *h, uint32_t tokens) {
+    return tokens * h->cfg.top_k <= 9 * h->cfg.num_experts || !stream_fits(h, 2, true) ? 1 : 2;
+}
+bool stream_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared) {
+    return tc_shape_ok(h, with_shared) && h->cfg.top_k <= (uint32_t)kMaxTopK && stream_fits(h, stream_blocks(h, tokens), with_shared);
 }
 
 // Which experts of a batched call the streaming kernel has: those with up to `heavy` rows (>= the call's rows: all, 0: none).
@@ -912,6 +920,7 @@ struct ExpertSplit { uint32_t heavy; };
 ExpertSplit expert_split(const nvmai_cuda_moe *h, uint32_t tokens, const PrefillMode &mode) {
     if (!stream_ok(h, tokens, !mode.routed_only)) return {0};
     if (h->stream_max_rows != ~0u) return {h->stream_max_rows};
+    if (mode.decode_order && tokens < kExactRows) return {~0u};      // the bits of the single-row stages
     const auto &c = h->cfg;
     const uint64_t passes = (c.routed_bits / 4) * (mode.decode_order && c.meta_dtype == NVMAI_META_FP16 ? 2 : 1);
     const uint64_t P = (uint64_t)tokens * c.top_k, E = c.num_experts;
@@ -967,7 +976,7 @@ int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32
     uint32_t *idx = out_idx ? out_idx : h->idx;
     __half *w = out_w ? out_w : h->w;
     const uint32_t cap = 8 * stream_blocks(h, tokens), caps[3] = {cap, cap, cap};
-    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, PackXParams{}, caps, ~0u, mode.routed_only, st))) return rc;
+    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, PackXParams{}, caps, ~0u, mode, st))) return rc;
     for (int phase = 0; phase < 2; ++phase)
         if ((rc = stream_phase(h, lv, c, phase, x, tokens, false, st))) return rc;
     CombineRowsParams pc{};
@@ -1015,7 +1024,7 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     PackXParams px{};
     px.dst = h->pf_x; px.dst2 = two_orders ? h->pf_xs : nullptr; px.permute = c.routed_bits == 4 ? 1 : 0;
     const uint32_t caps[3] = {plan0.cap, plan1.cap, 8 * stream_blocks(h, tokens)};
-    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, px, caps, mixed ? heavy : 0, mode.routed_only, st))) return rc;
+    if ((rc = route_rows(h, lv, c, x, tokens, idx, w, px, caps, mixed ? heavy : 0, mode, st))) return rc;
 
     const uint32_t shared_rows = merged ? tokens : 0;
     auto set_common = [&](EgParams &g, const EgPlan &plan) {
@@ -1124,6 +1133,8 @@ bool tc_batch_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared, cud
         if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
     }
     if (c.top_k > (uint32_t)kMaxTopK) return false;
+    // few rows: only where the streaming kernel takes them (it has the bits of the per-row kernels)
+    if (tokens < kExactRows && h->stream_max_rows == ~0u && !stream_ok(h, tokens, with_shared)) return false;
     return tc_shape_ok(h, with_shared);
 }
 

@@ -2,7 +2,6 @@
 import sys
 from pathlib import Path
 
-import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -82,3 +81,16 @@ def test_long_rows_equal_calls_of_their_own(bits, meta, out, rows, d, f):
 def test_rows_of_an_affine_router_equal_calls_of_their_own(bits, meta, out, rows, router):
     cfg = _config(bits, meta, out, rows, 512, 256, 256, router)
     _check_rows_alone(cfg, rows, seed=200 + rows)
+
+
+# Dense routers: up to 31 rows the single-row router's order of additions and the streaming kernel, also where few experts
+# hold the rows (8 experts: 31 rows each); a shape of the streaming kernel's (2048 / 512) and others; no shared expert; a
+# shared expert of its own bit width.
+@pytest.mark.parametrize("bits,meta,out,rows,d,f,experts,other", [
+    (4, BF16, fmt.OUT_FP32, 4, 2048, 512, 256, {}), (8, BF16, fmt.OUT_FP16, 9, 2048, 512, 64, {}),
+    (4, FP16, fmt.OUT_FP16, 31, 2048, 512, 256, {}), (4, BF16, fmt.OUT_FP32, 31, 512, 128, 8, {}),
+    (8, FP16, fmt.OUT_FP32, 13, 768, 384, 128, {}), (4, BF16, fmt.OUT_FP16, 7, 256, 128, 128, {"shared_f": 0}),
+    (4, BF16, fmt.OUT_FP32, 11, 512, 256, 128, {"shared_bits": 8, "shared_f": 128}), (4, BF16, fmt.OUT_FP16, 20, 4096, 512, 16, {})])
+def test_rows_of_a_dense_router_equal_calls_of_their_own(bits, meta, out, rows, d, f, experts, other):
+    cfg = _config(bits, meta, out, rows, d, f, experts, DENSE, **other)
+    _check_rows_alone(cfg, rows, seed=300 + rows)
