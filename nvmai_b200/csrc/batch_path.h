@@ -98,12 +98,13 @@ cudaError_t bp_pack_x(const PackXParams &p, cudaStream_t st);
 struct RouterParams { float *logits; uint32_t tokens, experts, kdim, splits; unsigned int *status; };
 struct alignas(64) RouterArgs { CUtensorMap w, x; RouterParams p; };
 constexpr uint32_t kRouterTileTokens = 64;
+constexpr uint32_t kRouterParts = 4;      // sums over K that the logits add up from; splits: 1, 2 or 4 of them a block
 cudaError_t bp_router(const RouterArgs &args, cudaStream_t st);
 
 // top-k of every row (or the given experts), histograms per block, and in the last block the scan: offsets per expert,
 // first positions per block, the GEMMs' work lists
 struct RouteParams {
-    const float *logits; uint32_t splits;     // nullptr: idx is given
+    const float *logits; uint32_t splits;     // nullptr: idx is given; splits <= kRouterParts
     const uint16_t *pes;
     uint32_t *idx; __half *w;
     uint32_t tokens, E, K;

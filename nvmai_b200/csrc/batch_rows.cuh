@@ -82,7 +82,9 @@ __global__ void __launch_bounds__(256) pack_x_kernel(PackXParams p) {
 // ---- dense router ---------------------------------------------------------------------------
 // logits[split][token][expert]: 128 router rows x 64 token rows per block, K split over blockIdx.z so that a small
 // batch still spreads over the chip (one block per 256 tokens took 20-29 us at any batch size).  Products of two fp16
-// values are exact in fp32: only the order of the additions differs from the decode router's.
+// values are exact in fp32: only the order of the additions differs from the decode router's.  That order is the same
+// for any number of splits, so a row's logits do not depend on the rows beside it: K always adds up in four quarters,
+// (q0 + q1) + (q2 + q3), a block keeping each of its quarters in an accumulator of its own.
 constexpr uint32_t kRouterStages = 4;
 constexpr uint32_t kRouterStageBytes = 128 * 128 + kRouterTileTokens * 128;
 constexpr size_t kRouterSmem = 2048 + kRouterStages * kRouterStageBytes;
@@ -100,13 +102,14 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
         mbar_init(&bars->done, 1);
         mbar_fence_init();
     }
-    if (warp == 1) { tmem_alloc(&bars->tmem_slot, kRouterTileTokens); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(&bars->tmem_slot, kRouterParts * kRouterTileTokens); tmem_relinquish(); }      // (two blocks per SM)
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&bars->tmem_slot);
     // x was complete before the kernel in front of this one (which packs it) could pass its own wait
     const uint32_t n_kb = p.kdim / 64u / p.splits, kb0 = blockIdx.z * n_kb;
+    const uint32_t quarters = kRouterParts / p.splits, quarter_kb = p.kdim / 64u / kRouterParts;      // this block's
     const uint32_t e0 = blockIdx.x * 128u, t0 = blockIdx.y * kRouterTileTokens;
     bool ok = *reinterpret_cast<volatile unsigned int *>(p.status) == 0u;
     ok = __syncthreads_and(ok);
@@ -125,6 +128,7 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
     } else if (warp == 1) {
         if (elect_one()) {
             const uint32_t idesc = umma_idesc_f16(128u, kRouterTileTokens);
+            uint32_t acc = tmem, in_quarter = 0;
             for (uint32_t k = 0; k < n_kb && ok; ++k) {
                 const uint32_t s = k % kRouterStages, st = ring + s * kRouterStageBytes;
                 ok = mbar_wait(&bars->full[s], (k / kRouterStages) & 1u, p.status);
@@ -132,8 +136,9 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
                 tc_fence_after_sync();
                 const uint64_t da = umma_desc_sw128(st), db = umma_desc_sw128(st + 128u * 128u);
 #pragma unroll
-                for (uint32_t j = 0; j < 4u; ++j) umma_f16_ss(tmem, da + 2u * j, db + 2u * j, idesc, (k | j) != 0u);
+                for (uint32_t j = 0; j < 4u; ++j) umma_f16_ss(acc, da + 2u * j, db + 2u * j, idesc, (in_quarter | j) != 0u);
                 umma_commit(&bars->empty[s]);
+                if (++in_quarter == quarter_kb) { in_quarter = 0; acc += kRouterTileTokens; }
             }
             if (ok) umma_commit(&bars->done);
         }
@@ -145,17 +150,29 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
         tc_fence_after_sync();
         float *out = p.logits + ((size_t)blockIdx.z * p.tokens + t0) * p.experts + e0 + warp * 32u + lane;
         for (uint32_t cb = 0; cb < kRouterTileTokens && t0 + cb < p.tokens; cb += 8u) {
-            uint32_t r[8];
-            tmem_ld8(tmem + ((warp * 32u) << 16) + cb, r);
-            tmem_ld_wait();
+            float v[8];
+            auto load = [&](uint32_t q, float (&o)[8]) {
+                uint32_t r[8];
+                tmem_ld8(tmem + ((warp * 32u) << 16) + q * kRouterTileTokens + cb, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[i]);
+            };
+            auto add = [&](float (&a)[8], const float (&b)[8]) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a[i] += b[i];
+            };
+            load(0u, v);
+            if (quarters >= 2u) { float q1[8]; load(1u, q1); add(v, q1); }
+            if (quarters == 4u) { float q2[8], q3[8]; load(2u, q2); load(3u, q3); add(q2, q3); add(v, q2); }
 #pragma unroll
             for (uint32_t i = 0; i < 8u; ++i)
-                if (t0 + cb + i < p.tokens) out[(size_t)(cb + i) * p.experts] = __uint_as_float(r[i]);
+                if (t0 + cb + i < p.tokens) out[(size_t)(cb + i) * p.experts] = v[i];
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, kRouterTileTokens);
+    if (warp == 1) tmem_dealloc(tmem, kRouterParts * kRouterTileTokens);
     pdl_wait();                     // the kernel after this one relies on the one before it being complete
     pdl_launch_dependents();
 }
@@ -192,23 +209,20 @@ __device__ __forceinline__ uint32_t heavy_limit(const RouteParams &p, uint32_t r
     return many ? p.heavy : ~0u;
 }
 
-// v[i] = logit of expert lane + 32 i: the splits added in order, up to 32 loads in flight
+// v[i] = logit of expert lane + 32 i: the splits of K added as (s0 + s1) + (s2 + s3), all 32 loads in flight
 __device__ __forceinline__ void add_splits(float (&v)[kMaxExperts / 32], const RouteParams &p, uint32_t tok, uint32_t lane) {
-    for (uint32_t sp = 0; sp < p.splits; sp += 4u) {
-        float a[4][kMaxExperts / 32];
+    static_assert(kRouterParts == 4, "the sum has four terms");
+    float a[4][kMaxExperts / 32];
 #pragma unroll
-        for (uint32_t k = 0; k < 4u; ++k)
+    for (uint32_t k = 0; k < 4u; ++k)
 #pragma unroll
-            for (int i = 0; i < kMaxExperts / 32; ++i) {
-                const uint32_t e = lane + 32u * i;
-                a[k][i] = e < p.E && sp + k < p.splits ? __ldcg(p.logits + ((size_t)(sp + k) * p.tokens + tok) * p.E + e) : 0.0f;
-            }
+        for (int i = 0; i < kMaxExperts / 32; ++i) {
+            const uint32_t e = lane + 32u * i;
+            a[k][i] = e < p.E && k < p.splits ? __ldcg(p.logits + ((size_t)k * p.tokens + tok) * p.E + e) : 0.0f;
+        }
 #pragma unroll
-        for (uint32_t k = 0; k < 4u; ++k)
-#pragma unroll
-            for (int i = 0; i < kMaxExperts / 32; ++i)
-                if (sp + k < p.splits) v[i] += a[k][i];
-    }
+    for (int i = 0; i < kMaxExperts / 32; ++i)
+        if (lane + 32u * i < p.E) v[i] = (a[0][i] + a[1][i]) + (a[2][i] + a[3][i]);
 }
 
 // Router semantics of router_topk_select_k8 (moe.metal:233-285); the pairs end up in (expert, token, rank) order, as

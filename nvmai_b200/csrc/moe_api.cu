@@ -704,13 +704,13 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
 }
 
 // ---- prefill: grouped GEMMs on the tensor cores ----------------------------------
-// Splits of the router's K over blocks: up to four, while they fill the chip once (the top-k reads every split: with
+// Splits of the router's K over blocks: up to four, while they fill the chip once (the top-k adds the splits: with
 // sixteen it took 10 us for 13 rows, most of it one SM reading partial logits).
 uint32_t router_splits(const nvmai_cuda_moe *h, uint32_t tokens) {
     const auto &c = h->cfg;
     const uint32_t tiles = (c.num_experts / 128) * ((tokens + kRouterTileTokens - 1) / kRouterTileTokens);
     uint32_t s = 1;
-    while (s < 4 && 2 * s * tiles <= (uint32_t)h->sm_count && (c.d / 64) % (2 * s) == 0) s *= 2;
+    while (s < kRouterParts && 2 * s * tiles <= (uint32_t)h->sm_count) s *= 2;      // (d is a multiple of 256: tc_shape_ok)
     return s;
 }
 

@@ -94,3 +94,29 @@ def test_rows_of_an_affine_router_equal_calls_of_their_own(bits, meta, out, rows
 def test_rows_of_a_dense_router_equal_calls_of_their_own(bits, meta, out, rows, d, f, experts, other):
     cfg = _config(bits, meta, out, rows, d, f, experts, DENSE, **other)
     _check_rows_alone(cfg, rows, seed=300 + rows)
+
+
+# From 32 rows on the dense router is a GEMM whose K is split over four, two or one block by the number of rows (32 to 1152,
+# to 2368 and more, at 256 experts on 148 SMs): the logits, and so the routing, are the same for any number.
+@pytest.mark.parametrize("d", [256, 1280])
+def test_routing_of_a_row_does_not_depend_on_the_rows_beside_it(d):
+    torch = gu.torch_cuda()
+    most = 2500
+    cfg = _config(4, BF16, fmt.OUT_FP16, most, d, 128, 256, DENSE)
+    moe = MoE(cfg)
+    dev = _layer(17, cfg)
+    synthetic.register_device_layer(moe, 0, dev)
+    x = torch.randn((most, d), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).half()
+
+    def routing(rows):
+        idx = torch.zeros((rows, 8), dtype=torch.int32, device="cuda")
+        w = torch.zeros((rows, 8), dtype=torch.float16, device="cuda")
+        y = torch.zeros((rows, d), dtype=torch.float16, device="cuda")
+        moe.layer_prefill(0, x, rows, y_out=y, out_idx=idx, out_w=w)
+        moe.synchronize()
+        return idx, w
+
+    idx, w = routing(most)
+    for rows in (40, 1100, 1500):
+        some_idx, some_w = routing(rows)
+        assert torch.equal(some_idx, idx[:rows]) and torch.equal(some_w, w[:rows]), rows
