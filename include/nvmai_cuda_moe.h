@@ -390,6 +390,10 @@ NVMAI_API int nvmai_cuda_moe_debug_drop_prefill_copy(nvmai_cuda_moe *h);
  * device stays idle), so that a test can watch a host-side wait run out. */
 NVMAI_API int nvmai_cuda_moe_debug_host_delay(nvmai_cuda_moe *h, void *stream, uint32_t ms);
 
+/* Test hook: how many CUDA graphs of stack steps the handle holds (one per row count and kind
+ * of launches, at most 32; none is kept by the address of a buffer). */
+NVMAI_API int nvmai_cuda_moe_debug_stack_graphs(const nvmai_cuda_moe *h, uint32_t *out_count);
+
 /* Test hook for the failure path of the resident kernel: block `block` keeps its phase-1
  * results (router logits, shared-expert activations or the gate value) to itself, so that
  * every other block's bounded wait for them runs out and the step ends with

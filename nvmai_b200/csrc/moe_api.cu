@@ -71,12 +71,15 @@ struct Slab {
     }
 };
 
-struct StackGraphKey {
-    const void *x0; void *y; uint32_t tokens; cudaStream_t stream; bool batched, logged;
-    bool operator<(const StackGraphKey &o) const {
-        return std::tie(x0, y, tokens, stream, batched, logged) < std::tie(o.x0, o.y, o.tokens, o.stream, o.batched, o.logged);
-    }
+struct EpGraphKey {
+    const void *x0; void *y; uint32_t tokens; cudaStream_t stream;
+    bool operator<(const EpGraphKey &o) const { return std::tie(x0, y, tokens, stream) < std::tie(o.x0, o.y, o.tokens, o.stream); }
 };
+// The inner layers of a stack step as a graph, by what its launches depend on: rows, the batched kernels or the staged
+// ones, route log or not.
+using StackGraphKey = std::tuple<uint32_t, bool, bool>;
+constexpr size_t kMaxStackGraphs = 32;
+constexpr uint32_t kMinGraphLayers = 8;
 
 struct nvmai_cuda_moe {
     nvmai_cuda_moe_config cfg{};
@@ -161,7 +164,7 @@ struct nvmai_cuda_moe {
                                                 // [2 ..] this rank's block counters per layer
     size_t ep_buf_elems = 0;
     struct EpGraph { cudaGraphExec_t exec = nullptr; uint32_t calls = 0; };
-    std::map<StackGraphKey, EpGraph> ep_graphs;
+    std::map<EpGraphKey, EpGraph> ep_graphs;
     // one-launch decode step (persistent_decode.cuh): per-layer views on the device, the tagged exchange words,
     // the epoch word and the experts each layer selected
     PdLayer *pd_layers = nullptr;
@@ -1830,11 +1833,13 @@ int nvmai_cuda_moe_rms_renorm(nvmai_cuda_moe *h, const void *y, uint32_t tokens,
 // stage 2), so a layer is exactly three launches.
 // batched: through the batched experts' kernels, whose reduction normalises the rows for the next layer.
 // route_log: where the selected experts go, [num_layers][tokens][top_k], or nullptr.
-static int stack_enqueue(nvmai_cuda_moe *h, const __half *x0, uint32_t tokens, void *y_last, cudaStream_t st, bool batched, uint32_t *route_log) {
+// begin, end: the layers to run (x0 is read by the first layer, y_last written by the last one).
+static int stack_enqueue(nvmai_cuda_moe *h, const __half *x0, uint32_t tokens, void *y_last, cudaStream_t st, bool batched, uint32_t *route_log,
+                         uint32_t begin, uint32_t end) {
     const auto &c = h->cfg;
     auto log = [&](uint32_t l) { return route_log ? route_log + (size_t)l * tokens * c.top_k : nullptr; };
     if (batched) {
-        for (uint32_t l = 0; l < c.num_layers; ++l) {
+        for (uint32_t l = begin; l < end; ++l) {
             const bool last = l + 1 == c.num_layers;
             PrefillMode mode;
             mode.decode_order = true;
@@ -1844,7 +1849,7 @@ static int stack_enqueue(nvmai_cuda_moe *h, const __half *x0, uint32_t tokens, v
         }
         return NVMAI_CUDA_OK;
     }
-    for (uint32_t l = 0; l < c.num_layers; ++l) {
+    for (uint32_t l = begin; l < end; ++l) {
         const bool last = l + 1 == c.num_layers;
         void *y = last ? y_last : h->y;
         XSource xsrc{};
@@ -1867,9 +1872,11 @@ int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16, uint32_t 
     for (uint32_t l = 0; l < c.num_layers; ++l)
         if (!h->layers[l].registered) return NVMAI_CUDA_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // Launch-bound chain (3 small kernels per layer): replay it as a CUDA graph.
-    // The graph is captured once per (x0, y, tokens, stream); a stream that is
-    // itself being captured, or the legacy default stream, gets plain launches.
+    // Launch-bound chain (3 to 6 small kernels per layer): the inner layers are replayed as a CUDA graph, which saves 1 to 2 us
+    // a layer and costs about 6 where it meets the plain launches (40 layers, graph / plain: 2 rows 975 / 1016 us, 5 rows
+    // 1696 / 1840; 4 layers: 2 rows 106 / 100).  The first and the last layer, which touch the caller's buffers, are plain
+    // launches: a graph that holds them has to be made anew for every pair of buffers (5 rows: 0.15 ms for 4 layers, 1.4 ms
+    // for 40).  A stream that is itself being captured, and the legacy default stream, get plain launches only.
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (st != nullptr) cudaStreamIsCapturing(st, &cs);
     // One token and a shape the resident kernel covers: the whole step is one launch (no graph needed).  A stream
@@ -1895,8 +1902,10 @@ int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16, uint32_t 
         route_log = h->pd_route_log;
         h->pd_route_rows = tokens;
     }
-    if (st == nullptr || cs != cudaStreamCaptureStatusNone)
-        return stack_enqueue(h, static_cast<const __half *>(x0_f16), tokens, y_last, st, batched, route_log);
+    const __half *x0 = static_cast<const __half *>(x0_f16);
+    auto enqueue = [&](uint32_t begin, uint32_t end) { return stack_enqueue(h, x0, tokens, y_last, st, batched, route_log, begin, end); };
+    const uint32_t L = c.num_layers;
+    if (st == nullptr || cs != cudaStreamCaptureStatusNone || L < kMinGraphLayers) return enqueue(0, L);
     if (batched) {       // what a capture may not do: scratch
         int rc = ensure_prefill_scratch(h, st);
         if (rc) return rc;
@@ -1906,13 +1915,14 @@ int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16, uint32_t 
         h->stack_graphs.clear();
         h->graphs_stale = false;
     }
-    StackGraphKey key{x0_f16, y_last, tokens, st, batched, route_log != nullptr};
+    const StackGraphKey key{tokens, batched, route_log != nullptr};
     auto it = h->stack_graphs.find(key);
     if (it == h->stack_graphs.end()) {
+        if (h->stack_graphs.size() >= kMaxStackGraphs) return enqueue(0, L);
         int rc = record(h, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         if (rc) return rc;
         const uint64_t launches_before = g_launches.load();
-        rc = stack_enqueue(h, static_cast<const __half *>(x0_f16), tokens, y_last, st, batched, route_log);
+        rc = enqueue(1, L - 1);
         const uint64_t captured = g_launches.load() - launches_before;
         g_launches.store(launches_before);        // captured, not launched
         cudaGraph_t graph = nullptr;
@@ -1925,9 +1935,16 @@ int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16, uint32_t 
         if ((rc = record(h, e))) return rc;
         it = h->stack_graphs.emplace(key, std::make_pair(exec, captured)).first;
     }
-    int rc = record(h, cudaGraphLaunch(it->second.first, st));
-    if (rc == NVMAI_CUDA_OK) g_launches.fetch_add(it->second.second, std::memory_order_relaxed);
-    return rc;
+    int rc = enqueue(0, 1);
+    if (rc || (rc = record(h, cudaGraphLaunch(it->second.first, st)))) return rc;
+    g_launches.fetch_add(it->second.second, std::memory_order_relaxed);
+    return enqueue(L - 1, L);
+}
+
+int nvmai_cuda_moe_debug_stack_graphs(const nvmai_cuda_moe *h, uint32_t *out_count) {
+    if (!h || !out_count) return NVMAI_CUDA_EINVAL;
+    *out_count = (uint32_t)h->stack_graphs.size();
+    return NVMAI_CUDA_OK;
 }
 
 int nvmai_cuda_moe_stack_decode_host(nvmai_cuda_moe *h, const void *x0_f16_host, uint32_t tokens, void *y_last_host,
@@ -2222,7 +2239,7 @@ int nvmai_cuda_moe_ep_stack_decode(nvmai_cuda_moe *h, const void *x_own_f16, uin
         h->ep_graphs.clear();
         h->ep_graphs_stale = false;
     }
-    auto &g = h->ep_graphs[StackGraphKey{x_own_f16, y_own, rows_own, st}];
+    auto &g = h->ep_graphs[EpGraphKey{x_own_f16, y_own, rows_own, st}];
     // First call per key: plain launches (NCCL sets up its channels on first use).
     // Second call: capture.  Every rank takes the same branch, since all count alike.
     if (g.calls++ == 0) return (ep_replicated_mode(h, rows_own) ? ep_stack_enqueue_replicated(h, x, rows_own, y_own, st) : ep_stack_enqueue(h, x, rows_own, y_own, st));

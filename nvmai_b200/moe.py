@@ -267,6 +267,11 @@ class MoE:
         """How a stack step runs: auto (one row: one resident kernel), the staged launches, or the resident kernel forced."""
         check(self._lib.nvmai_cuda_moe_set_decode_mode(self._h, int(mode)), "set_decode_mode")
 
+    def debug_stack_graphs(self) -> int:
+        n = C.c_uint32(0)
+        check(self._lib.nvmai_cuda_moe_debug_stack_graphs(self._h, C.byref(n)), "debug_stack_graphs")
+        return n.value
+
     def debug_mute_block(self, block: int = 0xFFFFFFFF) -> None:
         """Test hook: one block of the resident kernel withholds its phase-1 results (bounded waits then expire)."""
         check(self._lib.nvmai_cuda_moe_debug_mute_block(self._h, block & 0xFFFFFFFF), "debug_mute_block")

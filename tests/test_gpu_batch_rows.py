@@ -120,3 +120,54 @@ def test_routing_of_a_row_does_not_depend_on_the_rows_beside_it(d):
     for rows in (40, 1100, 1500):
         some_idx, some_w = routing(rows)
         assert torch.equal(some_idx, idx[:rows]) and torch.equal(some_w, w[:rows]), rows
+
+
+# A stack of rows on buffers it has not seen: the graph belongs to the row count, not to the buffers, and the caller's rows
+# are read and written.  2: the staged kernels, 5: the batched ones.
+@pytest.mark.parametrize("rows", [2, 5])
+def test_stack_graphs_are_not_kept_by_buffer(rows):
+    torch = gu.torch_cuda()
+    cfg = _config(4, BF16, fmt.OUT_FP32, 40, 256, 128, 128, DENSE, num_layers=9)
+    moe = MoE(cfg)
+    keep = [_layer(31 + l, cfg) for l in range(9)]
+    for l, dev in enumerate(keep):
+        synthetic.register_device_layer(moe, l, dev)
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        x = torch.randn((6, rows, cfg.d), device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).half()
+        y = torch.zeros((6, rows, cfg.d), device="cuda")
+        for i in range(6):
+            moe.stack_decode(x[i], rows, y[i], stream=st)
+        again = torch.zeros_like(y)
+        for i in (3, 0, 5, 1, 4, 2):
+            moe.stack_decode(x[i], rows, again[i], stream=st)
+        moe.synchronize(st)
+    plain = torch.zeros_like(y)
+    torch.cuda.synchronize()
+    for i in range(6):                                    # the default stream: plain launches, the caller's buffers
+        moe.stack_decode(x[i], rows, plain[i], stream=0)
+    moe.synchronize()
+    assert moe.debug_stack_graphs() == 1
+    assert torch.equal(y, again) and torch.equal(y, plain) and bool((y != 0).any())
+
+
+def test_stack_graphs_are_bounded():
+    torch = gu.torch_cuda()
+    cfg = _config(4, BF16, fmt.OUT_FP32, 40, 256, 128, 128, DENSE, num_layers=8)
+    moe = MoE(cfg)
+    keep = [_layer(41 + l, cfg) for l in range(8)]
+    for l, dev in enumerate(keep):
+        synthetic.register_device_layer(moe, l, dev)
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        x = torch.randn((40, cfg.d), device="cuda").half()
+        y = torch.zeros((40, cfg.d), device="cuda")
+        for rows in range(2, 41):                         # the last of them as plain launches
+            moe.stack_decode(x, rows, y, stream=st)
+        moe.synchronize(st)
+    plain = torch.zeros_like(y)
+    torch.cuda.synchronize()
+    moe.stack_decode(x, 40, plain, stream=0)
+    moe.synchronize()
+    assert moe.debug_stack_graphs() == 32
+    assert torch.equal(y, plain)
