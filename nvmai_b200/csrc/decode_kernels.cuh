@@ -42,20 +42,13 @@ struct RoutedSource {
     const uint16_t *pes;      // per-expert scale (bf16) for the routing weights, or nullptr
     uint32_t *publish_idx;    // [tokens][top_k]: one block per token stores what it selected
     __half *publish_w;
-    // Expert parallelism (deferred selection only): global expert id -> index of the blob this rank holds, or
-    // 0xFFFFFFFF.  Experts held elsewhere yield no blob: their blocks do nothing, their slots add nothing.
+    // Expert parallelism: global expert id -> index of the blob this rank holds, or 0xFFFFFFFF.  Experts held elsewhere
+    // yield no blob: their blocks do nothing, their slots add nothing.
     const uint32_t *expert_map;
 };
 
 struct ExpertOffsets { uint32_t o[9]; };
 
-__device__ __forceinline__ const uint8_t *routed_blob(const RoutedSource &src, uint32_t token, uint32_t slot,
-                                                       uint32_t top_k) {
-    if (src.idx == nullptr) return src.blob[slot];
-    uint32_t e = src.idx[(size_t)token * top_k + slot];
-    e = min(e, src.num_experts - 1u);
-    return src.base + (size_t)e * src.stride;
-}
 __device__ __forceinline__ const uint8_t *expert_blob(const RoutedSource &src, uint32_t e) {
     e = min(e, src.num_experts - 1u);
     if (src.expert_map != nullptr) {
@@ -63,6 +56,13 @@ __device__ __forceinline__ const uint8_t *expert_blob(const RoutedSource &src, u
         if (e == 0xFFFFFFFFu) return nullptr;
     }
     return src.base + (size_t)e * src.stride;
+}
+// sel: the block's own selection, used when logits are given
+__device__ __forceinline__ const uint8_t *routed_blob(const RoutedSource &src, const uint32_t *sel, uint32_t token, uint32_t slot,
+                                                       uint32_t top_k) {
+    if (src.logits != nullptr) return expert_blob(src, sel[slot]);
+    if (src.idx == nullptr) return src.blob[slot];
+    return expert_blob(src, src.idx[(size_t)token * top_k + slot]);
 }
 
 // the same as an index into the layer's blobs (no expert map): `sel` = the block's own selection, used when logits are given

@@ -585,13 +585,15 @@ __global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
         if (p.prefill) {
             const float h1 = acc;
             float h2 = 0.0f;
-            for (uint32_t r = 0; r < p.K; ++r) h2 = fmaf(wk[r], round_out<OUT>(p.partial[(size_t)pos[r] * p.D + d]), h2);
+            for (uint32_t r = 0; r < p.K; ++r)
+                if (pos[r] != kNotLocal) h2 = fmaf(wk[r], round_out<OUT>(p.partial[(size_t)pos[r] * p.D + d]), h2);
             h2 = round_out<OUT>(h2);
             if (p.y != nullptr) store_out<OUT>(p.y, i, h1 + h2);
             if (p.hidden != nullptr) store_out<OUT>(p.hidden, i, round_out<OUT>(load_out<OUT>(p.hidden, i) + h1) + h2);
             continue;
         }
-        for (uint32_t r = 0; r < p.K; ++r) acc += wk[r] * p.partial[(size_t)pos[r] * p.D + d];
+        for (uint32_t r = 0; r < p.K; ++r)
+            if (pos[r] != kNotLocal) acc += wk[r] * p.partial[(size_t)pos[r] * p.D + d];
         const float yv = round_out<OUT>(acc);
         if (p.y != nullptr) store_out<OUT>(p.y, i, yv);
         if (p.hidden != nullptr) {

@@ -233,6 +233,7 @@ RoutedSource source_from_layer(const nvmai_cuda_moe *h, const LayerViews &lv, co
     s.base = static_cast<const uint8_t *>(lv.w.experts);
     s.stride = lv.w.expert_stride;
     s.num_experts = h->cfg.num_experts;
+    s.expert_map = h->expert_map;
     return s;
 }
 
@@ -576,7 +577,7 @@ int grouped_tail(nvmai_cuda_moe *h, const LayerViews &lv, const __half *x_rows, 
                  const __half *hidden_delta = nullptr, bool prefill_rounding = false) {
     const auto &c = h->cfg;
     const bool ep = partial_y != nullptr;
-    int rc = launch_group_pairs(h, idx, w, tokens, nullptr, nullptr, nullptr, true, !ep, st, !ep, ep);
+    int rc = launch_group_pairs(h, idx, w, tokens, nullptr, nullptr, nullptr, true, !ep, st, !ep, true);
     if (rc) return rc;
     const uint32_t P = tokens * c.top_k;
     const uint32_t routed_bound = std::min(P, c.num_experts + P / kPairsPerItem);
@@ -1759,7 +1760,8 @@ int nvmai_cuda_moe_group_pairs(nvmai_cuda_moe *h, const uint32_t *idx, const voi
 int nvmai_cuda_moe_set_expert_map(nvmai_cuda_moe *h, const uint32_t *map_host, uint32_t n_local) {
     if (!h) return NVMAI_CUDA_EINVAL;
     const auto &c = h->cfg;
-    h->pd_layers_stale = true;              // the tensor maps span the blobs this rank holds
+    h->pd_layers_stale = true;              // the tensor maps span the blobs this rank holds,
+    h->graphs_stale = true;                 // captured launches carry the map
     for (auto &lv : h->layers) { lv.tc_maps = false; lv.tile_maps = 0; }
     if (map_host == nullptr) {              // back to "every expert is local"
         cudaFree(h->expert_map);

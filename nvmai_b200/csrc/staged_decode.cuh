@@ -622,7 +622,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) stage2_kernel(const __grid_
         trace_mark(p.trace, 1);
     }
     // an expert held by another rank (expert parallelism): nothing to do here beyond block (0, 0)'s publication
-    const bool local = p.src.logits == nullptr || expert_blob(p.src, sel_idx[slot]) != nullptr;
+    const uint8_t *blob = BOXED ? nullptr : routed_blob(p.src, sel_idx, tok, slot, p.top_k);
+    const bool local = BOXED || blob != nullptr;             // (the boxes are for handles that hold every expert)
     if (warp == 0) {
         if (BOXED) {
             if (lane == 0) {
@@ -634,7 +635,6 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) stage2_kernel(const __grid_
                 }
             }
         } else if (local) {
-            const uint8_t *blob = p.src.logits != nullptr ? expert_blob(p.src, sel_idx[slot]) : routed_blob(p.src, tok, slot, p.top_k);
             const AffineMat gate = {blob + p.off.o[0], reinterpret_cast<const uint16_t *>(blob + p.off.o[1]),
                                     reinterpret_cast<const uint16_t *>(blob + p.off.o[2])};
             const AffineMat up = {blob + p.off.o[3], reinterpret_cast<const uint16_t *>(blob + p.off.o[4]),
@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) stage2_kernel(const __grid_
     if (!local) { trace_end(p.trace); return; }
     const uint8_t *pf_blob = nullptr;
     if (p.prefetch_down && warp == 0) {
-        pf_blob = p.src.logits != nullptr ? expert_blob(p.src, sel_idx[slot]) : routed_blob(p.src, tok, slot, p.top_k);
+        pf_blob = routed_blob(p.src, sel_idx, tok, slot, p.top_k);
     }
     // once this block's own tile is in: warm the L2 with its share of the expert's down projection (stage 3 reads it next)
     auto late = [&]() {
@@ -863,15 +863,13 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32, 2) stage3_ke
                           reinterpret_cast<uint32_t *>(part), part + 32, part + 64);
     }
     // a slot whose expert another rank holds (expert parallelism) loads nothing and adds nothing
-    bool local = true;
-    if (routed && p.src.logits != nullptr) local = expert_blob(p.src, reinterpret_cast<uint32_t *>(part)[unit]) != nullptr;
+    const uint8_t *blob = routed && !BOXED ? routed_blob(p.src, reinterpret_cast<uint32_t *>(part), tok, unit, p.top_k) : nullptr;
+    const bool local = BOXED || blob != nullptr;
     if (half == 0) {
         if (routed && BOXED) {
             if (lane == 0)
                 issue_down_boxes<BITS>(region, L, maps, row0, routed_expert(p.src, reinterpret_cast<uint32_t *>(part), tok, unit, p.top_k), p.F);
         } else if (routed && local) {
-            const uint8_t *blob = p.src.logits != nullptr ? expert_blob(p.src, reinterpret_cast<uint32_t *>(part)[unit])
-                                                          : routed_blob(p.src, tok, unit, p.top_k);
             const AffineMat mat{blob + p.off.o[6], reinterpret_cast<const uint16_t *>(blob + p.off.o[7]),
                                 reinterpret_cast<const uint16_t *>(blob + p.off.o[8])};
             issue_down_copies<BITS>(region, L, mat, row0, p.F);

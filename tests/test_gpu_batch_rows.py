@@ -171,3 +171,39 @@ def test_stack_graphs_are_bounded():
     moe.synchronize()
     assert moe.debug_stack_graphs() == 32
     assert torch.equal(y, plain)
+
+
+# A handle that holds a part of the experts (set_expert_map): the whole-block calls leave the others out, as if their
+# weights were zero, on every path: 1 row, a few, grouped, a stack; top-2 without a shared expert: the stages that read the
+# indices instead of selecting.
+@pytest.mark.parametrize("rows,other", [(1, {}), (3, {}), (6, {}), (30, {}), (3, {"top_k": 2, "shared_f": 0})])
+@pytest.mark.parametrize("entry", ["layer", "stack"])
+def test_calls_on_a_part_of_the_experts_leave_the_others_out(rows, other, entry):
+    torch = gu.torch_cuda()
+    cfg = _config(4, BF16, fmt.OUT_FP32, 32, 256, 128, 64, DENSE, **other)
+    dev = _layer(53, cfg)
+    held = [e for e in range(64) if e % 3 != 1]
+    gone = [e for e in range(64) if e % 3 == 1]
+    part = dict(dev, experts=dev["experts"][held].clone())
+    off, meta_bytes = dev["offsets"], 128 * (256 // 64) * 2
+    for name in ("gate_s", "gate_b", "up_s", "up_b", "down_s", "down_b"):      # (all six are as long: 256 x 128 / 64)
+        dev["experts"][gone, off[name]:off[name] + meta_bytes] = 0
+    x = torch.randn((rows, cfg.d), device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).half()
+
+    def run(weights, expert_map):
+        moe = MoE(cfg)
+        if expert_map is not None:
+            moe.set_expert_map(expert_map)
+        synthetic.register_device_layer(moe, 0, weights)
+        y = torch.zeros((rows, cfg.d), device="cuda")
+        if entry == "layer":
+            moe.layer_decode(0, x, rows, h2_out=y)
+        else:
+            moe.stack_decode(x, rows, y)
+        moe.synchronize()
+        return y
+
+    want = run(dev, None)
+    got = run(part, [held.index(e) if e in held else 0xFFFFFFFF for e in range(64)])
+    assert bool(torch.isfinite(want).all()) and bool((want != 0).any())
+    assert torch.equal(got, want) or float((got - want).norm() / want.norm()) < 1e-6
