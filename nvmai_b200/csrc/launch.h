@@ -31,6 +31,15 @@ inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
 
 // pdl: launch with programmatic stream serialization, so that the kernel's
 // prologue (its weight copies) may overlap the previous kernel's tail.
+//
+// What every kernel launched here keeps to, and what those that start early lean on:
+//   1. Each block waits for the kernel in front (pdl_wait) before it lets the one behind start (pdl_launch_dependents),
+//      and no block ends without having waited.  So whatever ran before the kernel in front is complete, and its writes
+//      are visible, as soon as a kernel has started at all; the kernel in front itself is complete behind pdl_wait.
+//   2. A kernel that puts its own wait off may read, until then, only what kernels before the one in front wrote, and
+//      write only what none of them and not the one in front touches: the router GEMM beside the packing of the rows
+//      (batch_rows.cuh), a streaming kernel beside the grouped GEMM of the same phase (SgParams::beside).
+// A kernel that lets its dependents start without having waited would break both without any sign of it.
 template <typename Kern, typename... Params>
 inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
     cudaError_t e = ensure_smem(kern, smem);

@@ -141,8 +141,10 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
         for (uint32_t i = 0; i < 16; ++i) mbar_init(&bars->h_full[i >> 3][i & 7], 1);
         mbar_fence_init();
     }
-    if (!p.beside) pdl_wait();
-    pdl_launch_dependents();
+    if (!p.beside) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     bool ok = __syncthreads_and(*reinterpret_cast<volatile unsigned int *>(p.status) == 0u);
     // the units of the launch: those of the shared items come first and are skipped where another kernel has them
     const uint32_t skip = *p.shared_on != 0u ? 0u : p.shared_items * p.units_per_item;
@@ -448,7 +450,10 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
         const unsigned long long t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
-    if (p.beside) pdl_wait();              // the kernel after this one relies on the one before it being complete
+    if (p.beside) {                        // the kernel after this one relies on the one before it being complete
+        pdl_wait();
+        pdl_launch_dependents();
+    }
 }
 
 }  // namespace nvmai
