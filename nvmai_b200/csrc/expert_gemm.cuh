@@ -63,18 +63,18 @@ static_assert(sizeof(EgBarriers) <= 1024, "the barriers have 1 KB");
 // One unit of the launch.
 struct EgUnit { uint32_t shared, expert, start, count, j; };
 
-__device__ __forceinline__ EgUnit eg_unit(const EgParams &p, uint32_t u) {
+__device__ __forceinline__ EgUnit eg_unit(const EgParams &p, uint32_t u, uint32_t shared_items) {
     EgUnit r;
     const uint32_t item = u / p.units_per_item;
     r.j = u - item * p.units_per_item;
-    r.shared = item < p.shared_items ? 1u : 0u;
+    r.shared = item < shared_items ? 1u : 0u;
     if (r.shared) {       // the shared expert sees every token: even runs of token rows, first because they are the longest
         const uint32_t even = p.tokens / p.shared_items, extra = p.tokens - even * p.shared_items;
         r.expert = 0;
         r.start = item * even + min(item, extra);
         r.count = even + (item < extra ? 1u : 0u);
     } else {
-        const WorkItem w = p.work[item - p.shared_items];
+        const WorkItem w = p.work[item - shared_items];
         r.expert = min(w.expert, p.num_experts - 1u);
         r.start = w.start;
         r.count = min(w.count, p.cap);
@@ -83,9 +83,9 @@ __device__ __forceinline__ EgUnit eg_unit(const EgParams &p, uint32_t u) {
 }
 
 // For roles that must not wait for the work list between two units: the next unit is requested a unit ahead.
-__device__ __forceinline__ EgUnit eg_unit_or_last(const EgParams &p, uint32_t u, uint32_t total) {
+__device__ __forceinline__ EgUnit eg_unit_or_last(const EgParams &p, uint32_t u, uint32_t total, uint32_t shared_items) {
     if (total == 0u) return EgUnit{};
-    return eg_unit(p, min(u, total - 1u));
+    return eg_unit(p, min(u, total - 1u), shared_items);
 }
 
 // The scale a stage multiplies by, twice in a register: the low (odd = 0) or high half of `word`, pass 0 .. PASSES-1 =
@@ -350,9 +350,9 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
     const uint32_t n_pair = PHASE == 0 ? n_v : (n_v + 1u) / 2u;
     const uint32_t n_chunk = (n_main + kChunkBlocks - 1u) / kChunkBlocks;     // chunks per tile
     const uint32_t n_sub = PHASE == 0 ? 1u : p.tiles_per_unit;                // accumulator turns per unit
-    // the units of the launch: those of the shared items come first and are skipped where another kernel has them
-    const uint32_t skip = *p.shared_on != 0u ? 0u : p.shared_items * p.units_per_item;
-    const uint32_t total = ok ? (p.shared_items + p.n_work[0]) * p.units_per_item : 0u;
+    // the units of the launch: those of the shared items come first, and there are none where another kernel has them
+    const uint32_t shared_items = *p.shared_on != 0u ? p.shared_items : 0u;
+    const uint32_t total = ok ? (shared_items + p.n_work[0]) * p.units_per_item : 0u;
     const uint32_t meta_bytes = 128u * n_main * 2u;                           // scales (or biases) of a tile
 
     if (warp < kEgProducerWarps) {
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
         // pass0 + 2 where it has two): its share of the stages in slot order.
         constexpr uint32_t kStep = PHASE == 0 ? (kPasses == 1u ? 2u : 1u) : (kPasses == 1u ? 4u : kPasses == 2u ? 2u : 1u);
         constexpr uint32_t kTwo = PHASE == 0 && kPasses == 4u ? 2u : 1u;
-        for (uint32_t u = skip + blockIdx.x; u < total && ok; u += gridDim.x) {
+        for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
             for (uint32_t sub = 0; sub < n_sub; ++sub) {
                 const uint32_t tile = PHASE == 0 ? half : 0u;
                 uint32_t ms = m_slot + tile, mp = m_phase;
@@ -471,8 +471,8 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
         // ---------------- packed codes and scales: one thread, running ahead ----------------
         if (elect_one()) {
             uint32_t c = 0, m_slot = 0, m_phase = 0;
-            for (uint32_t u = skip + blockIdx.x; u < total && ok; u += gridDim.x) {
-                const EgUnit un = eg_unit(p, u);
+            for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
+                const EgUnit un = eg_unit(p, u, shared_items);
                 const uint8_t *blob = p.experts + (size_t)un.expert * p.stride;
                 for (uint32_t sub = 0; sub < n_sub && ok; ++sub) {
                     const uint32_t row0 = (PHASE == 0 ? un.j : un.j * n_sub + sub) * 128u;
@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
             const uint32_t w = warp - kEgRowWarp0, piece = lane & 7u, r0 = 4u * w + (lane >> 3);
             const uint32_t dst0 = row_ring + r0 * 128u + ((piece ^ (r0 & 7u)) << 4);
             const uint32_t row_bytes = (p.kdim + bp_extra_cols(p.kdim, 1)) * 2u;
-            EgUnit next = eg_unit_or_last(p, skip + blockIdx.x, total);
-            for (uint32_t u = skip + blockIdx.x; u < total && ok; u += gridDim.x) {
+            EgUnit next = eg_unit_or_last(p, blockIdx.x, total, shared_items);
+            for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
                 const EgUnit un = next;
                 const uint32_t n_i = (un.count + 15u) / 16u;
                 uint32_t off[kMaxRows];                // byte offsets; rows past the item's end repeat its last one
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                     const uint32_t n = un.start + min(16u * i + r0, un.count - 1u);
                     off[i] = i < n_i ? (un.shared ? n : p.sorted_pair[n] / p.top_k) * row_bytes + piece * 16u : 0u;
                 }
-                next = eg_unit_or_last(p, u + gridDim.x, total);
+                next = eg_unit_or_last(p, u + gridDim.x, total, shared_items);
                 const uint8_t *src = reinterpret_cast<const uint8_t *>(un.shared ? p.shared_rows : p.rows);
                 for (uint32_t kb = 0; kb < n_kb; ++kb, src += 128) {
                     ok = __all_sync(0xffffffffu, wait(&bars->b_empty[slot], phase ^ 1u));
@@ -547,8 +547,8 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
             cp_async_wait_all();
         } else if (warp == kEgRowWarp0) {
             // consecutive rows: one 16-row box per lane
-            for (uint32_t u = skip + blockIdx.x; u < total && ok; u += gridDim.x) {
-                const EgUnit un = eg_unit(p, u);
+            for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
+                const EgUnit un = eg_unit(p, u, shared_items);
                 const uint32_t n_cols = (un.count + 15u) & ~15u;
                 const uint32_t loads = p.resident ? 1u : n_sub;
                 for (uint32_t sub = 0; sub < loads && ok; ++sub) {
@@ -571,10 +571,10 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
             uint32_t pair = 0, slot = 0, phase = 0, acc = 0, acc_phase = 0;
             const uint64_t db0 = umma_desc_sw128(row_ring);
             const uint32_t slot_step = p.row_slot_bytes >> 4;
-            EgUnit next = eg_unit_or_last(p, skip + blockIdx.x, total);
-            for (uint32_t u = skip + blockIdx.x; u < total && ok; u += gridDim.x) {
+            EgUnit next = eg_unit_or_last(p, blockIdx.x, total, shared_items);
+            for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
                 const EgUnit un = next;
-                next = eg_unit_or_last(p, u + gridDim.x, total);
+                next = eg_unit_or_last(p, u + gridDim.x, total, shared_items);
                 const uint32_t idesc = umma_idesc_f16(128u, (un.count + 15u) & ~15u);
                 for (uint32_t sub = 0; sub < n_sub && ok; ++sub) {
                     ok = wait(&bars->d_empty[acc], acc_phase ^ 1u);
@@ -644,10 +644,10 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
         // ---------------- epilogue ----------------
         const uint32_t q = warp & 3u, h = (warp - kEgProducerWarps) >> 2;      // lane quarter; every other 8 columns
         uint32_t acc = 0, acc_phase = 0;
-        EgUnit next = eg_unit_or_last(p, skip + blockIdx.x, total);
-        for (uint32_t u = skip + blockIdx.x; u < total && ok; u += gridDim.x) {
+        EgUnit next = eg_unit_or_last(p, blockIdx.x, total, shared_items);
+        for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
             const EgUnit un = next;
-            next = eg_unit_or_last(p, u + gridDim.x, total);
+            next = eg_unit_or_last(p, u + gridDim.x, total, shared_items);
             for (uint32_t sub = 0; sub < n_sub && ok; ++sub) {
                 ok = __all_sync(0xffffffffu, wait_patient(&bars->d_full[acc], acc_phase));
                 if (!ok) break;
