@@ -94,17 +94,18 @@ struct PackXParams {
 };
 cudaError_t bp_pack_x(const PackXParams &p, cudaStream_t st);
 
-// dense fp16 router: logits as `splits` partial sums [split][tokens][experts]
+// dense fp16 router: logits as partial sums [term][tokens][experts]
 struct RouterParams { float *logits; uint32_t tokens, experts, kdim, splits; unsigned int *status; };
 struct alignas(64) RouterArgs { CUtensorMap w, x; RouterParams p; };
 constexpr uint32_t kRouterTileTokens = 64;
-constexpr uint32_t kRouterParts = 4;      // sums over K that the logits add up from; splits: 1, 2 or 4 of them a block
+constexpr uint32_t kRouterParts = 4;      // quarters of K that the logits add up from; splits: 1, 2 or 4 blocks share them
+inline uint32_t bp_router_terms(uint32_t splits) { return splits == 1 ? 1 : splits == 2 ? 3 : 4; }     // see router_gemm_kernel
 cudaError_t bp_router(const RouterArgs &args, cudaStream_t st);
 
 // top-k of every row (or the given experts), histograms per block, and in the last block the scan: offsets per expert,
 // first positions per block, the GEMMs' work lists
 struct RouteParams {
-    const float *logits; uint32_t splits;     // nullptr: idx is given; splits <= kRouterParts
+    const float *logits; uint32_t terms;      // [term][tokens][E], 1 to 4 terms; nullptr: idx is given
     const uint16_t *pes;
     uint32_t *idx; __half *w;
     uint32_t tokens, E, K;

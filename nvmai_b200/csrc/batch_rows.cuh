@@ -84,7 +84,8 @@ __global__ void __launch_bounds__(256) pack_x_kernel(PackXParams p) {
 // batch still spreads over the chip (one block per 256 tokens took 20-29 us at any batch size).  Products of two fp16
 // values are exact in fp32: only the order of the additions differs from the decode router's.  That order is the same
 // for any number of splits, so a row's logits do not depend on the rows beside it: K always adds up in four quarters,
-// (q0 + q1) + (q2 + q3), a block keeping each of its quarters in an accumulator of its own.
+// ((q0 + q1) + q2) + q3, a block keeping each of its quarters in an accumulator of its own.  The first block hands over the
+// sum of its quarters, the others each quarter: 1, 3 or 4 terms for 1, 2 or 4 splits (bp_router_terms).
 constexpr uint32_t kRouterStages = 4;
 constexpr uint32_t kRouterStageBytes = 128 * 128 + kRouterTileTokens * 128;
 constexpr size_t kRouterSmem = 2048 + kRouterStages * kRouterStageBytes;
@@ -148,26 +149,23 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
         tc_fence_after_sync();
-        float *out = p.logits + ((size_t)blockIdx.z * p.tokens + t0) * p.experts + e0 + warp * 32u + lane;
+        const uint32_t term = blockIdx.z == 0u ? 0u : p.splits == 2u ? 1u : blockIdx.z;
+        const size_t term_step = (size_t)p.tokens * p.experts;
+        float *out = p.logits + term * term_step + (size_t)t0 * p.experts + e0 + warp * 32u + lane;
         for (uint32_t cb = 0; cb < kRouterTileTokens && t0 + cb < p.tokens; cb += 8u) {
             float v[8];
-            auto load = [&](uint32_t q, float (&o)[8]) {
+            for (uint32_t q = 0; q < quarters; ++q) {
                 uint32_t r[8];
                 tmem_ld8(tmem + ((warp * 32u) << 16) + q * kRouterTileTokens + cb, r);
                 tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[i]);
-            };
-            auto add = [&](float (&a)[8], const float (&b)[8]) {
+                for (int i = 0; i < 8; ++i) v[i] = q != 0u && blockIdx.z == 0u ? v[i] + __uint_as_float(r[i]) : __uint_as_float(r[i]);
+                if (blockIdx.z == 0u && q + 1u < quarters) continue;
+                float *at = out + (blockIdx.z == 0u ? 0u : q * term_step);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) a[i] += b[i];
-            };
-            load(0u, v);
-            if (quarters >= 2u) { float q1[8]; load(1u, q1); add(v, q1); }
-            if (quarters == 4u) { float q2[8], q3[8]; load(2u, q2); load(3u, q3); add(q2, q3); add(v, q2); }
-#pragma unroll
-            for (uint32_t i = 0; i < 8u; ++i)
-                if (t0 + cb + i < p.tokens) out[(size_t)(cb + i) * p.experts] = v[i];
+                for (uint32_t i = 0; i < 8u; ++i)
+                    if (t0 + cb + i < p.tokens) at[(size_t)(cb + i) * p.experts] = v[i];
+            }
         }
     }
     tc_fence_before_sync();
@@ -209,8 +207,8 @@ __device__ __forceinline__ uint32_t heavy_limit(const RouteParams &p, uint32_t r
     return many ? p.heavy : ~0u;
 }
 
-// v[i] = logit of expert lane + 32 i: the splits of K added as (s0 + s1) + (s2 + s3), all 32 loads in flight
-__device__ __forceinline__ void add_splits(float (&v)[kMaxExperts / 32], const RouteParams &p, uint32_t tok, uint32_t lane) {
+// v[i] = logit of expert lane + 32 i: its terms added in order, all 32 loads in flight
+__device__ __forceinline__ void add_terms(float (&v)[kMaxExperts / 32], const RouteParams &p, uint32_t tok, uint32_t lane) {
     static_assert(kRouterParts == 4, "the sum has four terms");
     float a[4][kMaxExperts / 32];
 #pragma unroll
@@ -218,11 +216,11 @@ __device__ __forceinline__ void add_splits(float (&v)[kMaxExperts / 32], const R
 #pragma unroll
         for (int i = 0; i < kMaxExperts / 32; ++i) {
             const uint32_t e = lane + 32u * i;
-            a[k][i] = e < p.E && k < p.splits ? __ldcg(p.logits + ((size_t)k * p.tokens + tok) * p.E + e) : 0.0f;
+            a[k][i] = e < p.E && k < p.terms ? __ldcg(p.logits + ((size_t)k * p.tokens + tok) * p.E + e) : 0.0f;
         }
 #pragma unroll
     for (int i = 0; i < kMaxExperts / 32; ++i)
-        if (lane + 32u * i < p.E) v[i] = (a[0][i] + a[1][i]) + (a[2][i] + a[3][i]);
+        if (lane + 32u * i < p.E) v[i] = ((a[0][i] + a[1][i]) + a[2][i]) + a[3][i];
 }
 
 // Router semantics of router_topk_select_k8 (moe.metal:233-285); the pairs end up in (expert, token, rank) order, as
@@ -244,7 +242,7 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
             float v[kMaxExperts / 32];
 #pragma unroll
             for (int i = 0; i < kMaxExperts / 32; ++i) v[i] = lane + 32u * i < p.E ? 0.0f : -INFINITY;
-            add_splits(v, p, tok, lane);
+            add_terms(v, p, tok, lane);
             topk_softmax_warp_vals(v, (int)p.E, (int)p.K, p.pes, p.idx + (size_t)tok * p.K, p.w + (size_t)tok * p.K);
         }
         if ((uint32_t)lane < p.K) {
@@ -368,7 +366,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(RouteParams p) {
             float v[kMaxExperts / 32];
 #pragma unroll
             for (int i = 0; i < kMaxExperts / 32; ++i) v[i] = lane + 32u * i < p.E ? 0.0f : -INFINITY;
-            add_splits(v, p, tok, lane);
+            add_terms(v, p, tok, lane);
             topk_softmax_warp_vals(v, (int)p.E, (int)p.K, p.pes, p.idx + (size_t)tok * p.K, p.w + (size_t)tok * p.K);
         }
         if ((uint32_t)lane < p.K) {

@@ -138,7 +138,7 @@ struct nvmai_cuda_moe {
     __half *pf_acts16 = nullptr;     // [T*K][F + extra] routed activations as the down GEMM reads them
     __half *pf_sacts16 = nullptr;    // [T][Fs + extra] the shared expert's
     float *pf_rowscale = nullptr, *pf_srowscale = nullptr;   // per row: power of two taken out of a wide-range row
-    float *pf_logits = nullptr;      // [splits][T][E]
+    float *pf_logits = nullptr;      // [terms][T][E]
     uint32_t *pf_hist = nullptr;     // [routing blocks][256]
     WorkItem *pf_work2 = nullptr;    // the down GEMM's work list (h->work is the gate/up GEMM's)
     WorkItem *pf_work3 = nullptr;    // the streaming kernel's
@@ -798,7 +798,8 @@ int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
     const size_t T = c.max_tokens, P = T * c.top_k;
     const size_t dx = c.d + bp_extra_cols(c.d, 1), fx = c.f + bp_extra_cols(c.f, 2), sfx = c.shared_f + bp_extra_cols(c.shared_f, 2);
     const bool two_orders = c.shared_f != 0 && c.shared_bits != c.routed_bits;
-    const size_t logit_rows = std::min<size_t>(4 * T, std::max<size_t>(T, (size_t)h->sm_count * kRouterTileTokens));
+    // (router_splits: 4 terms of up to 64 rows for a quarter of the SMs, 3 for half of them, else one)
+    const size_t logit_rows = std::min<size_t>(4 * T, std::max<size_t>(T, (size_t)h->sm_count * kRouterTileTokens * 3 / 2));
     const size_t blocks = std::max(bp_route_blocks(c.max_tokens), bp_route_blocks(std::min(c.max_tokens, 1024u)));
     Slab slab;
     slab.want(&h->pf_x, T * dx * 2); slab.want(&h->pf_xs, two_orders ? T * dx * 2 : 0);
@@ -878,15 +879,16 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
         RouterArgs ra{};
         ra.w = lv.router;
         if ((rc = make_rows_tmap(h, &ra.x, x, tokens, c.d, kRouterTileTokens))) return rc;
-        r.splits = router_splits(h, tokens);
+        const uint32_t splits = router_splits(h, tokens);
+        r.terms = bp_router_terms(splits);
         r.logits = h->pf_logits;
-        ra.p = RouterParams{h->pf_logits, tokens, c.num_experts, c.d, r.splits, h->status};
+        ra.p = RouterParams{h->pf_logits, tokens, c.num_experts, c.d, splits, h->status};
         if ((rc = launched(h, bp_router(ra, st)))) return rc;
         if (gated && !gate_here && (rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, false, false, true, false, st))) return rc;
     } else if (!routed_only) {
         // (top-k in the routing kernel: left to this one's last block of every eight rows, and after the packing instead of
         // beside what came before, four rows of an 8-bit router took 57.7 us for the block, 47.1 as separate rows)
-        r.splits = 1;
+        r.terms = 1;
         r.logits = h->logits;
         if ((rc = launch_stage1(h, lv, xsrc, tokens, nullptr, nullptr, true, false, gated, true, st, true, true))) return rc;
     }

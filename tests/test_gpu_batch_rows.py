@@ -96,13 +96,14 @@ def test_rows_of_a_dense_router_equal_calls_of_their_own(bits, meta, out, rows, 
     _check_rows_alone(cfg, rows, seed=300 + rows)
 
 
-# From 32 rows on the dense router is a GEMM whose K is split over four, two or one block by the number of rows (32 to 1152,
-# to 2368 and more, at 256 experts on 148 SMs): the logits, and so the routing, are the same for any number.
-@pytest.mark.parametrize("d", [256, 1280])
-def test_routing_of_a_row_does_not_depend_on_the_rows_beside_it(d):
+# From 32 rows on the dense router is a GEMM whose K is split over four, two or one block by the number of rows (at 256
+# experts on 148 SMs up to 1152, 2368 and more rows; at 128 experts up to 2368, 4736 and more): the logits, and so the
+# routing, are the same for any number.
+@pytest.mark.parametrize("d,experts,some,most", [(256, 256, (40, 1100, 1500, 2368), 2500), (1280, 256, (40, 1152, 1500), 2500),
+                                                 (256, 128, (40, 2368, 2369, 4736), 4800)])
+def test_routing_of_a_row_does_not_depend_on_the_rows_beside_it(d, experts, some, most):
     torch = gu.torch_cuda()
-    most = 2500
-    cfg = _config(4, BF16, fmt.OUT_FP16, most, d, 128, 256, DENSE)
+    cfg = _config(4, BF16, fmt.OUT_FP16, most, d, 128, experts, DENSE)
     moe = MoE(cfg)
     dev = _layer(17, cfg)
     synthetic.register_device_layer(moe, 0, dev)
@@ -117,7 +118,7 @@ def test_routing_of_a_row_does_not_depend_on_the_rows_beside_it(d):
         return idx, w
 
     idx, w = routing(most)
-    for rows in (40, 1100, 1500):
+    for rows in some:
         some_idx, some_w = routing(rows)
         assert torch.equal(some_idx, idx[:rows]) and torch.equal(some_w, w[:rows]), rows
 
