@@ -153,18 +153,25 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
         const size_t term_step = (size_t)p.tokens * p.experts;
         float *out = p.logits + term * term_step + (size_t)t0 * p.experts + e0 + warp * 32u + lane;
         for (uint32_t cb = 0; cb < kRouterTileTokens && t0 + cb < p.tokens; cb += 8u) {
-            float v[8];
-            for (uint32_t q = 0; q < quarters; ++q) {
-                uint32_t r[8];
-                tmem_ld8(tmem + ((warp * 32u) << 16) + q * kRouterTileTokens + cb, r);
-                tmem_ld_wait();
+            uint32_t r[kRouterParts][8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = q != 0u && blockIdx.z == 0u ? v[i] + __uint_as_float(r[i]) : __uint_as_float(r[i]);
+            for (uint32_t q = 0; q < kRouterParts; ++q)
+                if (q < quarters) tmem_ld8(tmem + ((warp * 32u) << 16) + q * kRouterTileTokens + cb, r[q]);
+            tmem_ld_wait();
+            float *at = out + (size_t)cb * p.experts;
+#pragma unroll
+            for (uint32_t q = 0; q < kRouterParts; ++q) {
+                if (q >= quarters) break;
+                if (q != 0u) {
+                    if (blockIdx.z != 0u) at += term_step;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (blockIdx.z == 0u) r[q][i] = __float_as_uint(__uint_as_float(r[q - 1u][i]) + __uint_as_float(r[q][i]));
+                }
                 if (blockIdx.z == 0u && q + 1u < quarters) continue;
-                float *at = out + (blockIdx.z == 0u ? 0u : q * term_step);
 #pragma unroll
                 for (uint32_t i = 0; i < 8u; ++i)
-                    if (t0 + cb + i < p.tokens) at[(size_t)(cb + i) * p.experts] = v[i];
+                    if (t0 + cb + i < p.tokens) at[(size_t)i * p.experts] = __uint_as_float(r[q][i]);
             }
         }
     }
