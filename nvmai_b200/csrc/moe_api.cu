@@ -331,8 +331,8 @@ int launch_stage1(nvmai_cuda_moe *h, const LayerViews &lv, const XSource &xsrc, 
     p.status = h->status;
     p.router_row_blocks = (c.num_experts + kRowsPerRouterBlock - 1) / kRowsPerRouterBlock;
     p.tokens_per_chunk = tokens <= 8 ? tokens : 8;
-    if (spread_rows) {      // fewer rows a block where that still is one wave of blocks
-        const uint32_t wave = std::max(1u, (uint32_t)h->sm_count / p.router_row_blocks);
+    if (spread_rows) {      // fewer rows a block while two blocks an SM hold them all (one: 31 rows 97.6 us instead of 94.8)
+        const uint32_t wave = std::max(1u, 2u * (uint32_t)h->sm_count / p.router_row_blocks);
         p.tokens_per_chunk = std::min(p.tokens_per_chunk, (tokens + wave - 1) / wave);
     }
     const uint32_t chunks = (tokens + p.tokens_per_chunk - 1) / p.tokens_per_chunk;
@@ -855,7 +855,7 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
     // A dense fp16 router without an input scale is a plain GEMM (products of two fp16 values are
     // exact in fp32, so only the order of the fp32 additions differs from the decode router's);
     // affine routers keep the exact code-times-activation kernel, and so do decode calls of a few rows (4-bit block with the
-    // GEMM / this kernel: 4 rows 41.3 / 38.6 us, 13 rows 64.4 / 65.4, 31 rows 94.7 / 97.7).
+    // GEMM / this kernel: 4 rows 41.1 / 38.2 us, 13 rows 64.9 / 63.7, 31 rows 94.9 / 94.8).
     const bool gemm = !routed_only && !(mode.decode_order && tokens < kExactRows) && c.router_kind == NVMAI_ROUTER_DENSE_F16 && lv.w.effective_scale == nullptr && c.num_experts % 128 == 0;
     const bool gate_here = gemm && gated && c.shared_gate_kind == NVMAI_ROUTER_DENSE_F16;      // else stage 1 has the gate
     px.x = x; px.rows = tokens; px.n = c.d;
