@@ -306,8 +306,8 @@ def test_layer_decode_reference_format_fp16_out():
 
 @pytest.mark.parametrize("tokens,grouped_min", [(2, None), (4, None), (16, None), (64, None), (4, 4), (16, 4)])
 def test_layer_decode_batch(tokens, grouped_min, monkeypatch):
-    """independent rows, 8-bit.  Small batches run every row's blocks separately; from 24 rows on
-    (or from NVMAI_CUDA_GROUPED_MIN on) rows that picked the same expert are grouped and share one read of its weights"""
+    """independent rows, 8-bit.  From 4 rows on the batched experts' kernels; with NVMAI_CUDA_GROUPED_MIN (which
+    moves those to 32 rows) the exact kernels that group rows of the same expert"""
     if grouped_min is not None:
         monkeypatch.setenv("NVMAI_CUDA_GROUPED_MIN", str(grouped_min))
     host, cfg = _layer_case(8, fmt.META_FP16, fmt.OUT_FP32, tokens, seed=5)
@@ -323,7 +323,8 @@ def test_layer_decode_batch_4bit_reference_rounding(monkeypatch):
 
 
 def test_batched_result_equals_row_by_row(monkeypatch):
-    """grouping must not change a row's result: batch of 9 == nine single-row calls, bitwise"""
+    """grouping must not change a row's result: batch of 9 on the exact grouped kernels == nine single-row calls, bitwise
+    (the kernels a call takes by default: test_gpu_batch_rows.py)"""
     monkeypatch.setenv("NVMAI_CUDA_GROUPED_MIN", "4")
     host, cfg = _layer_case(4, fmt.META_BF16, fmt.OUT_FP32, 9, seed=41, d=256, f=128, e=32)
     moe = MoE(cfg)

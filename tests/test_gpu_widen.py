@@ -359,7 +359,7 @@ def test_zipf_batch_on_a_rank_that_holds_a_part_of_the_experts(placement):
 
 @pytest.mark.parametrize("out_dtype", [fmt.OUT_FP32, fmt.OUT_FP16])
 def test_large_decode_batch_on_tensor_cores_keeps_decode_semantics(out_dtype, monkeypatch):
-    """from 32 rows on a 4-bit batched decode call runs the grouped GEMMs of the prefill path; indices stay exact,
+    """a 4-bit batched decode call of 40 rows runs the launches of the prefill path; indices stay exact,
     every row stays within the bars of the decode oracle, the residual add keeps the decode order (one add of the
     rounded block output), and the result agrees with the per-row kernels' result for the same call"""
     tokens = 40
