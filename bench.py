@@ -907,8 +907,8 @@ def run_prefill(args) -> None:
         raise SystemExit("parity check of the timed path failed: " + json.dumps(parity))
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one stage2_kernel launch, from an ncu capture of the 4-bit
-# kernel (the 8-bit kernel has not been captured)
+# dram__bytes_read.sum + dram__bytes_write.sum of one stage2_kernel launch over the routed experts alone, from an ncu
+# capture of the 4-bit kernel (the 8-bit kernel has not been captured)
 STAGE2_DRAM_BYTES_PER_LAUNCH = {4: 9508352, 8: None}
 # the same for the resident decode kernel, per LAYER: an ncu capture of a 4-layer, 4-bit step read 68,057,600 B
 # and wrote 1,360,384 B; the traffic of a step grows with its number of layers
@@ -942,7 +942,7 @@ def resident_roofline(moe, args, xs, x_in, y, stream, peak: float, which: str) -
 
 
 def batch_roofline(moe, args, tokens: int, ms_per_step: float, peak: float, which: str) -> dict:
-    """2..8 rows per step run as one launch of the resident batch kernel.  Its algorithmic bytes follow the routing:
+    """2..8 rows per step.  The algorithmic bytes follow the routing:
     per layer every DISTINCT expert the rows selected (read back from the step's own routing record) once, plus the
     shared expert, the router, the gate row and the rows themselves."""
     log = moe.read_route_log_rows(tokens)                     # [layers][rows][K] of the last step
@@ -951,7 +951,9 @@ def batch_roofline(moe, args, tokens: int, ms_per_step: float, peak: float, whic
     distinct = [int(np.unique(log[l]).size) for l in range(log.shape[0])]
     nbytes = sum(d * blob + fixed for d in distinct)
     achieved = nbytes / (ms_per_step * 1e-3) / 1e9
-    return {"bound": "hbm", "kernel": "persistent_batch_kernel (one launch = all layers of the step, %d rows)" % tokens,
+    return {"bound": "hbm", "kernel": "all layers of the step, %d rows (%s)" % (
+                tokens, "persistent_batch_kernel" if os.environ.get("NVMAI_CUDA_DECODE_MODE") == "2" else
+                "stage kernels" if tokens < 4 else "batched experts' kernels"),
             "achieved": achieved, "peak": peak, "peak_source": which, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
             "bytes_per_launch": nbytes, "us_per_launch": ms_per_step * 1e3,
             "distinct_experts_per_layer_mean": float(np.mean(distinct))}

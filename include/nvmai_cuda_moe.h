@@ -191,7 +191,10 @@ NVMAI_API int nvmai_cuda_moe_routed_phase2(nvmai_cuda_moe *h, const void *const 
  * router -> shared expert -> phase 1 -> phase 2 (h1 as residual) -> hidden += h2.
  * x is the normalised input fp16[tokens][d]; hidden_inout out_dtype[tokens][d] may be
  * NULL; h2_out (optional) receives the block output before the residual add.
- * out_idx / out_w optional.  Experts stay on the device: no host read-back. */
+ * out_idx / out_w optional.  Experts stay on the device: no host read-back.
+ * Below 32 rows every row has the bits of a call of its own.  From 32 rows on its experts and
+ * weights still do not depend on the number of rows, but a dense router's logits and the
+ * experts' sums may be added up in another order than a single row's. */
 NVMAI_API int nvmai_cuda_moe_layer_decode(nvmai_cuda_moe *h, uint32_t layer, const void *x_f16, uint32_t tokens,
                                 void *hidden_inout, void *h2_out, uint32_t *out_idx, void *out_w_f16,
                                 void *stream);
@@ -258,7 +261,8 @@ NVMAI_API int nvmai_cuda_moe_read_file_to_device(const char *path, uint64_t file
  * local-index order; map_host[e] = local index of global expert e or 0xFFFFFFFF.
  * The map is validated: every local index below n_local is named by exactly one expert
  * (NVMAI_CUDA_EINVAL for a duplicate or a gap, NVMAI_CUDA_ERANGE for an index >= n_local).
- * NULL resets. */
+ * NULL resets.  The decode entry points on a handle with a map leave the other ranks'
+ * experts out of the sum; prefill refuses one (NVMAI_CUDA_EINVAL). */
 NVMAI_API int nvmai_cuda_moe_set_expert_map(nvmai_cuda_moe *h, const uint32_t *map_host, uint32_t n_local);
 
 /* This rank's share of the routed experts for `tokens` rows that every rank holds:
@@ -358,10 +362,14 @@ NVMAI_API int nvmai_cuda_moe_stack_decode(nvmai_cuda_moe *h, const void *x0_f16,
  *   0  (default) one row: one resident kernel for the whole step when the shape allows it
  *      (top_k <= 8, shared_bits == routed_bits, d <= 16 * SM count, f and shared_f <= 1024,
  *      no expert map, stream not under capture), the staged kernels otherwise; several rows:
- *      the kernels nvmai_cuda_moe_layer_decode runs for that many rows, as a CUDA graph;
- *   1  always the staged kernels (three launches per layer, replayed as a CUDA graph);
+ *      the kernels nvmai_cuda_moe_layer_decode runs for that many rows;
+ *   1  always the staged kernels (three launches per layer);
  *   2  the resident kernel, or NVMAI_CUDA_EINVAL when the shape does not allow it.
- * Both paths give bit-identical results.  NVMAI_CUDA_DECODE_MODE in the environment sets
+ * From 8 layers on the inner layers of a step in modes 0 and 1 are replayed as a CUDA graph.
+ * One row has the same bits in all three modes, and up to 31 rows have the same in modes 0
+ * and 1; the resident kernel's 2..8 rows add a row's sum of squares up in another order
+ * between layers, which moves single fp16 values of the next layer's input by one unit in the
+ * last place.  NVMAI_CUDA_DECODE_MODE in the environment sets
  * the initial value. */
 NVMAI_API int nvmai_cuda_moe_set_decode_mode(nvmai_cuda_moe *h, int mode);
 

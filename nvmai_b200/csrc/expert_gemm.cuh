@@ -13,11 +13,11 @@
 //            memory for all tiles of a unit; epilogue -> partial[row][d]
 //
 // One block per SM runs for the whole launch and walks the units (item x feature tile, item x run of down tiles).
-// Roles (27 warps):
+// Roles (30 warps):
 //   16 producer warps  codes -> fp16 A tiles in TENSOR memory (tcgen05.st), four groups of four warps, each group every
 //                      fourth A stage (128 rows x 64 K values)
 //   8 epilogue warps   accumulators -> activations / partial rows, while the next unit's MMAs run
-//   1 MMA thread, 1 warp for the TMA loads of the packed codes and scales, 1 warp for the token rows
+//   4 warps for the token rows, 1 MMA thread, 1 warp for the TMA loads of the packed codes and scales
 //
 // Why A goes through tensor memory: with both operands in shared memory an MMA of N <= 128 columns is bound by reading
 // the 4 KB of A per instruction (measured 39 cycles at N = 16, 48 at N = 64, 64 at N = 128, and the producers' stores

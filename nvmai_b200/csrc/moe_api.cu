@@ -919,7 +919,8 @@ bool stream_ok(const nvmai_cuda_moe *h, uint32_t tokens, bool with_shared) {
 // Which experts of a batched call the streaming kernel has: those with up to `heavy` rows (>= the call's rows: all, 0: none).
 // tcgen05 pays for converting an expert's codes once per pass (4 bits of a code, parts of a scale), mma.sync for every 8
 // rows; they are level at 16 rows.  Below 6 rows per expert, evenly routed, few experts can have more and the grouped
-// launches (10 us, empty) are not worth it; above 12 per pass few have less.  Measured per layer, streaming / mixed /
+// launches (10 us, empty) are not worth it; above 12 per pass few have less.  In between the launches are made before the
+// counts are known: an evenly routed call, where no expert is taken as heavy after all (heavy_min), pays for the empty ones.  Measured per layer, streaming / mixed /
 // tcgen05, 4-bit: 256 rows even 182 / 191 / 231; skewed (popularity 1 / rank^0.6) 183 / 156 / 189, 1 / rank^1.1 159 / 117 / 130;
 // 450 rows even 257 / 239 / 240; 8-bit 256 rows (1.1) 186 / 140 / 183, 700 rows (0.4) 456 / 352 / 421.
 struct ExpertSplit { uint32_t heavy; };

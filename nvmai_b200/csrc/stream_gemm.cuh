@@ -1,9 +1,9 @@
 // Few rows per expert: the weights streamed once through the warps' own tensor-core steps (mma.sync on the codes).
 //
 // With up to 16 rows per expert the conversion of the codes to fp16 operands is what the grouped GEMMs of
-// expert_gemm.cuh spend their time on (about 90 issue slots per 1,024 codes).  mma.sync takes the codes as they are
+// expert_gemm.cuh spend their time on (154 issue slots per 1,024 codes in gate/up, everything included).  mma.sync takes the codes as they are
 // (tile_gemv.cuh: a code in the low mantissa bits of a half is an exact subnormal) and applies scale and bias once per
-// group in fp32: about 52 slots per 1,024 codes for 8 rows, 67 for 16, and nothing is rounded.  Every row's result has
+// group in fp32: 75 slots per 1,024 8-bit codes for 8 rows, everything included, and nothing is rounded.  Every row's result has
 // the bits of the single-row stages: the fp32 chains of the parts of a row (an eighth of the groups each in gate/up, a
 // half in down) and their sum run in the same order (gate_up_compute, down_warp in staged_decode.cuh).
 //
@@ -11,7 +11,8 @@
 // rows as tensor-core columns) x 64 or 128 features (phase 0: gate and up rows of each) or 256 rows of the down
 // projection (phase 1); a block takes consecutive units, so the rows of an item are staged once for several of them.
 // The codes come as boxes of 64 rows x 128 bytes, 32 KB a stage, as many stages (two to six) as the shared memory holds.  KS = 2: two warps
-// share a tile, each half of K, so that a unit is small enough to balance over the chip.
+// share a tile, each half of K, so that a unit is small enough to balance over the chip.  96 registers a thread are what 18
+// warps leave; two column blocks (NB = 2) spill 28 to 200 bytes of them.
 #pragma once
 
 #include "batch_path.h"
