@@ -44,6 +44,7 @@ struct EgParams {
     uint32_t resident;                        // phase 1: an item's rows fit the ring and stay for all tiles of a unit
     uint32_t row_slots, row_slot_bytes, row_ring_off, meta_slots, meta_slot_bytes;
     uint32_t acc_slots, acc_stride, acc_tile_off;
+    uint32_t list_ready;                      // 1: the work list was complete before the kernel in front of this one could start
     uint32_t debug_drop_rows;                 // test hook: block 0 never announces its second K block of rows, so waits run out
     unsigned int *status;
     unsigned long long *trace;
@@ -72,6 +73,7 @@ struct SgParams {
     uint32_t shared_items, units_per_item, tokens, top_k, cap, kdim, out_cols, act;
     void *out, *shared_out;                   // phase 0: activations [row][F]; phase 1: fp32 partial rows [row][D]
     uint32_t stages, meta_off, meta_bytes, x_off, raw_off, sum_off, scale_off;
+    uint32_t list_ready;                      // as in EgParams
     uint32_t beside;                          // 1: runs beside the kernel in front of it, needs only what that one waited for
     unsigned int *status;
 };

@@ -309,12 +309,17 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
     __syncthreads();
     tc_fence_after_sync();
     constexpr uint32_t tmem = 0;           // an allocation of all 512 columns starts at column 0 (checked below)
-    // the work list and the rows were written by earlier kernels in the stream
-    pdl_wait();
-    pdl_launch_dependents();
+    // The rows and what the epilogue reads come from the kernel in front; with list_ready the work list does not, so the
+    // code loads and the conversion run ahead of the wait (see stream_gemm_kernel).
+    auto wait_in_front = [&]() {
+        pdl_wait();
+        pdl_launch_dependents();
+    };
+    if (!p.list_ready) wait_in_front();
     // an earlier wait gave up: do not pile on
     bool ok = __syncthreads_and(*reinterpret_cast<volatile unsigned int *>(p.status) == 0u &&
                                 *reinterpret_cast<volatile uint32_t *>(&bars->tmem_slot) == tmem);
+    if (p.list_ready && warp >= kEgProducerWarps && warp != kEgCodeWarp) wait_in_front();
     trace_begin(p.trace);
 
     // bounded by the GPU's nanosecond timer (one second unless a test shortens it), looked at every 16 tries

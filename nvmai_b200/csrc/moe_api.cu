@@ -934,6 +934,10 @@ ExpertSplit expert_split(const nvmai_cuda_moe *h, uint32_t tokens, const Prefill
     return {P < 6 * E ? ~0u : P <= 12 * passes * E ? 16u : 0u};
 }
 
+// Was the work list complete before the kernel in front of a phase's first launch could start?  In front of gate/up stands the
+// scatter of the pairs (behind route_kernel, which makes the lists) or, for a few rows, the routing kernel itself.
+bool list_ready(int phase, uint32_t tokens) { return phase == 1 || bp_route_launches(tokens) > 1; }
+
 // One phase (0 gate/up, 1 down) of the streaming kernel over its work list and the shared expert; c as in route_rows.
 // beside: next to the grouped GEMM that was launched just before.
 int stream_phase(nvmai_cuda_moe *h, const LayerViews &lv, const nvmai_cuda_moe_config &c, int phase, const __half *x, uint32_t tokens, bool beside,
@@ -947,7 +951,7 @@ int stream_phase(nvmai_cuda_moe *h, const LayerViews &lv, const nvmai_cuda_moe_c
     p.kdim = phase == 0 ? c.d : c.f; p.out_cols = phase == 0 ? c.f : c.d;
     p.experts = u8(lv.w.experts); p.stride = lv.w.expert_stride; p.num_experts = experts;
     p.work = h->pf_work3; p.n_work = h->n_work + 1; p.sorted_pair = h->sorted_pair;
-    p.tokens = tokens; p.top_k = c.top_k; p.act = c.activation; p.status = h->status; p.beside = beside ? 1 : 0;
+    p.tokens = tokens; p.top_k = c.top_k; p.act = c.activation; p.status = h->status; p.beside = beside ? 1 : 0; p.list_ready = list_ready(phase, tokens) ? 1 : 0;
     p.shared_on = h->pf_counter + 2;
     if (phase == 0) {
         p.off_s[0] = lv.w.offsets.gate_s; p.off_b[0] = lv.w.offsets.gate_b; p.off_s[1] = lv.w.offsets.up_s; p.off_b[1] = lv.w.offsets.up_b;
@@ -1062,6 +1066,7 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     EgArgs args{};
     // gate/up
     set_common(g0, plan0); set_shared(g0, 0);
+    g0.list_ready = list_ready(0, tokens) ? 1 : 0; g1.list_ready = 1;
     g0.work = h->work; g0.n_work = h->n_work;
     g0.off_s[0] = lv.w.offsets.gate_s; g0.off_b[0] = lv.w.offsets.gate_b; g0.off_s[1] = lv.w.offsets.up_s; g0.off_b[1] = lv.w.offsets.up_b;
     g0.units_per_item = c.f / 128; g0.kfeat = c.f;

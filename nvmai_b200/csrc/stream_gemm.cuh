@@ -142,10 +142,15 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
         for (uint32_t i = 0; i < 16; ++i) mbar_init(&bars->h_full[i >> 3][i & 7], 1);
         mbar_fence_init();
     }
-    if (!p.beside) {
+    // Codes, scales and the work list do not come from the kernel in front (list_ready): the warp that requests them then does
+    // so without waiting for it, and only those that touch rows wait.  As much of a block's weights as the ring holds (up to
+    // 192 KB) is on its way while the slowest block of the kernel in front still runs and while its writes are flushed.
+    auto wait_in_front = [&]() {
         pdl_wait();
         pdl_launch_dependents();
-    }
+    };
+    if (!p.beside && !p.list_ready) wait_in_front();
+    const bool late_wait = !p.beside && p.list_ready;
     bool ok = __syncthreads_and(*reinterpret_cast<volatile unsigned int *>(p.status) == 0u);
     // the units of the launch: those of the shared items come first and are skipped where another kernel has them
     const uint32_t skip = *p.shared_on != 0u ? 0u : p.shared_items * p.units_per_item;
@@ -195,6 +200,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
         __syncwarp();
     } else if (warp == kSgWarps + 1) {
         // ---------------- rows of an item ----------------
+        if (late_wait) wait_in_front();
         uint32_t ph = 0;
         const uint32_t bytes = p.kdim * (kWideRows ? 4u : 2u);
         for (uint32_t u = u0; u < u1 && ok; u = (u / p.units_per_item + 1u) * p.units_per_item) {
@@ -215,6 +221,7 @@ __global__ void __launch_bounds__(kSgThreads + 32, 1) stream_gemm_kernel(const _
         }
     } else {
         // ---------------- compute ----------------
+        if (late_wait) wait_in_front();
         const uint32_t g = lane >> 2, t = lane & 3u;
         const uint32_t ks = KS == 2u ? warp >> 3 : 0u, tl = KS == 2u ? warp & 7u : warp;
         // the lane's rows: phase 0 gate and up of feature 8 tl + g, phase 1 rows 16 tl + g and + 8
