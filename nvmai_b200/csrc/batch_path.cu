@@ -153,7 +153,8 @@ uint32_t bp_route_blocks(uint32_t tokens) {
 cudaError_t bp_route(const RouteParams &p, cudaStream_t st) {
     if (p.tokens <= kSmallRoute) return launch_pdl(route_small_kernel, dim3(1), dim3(1024), 0, st, true, p);
     const dim3 grid(bp_route_blocks(p.tokens));
-    cudaError_t e = launch_pdl(route_kernel, grid, dim3(256), 0, st, true, p);
+    cudaError_t e = bp_tokens_per_block(p.tokens) == 8 ? launch_pdl(route_kernel<8>, grid, dim3(256), 0, st, true, p)
+                                                       : launch_pdl(route_kernel<32>, grid, dim3(1024), 0, st, true, p);
     if (e != cudaSuccess) return e;
     return launch_pdl(route_scatter_kernel, grid, dim3(256), 0, st, true, p);
 }

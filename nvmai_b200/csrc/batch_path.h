@@ -112,7 +112,9 @@ struct RouteParams {
     uint32_t *idx; __half *w;
     uint32_t tokens, E, K;
     const uint32_t *expert_map; uint32_t n_local;
-    uint32_t *block_hist; unsigned int *counter;
+    uint16_t *block_hist;                     // [block][kMaxExperts] pairs
+    uint32_t *totals, *first;                 // per expert: pairs (zero between calls), first row
+    unsigned int *counter;
     uint32_t *sorted_pair, *inv;
     // work lists: 0, 1 the grouped GEMMs' (gate/up, down) of the experts with more than `heavy` rows, 2 the streaming
     // kernel's of the others (both phases).  `heavy` is taken as "none" where those experts hold fewer than

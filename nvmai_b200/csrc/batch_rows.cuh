@@ -183,8 +183,7 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
 }
 
 // ---- top-k and grouping -----------------------------------------------------------------------
-// Tokens per block: 8 up to 1024 tokens (a warp per token), 32 above, so that the last block scans at most 128
-// histograms for a chunk of 4096.
+// Tokens (and warps) per block: 8 up to 1024 tokens, 32 above, so that a chunk of 4096 is one wave of 128 blocks.
 __host__ __device__ constexpr uint32_t bp_tokens_per_block(uint32_t tokens) { return tokens <= 1024u ? 8u : 32u; }
 
 // Expert e's work items in list j: its rows split evenly over them (two items of 70 instead of 128 + 12).
@@ -231,20 +230,24 @@ __device__ __forceinline__ void add_terms(float (&v)[kMaxExperts / 32], const Ro
 }
 
 // Router semantics of router_topk_select_k8 (moe.metal:233-285); the pairs end up in (expert, token, rank) order, as
-// PrefillMoEGrouping.groupTokenExpertPairs has them (PrefillMoEGrouping.swift:90-192).
-__global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
+// PrefillMoEGrouping.groupTokenExpertPairs has them (PrefillMoEGrouping.swift:90-192).  A warp per token.  The whole chip
+// waits while the last block makes the work lists, so that block gets by with 256 totals, which the blocks have added up
+// with atomics; where a block's own pairs begin, the scatter works out from the counts of the blocks before it.  (With four
+// tokens per warp and a last block that scanned every block's counts, 4096 rows took 33 us from the router's end to this
+// kernel's, 1531 rows 29, 256 rows 14.)
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
+    static_assert(WARPS * 32 >= kMaxExperts, "a thread per expert");
     __shared__ uint32_t hist[kMaxExperts];
     __shared__ uint32_t warp_tot[4][kMaxExperts / 32];
     __shared__ bool last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    hist[tid] = 0;
+    if (tid < kMaxExperts) hist[tid] = 0;
     pdl_wait();
     pdl_launch_dependents();
     __syncthreads();
-    const uint32_t tpb = bp_tokens_per_block(p.tokens);
-    for (uint32_t t = warp; t < tpb; t += 8u) {
-        const uint32_t tok = blockIdx.x * tpb + t;
-        if (tok >= p.tokens) break;
+    const uint32_t tok = blockIdx.x * WARPS + warp;
+    if (tok < p.tokens) {
         if (p.logits != nullptr) {
             float v[kMaxExperts / 32];
 #pragma unroll
@@ -259,42 +262,42 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
         }
     }
     __syncthreads();
-    p.block_hist[(size_t)blockIdx.x * kMaxExperts + tid] = hist[tid];
+    if (tid < kMaxExperts && hist[tid] != 0u) atomicAdd(p.totals + tid, hist[tid]);
+    if (tid < kMaxExperts / 4)      // at most 32 * kMaxTopK pairs of an expert (a caller's list may repeat one)
+        reinterpret_cast<uint2 *>(p.block_hist)[(size_t)blockIdx.x * (kMaxExperts / 4) + tid] =
+            make_uint2(hist[4 * tid] | hist[4 * tid + 1] << 16, hist[4 * tid + 2] | hist[4 * tid + 3] << 16);
     __threadfence();
     __syncthreads();
     if (tid == 0) last = atomicAdd(p.counter, 1u) == gridDim.x - 1u;
     __syncthreads();
     if (!last) return;
-    // thread e owns expert e: total, exclusive scans of the pairs and of both launches' work items
+    // thread e owns expert e: exclusive scans of the pairs and of the launches' work items
     __threadfence();
     if (tid == 0) *p.counter = 0u;
-    // (the blocks' counts come 32 at a time: this runs in one block while the chip waits; eight at a time the
-    // kernel took 24 us at 4096 rows, now 20.7)
-    constexpr uint32_t kBatch = 32;
-    uint32_t total = 0, counts[kBatch];
-    auto fetch = [&](uint32_t b0) {
-#pragma unroll
-        for (uint32_t k = 0; k < kBatch; ++k)
-            counts[k] = b0 + k < gridDim.x ? __ldcg(p.block_hist + (size_t)(b0 + k) * kMaxExperts + tid) : 0u;
-    };
-    for (uint32_t b0 = 0; b0 < gridDim.x; b0 += kBatch) {
-        fetch(b0);
-#pragma unroll
-        for (uint32_t k = 0; k < kBatch; ++k) total += counts[k];
+    uint32_t total = 0;
+    if (tid < kMaxExperts) {
+        total = __ldcg(p.totals + tid);
+        p.totals[tid] = 0u;
     }
     const uint32_t heavy = heavy_limit(p, total);
-    uint32_t mine[4] = {total, item_count(p, 0, total, heavy), item_count(p, 1, total, heavy), item_count(p, 2, total, heavy)}, pre[4];
+    uint32_t mine[4] = {}, pre[4];
+    if (tid < kMaxExperts) {
+        mine[0] = total;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        pre[j] = mine[j];
+        for (int j = 0; j < 3; ++j) mine[1 + j] = item_count(p, j, total, heavy);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, pre[j], o);
-            if (lane >= o) pre[j] += v;
+        for (int j = 0; j < 4; ++j) {
+            pre[j] = mine[j];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, pre[j], o);
+                if (lane >= o) pre[j] += v;
+            }
+            if (lane == 31) warp_tot[j][warp] = pre[j];
         }
-        if (lane == 31) warp_tot[j][warp] = pre[j];
     }
     __syncthreads();
+    if (tid >= kMaxExperts) return;
     uint32_t all[4] = {};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -304,26 +307,18 @@ __global__ void __launch_bounds__(256) route_kernel(RouteParams p) {
             all[j] += warp_tot[j][w];
         }
     }
+    p.first[tid] = pre[0];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         write_items(p, j, tid, total, mine[1 + j], pre[0], pre[1 + j]);
         if (tid == 0) p.n_work[j][0] = all[1 + j];
-    }
-    uint32_t run = pre[0];
-    for (uint32_t b0 = 0; b0 < gridDim.x; b0 += kBatch) {
-        if (gridDim.x > kBatch) fetch(b0);         // else they are still there
-#pragma unroll
-        for (uint32_t k = 0; k < kBatch; ++k)
-            if (b0 + k < gridDim.x) {
-                p.block_hist[(size_t)(b0 + k) * kMaxExperts + tid] = run;
-                run += counts[k];
-            }
     }
 }
 
 // stable scatter of a block's pairs
 __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
     __shared__ uint16_t cnt[8][kMaxExperts];
+    __shared__ uint32_t before[4][kMaxExperts];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
     for (int w = 0; w < 8; ++w) cnt[w][tid] = 0;
@@ -337,6 +332,23 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
         const uint32_t g = min(p.idx[i], p.E - 1u);
         e = p.expert_map != nullptr ? p.expert_map[g] : g;
     }
+    // the pairs of the blocks in front: a quarter of the blocks a thread, four experts each, 32 blocks' counts in flight
+    {
+        constexpr uint32_t kBatch = 32;
+        const uint32_t part = tid >> 6, quad = tid & 63;
+        uint32_t n[4] = {};
+        for (uint32_t b0 = part; b0 < blockIdx.x; b0 += 4u * kBatch) {
+            uint2 c[kBatch], sum = make_uint2(0u, 0u);
+#pragma unroll
+            for (uint32_t k = 0; k < kBatch; ++k)
+                c[k] = b0 + 4u * k < blockIdx.x
+                           ? __ldcg(reinterpret_cast<const uint2 *>(p.block_hist) + (size_t)(b0 + 4u * k) * (kMaxExperts / 4) + quad) : make_uint2(0u, 0u);
+#pragma unroll
+            for (uint32_t k = 0; k < kBatch; ++k) { sum.x += c[k].x; sum.y += c[k].y; }      // (32 x 256 fits 16 bits)
+            n[0] += sum.x & 0xFFFFu; n[1] += sum.x >> 16; n[2] += sum.y & 0xFFFFu; n[3] += sum.y >> 16;
+        }
+        *reinterpret_cast<uint4 *>(&before[part][4 * quad]) = make_uint4(n[0], n[1], n[2], n[3]);
+    }
     const bool live = e != kBpNotLocal;
     if (mine && !live) p.inv[i] = kBpNotLocal;
     const uint32_t peers = __match_any_sync(0xffffffffu, e);
@@ -345,7 +357,9 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
     if (live && rank == 0u) cnt[warp][e] = (uint16_t)__popc(peers);
     __syncthreads();
     if (live) {
-        uint32_t pos = p.block_hist[(size_t)blockIdx.x * kMaxExperts + e] + rank;
+        uint32_t pos = __ldcg(p.first + e) + rank;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) pos += before[q][e];
         for (int w = 0; w < warp; ++w) pos += cnt[w][e];
         p.sorted_pair[pos] = i;
         p.inv[i] = pos;

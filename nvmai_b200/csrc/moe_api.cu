@@ -139,7 +139,8 @@ struct nvmai_cuda_moe {
     __half *pf_sacts16 = nullptr;    // [T][Fs + extra] the shared expert's
     float *pf_rowscale = nullptr, *pf_srowscale = nullptr;   // per row: power of two taken out of a wide-range row
     float *pf_logits = nullptr;      // [terms][T][E]
-    uint32_t *pf_hist = nullptr;     // [routing blocks][256]
+    uint16_t *pf_hist = nullptr;     // [routing blocks][256]
+    uint32_t *pf_totals = nullptr, *pf_first = nullptr;     // [256]
     WorkItem *pf_work2 = nullptr;    // the down GEMM's work list (h->work is the gate/up GEMM's)
     WorkItem *pf_work3 = nullptr;    // the streaming kernel's
     unsigned int *pf_counter = nullptr;
@@ -806,7 +807,8 @@ int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
     // (the columns behind the sums are never written: they stay the zeros put there now)
     slab.want(&h->pf_acts16, P * fx * 2, true); slab.want(&h->pf_sacts16, std::max<size_t>(T * sfx * 2, 16), true);
     slab.want(&h->pf_rowscale, P * 4); slab.want(&h->pf_srowscale, T * 4);
-    slab.want(&h->pf_logits, logit_rows * c.num_experts * 4); slab.want(&h->pf_hist, blocks * kMaxExperts * 4);
+    slab.want(&h->pf_logits, logit_rows * c.num_experts * 4); slab.want(&h->pf_hist, blocks * kMaxExperts * 2);
+    slab.want(&h->pf_totals, kMaxExperts * 4, true); slab.want(&h->pf_first, kMaxExperts * 4);
     slab.want(&h->pf_work2, (size_t)h->max_work * sizeof(WorkItem)); slab.want(&h->pf_work3, (size_t)h->max_work * sizeof(WorkItem));
     slab.want(&h->pf_counter, 16, true);
     const bool ok = slab.make(h->pf_slab, st) == cudaSuccess &&
@@ -867,7 +869,7 @@ int route_rows(nvmai_cuda_moe *h, LayerViews &lv, const nvmai_cuda_moe_config &c
     r.pes = static_cast<const uint16_t *>(lv.w.per_expert_scale);
     r.idx = idx; r.w = w; r.tokens = tokens; r.E = c.num_experts; r.K = c.top_k;
     r.expert_map = h->expert_map; r.n_local = h->expert_map ? h->n_local : c.num_experts;
-    r.block_hist = h->pf_hist; r.counter = h->pf_counter; r.sorted_pair = h->sorted_pair; r.inv = h->inv;
+    r.block_hist = h->pf_hist; r.totals = h->pf_totals; r.first = h->pf_first; r.counter = h->pf_counter; r.sorted_pair = h->sorted_pair; r.inv = h->inv;
     r.work[0] = h->work; r.work[1] = h->pf_work2; r.work[2] = h->pf_work3;
     r.n_work[0] = h->n_work; r.n_work[1] = h->n_work + 2; r.n_work[2] = h->n_work + 1;      // n_work[3] stays 0
     for (int j = 0; j < 3; ++j) r.cap[j] = caps[j];
