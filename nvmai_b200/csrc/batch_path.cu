@@ -167,7 +167,8 @@ cudaError_t bp_combine(const CombineRowsParams &in, uint32_t out_dtype, cudaStre
     CombineRowsParams p = in;
     p.aligned = ((reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.hidden) | reinterpret_cast<uintptr_t>(p.hidden_delta) |
                   reinterpret_cast<uintptr_t>(p.partial_y)) & 15u) == 0 ? 1u : 0u;
-    const dim3 grid(p.tokens), block(256);
+    const bool half_rows = p.x_next == nullptr && out_dtype == OUT_F16 && p.partial_half;
+    const dim3 grid(std::min(p.tokens, p.sms * kCombineBlocks[half_rows ? 0 : 1])), block(256);
     if (p.x_next != nullptr)
         return out_dtype == OUT_F16 ? launch_pdl(combine_rows_kernel<OUT_F16, OUT_F32, true>, grid, block, 0, st, true, p)
                                     : launch_pdl(combine_rows_kernel<OUT_F32, OUT_F32, true>, grid, block, 0, st, true, p);

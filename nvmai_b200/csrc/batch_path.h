@@ -145,6 +145,7 @@ struct CombineRowsParams {
     float *partial_y;             // this rank's share only
     __half *x_next;               // or nullptr: the next block's input, half(y * rsqrt(mean(y^2) + 1e-6)); D <= kBpNormRow, decode order
     uint32_t tokens, D, K, prefill;
+    uint32_t sms;                 // SMs of the device
     uint32_t aligned;             // set by bp_combine
 };
 cudaError_t bp_combine(const CombineRowsParams &p, uint32_t out_dtype, cudaStream_t st);

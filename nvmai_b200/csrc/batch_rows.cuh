@@ -573,7 +573,7 @@ template <int PART> struct Part8 {
     }
 };
 
-// One block per token, 8 values per thread; every slot's partial row is requested before any is used (the version that
+// A block walks every gridDim-th token, 8 values per thread; every slot's partial row is requested before any is used (the version that
 // walked the slots value by value took 19-23 us for any batch).  Slot order, so the result does not depend on the
 // grouping.  PART: type of the partial rows.  Prefill rounding (prefill.metal:437-458, RealForwardRunner.swift:3560-3569):
 // every partial is rounded to the output type, h2 = out(sum_r fma(w, partial)) on its own, and the residual takes two
@@ -581,100 +581,121 @@ template <int PART> struct Part8 {
 // NORM: the row's RMS-normalised form is stored as the next block's input.  Its own variant: with the norm's code in it the
 // plain reduction of 1531 rows took 47 us instead of 26; with the partial rows kept as loaded (80 registers, three blocks
 // per SM, for half rows) it takes 20, 46 at 4096 rows.
+// The grid is what is resident at once; a row's positions and weights are requested while the row before it is added up, the
+// first one's before the wait: with a block per token and all of it behind the wait, a stack of 5 rows took 163.7 us instead of
+// 159.3, 13 rows 60.0 instead of 58.2, the reduction of 4096 rows 57 instead of 54.
+constexpr int kCombineBlocks[2] = {3, 2};      // resident per SM: half, fp32 partial rows
 template <int OUT, int PART, bool NORM>
-__global__ void __launch_bounds__(256, PART == OUT_F16 ? 3 : 2) combine_rows_kernel(CombineRowsParams p) {
-    __shared__ uint32_t pos[kMaxTopK];
-    __shared__ float wk[kMaxTopK];
+__global__ void __launch_bounds__(256, kCombineBlocks[PART == OUT_F16 ? 0 : 1]) combine_rows_kernel(CombineRowsParams p) {
+    __shared__ uint32_t pos_of[2][kMaxTopK];
+    __shared__ float weight_of[2][kMaxTopK];
     __shared__ float row[NORM ? kBpNormRow : 1];
     __shared__ float wsum[8];
+    uint32_t next_pos = 0;
+    float next_weight = 0.0f;
+    auto request = [&](uint32_t t) {
+        if (threadIdx.x >= p.K) return;
+        next_pos = p.inv[(size_t)t * p.K + threadIdx.x];
+        next_weight = __half2float(p.routing_w[(size_t)t * p.K + threadIdx.x]);
+    };
+    auto keep_requested = [&](uint32_t b) {
+        if (threadIdx.x < p.K) { pos_of[b][threadIdx.x] = next_pos; weight_of[b][threadIdx.x] = next_weight; }
+    };
+    // (the routing is from before the kernel in front)
+    request(blockIdx.x);
+    keep_requested(0);
     pdl_wait();
     pdl_launch_dependents();
-    const uint32_t tok = blockIdx.x;
-    if (threadIdx.x < p.K) {
-        pos[threadIdx.x] = p.inv[tok * p.K + threadIdx.x];
-        wk[threadIdx.x] = __half2float(p.routing_w[tok * p.K + threadIdx.x]);
-    }
     __syncthreads();
-    const float gate = p.gate_val != nullptr ? p.gate_val[tok] : 0.0f;
-    for (uint32_t d = threadIdx.x * 8u; d < p.D; d += 2048u) {
-        const size_t i = (size_t)tok * p.D + d;
-        Part8<PART> v[kMaxTopK];
-#pragma unroll
-        for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
-            if (r < p.K && pos[r] != kBpNotLocal) v[r].load(p.partial, (size_t)pos[r] * p.D + d);
-        if (p.partial_y != nullptr) {          // expert parallelism: this rank's share of the sum
-            float acc[8] = {};
+    for (uint32_t tok = blockIdx.x, buf = 0; tok < p.tokens; tok += gridDim.x, buf ^= 1u) {
+        const uint32_t *pos = pos_of[buf];
+        const float *wk = weight_of[buf];
+        const bool more = tok + gridDim.x < p.tokens;
+        if (more) request(tok + gridDim.x);
+        const float gate = p.gate_val != nullptr ? p.gate_val[tok] : 0.0f;
+        for (uint32_t d = threadIdx.x * 8u; d < p.D; d += 2048u) {
+            const size_t i = (size_t)tok * p.D + d;
+            Part8<PART> v[kMaxTopK];
 #pragma unroll
             for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
-                if (r < p.K && pos[r] != kBpNotLocal)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) acc[k] += wk[r] * v[r].at(k);
-            store_out8<OUT_F32>(p.partial_y, i, acc, p.aligned);
-            continue;
-        }
-        float h1[8] = {};
-        if (p.shared_partial != nullptr) {
-            if (p.shared_half) load_out8<OUT_F16>(p.shared_partial, i, h1); else load_out8<OUT_F32>(p.shared_partial, i, h1);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                h1[k] = round_out<OUT>(h1[k]);
-                if (p.gate_val != nullptr) h1[k] = round_out<OUT>(sigmoid_div(h1[k], gate));
-            }
-        }
-        float y[8], hid[8] = {}, delta[8] = {};
-        if (p.hidden != nullptr) load_out8<OUT>(p.hidden, i, hid, p.aligned);
-        if (p.prefill) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                float h2 = 0.0f;
+                if (r < p.K && pos[r] != kBpNotLocal) v[r].load(p.partial, (size_t)pos[r] * p.D + d);
+            if (p.partial_y != nullptr) {          // expert parallelism: this rank's share of the sum
+                float acc[8] = {};
 #pragma unroll
                 for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
-                    if (r < p.K) h2 = fmaf(wk[r], round_out<OUT>(v[r].at(k)), h2);
-                h2 = round_out<OUT>(h2);
-                y[k] = h1[k] + h2;
-                hid[k] = round_out<OUT>(hid[k] + h1[k]) + h2;
+                    if (r < p.K && pos[r] != kBpNotLocal)
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) acc[k] += wk[r] * v[r].at(k);
+                store_out8<OUT_F32>(p.partial_y, i, acc, p.aligned);
+                continue;
             }
-        } else {
+            float y[8], hid[8] = {}, delta[8] = {};
+            if (p.hidden != nullptr) load_out8<OUT>(p.hidden, i, hid, p.aligned);
             if (p.hidden_delta != nullptr) load_out8<OUT_F16>(p.hidden_delta, i, delta, p.aligned);
+            float h1[8] = {};
+            if (p.shared_partial != nullptr) {
+                if (p.shared_half) load_out8<OUT_F16>(p.shared_partial, i, h1); else load_out8<OUT_F32>(p.shared_partial, i, h1);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                float acc = h1[k];
+                for (int k = 0; k < 8; ++k) {
+                    h1[k] = round_out<OUT>(h1[k]);
+                    if (p.gate_val != nullptr) h1[k] = round_out<OUT>(sigmoid_div(h1[k], gate));
+                }
+            }
+            if (p.prefill) {
 #pragma unroll
-                for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
-                    if (r < p.K) acc += wk[r] * v[r].at(k);
-                y[k] = round_out<OUT>(acc);
-                if (p.hidden_delta != nullptr) hid[k] = round_out<OUT>(hid[k] + delta[k]);
-                hid[k] += y[k];
+                for (int k = 0; k < 8; ++k) {
+                    float h2 = 0.0f;
+#pragma unroll
+                    for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
+                        if (r < p.K) h2 = fmaf(wk[r], round_out<OUT>(v[r].at(k)), h2);
+                    h2 = round_out<OUT>(h2);
+                    y[k] = h1[k] + h2;
+                    hid[k] = round_out<OUT>(hid[k] + h1[k]) + h2;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    float acc = h1[k];
+#pragma unroll
+                    for (uint32_t r = 0; r < (uint32_t)kMaxTopK; ++r)
+                        if (r < p.K) acc += wk[r] * v[r].at(k);
+                    y[k] = round_out<OUT>(acc);
+                    if (p.hidden_delta != nullptr) hid[k] = round_out<OUT>(hid[k] + delta[k]);
+                    hid[k] += y[k];
+                }
+            }
+            if (p.y != nullptr) store_out8<OUT>(p.y, i, y, p.aligned);
+            if (p.hidden != nullptr) store_out8<OUT>(p.hidden, i, hid, p.aligned);
+            if constexpr (NORM)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) row[d + k] = y[k];
+        }
+        if (more) keep_requested(buf ^ 1u);
+        if constexpr (NORM) {
+            // the reduction tree of stage_x (staged_decode.cuh), so that a stack's rows have the bits of its layers run one by one
+            __syncthreads();
+            float keep[kBpNormRow / 256], ss = 0.0f;
+#pragma unroll
+            for (uint32_t j = 0; j < kBpNormRow / 256; ++j) {
+                const uint32_t i = threadIdx.x + j * 256u;
+                keep[j] = i < p.D ? row[i] : 0.0f;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kBpNormRow / 256; ++j) ss = fmaf(keep[j], keep[j], ss);
+            ss = warp_sum(ss);
+            if ((threadIdx.x & 31u) == 0) wsum[threadIdx.x >> 5] = ss;
+            __syncthreads();
+            float tot = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) tot += wsum[i];
+            const float sc = rsqrtf(tot / (float)p.D + 1e-6f);
+#pragma unroll
+            for (uint32_t j = 0; j < kBpNormRow / 256; ++j) {
+                const uint32_t i = threadIdx.x + j * 256u;
+                if (i < p.D) p.x_next[(size_t)tok * p.D + i] = __float2half_rn(keep[j] * sc);
             }
         }
-        if (p.y != nullptr) store_out8<OUT>(p.y, i, y, p.aligned);
-        if (p.hidden != nullptr) store_out8<OUT>(p.hidden, i, hid, p.aligned);
-        if constexpr (NORM)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) row[d + k] = y[k];
-    }
-    if constexpr (!NORM) return;
-    // the reduction tree of stage_x (staged_decode.cuh), so that a stack's rows have the bits of its layers run one by one
-    __syncthreads();
-    float keep[kBpNormRow / 256], ss = 0.0f;
-#pragma unroll
-    for (uint32_t j = 0; j < kBpNormRow / 256; ++j) {
-        const uint32_t i = threadIdx.x + j * 256u;
-        keep[j] = i < p.D ? row[i] : 0.0f;
-    }
-#pragma unroll
-    for (uint32_t j = 0; j < kBpNormRow / 256; ++j) ss = fmaf(keep[j], keep[j], ss);
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31u) == 0) wsum[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    float tot = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) tot += wsum[i];
-    const float sc = rsqrtf(tot / (float)p.D + 1e-6f);
-#pragma unroll
-    for (uint32_t j = 0; j < kBpNormRow / 256; ++j) {
-        const uint32_t i = threadIdx.x + j * 256u;
-        if (NORM && i < p.D) p.x_next[(size_t)tok * p.D + i] = __float2half_rn(keep[j] * sc);
+        __syncthreads();
     }
 }
 

@@ -996,7 +996,7 @@ int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32
     pc.partial = h->partial; pc.shared_partial = c.shared_f ? h->shared_partial : nullptr;
     pc.inv = h->inv; pc.routing_w = w; pc.gate_val = c.shared_f != 0 && c.shared_gate_kind != NVMAI_GATE_NONE ? h->gate_val : nullptr;
     pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y; pc.x_next = mode.x_next;
-    pc.tokens = tokens; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
+    pc.tokens = tokens; pc.sms = (uint32_t)h->sm_count; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
     return launched(h, bp_combine(pc, c.out_dtype, st));
 }
 
@@ -1128,7 +1128,7 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     pc.shared_partial = c.shared_f ? h->shared_partial : nullptr; pc.shared_half = wide || mixed ? 0 : 1;
     pc.inv = h->inv; pc.routing_w = w; pc.gate_val = gated ? h->gate_val : nullptr;
     pc.y = y; pc.hidden = hidden; pc.hidden_delta = mode.hidden_delta; pc.partial_y = mode.partial_y; pc.x_next = mode.x_next;
-    pc.tokens = tokens; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
+    pc.tokens = tokens; pc.sms = (uint32_t)h->sm_count; pc.D = c.d; pc.K = c.top_k; pc.prefill = mode.decode_order ? 0 : 1;
     return launched(h, bp_combine(pc, c.out_dtype, st));
 }
 
