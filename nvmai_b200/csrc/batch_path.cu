@@ -20,9 +20,10 @@ EgPlan eg_plan(EgParams &p, int phase, uint32_t want_cap) {
     const size_t fixed = 2048 + (size_t)kEgChunks * kEgChunkBytes;           // alignment slack, barriers, code ring
     p.meta_slot_bytes = 128 * n_main * 4;
     p.meta_slots = (size_t)4 * p.meta_slot_bytes <= 64 * 1024 ? 4 : 2;
-    const size_t meta = ((size_t)p.meta_slots * p.meta_slot_bytes + 1023) & ~(size_t)1023;
+    auto meta_ring = [&]() { return ((size_t)p.meta_slots * p.meta_slot_bytes + 1023) & ~(size_t)1023; };
+    size_t meta = meta_ring();
     if (fixed + meta + 2 * 2048 > kMaxBlockSmem) return EgPlan{0, 0};
-    const size_t avail = kMaxBlockSmem - fixed - meta;
+    size_t avail = kMaxBlockSmem - fixed - meta;
     uint32_t cap = (want_cap + 15) / 16 * 16;
     if (phase == 0) {
         // three K blocks of rows in flight at least
@@ -35,18 +36,21 @@ EgPlan eg_plan(EgParams &p, int phase, uint32_t want_cap) {
         cap = std::min(cap, p.resident ? fits : (uint32_t)(avail / 3 / 128) / 16 * 16);
     }
     if (cap == 0) return EgPlan{0, 0};
+    p.acc_tile_off = phase == 0 ? cap : 0;
+    p.acc_stride = phase == 0 ? 2 * cap : cap;
+    // two sets of accumulators where at least two A slots remain beside them; what is left goes to the A slots
+    p.acc_slots = 2 * p.acc_stride + 2 * kEgSlotCols <= kEgCols ? 2 : 1;
+    p.a_slots = std::min(kEgMaxPairs, (kEgCols - p.acc_slots * p.acc_stride) / kEgSlotCols);
+    p.a_col = kEgCols - p.a_slots * kEgSlotCols;
+    p.acc_slots = std::min(kEgMaxAcc, p.a_col / p.acc_stride);
+    if (phase == 0 && p.acc_slots == 1) {       // the scales of the next unit come while the accumulators are emptied
+        p.meta_slots = 2;
+        meta = meta_ring();
+        avail = kMaxBlockSmem - fixed - meta;
+    }
     p.row_slot_bytes = cap * 128;
     p.row_slots = (uint32_t)std::min<size_t>(kEgMaxRowSlots, avail / p.row_slot_bytes);
     p.row_ring_off = (uint32_t)(1024 + (size_t)kEgChunks * kEgChunkBytes + meta);
-    if (phase == 0) {
-        p.acc_slots = std::min(kEgMaxAcc, kEgAccCols / (2 * cap));
-        p.acc_stride = kEgAccCols / p.acc_slots / 32 * 32;
-        p.acc_tile_off = p.acc_stride / 2;
-    } else {
-        p.acc_slots = std::min(kEgMaxAcc, kEgAccCols / cap);
-        p.acc_stride = kEgAccCols / p.acc_slots / 16 * 16;
-        p.acc_tile_off = 0;
-    }
     p.cap = cap;
     return EgPlan{cap, fixed + meta + (size_t)p.row_slots * p.row_slot_bytes};
 }

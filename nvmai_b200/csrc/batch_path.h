@@ -44,6 +44,7 @@ struct EgParams {
     uint32_t resident;                        // phase 1: an item's rows fit the ring and stay for all tiles of a unit
     uint32_t row_slots, row_slot_bytes, row_ring_off, meta_slots, meta_slot_bytes;
     uint32_t acc_slots, acc_stride, acc_tile_off;
+    uint32_t a_slots, a_col;                  // A slots and the tensor-memory column of the first one (the last ends at 512)
     uint32_t list_ready;                      // 1: the work list was complete before the kernel in front of this one could start
     uint32_t debug_drop_rows;                 // test hook: block 0 never announces its second K block of rows, so waits run out
     unsigned int *status;

@@ -13,11 +13,15 @@
 //            memory for all tiles of a unit; epilogue -> partial[row][d]
 //
 // One block per SM runs for the whole launch and walks the units (item x feature tile, item x run of down tiles).
-// Roles (30 warps):
+// Roles (31 warps):
 //   16 producer warps  codes -> fp16 A tiles in TENSOR memory (tcgen05.st), four groups of four warps, each group every
 //                      fourth A stage (128 rows x 64 K values)
 //   8 epilogue warps   accumulators -> activations / partial rows, while the next unit's MMAs run
-//   4 warps for the token rows, 1 MMA thread, 1 warp for the TMA loads of the packed codes and scales
+//   4 warps for the token rows, 2 threads that issue MMAs (phase 0: one per tile; phase 1: one), 1 warp for the TMA loads of
+//   the packed codes and scales
+//
+// Where an item leaves room for one set of accumulators only (more than 96 rows), the MMAs wait until the epilogue has emptied
+// them and the producers have nothing to convert for, so all 24 warps empty them.
 //
 // Why A goes through tensor memory: with both operands in shared memory an MMA of N <= 128 columns is bound by reading
 // the 4 KB of A per instruction (measured 39 cycles at N = 16, 48 at N = 64, 64 at N = 128, and the producers' stores
@@ -42,16 +46,16 @@
 namespace nvmai {
 
 constexpr int kEgProducerWarps = 16, kEgEpilogueWarps = 8, kEgRowWarps = 4;
-constexpr int kEgRowWarp0 = 24, kEgMmaWarp = 28, kEgCodeWarp = 29;
-constexpr int kEgThreads = 30 * 32;
-constexpr uint32_t kEgPairs = 2;              // A slots: two stages of 128 rows x 64 fp16, 32 tensor-memory columns each
-constexpr uint32_t kEgAccCols = 384;          // accumulators: columns 0..383, A slots: 384..511
-constexpr uint32_t kEgStageCols = 32;
+constexpr int kEgRowWarp0 = 24, kEgMmaWarp = 28, kEgCodeWarp = 29, kEgMmaWarp1 = 30;
+constexpr int kEgThreads = 31 * 32;
+// Tensor memory: accumulators from column 0 on, A slots (two stages of 128 rows x 64 fp16 each) at the end.
+constexpr uint32_t kEgMaxPairs = 6;
+constexpr uint32_t kEgCols = 512, kEgStageCols = 32, kEgSlotCols = 2 * kEgStageCols;
 constexpr uint32_t kEgChunkBytes = 128 * 128; // codes of 128 rows: 128 bytes of each
 constexpr uint32_t kEgMaxRowSlots = 16, kEgMaxMeta = 4, kEgMaxAcc = 8;
 
 struct EgBarriers {
-    uint64_t a_full[kEgPairs], a_empty[kEgPairs];
+    uint64_t a_full[kEgMaxPairs][2], a_empty[kEgMaxPairs][2];      // phase 0: per tile; phase 1: [.][0]
     uint64_t c_full[kEgChunks], c_empty[kEgChunks];
     uint64_t m_full[kEgMaxMeta], m_empty[kEgMaxMeta];
     uint64_t b_full[kEgMaxRowSlots], b_empty[kEgMaxRowSlots];
@@ -252,6 +256,16 @@ __device__ __forceinline__ void eg_correction(uint32_t meta, uint32_t bias_off, 
     }
 }
 
+// g / (1 + exp(-g)) through the hardware's approximations (1 to 2 ulp: far below the fp16 operand rounding).  exp overflows to
+// infinity and a quotient below 2^-126 is flushed, 0 either way; the intrinsics' handling of subnormal arguments cost a third
+// of an epilogue.
+__device__ __forceinline__ float eg_silu(float g) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return g * r;
+}
+
 // Sum of 8 columns over the 32 lanes: lane l ends up with the sum of column (l >> 2), which column order the halving
 // steps below give: bit 4 of the lane picks columns 4-7, bit 3 the upper two of those, bit 2 the upper one.
 __device__ __forceinline__ float eg_column_sums(const float (&v)[8], uint32_t lane) {
@@ -283,6 +297,7 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
     const EgParams &p = args.p;
     constexpr uint32_t kPasses = (BITS == 8 ? 2u : 1u) * (SPLIT ? 2u : 1u);
     constexpr uint32_t kTiles = PHASE == 0 ? 2u : 1u;             // weight tiles that share a K block of rows
+    constexpr uint32_t kStreams = kTiles;                         // threads that issue MMAs, each those of a tile
     constexpr uint32_t kChunkBlocks = BITS == 4 ? 4u : 2u;        // K blocks in a chunk of 128 bytes per row
     constexpr int kSpg = PHASE == 0 ? 1 : 2;                      // correction slots per quantisation group
     extern __shared__ unsigned char eg_smem_raw[];
@@ -292,13 +307,14 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
     const uint32_t chunk_ring = base + 1024u, meta_ring = chunk_ring + kEgChunks * kEgChunkBytes;
     const uint32_t row_ring = base + p.row_ring_off;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const bool all_drain = PHASE == 0 && p.acc_slots == 1u;
 
     if (tid == 0) {
-        for (uint32_t i = 0; i < kEgPairs; ++i) { mbar_init(&bars->a_full[i], 8); mbar_init(&bars->a_empty[i], 1); }
+        for (uint32_t i = 0; i < 2 * kEgMaxPairs; ++i) { mbar_init(&bars->a_full[i / 2][i % 2], PHASE == 0 ? 4 : 8); mbar_init(&bars->a_empty[i / 2][i % 2], 1); }
         for (uint32_t i = 0; i < kEgChunks; ++i) { mbar_init(&bars->c_full[i], 1); mbar_init(&bars->c_empty[i], kEgProducerWarps); }
         for (uint32_t i = 0; i < kEgMaxMeta; ++i) { mbar_init(&bars->m_full[i], 1); mbar_init(&bars->m_empty[i], kEgProducerWarps); }
-        for (uint32_t i = 0; i < kEgMaxRowSlots; ++i) { mbar_init(&bars->b_full[i], PHASE == 0 ? kEgRowWarps * 32 : 1); mbar_init(&bars->b_empty[i], 1); }
-        for (uint32_t i = 0; i < kEgMaxAcc; ++i) { mbar_init(&bars->d_full[i], 1); mbar_init(&bars->d_empty[i], kEgEpilogueWarps); }
+        for (uint32_t i = 0; i < kEgMaxRowSlots; ++i) { mbar_init(&bars->b_full[i], PHASE == 0 ? kEgRowWarps * 32 : 1); mbar_init(&bars->b_empty[i], kStreams); }
+        for (uint32_t i = 0; i < kEgMaxAcc; ++i) { mbar_init(&bars->d_full[i], kStreams); mbar_init(&bars->d_empty[i], kEgEpilogueWarps + (all_drain ? kEgProducerWarps : 0)); }
         mbar_fence_init();
     }
     if (warp == kEgMmaWarp) {
@@ -351,6 +367,9 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
     const uint32_t n_corr = bp_extra_cols(p.kdim, kSpg) / 64u;                // correction K blocks
     const uint32_t n_kb = n_main + n_corr;
     const uint32_t n_mainv = n_main * kPasses, n_v = n_mainv + n_corr;        // A stages per tile
+    // One set of accumulators: the MMAs of the next unit wait for them, so the producers, which would wait for those, help the
+    // epilogue warps to empty it.
+    constexpr uint32_t kDrains = kEgEpilogueWarps / 4, kAllDrains = kDrains + kEgProducerWarps / 4;
     // A slots per sub-unit: phase 0 the two tiles' stages of one K block (and pass), phase 1 two consecutive stages
     const uint32_t n_pair = PHASE == 0 ? n_v : (n_v + 1u) / 2u;
     const uint32_t n_chunk = (n_main + kChunkBlocks - 1u) / kChunkBlocks;     // chunks per tile
@@ -360,29 +379,125 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
     const uint32_t total = ok ? (shared_items + p.n_work[0]) * p.units_per_item : 0u;
     const uint32_t meta_bytes = 128u * n_main * 2u;                           // scales (or biases) of a tile
 
+    // v[c] of column c -> half at `at` + c * stride, this lane's place; the lane `partner` away has the half beside it
+    auto store_pairs = [&](unsigned char *at, uint32_t stride, uint32_t live, const float (&v)[8], uint32_t partner) {
+        const bool upper = (lane & partner) != 0u;
+        const uint32_t pick = upper ? 0x3276u : 0x5410u;
+        at += upper ? stride - 2u : 0u;
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i) {
+            const __half2 own = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+            const uint32_t mine = *reinterpret_cast<const uint32_t *>(&own);
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, partner);
+            if (2u * i + (upper ? 1u : 0u) < live) *reinterpret_cast<uint32_t *>(at + 2u * i * stride) = __byte_perm(mine, other, pick);
+        }
+    };
+    // Accumulators -> activations / partial rows: every hs-th block of 8 columns from the h-th on, the warp's lane quarter.
+    // Two neighbouring columns at a time change hands between the two lanes whose features lie side by side in a row, so
+    // that a lane stores two features of one row.
+    auto drain = [&](const EgUnit &un, uint32_t sub, uint32_t acc, uint32_t h, uint32_t hs) {
+        const uint32_t q = warp & 3u;
+        const uint32_t d0 = tmem + ((q * 32u) << 16) + acc * p.acc_stride;
+        if (PHASE == 0) {
+            const uint32_t f = un.j * 128u + q * 32u + lane;
+            // byte offsets inside the unit fit 32 bits
+            const uint32_t stride = OUT == OUT_F32 ? p.kfeat * 4u : (p.kfeat + bp_extra_cols(p.kfeat, 2)) * 2u;
+            unsigned char *rows = static_cast<unsigned char *>(un.shared ? p.shared_out : p.out) + (size_t)un.start * stride;
+            const bool permuted = (un.shared ? p.shared_permute : p.permute) != 0u;
+            const uint32_t partner = permuted ? 4u : 1u;       // bp_k_position puts k and k + 4 side by side
+            const uint32_t pos = OUT == OUT_F32 ? f * 4u : (permuted ? bp_k_position(f) : f) * 2u;
+            const uint32_t slots = p.kfeat / 32u, part = lane & 3u;
+            const uint32_t sum_pos = (p.kfeat + part * slots + f / 32u) * 2u;
+            for (uint32_t cb = h * 8u; cb < un.count; cb += hs * 8u) {
+                uint32_t g8[8], u8[8];
+                tmem_ld8(d0 + cb, g8);
+                tmem_ld8(d0 + p.acc_tile_off + cb, u8);
+                tmem_ld_wait();
+                float act[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    float g = __uint_as_float(g8[i]), up = __uint_as_float(u8[i]);
+                    if (un.shared) { g = round_mid<OUT>(g); up = round_mid<OUT>(up); }     // the shared expert rounds both
+                    const float a = p.act == ACT_SILU ? eg_silu(g) : act_gelu_tanh(g);
+                    act[i] = round_mid<OUT>(a * up);
+                }
+                const uint32_t live = min(un.count - cb, 8u);
+                if (OUT == OUT_F16) {
+                    store_pairs(rows + cb * stride + pos, stride, live, act, partner);
+                } else {
+                    uint32_t at = cb * stride + pos;
+#pragma unroll
+                    for (uint32_t i = 0; i < 8u; ++i, at += stride)
+                        if (i < live) *reinterpret_cast<float *>(rows + at) = act[i];          // scaled and packed by pack_acts_kernel
+                }
+                if (OUT == OUT_F16) {          // rows as the down GEMM reads them, with their half-group sums
+                    const float sum = eg_column_sums(act, lane) * kBpSumScale;
+                    const uint32_t col = lane >> 2;
+                    const __half hi = __float2half_rn(sum);
+                    const __half lo = __float2half_rn(sum - __half2float(hi));
+                    if (part < 3u && col < live)
+                        *reinterpret_cast<__half *>(rows + (cb + col) * stride + sum_pos) = part == 1u ? lo : hi;
+                }
+            }
+        } else {
+            const uint32_t d = (un.j * n_sub + sub) * 128u + q * 32u + lane;
+            const float *scale = un.shared ? p.shared_row_scale : p.row_scale;
+            const bool half_out = un.shared ? p.shared_out_half : p.out_half;
+            const uint32_t stride = p.out_cols * (half_out ? 2u : 4u), pos = d * (half_out ? 2u : 4u);
+            unsigned char *rows = static_cast<unsigned char *>(un.shared ? p.shared_out : p.out) + (size_t)un.start * stride;
+            for (uint32_t cb = h * 8u; cb < un.count; cb += hs * 8u) {
+                uint32_t r8[8];
+                tmem_ld8(d0 + cb, r8);
+                tmem_ld_wait();
+                const uint32_t live = min(un.count - cb, 8u);
+                if (scale != nullptr) {
+                    const float mine = scale[un.start + cb + min((uint32_t)lane, live - 1u)];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) r8[i] = __float_as_uint(__uint_as_float(r8[i]) * __shfl_sync(0xffffffffu, mine, i));
+                }
+                if (half_out) {
+                    float v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r8[i]);
+                    store_pairs(rows + cb * stride + pos, stride, live, v, 1u);
+                } else {
+                    uint32_t at = cb * stride + pos;
+#pragma unroll
+                    for (uint32_t i = 0; i < 8u; ++i, at += stride)
+                        if (i < live) *reinterpret_cast<float *>(rows + at) = __uint_as_float(r8[i]);
+                }
+            }
+        }
+    };
+
     if (warp < kEgProducerWarps) {
         // ---------------- producers: codes -> fp16 tiles in tensor memory ----------------
-        // group g of four warps: A slot g >> 1, stage g & 1 of it (phase 0: the tile; phase 1: the earlier or later stage)
-        const uint32_t slot = warp >> 3, half = (warp >> 2) & 1u, row = (warp & 3u) * 32u + lane;
-        const uint32_t a_dst = (((warp & 3u) * 32u) << 16) + kEgAccCols + (warp >> 2) * kEgStageCols;
+        // group g of four warps: every other A slot from g >> 1 on, stage g & 1 of it (phase 0: the tile; phase 1: the earlier
+        // or later stage)
+        const uint32_t set = warp >> 3, half = (warp >> 2) & 1u, row = (warp & 3u) * 32u + lane;
+        const uint32_t a_dst = (((warp & 3u) * 32u) << 16) + p.a_col + half * kEgStageCols;
         // address of the row's 16-byte piece q in a chunk: (chunk + row_at) ^ (q << 4), the 128-byte swizzle
         const uint32_t row_at = chunk_ring + row * 128u + ((row & 7u) << 4);
         const uint32_t meta_at = meta_ring + row * n_main * 2u;
         const bool vec = (n_main & 7u) == 0u;
-        uint32_t pair_base = 0, use = 1;           // pairs of the launch so far; parity of the slot's next refill
+        const uint32_t mine_ab = PHASE == 0 ? half : 0u;
+        uint32_t pair_base = 0;                    // pairs of the launch so far
+        uint32_t slot = set, use = 1;              // A slot of the set's next pair; parity of its refill
+        auto next_slot = [&]() { if ((slot += 2u) >= p.a_slots) { slot -= p.a_slots; use ^= 1u; } };
         uint32_t c = 0;                            // chunks of the launch so far (all tiles')
         uint32_t m_slot = 0, m_phase = 0;          // scale tile of the sub-unit (its first one)
+        uint32_t d_phase = 0;
         // registers -> the group's stage, once the MMAs that read it last have finished
         auto publish = [&](const uint32_t (&o)[32]) {
-            ok = __all_sync(0xffffffffu, wait(&bars->a_empty[slot], use) && ok);
-            use ^= 1u;
+            ok = __all_sync(0xffffffffu, wait(&bars->a_empty[slot][mine_ab], use) && ok);
             if (!ok) return;
             tc_fence_after_sync();
-            tmem_st32(a_dst, o);
+            tmem_st32(a_dst + slot * kEgSlotCols, o);
             tmem_st_wait();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->a_full[slot]);
+            if (lane == 0) mbar_arrive(&bars->a_full[slot][mine_ab]);
+            next_slot();
         };
         // Of a chunk's K blocks j and passes a group takes every kStep-th block from `first` on, with pass `pass0` (and
         // pass0 + 2 where it has two): its share of the stages in slot order.
@@ -396,7 +511,7 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                 ok = __all_sync(0xffffffffu, wait(&bars->m_full[ms], mp));
                 if (!ok) break;
                 const uint32_t meta = meta_at + ms * p.meta_slot_bytes;
-                const uint32_t par = (pair_base ^ slot) & 1u;              // the sub-unit's pairs par, par + 2, ... use this slot
+                const uint32_t par = (pair_base ^ set) & 1u;               // the sub-unit's pairs par, par + 2, ... are this set's
                 const uint32_t first = PHASE == 0 ? (kPasses == 1u ? par : 0u) : (kPasses == 1u ? 2u * par + half : kPasses == 2u ? par : 0u);
                 const uint32_t pass0 = kPasses == 1u ? 0u : PHASE == 0 ? par : kPasses == 2u ? half : 2u * par + half;
                 uint4 scales = make_uint4(0u, 0u, 0u, 0u);
@@ -457,9 +572,9 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                         eg_correction<BITS, META, kSpg>(meta, meta_bytes, n_main, v - n_mainv, o);
                         publish(o);
                     } else {                       // an odd number of stages: the last slot is half empty
-                        ok = __all_sync(0xffffffffu, wait(&bars->a_empty[slot], use));
-                        use ^= 1u;
-                        if (ok && lane == 0) mbar_arrive(&bars->a_full[slot]);
+                        ok = __all_sync(0xffffffffu, wait(&bars->a_empty[slot][0], use));
+                        if (ok && lane == 0) mbar_arrive(&bars->a_full[slot][0]);
+                        next_slot();
                     }
                     if (!ok) break;
                 }
@@ -470,6 +585,17 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                     if (lane == 0) mbar_arrive(&bars->m_empty[m_slot]);
                     if (++m_slot == p.meta_slots) { m_slot = 0; m_phase ^= 1u; }
                 }
+            }
+            if (all_drain && ok) {
+                const EgUnit un = eg_unit(p, u, shared_items);
+                ok = __all_sync(0xffffffffu, wait(&bars->d_full[0], d_phase));
+                d_phase ^= 1u;
+                if (!ok) break;
+                tc_fence_after_sync();
+                drain(un, 0, 0, 2u + (warp >> 2), kAllDrains);
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->d_empty[0]);
             }
         }
     } else if (warp == kEgCodeWarp) {
@@ -570,10 +696,13 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                 }
             }
         }
-    } else if (warp == kEgMmaWarp) {
-        // ---------------- MMA issue: one thread ----------------
-        if (elect_one()) {
-            uint32_t pair = 0, slot = 0, phase = 0, acc = 0, acc_phase = 0;
+    } else if (warp == kEgMmaWarp || warp == kEgMmaWarp1) {
+        // ---------------- MMA issue: one thread, phase 0: one per tile ----------------
+        if ((PHASE == 0 || warp == kEgMmaWarp) && elect_one()) {
+            const uint32_t tile = PHASE == 0 && warp == kEgMmaWarp1 ? 1u : 0u;
+            uint32_t st = 0, a_phase = 0;                  // A slot of the next pair
+            auto next_pair = [&]() { if (++st == p.a_slots) { st = 0; a_phase ^= 1u; } };
+            uint32_t slot = 0, phase = 0, acc = 0, acc_phase = 0;
             const uint64_t db0 = umma_desc_sw128(row_ring);
             const uint32_t slot_step = p.row_slot_bytes >> 4;
             EgUnit next = eg_unit_or_last(p, blockIdx.x, total, shared_items);
@@ -584,26 +713,24 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                 for (uint32_t sub = 0; sub < n_sub && ok; ++sub) {
                     ok = wait(&bars->d_empty[acc], acc_phase ^ 1u);
                     if (!ok) break;
-                    const uint32_t d0 = tmem + acc * p.acc_stride, d1 = d0 + p.acc_tile_off;
+                    const uint32_t d0 = tmem + acc * p.acc_stride + tile * p.acc_tile_off;
                     if (PHASE == 0) {
                         for (uint32_t kb = 0; kb < n_kb; ++kb) {
                             ok = wait(&bars->b_full[slot], phase);
                             fence_proxy_async_smem();      // rows: generic-proxy writes -> the tensor core's reads
                             const uint64_t db = db0 + (uint64_t)(slot * slot_step);
                             const uint32_t passes = kb < n_main ? kPasses : 1u;
-                            for (uint32_t ps = 0; ps < passes; ++ps, ++pair) {
-                                const uint32_t st = pair & 1u;
-                                ok = ok && wait(&bars->a_full[st], (pair >> 1) & 1u);
+                            for (uint32_t ps = 0; ps < passes; ++ps, next_pair()) {
+                                ok = ok && wait(&bars->a_full[st][tile], a_phase);
                                 if (!ok) break;
                                 tc_fence_after_sync();
-                                const uint32_t ta = tmem + kEgAccCols + st * 2u * kEgStageCols;
+                                const uint32_t ta = tmem + p.a_col + st * kEgSlotCols + tile * kEgStageCols;
                                 const uint32_t more = (kb | ps) != 0u;
 #pragma unroll
                                 for (uint32_t k = 0; k < 4u; ++k) {      // 16 values = 8 columns of A = 32 bytes of a row of B
                                     umma_f16_ts(d0, ta + 8u * k, db + 2u * k, idesc, more | k);
-                                    umma_f16_ts(d1, ta + kEgStageCols + 8u * k, db + 2u * k, idesc, more | k);
                                 }
-                                umma_commit(&bars->a_empty[st]);
+                                umma_commit(&bars->a_empty[st][tile]);
                             }
                             if (!ok) break;
                             umma_commit(&bars->b_empty[slot]);
@@ -612,12 +739,11 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                     } else {
                         const bool keep = p.resident && sub + 1u < n_sub;     // the rows serve the next tile too
                         uint32_t bs = slot, bp = phase, kb = 0, ps = 0;
-                        for (uint32_t q = 0; q < n_pair; ++q, ++pair) {
-                            const uint32_t st = pair & 1u;
-                            ok = wait(&bars->a_full[st], (pair >> 1) & 1u);
+                        for (uint32_t q = 0; q < n_pair; ++q, next_pair()) {
+                            ok = wait(&bars->a_full[st][0], a_phase);
                             if (!ok) break;
                             tc_fence_after_sync();
-                            const uint32_t ta = tmem + kEgAccCols + st * 2u * kEgStageCols;
+                            const uint32_t ta = tmem + p.a_col + st * kEgSlotCols;
 #pragma unroll
                             for (uint32_t t = 0; t < 2u; ++t) {
                                 if (2u * q + t >= n_v) break;
@@ -634,7 +760,7 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                                 }
                             }
                             if (!ok) break;
-                            umma_commit(&bars->a_empty[st]);
+                            umma_commit(&bars->a_empty[st][0]);
                         }
                         if (!keep) { slot = bs; phase = bp; }
                     }
@@ -647,7 +773,7 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
         __syncwarp();
     } else {
         // ---------------- epilogue ----------------
-        const uint32_t q = warp & 3u, h = (warp - kEgProducerWarps) >> 2;      // lane quarter; every other 8 columns
+        const uint32_t h = (warp - kEgProducerWarps) >> 2;
         uint32_t acc = 0, acc_phase = 0;
         EgUnit next = eg_unit_or_last(p, blockIdx.x, total, shared_items);
         for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
@@ -657,75 +783,7 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
                 ok = __all_sync(0xffffffffu, wait_patient(&bars->d_full[acc], acc_phase));
                 if (!ok) break;
                 tc_fence_after_sync();
-                const uint32_t d0 = tmem + ((q * 32u) << 16) + acc * p.acc_stride;
-                if (PHASE == 0) {
-                    const uint32_t f = un.j * 128u + q * 32u + lane;
-                    // byte offsets inside the unit fit 32 bits
-                    const uint32_t stride = OUT == OUT_F32 ? p.kfeat * 4u : (p.kfeat + bp_extra_cols(p.kfeat, 2)) * 2u;
-                    unsigned char *rows = static_cast<unsigned char *>(un.shared ? p.shared_out : p.out) + (size_t)un.start * stride;
-                    const uint32_t pos = OUT == OUT_F32 ? f * 4u : ((un.shared ? p.shared_permute : p.permute) ? bp_k_position(f) : f) * 2u;
-                    const uint32_t slots = p.kfeat / 32u, part = lane & 3u;
-                    const uint32_t sum_pos = (p.kfeat + part * slots + f / 32u) * 2u;
-                    for (uint32_t cb = h * 8u; cb < un.count; cb += 16u) {
-                        uint32_t g8[8], u8[8];
-                        tmem_ld8(d0 + cb, g8);
-                        tmem_ld8(d0 + p.acc_tile_off + cb, u8);
-                        tmem_ld_wait();
-                        float act[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            float g = __uint_as_float(g8[i]), up = __uint_as_float(u8[i]);
-                            if (un.shared) { g = round_mid<OUT>(g); up = round_mid<OUT>(up); }     // the shared expert rounds both
-                            // exp and the quotient through the fast intrinsics (2 ulp): far below the fp16 operand rounding
-                            const float a = p.act == ACT_SILU ? __fdividef(g, 1.0f + __expf(-g)) : act_gelu_tanh(g);
-                            act[i] = round_mid<OUT>(a * up);
-                        }
-                        uint32_t at = cb * stride + pos;
-                        const uint32_t live = min(un.count - cb, 8u);
-#pragma unroll
-                        for (uint32_t i = 0; i < 8u; ++i, at += stride) {
-                            if (i < live) {
-                                if (OUT == OUT_F32) *reinterpret_cast<float *>(rows + at) = act[i];    // scaled and packed by pack_acts_kernel
-                                else *reinterpret_cast<__half *>(rows + at) = __float2half_rn(act[i]);
-                            }
-                        }
-                        if (OUT == OUT_F16) {          // rows as the down GEMM reads them, with their half-group sums
-                            const float sum = eg_column_sums(act, lane) * kBpSumScale;
-                            const uint32_t col = lane >> 2;
-                            const __half hi = __float2half_rn(sum);
-                            const __half lo = __float2half_rn(sum - __half2float(hi));
-                            if (part < 3u && col < live)
-                                *reinterpret_cast<__half *>(rows + (cb + col) * stride + sum_pos) = part == 1u ? lo : hi;
-                        }
-                    }
-                } else {
-                    const uint32_t d = (un.j * n_sub + sub) * 128u + q * 32u + lane;
-                    const float *scale = un.shared ? p.shared_row_scale : p.row_scale;
-                    const bool half_out = un.shared ? p.shared_out_half : p.out_half;
-                    const uint32_t stride = p.out_cols * (half_out ? 2u : 4u), pos = d * (half_out ? 2u : 4u);
-                    unsigned char *rows = static_cast<unsigned char *>(un.shared ? p.shared_out : p.out) + (size_t)un.start * stride;
-                    for (uint32_t cb = h * 8u; cb < un.count; cb += 16u) {
-                        uint32_t r8[8];
-                        tmem_ld8(d0 + cb, r8);
-                        tmem_ld_wait();
-                        const uint32_t live = min(un.count - cb, 8u);
-                        if (scale != nullptr) {
-                            const float mine = scale[un.start + cb + min((uint32_t)lane, live - 1u)];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) r8[i] = __float_as_uint(__uint_as_float(r8[i]) * __shfl_sync(0xffffffffu, mine, i));
-                        }
-                        uint32_t at = cb * stride + pos;
-                        if (half_out) {
-#pragma unroll
-                            for (uint32_t i = 0; i < 8u; ++i, at += stride)
-                                if (i < live) *reinterpret_cast<__half *>(rows + at) = __float2half_rn(__uint_as_float(r8[i]));
-                        } else {
-#pragma unroll
-                            for (uint32_t i = 0; i < 8u; ++i, at += stride)
-                                if (i < live) *reinterpret_cast<float *>(rows + at) = __uint_as_float(r8[i]);
-                        }
-                    }
-                }
+                drain(un, sub, acc, h, all_drain ? kAllDrains : kDrains);
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->d_empty[acc]);
