@@ -309,6 +309,13 @@ __global__ void __launch_bounds__(kEgThreads, 1) expert_gemm_kernel(const __grid
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const bool all_drain = PHASE == 0 && p.acc_slots == 1u;
 
+    // nothing here (a call whose experts all went to the streaming kernel): out of its way without the set-up
+    if (p.list_ready && *p.shared_on == 0u && p.n_work[0] == 0u) {
+        pdl_wait();
+        pdl_launch_dependents();
+        return;
+    }
+
     if (tid == 0) {
         for (uint32_t i = 0; i < 2 * kEgMaxPairs; ++i) { mbar_init(&bars->a_full[i / 2][i % 2], PHASE == 0 ? 4 : 8); mbar_init(&bars->a_empty[i / 2][i % 2], 1); }
         for (uint32_t i = 0; i < kEgChunks; ++i) { mbar_init(&bars->c_full[i], 1); mbar_init(&bars->c_empty[i], kEgProducerWarps); }

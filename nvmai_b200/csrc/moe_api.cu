@@ -1029,9 +1029,10 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     // Longest work item: two standard deviations above an evenly routed expert's rows, so that few experts are converted
     // twice; what the accumulators leave of the tensor memory goes to the A slots and to a second set of accumulators (up to
     // 96 rows).  Measured, 4-bit: 4096 rows 388 us (items of 160), 390 (192), 454 (128: half of the experts split); 3000 rows
-    // 308 (128), 312 (192), 372 (96); 8-bit 1531 rows 408 (64), 410 (80), 420 (96), 450 (192).
+    // 308 (128), 312 (192), 372 (96); 8-bit 1531 rows 408 (64), 410 (80), 420 (96), 450 (192).  Beside the streaming kernel an SM
+    // gets one unit or none: one set of accumulators and more A slots (256 skewed rows 109.6 us, items of 96: 111.7, of 64: 122).
     const float rows = (float)P / c.num_experts;
-    const uint32_t want = mixed ? 96 : std::min(192u, std::max(48u, ((uint32_t)(rows + 2.0f * std::sqrt(rows)) + 15) / 16 * 16));
+    const uint32_t want = mixed ? 112 : std::min(192u, std::max(48u, ((uint32_t)(rows + 2.0f * std::sqrt(rows)) + 15) / 16 * 16));
     EgParams g0{}, g1{};
     g0.kdim = c.d; g1.kdim = c.f;
     const EgPlan plan0 = eg_plan(g0, 0, want), plan1 = eg_plan(g1, 1, std::min(want, 128u));
