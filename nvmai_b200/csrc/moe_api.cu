@@ -469,7 +469,11 @@ int launch_stage2(nvmai_cuda_moe *h, const RoutedSource &src, const ExpertOffset
     }
     const uint32_t f = shared ? std::max(c.f, c.shared_f) : c.f;
     dim3 grid((f + kBlockFeatures - 1) / kBlockFeatures, n_slots + (shared ? 1 : 0), tokens);
-    const size_t smem = GateUpLayout(c.d, c.routed_bits, maps != nullptr).total;
+    size_t smem = GateUpLayout(c.d, c.routed_bits, maps != nullptr).total;
+    // Two blocks an SM hold the grid: no SM takes three then, which would leave no room for one of the next stage's blocks
+    // (26 SMs took three, and a quarter of stage 3's blocks started when these had left: 8 layers of one row 176.4 -> 172.8 us).
+    const size_t third = kMaxSmem / 3 + 1024, next = DownLayout(c.f, shared ? c.shared_f : 0, c.routed_bits, c.shared_bits, c.top_k + 1, true).total;
+    if (maps != nullptr && grid.x * grid.y * grid.z <= 2u * h->sm_count && smem < third && 2 * third + next <= kMaxSmem) smem = third;
     return dispatch_bits_meta(c.routed_bits, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
             constexpr int b = decltype(B)::value, m = decltype(M)::value, o = decltype(O)::value;
