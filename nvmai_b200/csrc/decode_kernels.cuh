@@ -320,19 +320,24 @@ __device__ __forceinline__ void topk_select_block(const float *logits, int E, in
 }
 
 // Routing weights of a selection (moe.metal:271-285): softmax over the K selected
-// scores summed in rank order, times the per-expert scale, rounded to half.
-__device__ __forceinline__ void routing_weights_warp(const uint32_t *sel_idx, const float *sel_score, int K,
-                                                     const uint16_t *pes, uint32_t *out_idx, __half *out_w) {
+// scores summed in rank order, times the per-expert scale, rounded to half.  One warp; lane k < K gets the k-th.
+__device__ __forceinline__ __half routing_weight(const uint32_t *sel_idx, const float *sel_score, int K, const uint16_t *pes) {
     const int lane = threadIdx.x & 31;
     const float top0 = sel_score[0];
     float sum_exp = 0.0f;
     for (int k = 0; k < K; ++k) sum_exp += expf(sel_score[k] - top0);
+    if (lane >= K) return __half{};
+    const float w = expf(sel_score[lane] - top0) / sum_exp;
+    const float gain = pes ? __uint_as_float(((uint32_t)ldg_u16(pes + sel_idx[lane])) << 16) : 1.0f;
+    return __float2half_rn(w * gain);
+}
+__device__ __forceinline__ void routing_weights_warp(const uint32_t *sel_idx, const float *sel_score, int K,
+                                                     const uint16_t *pes, uint32_t *out_idx, __half *out_w) {
+    const int lane = threadIdx.x & 31;
+    const __half w = routing_weight(sel_idx, sel_score, K, pes);
     if (lane < K) {
-        const uint32_t e = sel_idx[lane];
-        const float w = expf(sel_score[lane] - top0) / sum_exp;
-        const float gain = pes ? __uint_as_float(((uint32_t)ldg_u16(pes + e)) << 16) : 1.0f;
-        out_idx[lane] = e;
-        out_w[lane] = __float2half_rn(w * gain);
+        out_idx[lane] = sel_idx[lane];
+        out_w[lane] = w;
     }
 }
 
@@ -430,30 +435,24 @@ struct NextNorm {
     unsigned int *row_counter;   // [tokens], zero between calls (single-token stage only)
 };
 
-template <int OUT>
-__device__ __forceinline__ void next_norm_row(const NextNorm &nn, const void *hidden, uint32_t tok, int D, float *wsum) {
+// load(i): the row's i-th value, i < 2048 through `first`: all of a thread's at once
+template <typename First, typename Load>
+__device__ __forceinline__ bool next_norm_values(const NextNorm &nn, uint32_t tok, int D, float *wsum, First &&first, Load &&load) {
     // the first 2048 values stay in registers between the two passes, and they and their weights are requested in one
     // batch: this runs in one block while the chip waits for it
     constexpr int kKeep = 8;
     const size_t base = (size_t)tok * D;
-    auto load = [&](int i) {
-        return OUT == OUT_F16 ? __half2float(__ldcg(reinterpret_cast<const __half *>(hidden) + base + i))
-                              : __ldcg(reinterpret_cast<const float *>(hidden) + base + i);
-    };
     float keep[kKeep];
     uint16_t w[kKeep];
     float ss = 0.0f;
+    bool ok = true;
     if (threadIdx.x < 256) {
-#pragma unroll
-        for (int j = 0; j < kKeep; ++j) {
-            const int i = threadIdx.x + j * 256;
-            keep[j] = i < D ? load(i) : 0.0f;
-        }
 #pragma unroll
         for (int j = 0; j < kKeep; ++j) {
             const int i = threadIdx.x + j * 256;
             w[j] = i < D ? ldg_u16(nn.w + i) : (uint16_t)0;
         }
+        ok = first(keep);
 #pragma unroll
         for (int j = 0; j < kKeep; ++j) ss = fmaf(keep[j], keep[j], ss);
         for (int i = threadIdx.x + kKeep * 256; i < D; i += 256) {
@@ -463,7 +462,7 @@ __device__ __forceinline__ void next_norm_row(const NextNorm &nn, const void *hi
         ss = warp_sum(ss);
         if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = ss;
     }
-    __syncthreads();
+    if (!__syncthreads_and(ok)) return false;
     if (threadIdx.x < 256) {
         float tot = 0.0f;
 #pragma unroll
@@ -477,6 +476,24 @@ __device__ __forceinline__ void next_norm_row(const NextNorm &nn, const void *hi
         for (int i = threadIdx.x + kKeep * 256; i < D; i += 256)
             nn.x_next[base + i] = __float2half_rn(load(i) * sc * meta_to_float<META_BF16>(ldg_u16(nn.w + i)));
     }
+    return true;
+}
+
+template <int OUT>
+__device__ __forceinline__ void next_norm_row(const NextNorm &nn, const void *hidden, uint32_t tok, int D, float *wsum) {
+    const size_t base = (size_t)tok * D;
+    auto load = [&](int i) {
+        return OUT == OUT_F16 ? __half2float(__ldcg(reinterpret_cast<const __half *>(hidden) + base + i))
+                              : __ldcg(reinterpret_cast<const float *>(hidden) + base + i);
+    };
+    next_norm_values(nn, tok, D, wsum, [&](float (&keep)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int i = threadIdx.x + j * 256;
+            keep[j] = i < D ? load(i) : 0.0f;
+        }
+        return true;
+    }, load);
 }
 
 // Expert parallelism over peer memory (see ep_finalize_peer_kernel): where the ranks' receive buffers and

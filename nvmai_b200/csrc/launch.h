@@ -10,7 +10,7 @@ namespace nvmai {
 // Kernels here use more than the default 48 KB of dynamic shared memory; the
 // opt-in is per function and sticky, so it is raised once per (function, size).
 template <typename Kern>
-inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
+inline cudaError_t ensure_smem(Kern kern, size_t bytes, bool most_shared = false) {
     // the attribute is per device and handles may be driven from several host threads
     static std::map<std::pair<int, const void *>, size_t> granted;
     static std::mutex guard;
@@ -23,6 +23,12 @@ inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
     if (it != granted.end() && it->second >= bytes) return cudaSuccess;
     if (bytes > 40 * 1024) {        // the default limit counts the kernel's static shared memory too
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+    }
+    // An SM's split between L1 and shared memory is made for the kernel that runs and cannot change under its blocks: a kernel
+    // whose dependents are to fit beside it asks for all of the shared memory.
+    if (most_shared && it == granted.end()) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
     }
     granted[key] = bytes;
@@ -39,11 +45,11 @@ inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
 //   2. A kernel that puts its own wait off may read, until then, only what kernels before the one in front wrote, and
 //      write only what none of them and not the one in front touches: the router GEMM beside the packing of the rows
 //      (batch_rows.cuh), a streaming kernel beside the grouped GEMM of the same phase (SgParams::beside).
+//      Weights and the work list ahead of the wait (list_ready in batch_path.h) are of this kind.  Tagged words are the exception:
+//      stage 3 polls what stage 2 writes (Handover in staged_decode.cuh).
 // A kernel that lets its dependents start without having waited would break both without any sign of it.
 template <typename Kern, typename... Params>
-inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
-    cudaError_t e = ensure_smem(kern, smem);
-    if (e != cudaSuccess) return e;
+inline cudaError_t launch_granted(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -55,6 +61,11 @@ inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cud
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, p...);
+}
+template <typename Kern, typename... Params>
+inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
+    cudaError_t e = ensure_smem(kern, smem);
+    return e != cudaSuccess ? e : launch_granted(kern, grid, block, smem, st, pdl, p...);
 }
 
 }  // namespace nvmai

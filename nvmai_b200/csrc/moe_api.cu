@@ -80,6 +80,8 @@ struct EpGraphKey {
 using StackGraphKey = std::tuple<uint32_t, bool, bool>;
 constexpr size_t kMaxStackGraphs = 32;
 constexpr uint32_t kMinGraphLayers = 8;
+constexpr uint32_t kHandoverRows = 3;      // rows of a call whose decode stages hand over by tagged words
+constexpr uint32_t kHandoverNorm = 2048;   // longest row whose next norm is handed over too (next_norm_values)
 
 struct nvmai_cuda_moe {
     nvmai_cuda_moe_config cfg{};
@@ -139,6 +141,10 @@ struct nvmai_cuda_moe {
     __half *pf_sacts16 = nullptr;    // [T][Fs + extra] the shared expert's
     float *pf_rowscale = nullptr, *pf_srowscale = nullptr;   // per row: power of two taken out of a wide-range row
     float *pf_logits = nullptr;      // [terms][T][E]
+    // hand-over between the decode stages of a call: the words, the last tag given out, the call's (none between calls)
+    unsigned long long *hand_words = nullptr;
+    uint32_t hand_tag = 0;
+    Handover hand{};
     uint16_t *pf_hist = nullptr;     // [routing blocks][256]
     uint32_t *pf_totals = nullptr, *pf_first = nullptr;     // [256]
     WorkItem *pf_work2 = nullptr;    // the down GEMM's work list (h->work is the gate/up GEMM's)
@@ -290,6 +296,14 @@ int launch_kernel(nvmai_cuda_moe *h, Kern kern, dim3 grid, dim3 block, size_t sm
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return record(h, e);
 }
+// a decode stage's launch: the next stage's blocks are to fit beside its own
+template <typename Kern, typename... Params>
+int launch_stage(nvmai_cuda_moe *h, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
+    cudaError_t e = ensure_smem(kern, smem, true);
+    if (e == cudaSuccess) e = launch_granted(kern, grid, block, smem, st, pdl, p...);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return record(h, e);
+}
 // a launch made by batch_path.cu
 int launched(nvmai_cuda_moe *h, cudaError_t e, uint64_t launches = 1) {
     g_launches.fetch_add(launches, std::memory_order_relaxed);
@@ -352,7 +366,7 @@ int launch_stage1(nvmai_cuda_moe *h, const LayerViews &lv, const XSource &xsrc, 
     if (with_shared) smem = std::max(smem, GateUpLayout(c.d, c.shared_bits).total);
     return dispatch_bits_meta(c.shared_f ? c.shared_bits : 4, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
-            return launch_kernel(h, stage1_kernel<decltype(B)::value, decltype(M)::value, decltype(O)::value>,
+            return launch_stage(h, stage1_kernel<decltype(B)::value, decltype(M)::value, decltype(O)::value>,
                                  dim3(grid), dim3(kDecodeThreads), smem, st, pdl, p);
         });
     });
@@ -463,6 +477,7 @@ int launch_stage2(nvmai_cuda_moe *h, const RoutedSource &src, const ExpertOffset
     p.status = h->status;
     p.trace = h->cur_trace;
     p.n_slots = n_slots;
+    p.hand = h->hand;
     if (shared) {
         p.sgate = to_mat(shared->w.shared_gate_proj); p.sup = to_mat(shared->w.shared_up_proj);
         p.shared_f = c.shared_f; p.shared_act = h->shared_act;
@@ -477,8 +492,8 @@ int launch_stage2(nvmai_cuda_moe *h, const RoutedSource &src, const ExpertOffset
     return dispatch_bits_meta(c.routed_bits, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
             constexpr int b = decltype(B)::value, m = decltype(M)::value, o = decltype(O)::value;
-            return maps ? launch_kernel(h, stage2_kernel<b, m, o, true>, grid, dim3(kDecodeThreads), smem, st, pdl, p, *maps)
-                        : launch_kernel(h, stage2_kernel<b, m, o, false>, grid, dim3(kDecodeThreads), smem, st, pdl, p, TileMaps{});
+            return maps ? launch_stage(h, stage2_kernel<b, m, o, true>, grid, dim3(kDecodeThreads), smem, st, pdl, p, *maps)
+                        : launch_stage(h, stage2_kernel<b, m, o, false>, grid, dim3(kDecodeThreads), smem, st, pdl, p, TileMaps{});
         });
     });
 }
@@ -488,15 +503,18 @@ int launch_stage3(nvmai_cuda_moe *h, Stage3Params p, uint32_t tokens, bool pdl, 
     p.D = c.d; p.F = c.f;
     p.status = h->status;
     p.trace = h->cur_trace;
-    dim3 grid(c.d / kTileRows, tokens);
+    p.hand = h->hand;
+    if (p.next.w == nullptr || p.hidden == nullptr || c.d > kHandoverNorm) p.hand.hidden = nullptr;
+    dim3 grid(c.d / kTileRows + (p.hand.hidden != nullptr ? 1 : 0), tokens);
     const uint32_t units = p.top_k + (p.shared_f ? 1 : 0);
     const uint32_t threads = (units < 1 ? 1 : units) * kDownSplit * 32;
     const size_t smem = DownLayout(c.f, p.shared_f, c.routed_bits, p.shared_bits, units, maps != nullptr).total;
     return dispatch_bits_meta(c.routed_bits, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
             constexpr int b = decltype(B)::value, m = decltype(M)::value, o = decltype(O)::value;
-            return maps ? launch_kernel(h, stage3_kernel<b, m, o, true>, grid, dim3(threads), smem, st, pdl, p, *maps)
-                        : launch_kernel(h, stage3_kernel<b, m, o, false>, grid, dim3(threads), smem, st, pdl, p, TileMaps{});
+            if (maps && p.hand.tag != 0) return launch_stage(h, stage3_kernel<b, m, o, true, true>, grid, dim3(threads), smem, st, pdl, p, *maps);
+            return maps ? launch_stage(h, stage3_kernel<b, m, o, true, false>, grid, dim3(threads), smem, st, pdl, p, *maps)
+                        : launch_stage(h, stage3_kernel<b, m, o, false, false>, grid, dim3(threads), smem, st, pdl, p, TileMaps{});
         });
     });
 }
@@ -637,6 +655,33 @@ int grouped_tail(nvmai_cuda_moe *h, const LayerViews &lv, const __half *x_rows, 
 
 // xsrc: where stage 1 gets its rows; x_rows: the fp16 rows stages 2 reads (the
 // same buffer, or the buffer stage 1 writes its normalised rows to).
+// The words of the next call's hand-over from stage 2 to stage 3 (see Handover), or none: rows or activations that they have no
+// room for; a stream under capture, whose launches repeat with the parameters they were captured with.  The words come with the
+// first call that uses them (beside the resident kernel's exchange words they cost a stack step 3 %).
+Handover new_handover(nvmai_cuda_moe *h, uint32_t tokens, cudaStream_t st) {
+    const auto &c = h->cfg;
+    const uint32_t longest = c.out_dtype == NVMAI_OUT_FP32 ? kHandoverWide : kHandoverHalf;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (tokens > kHandoverRows || c.f > longest || c.shared_f > longest) return Handover{};
+    if (st != nullptr && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
+        cudaGetLastError();
+        return Handover{};
+    }
+    const size_t rows = std::min<size_t>(c.max_tokens, kHandoverRows), words = rows * ((size_t)c.top_k * c.f + c.shared_f + c.d);
+    if (h->hand_words == nullptr) {
+        void *w = nullptr;
+        if (cudaMalloc(&w, words * 8) != cudaSuccess || cudaMemsetAsync(w, 0, words * 8, st) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(w);
+            return Handover{};
+        }
+        h->hand_words = static_cast<unsigned long long *>(w);
+    }
+    if (++h->hand_tag == 0) ++h->hand_tag;
+    unsigned long long *acts = h->hand_words, *sact = acts + rows * c.top_k * c.f;
+    return Handover{h->hand_tag, acts, sact, sact + rows * c.shared_f};
+}
+
 int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, const __half *x_rows, uint32_t tokens,
                       void *hidden, void *h2_out, uint32_t *out_idx, __half *out_w, cudaStream_t st,
                       const LayerViews *next_layer = nullptr, const __half *hidden_delta = nullptr) {
@@ -653,6 +698,8 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
     // single-token path: the expert stages select the experts themselves from the logits
     // (the block-wide selection wants one thread per expert in the down stage's block too)
     const bool defer = !grouped && (c.top_k + (c.shared_f ? 1 : 0)) * kDownSplit * 32 >= (uint32_t)kMaxExperts;
+    struct HandGuard { nvmai_cuda_moe *h; ~HandGuard() { h->hand = Handover{}; } } hand_guard{h};
+    if (defer && maps != nullptr && (c.shared_f == 0 || shared_late)) h->hand = new_handover(h, tokens, st);
     int rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, c.shared_f != 0 && !grouped && !shared_late, c.shared_f != 0, true, st,
                            defer);
     if (rc) return rc;
@@ -1523,7 +1570,7 @@ void nvmai_cuda_moe_destroy(nvmai_cuda_moe *h) {
         for (void *p : lv.owned) cudaFree(p);
     cudaFree(h->logits); cudaFree(h->idx); cudaFree(h->w); cudaFree(h->acts); cudaFree(h->shared_act);
     cudaFree(h->gate_val); cudaFree(h->y); cudaFree(h->xnorm); cudaFree(h->counter); cudaFree(h->status);
-    cudaFree(h->stage_x); cudaFree(h->stage_y); cudaFree(h->row_counter);
+    cudaFree(h->stage_x); cudaFree(h->stage_y); cudaFree(h->row_counter); cudaFree(h->hand_words);
     cudaFree(h->sorted_pair); cudaFree(h->inv); cudaFree(h->expert_offsets); cudaFree(h->expert_counts);
     cudaFree(h->work); cudaFree(h->n_work); cudaFree(h->group_hist); cudaFree(h->trace); cudaFree(h->expert_map); cudaFree(h->partial); cudaFree(h->shared_partial);
     delete h;

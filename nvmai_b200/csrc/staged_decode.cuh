@@ -2,8 +2,21 @@
 // with bulk asynchronous copies and chained by programmatic dependent launch.
 #pragma once
 #include "decode_kernels.cuh"
+#include "tagged.cuh"
 
 namespace nvmai {
+
+// What stage 2 hands to stage 3, as tagged words (tagged.cuh): the blocks of stage 3, which are resident by then, poll the
+// activations instead of waiting until stage 2's grid has ended, its writes are flushed and the dependents are released, and then
+// fetching them (4-bit, one row: from the last block of stage 2 to the down products 2 us instead of 4).  Polling is safe because programmatic dependent launch lets
+// stage 3 start only once every block of stage 2 runs or has ended.  Stage 3 still waits for stage 2 before it lets the kernel
+// behind it start, only later.  The tag is new for every call, so that words of earlier calls never match; 0: no hand-over (a
+// captured launch, whose parameters repeat; rows or shapes that the words are not made for), plain arrays behind the wait then.
+struct Handover {
+    uint32_t tag;
+    unsigned long long *acts, *sact;     // [tokens][top_k][F], [tokens][shared_f]: fp16 outputs two halves a word, else a value a word
+    unsigned long long *hidden;          // [tokens][D] values: the new hidden state, for the next block's norm; nullptr: not wanted
+};
 
 constexpr int kRowsPerRouterBlock = 8;
 // A router block that ends with the block-wide top-k (topk_softmax_block) reuses its dynamic shared memory from
@@ -289,7 +302,7 @@ template <int BITS, int META, int OUT, bool BOXED = false, typename Late = NoLat
 __device__ __forceinline__ void gate_up_compute(unsigned char *smem, const GateUpLayout &L, int f0, int n_tiles,
                                                 int D, uint32_t act, bool round_gate_up, void *out_base,
                                                 size_t out_row_offset, unsigned int *status,
-                                                Late after_first_tile = Late()) {
+                                                Late after_first_tile = Late(), unsigned long long *words = nullptr, uint32_t tag = 0) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int groups = D / kGroup;
@@ -391,7 +404,16 @@ __device__ __forceinline__ void gate_up_compute(unsigned char *smem, const GateU
             usum += red[(tile * kDecodeWarps + w) * 16 + kTileFeatures + f];
         }
         if (round_gate_up) { gsum = round_mid<OUT>(gsum); usum = round_mid<OUT>(usum); }
-        store_mid<OUT>(out_base, out_row_offset + f0 + threadIdx.x, hidden_act(gsum, act) * usum);
+        const float v = hidden_act(gsum, act) * usum;
+        const size_t at = out_row_offset + f0 + threadIdx.x;
+        if (tag == 0) {
+            store_mid<OUT>(out_base, at, v);
+        } else if (OUT == OUT_F32) {
+            st_tagged(words + at, tag, round11(v));
+        } else {
+            const __half2 both = __floats2half2_rn(v, __shfl_down_sync((1u << (kTileFeatures * n_tiles)) - 1u, v, 1));
+            if ((threadIdx.x & 1) == 0) st_tagged_bits(words + at / 2, tag, *reinterpret_cast<const uint32_t *>(&both));
+        }
     }
 }
 
@@ -577,16 +599,19 @@ struct Stage2Params {
     AffineMat sgate, sup;
     uint32_t n_slots, shared_f;
     void *shared_act;                   // [tokens][shared_f]
+    Handover hand;
     unsigned int *status;
     unsigned long long *trace;   // optional {start, end} timestamps of this launch
 };
 
-// 64 registers, so that the next stage's blocks (which request their tiles ahead of this stage's end) fit beside two of
-// these blocks: at 101 they started when these had left, 2 us late.  It spills 48 to 124 bytes a thread, and stage 3 (56
-// registers, for the same reason) up to 190, which costs less than the late start; so it does where the tiles come as row
-// copies: 2048 / 192 without the caps, 1 row 15.3 us instead of 15.5, but 4 rows 37.3 instead of 31.6, 8 rows 65.6 instead of 54.5.
+// 56 registers where the tiles are boxes (64 elsewhere), so that a block of stage 3 fits beside two of these, which request their
+// tiles ahead of this stage's end: its 18 warps of 56 registers put five on a quarter of the SM, 8960 of 16384, and at 64 two of
+// these blocks take 8192 there.  Together with the shared memory's split (launch.h) and two blocks an SM (launch_stage2) all 128
+// blocks of stage 3 now start 1.2 to 1.8 us after this stage's selection begins; they used to start at 4.1 to 5.9, when these had
+// left (8 layers of one row: 173.6 us at 64, 171.3 at 56, 169.6 with the split).  It spills 64 to 168 bytes a thread.
+// Row copies without the caps: 2048 / 192, 1 row 15.3 us instead of 15.5, but 4 rows 37.3 instead of 31.6, 8 rows 65.6 instead of 54.5.
 template <int BITS, int META, int OUT, bool BOXED>
-__global__ void __launch_bounds__(kDecodeThreads, 4) stage2_kernel(const __grid_constant__ Stage2Params p, const __grid_constant__ TileMaps maps) {
+__global__ void __maxnreg__(BOXED ? 56 : 64) stage2_kernel(const __grid_constant__ Stage2Params p, const __grid_constant__ TileMaps maps) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *smem = BOXED ? smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u) : smem_raw;
     const GateUpLayout L(p.D, BITS, BOXED);
@@ -604,7 +629,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) stage2_kernel(const __grid_
         pdl_launch_dependents();
         if (n_tiles <= 0) return;
         if (threadIdx.x == 0) bulk_g2s(smem + L.xs, p.x + (size_t)tok * p.x_stride, p.D * 2, reinterpret_cast<uint64_t *>(smem));
-        gate_up_compute<BITS, META, OUT, BOXED>(smem, L, f0, n_tiles, p.D, p.act, true, p.shared_act, (size_t)tok * p.shared_f, p.status);
+        gate_up_compute<BITS, META, OUT, BOXED>(smem, L, f0, n_tiles, p.D, p.act, true, p.shared_act, (size_t)tok * p.shared_f, p.status,
+                                                NoLateWork(), p.hand.sact, p.hand.tag);
         trace_end(p.trace);
         return;
     }
@@ -665,7 +691,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) stage2_kernel(const __grid_
         l2_prefetch_slice(pf_blob + p.off.o[8], (size_t)p.D * (p.F / kGroup) * 2, blockIdx.x, gridDim.x, lane);
     };
     gate_up_compute<BITS, META, OUT, BOXED>(smem, L, f0, n_tiles, p.D, p.act, false, p.acts,
-                                            ((size_t)tok * p.top_k + slot) * p.F, p.status, late);
+                                            ((size_t)tok * p.top_k + slot) * p.F, p.status, late, p.hand.acts, p.hand.tag);
     trace_mark(p.trace, 4);
     trace_end(p.trace);
 }
@@ -700,6 +726,7 @@ struct Stage3Params {
     // weights): each block asks the L2 for its share
     const void *next_ptr[6]; unsigned long long next_bytes[6];
     NextNorm next;                      // optional: the block that finishes a row last also writes the next block's input
+    Handover hand;                      // with a tag: boxes, deferred selection; hand.hidden: a block past D / 16 makes the next norm
     uint32_t D, F, top_k;
     unsigned int *status;
     unsigned long long *trace;   // optional {start, end} timestamps of this launch
@@ -787,19 +814,98 @@ __device__ __forceinline__ const __half *stage_row_part(const void *rows, size_t
     return smem_row;
 }
 
+// The same from tagged words, polled.  fp32 rows, of up to kHandoverWide values: a scale is a property of the whole row, so a warp
+// polls the other warp's half too, for its magnitudes alone.
+constexpr int kHandoverHalf = 1024, kHandoverWide = 512;      // longest row handed over: fp16, fp32
+template <int OUT>
+__device__ __forceinline__ bool poll_row_part(const unsigned long long *words, uint32_t tag, int n, int begin, int count, __half *smem_row,
+                                              float &scale_up, unsigned int *status) {
+    const int lane = threadIdx.x & 31;
+    scale_up = 1.0f;
+    bool ok = true;
+    PollClock clk;
+    if (OUT == OUT_F16) {
+        for (int i = begin + lane * 8; i < begin + count && ok; i += 256) {
+            unsigned long long a, b, c, d;
+            for (;;) {
+                ld_tagged2(words + i / 2, a, b);
+                ld_tagged2(words + i / 2 + 2, c, d);
+                if (tag_is(a, tag) & tag_is(b, tag) & tag_is(c, tag) & tag_is(d, tag)) break;
+                if (clk.expired(status)) { atomicExch(status, 1u); ok = false; break; }
+            }
+            *reinterpret_cast<uint4 *>(smem_row + i) = make_uint4((uint32_t)a, (uint32_t)b, (uint32_t)c, (uint32_t)d);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        __syncwarp();
+        return ok;
+    }
+    // four pairs of values a lane: pair j at first + 64 j + 2 lane
+    auto fetch = [&](int first, int end, float (&v)[8]) {
+        for (;;) {
+            bool all = true;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = first + 64 * j + 2 * lane;
+                unsigned long long a = 0, b = 0;
+                if (i < end) {
+                    ld_tagged2(words + i, a, b);
+                    all = all & tag_is(a, tag) & tag_is(b, tag);
+                }
+                v[2 * j] = tag_val(a); v[2 * j + 1] = tag_val(b);
+            }
+            if (all) return;
+            if (clk.expired(status)) { atomicExch(status, 1u); ok = false; return; }
+        }
+    };
+    float v[8], m = 0.0f;
+    auto peak = [&]() {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) m = fmaxf(m, fabsf(v[j]));
+    };
+    const int other = begin == 0 ? begin + count : 0, other_end = begin == 0 ? n : begin;
+    fetch(other, other_end, v);
+    peak();
+    fetch(begin, begin + count, v);
+    peak();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const uint32_t ebits = (__float_as_uint(m) >> 23) & 0xFFu;
+    float scale_down = 1.0f;
+    if (ebits > 14u) {
+        scale_down = __uint_as_float((268u - ebits) << 23);
+        scale_up = __uint_as_float((ebits - 14u) << 23);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int i = begin + 64 * j + 2 * lane;
+        if (i < begin + count) *reinterpret_cast<__half2 *>(smem_row + i) = __floats2half2_rn(v[2 * j] * scale_down, v[2 * j + 1] * scale_down);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    __syncwarp();
+    return ok;
+}
+
 // one warp of the pair that owns (slot, tile): its half of the groups
-template <int BITS, int META, int OUT, bool BOXED>
+// tag != 0: act_rows are tagged words
+template <int BITS, int META, int OUT, bool BOXED, bool POLLED>
 __device__ __forceinline__ bool down_warp(unsigned char *region, const DownLayout &L, int n, int half,
                                           const void *act_rows, size_t act_offset, unsigned int *status,
-                                          float (&out)[2]) {
+                                          float (&out)[2], uint32_t tag) {
     const int lane = threadIdx.x & 31;
     const int groups = n / kGroup;
     const int gpw = (groups + kDownSplit - 1) / kDownSplit;
     const int g_begin = min(half * gpw, groups), g_end = min(g_begin + gpw, groups);
     uint64_t *bar = reinterpret_cast<uint64_t *>(region + L.bar);
     float scale_up;
-    const __half *arow = stage_row_part<OUT>(act_rows, act_offset, n, g_begin * kGroup, (g_end - g_begin) * kGroup,
-                                             reinterpret_cast<__half *>(region + L.act), scale_up);
+    const __half *arow = reinterpret_cast<const __half *>(region + L.act);
+    if constexpr (POLLED) {
+        if (!poll_row_part<OUT>(static_cast<const unsigned long long *>(act_rows) + (OUT == OUT_F16 ? act_offset / 2 : act_offset), tag, n,
+                                g_begin * kGroup, (g_end - g_begin) * kGroup, reinterpret_cast<__half *>(region + L.act), scale_up, status))
+            return false;
+    } else {
+        arow = stage_row_part<OUT>(act_rows, act_offset, n, g_begin * kGroup, (g_end - g_begin) * kGroup,
+                                   reinterpret_cast<__half *>(region + L.act), scale_up);
+    }
     float *xsum = reinterpret_cast<float *>(region + L.xsum);
     for (int base = g_begin; base < g_end; base += 4) {      // this warp's group sums of the activation row
         const int G = base + (lane >> 3);
@@ -841,7 +947,9 @@ __device__ __forceinline__ bool down_warp(unsigned char *region, const DownLayou
     return true;
 }
 
-template <int BITS, int META, int OUT, bool BOXED>
+// POLLED: the activations come as tagged words (Handover).  8 layers of one row, 4-bit: 169.6 us waiting for stage 2 and the last
+// block making the next norm, 157 like this; fp32 outputs 172 and 155.
+template <int BITS, int META, int OUT, bool BOXED, bool POLLED>
 __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32, 2) stage3_kernel(const __grid_constant__ Stage3Params p, const __grid_constant__ TileMaps maps) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *smem = BOXED ? smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u) : smem_raw;
@@ -857,6 +965,19 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32, 2) stage3_ke
     const bool routed = unit < (int)p.top_k;
     const bool shared = unit == (int)p.top_k && p.shared_f != 0;
     trace_begin(p.trace);
+    if (POLLED && row0 >= (int)p.D) {
+        // the next block's norm: a block of its own polls the row as the others finish it (the last of them to finish would
+        // have to find that out through an atomic first and then to fetch the row)
+        __shared__ float wsum_row[8];
+        for (uint32_t i = threadIdx.x * 64u; i < p.D; i += blockDim.x * 64u) l2_prefetch_line(p.next.w + i);
+        pdl_wait();
+        pdl_launch_dependents();
+        next_norm_values(p.next, tok, p.D, wsum_row, [&](float (&keep)[8]) {
+            return poll_strided<8, 256>(p.hand.hidden + (size_t)tok * p.D, threadIdx.x, p.D, p.hand.tag, keep, p.status);
+        }, [](int) { return 0.0f; });
+        trace_end(p.trace);
+        return;
+    }
     // expert tiles depend only on stage 1's indices, which are complete before this
     // kernel can start: request them before waiting for stage 2's activations
     if (p.src.logits != nullptr) {
@@ -886,13 +1007,19 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32, 2) stage3_ke
             if (p.next_ptr[i] != nullptr) l2_prefetch_slice(p.next_ptr[i], p.next_bytes[i], blockIdx.x, gridDim.x, lane);
     }
     if (p.next.w != nullptr && p.hidden != nullptr && blockIdx.x < p.D / 64 && threadIdx.x == 0) l2_prefetch_line(p.next.w + blockIdx.x * 64);
+    float *wk_s = part + (kMaxTopK + 1) * kDownSplit * 16;
+    if (POLLED && warp == 0) {       // (stage 2 publishes the same weights, too late for this one)
+        const __half w = routing_weight(reinterpret_cast<uint32_t *>(part), part + 32, p.top_k, p.src.pes);
+        if (lane < (int)p.top_k) wk_s[lane] = __half2float(w);
+    }
     __syncthreads();        // the barrier of each unit is initialised before its second warp waits on it
-    pdl_wait();
-    pdl_launch_dependents();
+    if constexpr (!POLLED) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     trace_mark(p.trace, 0);
     // routing weights for the final sum: fetched now, in parallel, instead of one dependent load per slot later
-    float *wk_s = part + (kMaxTopK + 1) * kDownSplit * 16;
-    if (threadIdx.x < p.top_k) wk_s[threadIdx.x] = __half2float(p.routing_w[(size_t)tok * p.top_k + threadIdx.x]);
+    if (!POLLED && threadIdx.x < p.top_k) wk_s[threadIdx.x] = __half2float(p.routing_w[(size_t)tok * p.top_k + threadIdx.x]);
     const float gate_v = (p.gate_val != nullptr && threadIdx.x < 16) ? p.gate_val[tok] : 0.0f;
     // likewise the hidden state and the delta this thread adds to (no other thread writes them)
     float hidden_v = 0.0f, delta_v = 0.0f;
@@ -904,12 +1031,19 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32, 2) stage3_ke
     bool ok = true;
     float v[2] = {0.0f, 0.0f};
     if (routed && local) {
-        ok = down_warp<BITS, META, OUT, BOXED>(region, L, p.F, half, p.acts, ((size_t)tok * p.top_k + unit) * p.F, p.status, v);
+        ok = down_warp<BITS, META, OUT, BOXED, POLLED>(region, L, p.F, half, POLLED ? p.hand.acts : p.acts, ((size_t)tok * p.top_k + unit) * p.F,
+                                                       p.status, v, p.hand.tag);
     } else if (shared) {
         if (p.shared_bits == 4)
-            ok = down_warp<4, META, OUT, false>(region, L, p.shared_f, half, p.shared_act, (size_t)tok * p.shared_f, p.status, v);
+            ok = down_warp<4, META, OUT, false, POLLED>(region, L, p.shared_f, half, POLLED ? p.hand.sact : p.shared_act, (size_t)tok * p.shared_f,
+                                                        p.status, v, p.hand.tag);
         else
-            ok = down_warp<8, META, OUT, false>(region, L, p.shared_f, half, p.shared_act, (size_t)tok * p.shared_f, p.status, v);
+            ok = down_warp<8, META, OUT, false, POLLED>(region, L, p.shared_f, half, POLLED ? p.hand.sact : p.shared_act, (size_t)tok * p.shared_f,
+                                                        p.status, v, p.hand.tag);
+    }
+    if (POLLED && (shared || p.shared_f == 0)) {       // one unit's warps, when their words are there: stage 2 is about to end
+        pdl_wait();
+        pdl_launch_dependents();
     }
     if (t == 0 && (routed || shared)) {
         part[(unit * kDownSplit + half) * 16 + g] = v[0];
@@ -968,11 +1102,13 @@ __global__ void __launch_bounds__((kMaxTopK + 1) * kDownSplit * 32, 2) stage3_ke
         const float yv = round_out<OUT>(acc);
         if (p.y != nullptr) store_out<OUT>(p.y, i, yv);
         if (p.hidden != nullptr) {                                                              // utility.metal:94-103
-            const float hv = p.hidden_delta != nullptr ? round_out<OUT>(hidden_v + delta_v) : hidden_v;
-            store_out<OUT>(p.hidden, i, hv + yv);
+            const float hv = round_out<OUT>((p.hidden_delta != nullptr ? round_out<OUT>(hidden_v + delta_v) : hidden_v) + yv);
+            store_out<OUT>(p.hidden, i, hv);
+            if (POLLED && p.hand.hidden != nullptr) st_tagged(p.hand.hidden + i, p.hand.tag, hv);
         }
     }
     trace_mark(p.trace, 3);
+    if (POLLED && p.hand.hidden != nullptr) { trace_end(p.trace); return; }
     if (p.next.w != nullptr && p.hidden != nullptr) {
         // the row's blocks count themselves; the one that finds the row complete normalises it for the next block
         __shared__ bool row_done;
