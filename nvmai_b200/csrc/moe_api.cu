@@ -346,6 +346,9 @@ int launch_stage1(nvmai_cuda_moe *h, const LayerViews &lv, const XSource &xsrc, 
     p.status = h->status;
     p.router_row_blocks = (c.num_experts + kRowsPerRouterBlock - 1) / kRowsPerRouterBlock;
     p.tokens_per_chunk = tokens <= 8 ? tokens : 8;
+    // few rows in front of the decode stages: a block per row and eight experts, beside the stages' other blocks (two rows one
+    // after the other, each with a norm, cost a layer 3 us)
+    if (defer_topk && !spread_rows && (p.router_row_blocks + 1) * tokens <= (uint32_t)h->sm_count) p.tokens_per_chunk = 1;
     if (spread_rows) {      // fewer rows a block while two blocks an SM hold them all (one: 31 rows 97.6 us instead of 94.8)
         const uint32_t wave = std::max(1u, 2u * (uint32_t)h->sm_count / p.router_row_blocks);
         p.tokens_per_chunk = std::min(p.tokens_per_chunk, (tokens + wave - 1) / wave);
