@@ -156,3 +156,47 @@ def test_stack_of_rows_equals_its_layers_one_by_one(rows, bits, out, d, f, exper
             x = x_next.clone()
     assert torch.equal(y, again) and bool(torch.isfinite(y).all())
     assert torch.equal(y, y1)
+
+
+# Items whose accumulators leave other numbers of A slots than the above (8 experts see every row): 62 rows, items of 80, two sets
+# and three slots; 90 rows, items of 112, one set that all warps empty and four slots; 150 rows, items of 176, one set, two slots.
+@pytest.mark.parametrize("bits,meta,out,tokens", [(4, BF16, fmt.OUT_FP16, 62), (8, FP16, fmt.OUT_FP32, 62), (4, BF16, fmt.OUT_FP32, 90),
+                                                  (8, FP16, fmt.OUT_FP16, 90), (4, FP16, fmt.OUT_FP16, 150), (8, BF16, fmt.OUT_FP16, 150)])
+@pytest.mark.parametrize("entry", ["decode", "prefill"])
+def test_items_of_every_tensor_memory_plan_match_the_oracle(bits, meta, out, tokens, entry, monkeypatch):
+    monkeypatch.setenv("NVMAI_CUDA_STREAM_ROWS", "0")
+    host = _host_layer(900 + tokens, bits, meta, 768, 384, 8)
+    cfg = MoEConfig(d=768, f=384, shared_f=384, num_experts=8, top_k=8, routed_bits=bits, shared_bits=bits, meta_dtype=meta,
+                    out_dtype=out, max_tokens=tokens)
+    assert _worst_error(host, cfg, entry, tokens, sorted({0, 31, tokens // 2, tokens - 1})) < _tol(meta, out, entry)
+
+
+# Routing in blocks of 8 tokens (up to 1024) and of 32, with a last block of one; the reduction walks more rows than its grid.
+@pytest.mark.parametrize("tokens", [33, 1024, 1025, 1409])
+def test_rows_at_the_borders_of_the_routing_blocks_match_the_oracle(tokens):
+    host = _host_layer(77, 4, BF16, 256, 128, 256)
+    cfg = MoEConfig(d=256, f=128, shared_f=128, num_experts=256, top_k=8, routed_bits=4, shared_bits=4, meta_dtype=BF16,
+                    out_dtype=fmt.OUT_FP32, max_tokens=tokens)
+    sample = sorted({t for t in (0, 7, 8, 31, 32, 443, 444, 445, 1023, 1024, tokens - 1) if t < tokens})
+    assert _worst_error(host, cfg, "prefill", tokens, sample) < _tol(BF16, fmt.OUT_FP32, "prefill")
+
+
+# A caller's routing may name one expert eight times in every row: 256 pairs of a block on one expert.  The row's share is then
+# that expert's output, eight eighths of it (fp32 additions: 8 x 2^-24).
+@pytest.mark.parametrize("tokens", [40, 1100])
+def test_an_expert_named_by_every_slot_of_every_row(tokens):
+    torch = gu.torch_cuda()
+    cfg = MoEConfig(d=256, f=128, shared_f=0, shared_gate_kind=fmt.GATE_NONE, num_experts=16, top_k=8, routed_bits=4, shared_bits=4,
+                    meta_dtype=BF16, out_dtype=fmt.OUT_FP32, max_tokens=tokens)
+    moe = MoE(cfg)
+    dev = synthetic.device_layer(5, d=256, f=128, shared_f=0, num_experts=16, routed_bits=4, shared_bits=4, meta=BF16)
+    synthetic.register_device_layer(moe, 0, dev)
+    x = torch.randn((tokens, 256), device="cuda", generator=torch.Generator(device="cuda").manual_seed(9)).half()
+    same = torch.full((tokens, 8), 3, dtype=torch.int32, device="cuda")
+    once = torch.arange(8, dtype=torch.int32, device="cuda").repeat(tokens, 1)
+    share, want = (torch.zeros((tokens, 256), device="cuda") for _ in range(2))
+    moe.routed_partial(0, x, tokens, same, torch.full((tokens, 8), 0.125, dtype=torch.float16, device="cuda"), share)
+    moe.routed_partial(0, x, tokens, once, (once == 3).half(), want)
+    moe.synchronize()
+    assert bool(torch.isfinite(want).all()) and float(want.abs().max()) > 0
+    assert float((share - want).norm() / want.norm()) < 2e-6
