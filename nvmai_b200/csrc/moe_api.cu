@@ -143,6 +143,7 @@ struct nvmai_cuda_moe {
     float *pf_logits = nullptr;      // [terms][T][E]
     // hand-over between the decode stages of a call: the words, the last tag given out, the call's (none between calls)
     unsigned long long *hand_words = nullptr;
+    bool hand_tried = false;         // asked for the words' memory
     uint32_t hand_tag = 0;
     Handover hand{};
     uint16_t *pf_hist = nullptr;     // [routing blocks][256]
@@ -671,15 +672,21 @@ Handover new_handover(nvmai_cuda_moe *h, uint32_t tokens, cudaStream_t st) {
         return Handover{};
     }
     const size_t rows = std::min<size_t>(c.max_tokens, kHandoverRows), words = rows * ((size_t)c.top_k * c.f + c.shared_f + c.d);
-    if (h->hand_words == nullptr) {
+    if (!h->hand_tried) {
+        // once, also where there is no memory for them; another stream's capture is not disturbed
+        h->hand_tried = true;
         void *w = nullptr;
-        if (cudaMalloc(&w, words * 8) != cudaSuccess || cudaMemsetAsync(w, 0, words * 8, st) != cudaSuccess) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const bool made = cudaMalloc(&w, words * 8) == cudaSuccess && cudaMemsetAsync(w, 0, words * 8, st) == cudaSuccess;
+        if (!made) {
             cudaGetLastError();
             cudaFree(w);
-            return Handover{};
         }
-        h->hand_words = static_cast<unsigned long long *>(w);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (made) h->hand_words = static_cast<unsigned long long *>(w);
     }
+    if (h->hand_words == nullptr) return Handover{};
     if (++h->hand_tag == 0) ++h->hand_tag;
     unsigned long long *acts = h->hand_words, *sact = acts + rows * c.top_k * c.f;
     return Handover{h->hand_tag, acts, sact, sact + rows * c.shared_f};
