@@ -1087,13 +1087,19 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     const bool use_map = h->expert_map != nullptr;
     const uint32_t experts = use_map ? h->n_local : c.num_experts;
 
-    // Longest work item: two standard deviations above an evenly routed expert's rows, so that few experts are converted
-    // twice; what the accumulators leave of the tensor memory goes to the A slots and to a second set of accumulators (up to
-    // 96 rows).  Measured, 4-bit: 4096 rows 388 us (items of 160), 390 (192), 454 (128: half of the experts split); 3000 rows
-    // 308 (128), 312 (192), 372 (96); 8-bit 1531 rows 408 (64), 410 (80), 420 (96), 450 (192).  Beside the streaming kernel an SM
-    // gets one unit or none: one set of accumulators and more A slots (256 skewed rows 109.6 us, items of 96: 111.7, of 64: 122).
+    // Longest work item: two standard deviations above an evenly routed expert's rows, and no shorter than 96 rows (128 above 64
+    // rows per expert), since every further item of a popular expert converts its codes again; what the accumulators leave of the
+    // tensor memory goes to the A slots and to a second set of accumulators (up to 96 rows).  Measured for items of 48 or 64 / 96 /
+    // 128 / 160 rows, evenly routed and with popularities 1 / rank^0.6 and 1 / rank^1.17:
+    //   437 rows 4-bit   217 / 220 / 226 / 215    219 / 201 / 210 / 207    130 / 112 / 116 / 119 us
+    //   1154 rows 4-bit  240 / 244 / 251 / 252    312 / 275 / 260 / 268    238 / 207 / 192 / 190
+    //   1531 rows 8-bit  408 / 415 / 422 / 422    546 / 499 / 472 / 470    408 / 398 / 351 / 327
+    //   3000 rows 4-bit  464 / 369 / 309 / 310    488 / 411 / 405 / 402    456 / 373 / 345 / 340
+    // 4096 rows 4-bit, items of 128 / 160 / 192: 422 / 386 / 399 us.  Beside the streaming kernel an SM gets one unit or none: one
+    // set of accumulators and more A slots (256 skewed rows 109.6 us, items of 96: 111.7, of 64: 122).
     const float rows = (float)P / c.num_experts;
-    const uint32_t want = mixed ? 112 : std::min(192u, std::max(48u, ((uint32_t)(rows + 2.0f * std::sqrt(rows)) + 15) / 16 * 16));
+    const uint32_t sure = ((uint32_t)(rows + 2.0f * std::sqrt(rows)) + 15) / 16 * 16;
+    const uint32_t want = mixed ? 112 : rows <= 12.0f ? 48 : std::min(192u, std::max(rows > 64.0f ? 128u : 96u, sure));
     EgParams g0{}, g1{};
     g0.kdim = c.d; g1.kdim = c.f;
     const EgPlan plan0 = eg_plan(g0, 0, want), plan1 = eg_plan(g1, 1, std::min(want, 128u));
