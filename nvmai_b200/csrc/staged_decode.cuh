@@ -605,10 +605,11 @@ struct Stage2Params {
 };
 
 // 56 registers where the tiles are boxes of 4-bit codes (64 elsewhere: two blocks of 8-bit tiles leave no shared memory; 8 layers of
-// two rows, 8-bit, 244 us at 56, 241 at 64), so that a block of stage 3 fits beside two of these, which request their tiles ahead of this stage's end: its 18 warps of 56 registers put five on a quarter of the SM, 8960 of 16384, and at 64 two of
-// these blocks take 8192 there.  Together with the shared memory's split (launch.h) and two blocks an SM (launch_stage2) all 128
-// blocks of stage 3 now start 1.2 to 1.8 us after this stage's selection begins; they used to start at 4.1 to 5.9, when these had
-// left (8 layers of one row: 173.6 us at 64, 171.3 at 56, 169.6 with the split).  It spills 64 to 168 bytes a thread.
+// two rows, 8-bit, 244 us at 56, 241 at 64), so that a block of stage 3 fits beside two of these, which request their tiles ahead of
+// this stage's end: its 18 warps of 56 registers put five on a quarter of the SM, 8960 of 16384, and at 64 two of these blocks take
+// 8192 there.  Together with the shared memory's split (launch.h) and two blocks an SM (launch_stage2) all 128 blocks of stage 3 now
+// start 1.2 to 1.8 us after this stage's selection begins; they used to start at 4.1 to 5.9, when these had left (8 layers of one row:
+// 173.6 us at 64, 171.3 at 56, 169.6 with the split).  It spills 64 to 168 bytes a thread.
 // Row copies without the caps: 2048 / 192, 1 row 15.3 us instead of 15.5, but 4 rows 37.3 instead of 31.6, 8 rows 65.6 instead of 54.5.
 template <int BITS, int META, int OUT, bool BOXED>
 __global__ void __maxnreg__(BOXED && BITS == 4 ? 56 : 64) stage2_kernel(const __grid_constant__ Stage2Params p, const __grid_constant__ TileMaps maps) {
