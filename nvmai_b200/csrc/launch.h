@@ -10,7 +10,7 @@ namespace nvmai {
 // Kernels here use more than the default 48 KB of dynamic shared memory; the
 // opt-in is per function and sticky, so it is raised once per (function, size).
 template <typename Kern>
-inline cudaError_t ensure_smem(Kern kern, size_t bytes, bool most_shared = false) {
+inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
     // the attribute is per device and handles may be driven from several host threads
     static std::map<std::pair<int, const void *>, size_t> granted;
     static std::mutex guard;
@@ -23,12 +23,6 @@ inline cudaError_t ensure_smem(Kern kern, size_t bytes, bool most_shared = false
     if (it != granted.end() && it->second >= bytes) return cudaSuccess;
     if (bytes > 40 * 1024) {        // the default limit counts the kernel's static shared memory too
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-    }
-    // An SM's split between L1 and shared memory is made for the kernel that runs and cannot change under its blocks: a kernel
-    // whose dependents are to fit beside it asks for all of the shared memory.
-    if (most_shared && it == granted.end()) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
     }
     granted[key] = bytes;
@@ -48,24 +42,35 @@ inline cudaError_t ensure_smem(Kern kern, size_t bytes, bool most_shared = false
 //      Weights and the work list ahead of the wait (list_ready in batch_path.h) are of this kind.  Tagged words are the exception:
 //      stage 3 polls what stage 2 writes (Handover in staged_decode.cuh).
 // A kernel that lets its dependents start without having waited would break both without any sign of it.
+//
+// whole_shared: an SM's split between L1 and shared memory is made for the kernel that runs and cannot change under its blocks, so a
+// kernel whose dependents are to fit beside it asks for all of the shared memory.  Asked for launch by launch: as an attribute of the
+// function it would also hold for the other handles whose layers the same function runs (six 8-bit layers of one row: 2048 / 768
+// 168 us, behind a handle of 2048 / 128 175; 1024 / 512 119, behind one of 2048 / 512 108).
 template <typename Kern, typename... Params>
-inline cudaError_t launch_granted(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
+inline cudaError_t launch_granted(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, bool whole_shared,
+                                  const Params &...p) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    if (pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (whole_shared) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[cfg.numAttrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    }
     return cudaLaunchKernelEx(&cfg, kern, p...);
 }
 template <typename Kern, typename... Params>
 inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
     cudaError_t e = ensure_smem(kern, smem);
-    return e != cudaSuccess ? e : launch_granted(kern, grid, block, smem, st, pdl, p...);
+    return e != cudaSuccess ? e : launch_granted(kern, grid, block, smem, st, pdl, false, p...);
 }
 
 }  // namespace nvmai

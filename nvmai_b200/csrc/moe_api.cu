@@ -306,8 +306,8 @@ bool stages_fit(const nvmai_cuda_moe_config &c) {
 // not: 8 layers of one row 194.8 us with the whole, 190.6 without).
 template <typename Kern, typename... Params>
 int launch_stage(nvmai_cuda_moe *h, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
-    cudaError_t e = ensure_smem(kern, smem, stages_fit(h->cfg));
-    if (e == cudaSuccess) e = launch_granted(kern, grid, block, smem, st, pdl, p...);
+    cudaError_t e = ensure_smem(kern, smem);
+    if (e == cudaSuccess) e = launch_granted(kern, grid, block, smem, st, pdl, stages_fit(h->cfg), p...);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return record(h, e);
 }
