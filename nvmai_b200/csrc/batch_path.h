@@ -114,7 +114,9 @@ struct RouteParams {
     uint32_t tokens, E, K;
     const uint32_t *expert_map; uint32_t n_local;
     uint16_t *block_hist;                     // [block][kMaxExperts] pairs
-    uint32_t *totals, *first;                 // per expert: pairs (zero between calls), first row
+    // [segment of blocks][kMaxExperts]: an expert's pairs (zero between calls); its first row and, behind the first segment's, the
+    // pairs of the segments in front
+    uint32_t *totals, *first;
     unsigned int *counter;
     uint32_t *sorted_pair, *inv;
     // work lists: 0, 1 the grouped GEMMs' (gate/up, down) of the experts with more than `heavy` rows, 2 the streaming
@@ -124,6 +126,8 @@ struct RouteParams {
     WorkItem *work[3]; uint32_t *n_work[3]; uint32_t cap[3]; uint32_t heavy, heavy_min;
 };
 uint32_t bp_route_blocks(uint32_t tokens);
+constexpr uint32_t kRouteSegment = 128;       // routing blocks whose counts a block of the scatter adds up itself
+__host__ __device__ constexpr uint32_t bp_route_segments(uint32_t blocks) { return (blocks + kRouteSegment - 1u) / kRouteSegment; }
 constexpr uint32_t kSmallRoute = 32;          // up to this many tokens one block does it all
 cudaError_t bp_route(const RouteParams &p, cudaStream_t st);
 inline uint64_t bp_route_launches(uint32_t tokens) { return tokens <= kSmallRoute ? 1 : 2; }

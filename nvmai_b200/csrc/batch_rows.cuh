@@ -231,10 +231,11 @@ __device__ __forceinline__ void add_terms(float (&v)[kMaxExperts / 32], const Ro
 
 // Router semantics of router_topk_select_k8 (moe.metal:233-285); the pairs end up in (expert, token, rank) order, as
 // PrefillMoEGrouping.groupTokenExpertPairs has them (PrefillMoEGrouping.swift:90-192).  A warp per token.  The whole chip
-// waits while the last block makes the work lists, so that block gets by with 256 totals, which the blocks have added up
-// with atomics; where a block's own pairs begin, the scatter works out from the counts of the blocks before it.  (With four
-// tokens per warp and a last block that scanned every block's counts, 4096 rows took 33 us from the router's end to this
-// kernel's, 1531 rows 29, 256 rows 14.)
+// waits while the last block makes the work lists, so that block gets by with 256 totals a segment of 128 blocks, which the
+// blocks have added up with atomics; where a block's own pairs begin, the scatter works out from the counts of the blocks before
+// it in its segment: one segment up to 4096 rows; counts of all blocks in front would grow with the square of the rows (256 /
+// 128 wide, 262,144 rows: 5519 us, 4940 with segments; 4096 rows 112 either way).  (With four tokens per warp and a last block that
+// scanned every block's counts, 4096 rows took 33 us from the router's end to this kernel's, 1531 rows 29, 256 rows 14.)
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
     static_assert(WARPS * 32 >= kMaxExperts, "a thread per expert");
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
         }
     }
     __syncthreads();
-    if (tid < kMaxExperts && hist[tid] != 0u) atomicAdd(p.totals + tid, hist[tid]);
+    if (tid < kMaxExperts && hist[tid] != 0u) atomicAdd(p.totals + blockIdx.x / kRouteSegment * kMaxExperts + tid, hist[tid]);
     if (tid < kMaxExperts / 4)      // at most 32 * kMaxTopK pairs of an expert (a caller's list may repeat one)
         reinterpret_cast<uint2 *>(p.block_hist)[(size_t)blockIdx.x * (kMaxExperts / 4) + tid] =
             make_uint2(hist[4 * tid] | hist[4 * tid + 1] << 16, hist[4 * tid + 2] | hist[4 * tid + 3] << 16);
@@ -276,8 +277,12 @@ __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
     if (tid == 0) *p.counter = 0u;
     uint32_t total = 0;
     if (tid < kMaxExperts) {
-        total = __ldcg(p.totals + tid);
-        p.totals[tid] = 0u;
+        for (uint32_t i = tid; i < bp_route_segments(gridDim.x) * kMaxExperts; i += kMaxExperts) {
+            const uint32_t n = __ldcg(p.totals + i);
+            p.totals[i] = 0u;
+            if (i >= (uint32_t)kMaxExperts) p.first[i] = total;
+            total += n;
+        }
     }
     const uint32_t heavy = heavy_limit(p, total);
     uint32_t mine[4] = {}, pre[4];
@@ -332,22 +337,19 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
         const uint32_t g = min(p.idx[i], p.E - 1u);
         e = p.expert_map != nullptr ? p.expert_map[g] : g;
     }
-    // the pairs of the blocks in front: a quarter of the blocks a thread, four experts each, 32 blocks' counts in flight
+    // the pairs of the segment's blocks in front: a quarter of the blocks a thread, four experts each, all counts in flight
+    const uint32_t segment = blockIdx.x / kRouteSegment;
     {
-        constexpr uint32_t kBatch = 32;
-        const uint32_t part = tid >> 6, quad = tid & 63;
-        uint32_t n[4] = {};
-        for (uint32_t b0 = part; b0 < blockIdx.x; b0 += 4u * kBatch) {
-            uint2 c[kBatch], sum = make_uint2(0u, 0u);
+        constexpr uint32_t kBatch = kRouteSegment / 4u;
+        const uint32_t part = tid >> 6, quad = tid & 63, b0 = segment * kRouteSegment + part;
+        uint2 c[kBatch], sum = make_uint2(0u, 0u);
 #pragma unroll
-            for (uint32_t k = 0; k < kBatch; ++k)
-                c[k] = b0 + 4u * k < blockIdx.x
-                           ? __ldcg(reinterpret_cast<const uint2 *>(p.block_hist) + (size_t)(b0 + 4u * k) * (kMaxExperts / 4) + quad) : make_uint2(0u, 0u);
+        for (uint32_t k = 0; k < kBatch; ++k)
+            c[k] = b0 + 4u * k < blockIdx.x
+                       ? __ldcg(reinterpret_cast<const uint2 *>(p.block_hist) + (size_t)(b0 + 4u * k) * (kMaxExperts / 4) + quad) : make_uint2(0u, 0u);
 #pragma unroll
-            for (uint32_t k = 0; k < kBatch; ++k) { sum.x += c[k].x; sum.y += c[k].y; }      // (32 x 256 fits 16 bits)
-            n[0] += sum.x & 0xFFFFu; n[1] += sum.x >> 16; n[2] += sum.y & 0xFFFFu; n[3] += sum.y >> 16;
-        }
-        *reinterpret_cast<uint4 *>(&before[part][4 * quad]) = make_uint4(n[0], n[1], n[2], n[3]);
+        for (uint32_t k = 0; k < kBatch; ++k) { sum.x += c[k].x; sum.y += c[k].y; }      // (32 x 256 fits 16 bits)
+        *reinterpret_cast<uint4 *>(&before[part][4 * quad]) = make_uint4(sum.x & 0xFFFFu, sum.x >> 16, sum.y & 0xFFFFu, sum.y >> 16);
     }
     const bool live = e != kBpNotLocal;
     if (mine && !live) p.inv[i] = kBpNotLocal;
@@ -358,6 +360,7 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
     __syncthreads();
     if (live) {
         uint32_t pos = __ldcg(p.first + e) + rank;
+        if (segment != 0u) pos += __ldcg(p.first + segment * kMaxExperts + e);
 #pragma unroll
         for (int q = 0; q < 4; ++q) pos += before[q][e];
         for (int w = 0; w < warp; ++w) pos += cnt[w][e];

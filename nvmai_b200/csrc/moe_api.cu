@@ -147,7 +147,7 @@ struct nvmai_cuda_moe {
     uint32_t hand_tag = 0;
     Handover hand{};
     uint16_t *pf_hist = nullptr;     // [routing blocks][256]
-    uint32_t *pf_totals = nullptr, *pf_first = nullptr;     // [256]
+    uint32_t *pf_totals = nullptr, *pf_first = nullptr;     // [segments of routing blocks][256]
     WorkItem *pf_work2 = nullptr;    // the down GEMM's work list (h->work is the gate/up GEMM's)
     WorkItem *pf_work3 = nullptr;    // the streaming kernel's
     unsigned int *pf_counter = nullptr;
@@ -876,7 +876,8 @@ int ensure_prefill_scratch(nvmai_cuda_moe *h, cudaStream_t st) {
     slab.want(&h->pf_acts16, P * fx * 2, true); slab.want(&h->pf_sacts16, std::max<size_t>(T * sfx * 2, 16), true);
     slab.want(&h->pf_rowscale, P * 4); slab.want(&h->pf_srowscale, T * 4);
     slab.want(&h->pf_logits, logit_rows * c.num_experts * 4); slab.want(&h->pf_hist, blocks * kMaxExperts * 2);
-    slab.want(&h->pf_totals, kMaxExperts * 4, true); slab.want(&h->pf_first, kMaxExperts * 4);
+    const size_t segments = bp_route_segments((uint32_t)blocks);
+    slab.want(&h->pf_totals, segments * kMaxExperts * 4, true); slab.want(&h->pf_first, segments * kMaxExperts * 4);
     slab.want(&h->pf_work2, (size_t)h->max_work * sizeof(WorkItem)); slab.want(&h->pf_work3, (size_t)h->max_work * sizeof(WorkItem));
     slab.want(&h->pf_counter, 16, true);
     const bool ok = slab.make(h->pf_slab, st) == cudaSuccess &&
