@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "batch_path.h"
+#include "stage_room.h"
 #include "ep_comm.cuh"
 #include "grouped_decode.cuh"
 #include "launch.h"
@@ -146,6 +147,7 @@ struct nvmai_cuda_moe {
     bool hand_tried = false;         // asked for the words' memory
     uint32_t hand_tag = 0;
     Handover hand{};
+    StageRoom room{};                // of the call's decode stages (between calls: nothing)
     uint16_t *pf_hist = nullptr;     // [routing blocks][256]
     uint32_t *pf_totals = nullptr, *pf_first = nullptr;     // [segments of routing blocks][256]
     WorkItem *pf_work2 = nullptr;    // the down GEMM's work list (h->work is the gate/up GEMM's)
@@ -298,16 +300,19 @@ int launch_kernel(nvmai_cuda_moe *h, Kern kern, dim3 grid, dim3 block, size_t sm
     return record(h, e);
 }
 constexpr size_t kMaxSmem = 227 * 1024;
-// Do a block of stage 3 and two of stage 2 fit on an SM (4-bit tiles of 2048 / 512 do, 8-bit ones do not)?
-bool stages_fit(const nvmai_cuda_moe_config &c) {
-    return 2 * GateUpLayout(c.d, c.routed_bits, true).total + DownLayout(c.f, c.shared_f, c.routed_bits, c.shared_bits, c.top_k + 1, true).total <= kMaxSmem;
+// The room of a call's decode stages (see StageRoom); with_shared: the shared expert's gate/up tiles run in stage 2.
+StageRoom decode_room(const nvmai_cuda_moe *h, uint32_t tokens, bool boxed, bool with_shared) {
+    const auto &c = h->cfg;
+    const uint32_t f = with_shared ? std::max(c.f, c.shared_f) : c.f, units = c.top_k + (c.shared_f ? 1 : 0);
+    const uint32_t blocks = (f + kBlockFeatures - 1) / kBlockFeatures * (c.top_k + (with_shared ? 1 : 0)) * tokens;
+    return stage_room(GateUpLayout(c.d, c.routed_bits, boxed).total, DownLayout(c.f, c.shared_f, c.routed_bits, c.shared_bits, units, boxed).total,
+                      blocks, (uint32_t)h->sm_count, units * kDownSplit, boxed);
 }
-// A decode stage's launch: where the next stage's blocks fit beside its own it asks for the whole shared memory (8-bit, where they do
-// not: 8 layers of one row 194.8 us with the whole, 190.6 without).
+// A decode stage's launch.
 template <typename Kern, typename... Params>
 int launch_stage(nvmai_cuda_moe *h, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const Params &...p) {
     cudaError_t e = ensure_smem(kern, smem);
-    if (e == cudaSuccess) e = launch_granted(kern, grid, block, smem, st, pdl, stages_fit(h->cfg), p...);
+    if (e == cudaSuccess) e = launch_granted(kern, grid, block, smem, st, pdl, h->room.whole_shared, p...);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return record(h, e);
 }
@@ -496,12 +501,13 @@ int launch_stage2(nvmai_cuda_moe *h, const RoutedSource &src, const ExpertOffset
     // Two blocks an SM hold the grid: no SM takes three then, which would leave no room for one of the next stage's blocks
     // (26 SMs took three, and a quarter of stage 3's blocks started when these had left: 8 layers of one row 176.4 -> 172.8 us).
     const size_t third = kMaxSmem / 3 + 1024, next = DownLayout(c.f, shared ? c.shared_f : 0, c.routed_bits, c.shared_bits, c.top_k + 1, true).total;
-    if (maps != nullptr && grid.x * grid.y * grid.z <= 2u * h->sm_count && smem < third && 2 * third + next <= kMaxSmem) smem = third;
+    if (h->room.early && grid.x * grid.y * grid.z <= 2u * h->sm_count && smem < third && 2 * third + next <= kMaxSmem) smem = third;
     return dispatch_bits_meta(c.routed_bits, c.meta_dtype, [&](auto B, auto M) {
         return dispatch_out(c.out_dtype, [&](auto O) {
             constexpr int b = decltype(B)::value, m = decltype(M)::value, o = decltype(O)::value;
-            return maps ? launch_stage(h, stage2_kernel<b, m, o, true>, grid, dim3(kDecodeThreads), smem, st, pdl, p, *maps)
-                        : launch_stage(h, stage2_kernel<b, m, o, false>, grid, dim3(kDecodeThreads), smem, st, pdl, p, TileMaps{});
+            if (maps && h->room.lean) return launch_stage(h, stage2_kernel<b, m, o, true, true>, grid, dim3(kDecodeThreads), smem, st, pdl, p, *maps);
+            return maps ? launch_stage(h, stage2_kernel<b, m, o, true, false>, grid, dim3(kDecodeThreads), smem, st, pdl, p, *maps)
+                        : launch_stage(h, stage2_kernel<b, m, o, false, false>, grid, dim3(kDecodeThreads), smem, st, pdl, p, TileMaps{});
         });
     });
 }
@@ -671,9 +677,14 @@ Handover new_handover(nvmai_cuda_moe *h, uint32_t tokens, cudaStream_t st) {
     const uint32_t longest = c.out_dtype == NVMAI_OUT_FP32 ? kHandoverWide : kHandoverHalf;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (tokens > kHandoverRows || c.f > longest || c.shared_f > longest) return Handover{};
-    // One row's blocks of stage 2 all start at once; where stage 3's find no room beside two of them (8-bit tiles), there is nothing to
-    // poll for (8 layers, fp16 / fp32 outputs: 189.6 / 199.6 us, 188.3 / 198.6 without; two rows 244 / 257, 255 / 261 without).
-    if (tokens == 1 && !stages_fit(c)) return Handover{};
+    if (!h->room.early) {
+        // One row's blocks of stage 2 all start at once; where stage 3's find no room beside two of them (8-bit tiles), there is
+        // nothing to poll for (8 layers, fp16 / fp32 outputs: 189.6 / 199.6 us, 188.3 / 198.6 without; two rows 244 / 257, 255 / 261
+        // without).  Nor does it pay where the last 256 halves that a warp polls are not whole (6 layers, 4-bit: 2048 / 768 158 us,
+        // 152 without; two rows 195, 188 without; 2048 / 1024 149 us, 158 without).
+        auto whole = [](uint32_t f) { return f <= 512u || f % 512u == 0; };
+        if ((tokens == 1 && !h->room.beside_two) || !whole(c.f) || !whole(c.shared_f)) return Handover{};
+    }
     if (st != nullptr && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
         cudaGetLastError();
         return Handover{};
@@ -715,7 +726,8 @@ int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, co
     // single-token path: the expert stages select the experts themselves from the logits
     // (the block-wide selection wants one thread per expert in the down stage's block too)
     const bool defer = !grouped && (c.top_k + (c.shared_f ? 1 : 0)) * kDownSplit * 32 >= (uint32_t)kMaxExperts;
-    struct HandGuard { nvmai_cuda_moe *h; ~HandGuard() { h->hand = Handover{}; } } hand_guard{h};
+    struct CallGuard { nvmai_cuda_moe *h; ~CallGuard() { h->hand = Handover{}; h->room = StageRoom{}; } } call_guard{h};
+    if (!grouped) h->room = decode_room(h, tokens, maps != nullptr, shared_late);
     if (defer && maps != nullptr && (c.shared_f == 0 || shared_late)) h->hand = new_handover(h, tokens, st);
     int rc = launch_stage1(h, lv, xsrc, tokens, idx, w, true, c.shared_f != 0 && !grouped && !shared_late, c.shared_f != 0, true, st,
                            defer);

@@ -2,6 +2,7 @@
 // with bulk asynchronous copies and chained by programmatic dependent launch.
 #pragma once
 #include "decode_kernels.cuh"
+#include "stage_room.h"
 #include "tagged.cuh"
 
 namespace nvmai {
@@ -604,15 +605,14 @@ struct Stage2Params {
     unsigned long long *trace;   // optional {start, end} timestamps of this launch
 };
 
-// 56 registers where the tiles are boxes of 4-bit codes (64 elsewhere: two blocks of 8-bit tiles leave no shared memory; 8 layers of
-// two rows, 8-bit, 244 us at 56, 241 at 64), so that a block of stage 3 fits beside two of these, which request their tiles ahead of
-// this stage's end: its 18 warps of 56 registers put five on a quarter of the SM, 8960 of 16384, and at 64 two of these blocks take
-// 8192 there.  Together with the shared memory's split (launch.h) and two blocks an SM (launch_stage2) all 128 blocks of stage 3 now
+// LEAN: 56 registers instead of 64, so that a block of stage 3 fits beside two of these (stage_room.h has the rule), which request
+// their tiles ahead of this stage's end: its 18 warps of 56 registers put five on a quarter of the SM, 8960 of 16384, and at 64 two
+// of these blocks take 8192 there.  Together with the shared memory's split (launch.h) and two blocks an SM (launch_stage2) all 128 blocks of stage 3 now
 // start 1.2 to 1.8 us after this stage's selection begins; they used to start at 4.1 to 5.9, when these had left (8 layers of one row:
 // 173.6 us at 64, 171.3 at 56, 169.6 with the split).  It spills 64 to 168 bytes a thread.
 // Row copies without the caps: 2048 / 192, 1 row 15.3 us instead of 15.5, but 4 rows 37.3 instead of 31.6, 8 rows 65.6 instead of 54.5.
-template <int BITS, int META, int OUT, bool BOXED>
-__global__ void __maxnreg__(BOXED && BITS == 4 ? 56 : 64) stage2_kernel(const __grid_constant__ Stage2Params p, const __grid_constant__ TileMaps maps) {
+template <int BITS, int META, int OUT, bool BOXED, bool LEAN>
+__global__ void __maxnreg__(LEAN ? kGateUpLeanRegs : kGateUpRegs) stage2_kernel(const __grid_constant__ Stage2Params p, const __grid_constant__ TileMaps maps) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *smem = BOXED ? smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u) : smem_raw;
     const GateUpLayout L(p.D, BITS, BOXED);
