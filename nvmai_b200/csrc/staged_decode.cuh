@@ -901,8 +901,10 @@ __device__ __forceinline__ bool down_warp(unsigned char *region, const DownLayou
     const __half *arow = reinterpret_cast<const __half *>(region + L.act);
     if constexpr (POLLED) {
         if (!poll_row_part<OUT>(static_cast<const unsigned long long *>(act_rows) + (OUT == OUT_F16 ? act_offset / 2 : act_offset), tag, n,
-                                g_begin * kGroup, (g_end - g_begin) * kGroup, reinterpret_cast<__half *>(region + L.act), scale_up, status))
+                                g_begin * kGroup, (g_end - g_begin) * kGroup, reinterpret_cast<__half *>(region + L.act), scale_up, status)) {
+            mbar_wait(bar, 0, status);       // the tile's copies land before the block may end
             return false;
+        }
     } else {
         arow = stage_row_part<OUT>(act_rows, act_offset, n, g_begin * kGroup, (g_end - g_begin) * kGroup,
                                    reinterpret_cast<__half *>(region + L.act), scale_up);
