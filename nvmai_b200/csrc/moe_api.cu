@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "batch_path.h"
+#include "handover_words.h"
 #include "stage_room.h"
 #include "ep_comm.cuh"
 #include "grouped_decode.cuh"
@@ -142,10 +143,8 @@ struct nvmai_cuda_moe {
     __half *pf_sacts16 = nullptr;    // [T][Fs + extra] the shared expert's
     float *pf_rowscale = nullptr, *pf_srowscale = nullptr;   // per row: power of two taken out of a wide-range row
     float *pf_logits = nullptr;      // [terms][T][E]
-    // hand-over between the decode stages of a call: the words, the last tag given out, the call's (none between calls)
-    unsigned long long *hand_words = nullptr;
-    bool hand_tried = false;         // asked for the words' memory
-    uint32_t hand_tag = 0;
+    // hand-over between the decode stages: the words, the call's (none between calls)
+    HandoverWords hand_words;
     Handover hand{};
     StageRoom room{};                // of the call's decode stages (between calls: nothing)
     uint16_t *pf_hist = nullptr;     // [routing blocks][256]
@@ -670,8 +669,7 @@ int grouped_tail(nvmai_cuda_moe *h, const LayerViews &lv, const __half *x_rows, 
 // xsrc: where stage 1 gets its rows; x_rows: the fp16 rows stages 2 reads (the
 // same buffer, or the buffer stage 1 writes its normalised rows to).
 // The words of the next call's hand-over from stage 2 to stage 3 (see Handover), or none: rows or activations that they have no
-// room for; a stream under capture, whose launches repeat with the parameters they were captured with.  The words come with the
-// first call that uses them (beside the resident kernel's exchange words they cost a stack step 3 %).
+// room for; a stream under capture, whose launches repeat with the parameters they were captured with.
 Handover new_handover(nvmai_cuda_moe *h, uint32_t tokens, cudaStream_t st) {
     const auto &c = h->cfg;
     const uint32_t longest = c.out_dtype == NVMAI_OUT_FP32 ? kHandoverWide : kHandoverHalf;
@@ -689,25 +687,12 @@ Handover new_handover(nvmai_cuda_moe *h, uint32_t tokens, cudaStream_t st) {
         cudaGetLastError();
         return Handover{};
     }
-    const size_t rows = std::min<size_t>(c.max_tokens, kHandoverRows), words = rows * ((size_t)c.top_k * c.f + c.shared_f + c.d);
-    if (!h->hand_tried) {
-        // once, also where there is no memory for them; another stream's capture is not disturbed
-        h->hand_tried = true;
-        void *w = nullptr;
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        const bool made = cudaMalloc(&w, words * 8) == cudaSuccess && cudaMemsetAsync(w, 0, words * 8, st) == cudaSuccess;
-        if (!made) {
-            cudaGetLastError();
-            cudaFree(w);
-        }
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        if (made) h->hand_words = static_cast<unsigned long long *>(w);
-    }
-    if (h->hand_words == nullptr) return Handover{};
-    if (++h->hand_tag == 0) ++h->hand_tag;
-    unsigned long long *acts = h->hand_words, *sact = acts + rows * c.top_k * c.f;
-    return Handover{h->hand_tag, acts, sact, sact + rows * c.shared_f};
+    const size_t rows = std::min<size_t>(c.max_tokens, kHandoverRows);
+    h->hand_words.make(rows * ((size_t)c.top_k * c.f + c.shared_f + c.d), st);
+    const uint32_t tag = h->hand_words.next_tag(st);
+    if (tag == 0) return Handover{};
+    unsigned long long *acts = h->hand_words.words(), *sact = acts + rows * c.top_k * c.f;
+    return Handover{tag, acts, sact, sact + rows * c.shared_f};
 }
 
 int layer_decode_impl(nvmai_cuda_moe *h, uint32_t layer, const XSource &xsrc, const __half *x_rows, uint32_t tokens,
@@ -1606,7 +1591,7 @@ void nvmai_cuda_moe_destroy(nvmai_cuda_moe *h) {
         for (void *p : lv.owned) cudaFree(p);
     cudaFree(h->logits); cudaFree(h->idx); cudaFree(h->w); cudaFree(h->acts); cudaFree(h->shared_act);
     cudaFree(h->gate_val); cudaFree(h->y); cudaFree(h->xnorm); cudaFree(h->counter); cudaFree(h->status);
-    cudaFree(h->stage_x); cudaFree(h->stage_y); cudaFree(h->row_counter); cudaFree(h->hand_words);
+    cudaFree(h->stage_x); cudaFree(h->stage_y); cudaFree(h->row_counter); h->hand_words.release();
     cudaFree(h->sorted_pair); cudaFree(h->inv); cudaFree(h->expert_offsets); cudaFree(h->expert_counts);
     cudaFree(h->work); cudaFree(h->n_work); cudaFree(h->group_hist); cudaFree(h->trace); cudaFree(h->expert_map); cudaFree(h->partial); cudaFree(h->shared_partial);
     delete h;
