@@ -394,6 +394,12 @@ NVMAI_API int nvmai_cuda_moe_debug_set_wait_limit(uint64_t nanoseconds);
  * call runs normally.  Nothing faults or hangs. */
 NVMAI_API int nvmai_cuda_moe_debug_drop_prefill_copy(nvmai_cuda_moe *h);
 
+/* Test hook for the failure path of the decode stages' hand-over: in the next decode call that
+ * polls (1 to 3 rows, outside a capture) the down stage waits for words that nobody writes, so
+ * its bounded waits run out, nvmai_cuda_moe_synchronize reports NVMAI_CUDA_ETIMEOUT, and the call
+ * after it runs normally.  Nothing faults or hangs. */
+NVMAI_API int nvmai_cuda_moe_debug_drop_handover(nvmai_cuda_moe *h);
+
 /* Test hook: holds `stream` for `ms` milliseconds with a host function (no kernel runs, the
  * device stays idle), so that a test can watch a host-side wait run out. */
 NVMAI_API int nvmai_cuda_moe_debug_host_delay(nvmai_cuda_moe *h, void *stream, uint32_t ms);

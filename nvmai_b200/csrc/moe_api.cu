@@ -146,6 +146,7 @@ struct nvmai_cuda_moe {
     // hand-over between the decode stages: the words, the call's (none between calls)
     HandoverWords hand_words;
     Handover hand{};
+    bool hand_debug_drop = false;    // test hook, see nvmai_cuda_moe_debug_drop_handover
     StageRoom room{};                // of the call's decode stages (between calls: nothing)
     uint16_t *pf_hist = nullptr;     // [routing blocks][256]
     uint32_t *pf_totals = nullptr, *pf_first = nullptr;     // [segments of routing blocks][256]
@@ -517,6 +518,11 @@ int launch_stage3(nvmai_cuda_moe *h, Stage3Params p, uint32_t tokens, bool pdl, 
     p.status = h->status;
     p.trace = h->cur_trace;
     p.hand = h->hand;
+    if (p.hand.tag != 0 && h->hand_debug_drop) {
+        p.hand.tag = h->hand_words.next_tag(st);        // which nobody writes
+        h->hand_debug_drop = false;
+        if (p.hand.tag == 0) return NVMAI_CUDA_ECUDA;
+    }
     if (p.next.w == nullptr || p.hidden == nullptr || c.d > kHandoverNorm) p.hand.hidden = nullptr;
     dim3 grid(c.d / kTileRows + (p.hand.hidden != nullptr ? 1 : 0), tokens);
     const uint32_t units = p.top_k + (p.shared_f ? 1 : 0);
@@ -2546,6 +2552,12 @@ int nvmai_cuda_moe_read_route_log_rows(nvmai_cuda_moe *h, uint32_t *out_host, ui
 int nvmai_cuda_moe_debug_drop_prefill_copy(nvmai_cuda_moe *h) {
     if (!h) return NVMAI_CUDA_EINVAL;
     h->pf_debug_drop = true;
+    return NVMAI_CUDA_OK;
+}
+
+int nvmai_cuda_moe_debug_drop_handover(nvmai_cuda_moe *h) {
+    if (!h) return NVMAI_CUDA_EINVAL;
+    h->hand_debug_drop = true;
     return NVMAI_CUDA_OK;
 }
 

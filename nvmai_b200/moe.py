@@ -211,6 +211,9 @@ class MoE:
     def debug_drop_prefill_copy(self) -> None:
         check(self._lib.nvmai_cuda_moe_debug_drop_prefill_copy(self._h), "debug_drop_prefill_copy")
 
+    def debug_drop_handover(self) -> None:
+        check(self._lib.nvmai_cuda_moe_debug_drop_handover(self._h), "debug_drop_handover")
+
     def debug_host_delay(self, ms: int, stream=None) -> None:
         check(self._lib.nvmai_cuda_moe_debug_host_delay(self._h, _stream(stream), int(ms)), "debug_host_delay")
 

@@ -65,3 +65,75 @@ def test_handed_over_rows_have_the_bits_of_plain_ones(rows, d, f, shared_f, bits
     for n in (1, rows, 1, rows) * 10:          # words of an earlier call, of more rows or fewer, lie in the way
         call(n, torch.cuda.current_stream())
         assert all(torch.equal(a[:n], b) for a, b in zip(first, result(n)))
+
+
+def _block(torch, rows, out, seed, next_norm=True):
+    """A handle with one polling layer and a decode call of it; -> (moe, call(stream), outputs)."""
+    d, f = 512, 256
+    cfg = MoEConfig(d=d, f=f, shared_f=f, num_experts=64, top_k=8, routed_bits=4, shared_bits=4,
+                    shared_gate_kind=fmt.ROUTER_DENSE_F16, out_dtype=out, max_tokens=3)
+    moe = MoE(cfg)
+    dev = synthetic.device_layer(seed, d=d, f=f, shared_f=f, num_experts=64, routed_bits=4, shared_bits=4)
+    synthetic.register_device_layer(moe, 0, dev)
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    kind = torch.float16 if out == F16 else torch.float32
+    start = (torch.randn((rows, d), device="cuda", generator=gen) * 4).to(kind)
+    norm = (torch.rand(d, device="cuda", generator=gen) + 0.5).to(torch.bfloat16)
+    hidden, x_next = start.clone(), torch.zeros((rows, d), dtype=torch.float16, device="cuda")
+
+    def call(stream):
+        hidden.copy_(start)
+        if next_norm:
+            moe.layer_decode_fused_norms(0, hidden, norm, 1e-6, rows, norm, 1e-6, x_next, stream=stream)
+        else:
+            moe.layer_decode_prenorm(0, hidden, norm, 1e-6, rows, stream=stream)
+
+    return moe, call, (hidden, x_next), dev
+
+
+# The polls of stage 3 (halves, fp32 values, the block of the next norm) run out, from the host side: stage 3 waits for words that
+# nobody writes.  Waits are cut to 20 ms; the call ends, the time-out is reported once, and the next call has the bits of the first.
+@pytest.mark.parametrize("rows,out,next_norm", [(1, F16, True), (3, F32, True), (2, F16, False)])
+def test_a_hand_over_that_never_comes_times_out_and_the_next_call_runs(rows, out, next_norm):
+    from nvmai_b200 import _lib
+    from nvmai_b200.moe import debug_set_wait_limit
+    torch = gu.torch_cuda()
+    moe, call, outs, _keep = _block(torch, rows, out, 31 + rows, next_norm)
+    st = torch.cuda.current_stream()
+    call(st)
+    moe.synchronize()
+    good = [t.clone() for t in outs]
+    debug_set_wait_limit(20_000_000)
+    try:
+        moe.debug_drop_handover()
+        call(st)
+        with pytest.raises(_lib.NvmaiError) as err:
+            moe.synchronize()
+        assert err.value.code == _lib.ETIMEOUT
+    finally:
+        debug_set_wait_limit(0)
+    for _ in range(2):
+        call(st)
+        moe.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(good, outs))
+
+
+def test_two_handles_poll_on_two_streams_at_once():
+    torch = gu.torch_cuda()
+    made = [_block(torch, rows, out, 50 + rows) for rows, out in ((1, F16), (3, F32))]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in made]
+    good = []
+    for (moe, call, outs, _keep), st in zip(made, streams):
+        with torch.cuda.stream(st):
+            call(st)
+        moe.synchronize(st)
+        good.append([t.clone() for t in outs])
+    torch.cuda.synchronize()
+    for _ in range(50):
+        for (moe, call, outs, _keep), st in zip(made, streams):
+            with torch.cuda.stream(st):
+                call(st)
+    for (moe, call, outs, _keep), st, want in zip(made, streams, good):
+        moe.synchronize(st)
+        assert all(torch.equal(a, b) for a, b in zip(want, outs))
