@@ -394,6 +394,11 @@ NVMAI_API int nvmai_cuda_moe_debug_set_wait_limit(uint64_t nanoseconds);
  * call runs normally.  Nothing faults or hangs. */
 NVMAI_API int nvmai_cuda_moe_debug_drop_prefill_copy(nvmai_cuda_moe *h);
 
+/* Test hook: the plan of a prefill call whose experts all go to the grouped GEMMs, phase 0 (gate/up)
+ * or 1 (down): out[0] = rows of the longest work item, out[1] = sets of accumulators, out[2] = slots
+ * of converted weights in tensor memory. */
+NVMAI_API int nvmai_cuda_moe_debug_item_plan(const nvmai_cuda_moe *h, uint32_t tokens, int phase, uint32_t *out);
+
 /* Test hook for the failure path of the decode stages' hand-over: in the next decode call that
  * polls (1 to 3 rows, outside a capture) the down stage waits for words that nobody writes, so
  * its bounded waits run out, nvmai_cuda_moe_synchronize reports NVMAI_CUDA_ETIMEOUT, and the call

@@ -1072,6 +1072,27 @@ int layer_stream_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32
     return launched(h, bp_combine(pc, c.out_dtype, st));
 }
 
+// Longest work item: two standard deviations above an evenly routed expert's rows, and no shorter than 96 rows (128 above 64
+// rows per expert), since every further item of a popular expert converts its codes again; what the accumulators leave of the
+// tensor memory goes to the A slots and to a second set of accumulators (up to 96 rows).  Measured for items of 48 or 64 / 96 /
+// 128 / 160 rows, evenly routed and with popularities 1 / rank^0.6 and 1 / rank^1.17:
+//   437 rows 4-bit   217 / 220 / 226 / 215    219 / 201 / 210 / 207    130 / 112 / 116 / 119 us
+//   1154 rows 4-bit  240 / 244 / 251 / 252    312 / 275 / 260 / 268    238 / 207 / 192 / 190
+//   1531 rows 8-bit  408 / 415 / 422 / 422    546 / 499 / 472 / 470    408 / 398 / 351 / 327
+//   3000 rows 4-bit  464 / 369 / 309 / 310    488 / 411 / 405 / 402    456 / 373 / 345 / 340
+// 4096 rows 4-bit, items of 128 / 160 / 192: 422 / 386 / 399 us.  Beside the streaming kernel an SM gets one unit or none: one
+// set of accumulators and more A slots (256 skewed rows 109.6 us, items of 96: 111.7, of 64: 122).
+uint32_t item_rows(uint32_t pairs, uint32_t experts, bool mixed) {
+    const float rows = (float)pairs / experts;
+    const uint32_t sure = ((uint32_t)(rows + 2.0f * std::sqrt(rows)) + 15) / 16 * 16;
+    return mixed ? 112 : rows <= 12.0f ? 48 : std::min(192u, std::max(rows > 64.0f ? 128u : 96u, sure));
+}
+// The grouped GEMMs' plans for such items: gate/up, down.
+EgPlan item_plan(const nvmai_cuda_moe_config &c, EgParams &g, int phase, uint32_t want) {
+    g.kdim = phase == 0 ? c.d : c.f;
+    return eg_plan(g, phase, phase == 0 ? want : std::min(want, 128u));
+}
+
 int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint32_t tokens, void *hidden, void *y,
                        uint32_t *out_idx, __half *out_w, cudaStream_t st, const PrefillMode mode = PrefillMode{}) {
     const ExpertSplit split_at = expert_split(h, tokens, mode);
@@ -1098,22 +1119,9 @@ int layer_prefill_impl(nvmai_cuda_moe *h, uint32_t layer, const __half *x, uint3
     const bool use_map = h->expert_map != nullptr;
     const uint32_t experts = use_map ? h->n_local : c.num_experts;
 
-    // Longest work item: two standard deviations above an evenly routed expert's rows, and no shorter than 96 rows (128 above 64
-    // rows per expert), since every further item of a popular expert converts its codes again; what the accumulators leave of the
-    // tensor memory goes to the A slots and to a second set of accumulators (up to 96 rows).  Measured for items of 48 or 64 / 96 /
-    // 128 / 160 rows, evenly routed and with popularities 1 / rank^0.6 and 1 / rank^1.17:
-    //   437 rows 4-bit   217 / 220 / 226 / 215    219 / 201 / 210 / 207    130 / 112 / 116 / 119 us
-    //   1154 rows 4-bit  240 / 244 / 251 / 252    312 / 275 / 260 / 268    238 / 207 / 192 / 190
-    //   1531 rows 8-bit  408 / 415 / 422 / 422    546 / 499 / 472 / 470    408 / 398 / 351 / 327
-    //   3000 rows 4-bit  464 / 369 / 309 / 310    488 / 411 / 405 / 402    456 / 373 / 345 / 340
-    // 4096 rows 4-bit, items of 128 / 160 / 192: 422 / 386 / 399 us.  Beside the streaming kernel an SM gets one unit or none: one
-    // set of accumulators and more A slots (256 skewed rows 109.6 us, items of 96: 111.7, of 64: 122).
-    const float rows = (float)P / c.num_experts;
-    const uint32_t sure = ((uint32_t)(rows + 2.0f * std::sqrt(rows)) + 15) / 16 * 16;
-    const uint32_t want = mixed ? 112 : rows <= 12.0f ? 48 : std::min(192u, std::max(rows > 64.0f ? 128u : 96u, sure));
     EgParams g0{}, g1{};
-    g0.kdim = c.d; g1.kdim = c.f;
-    const EgPlan plan0 = eg_plan(g0, 0, want), plan1 = eg_plan(g1, 1, std::min(want, 128u));
+    const uint32_t want = item_rows(P, c.num_experts, mixed);
+    const EgPlan plan0 = item_plan(c, g0, 0, want), plan1 = item_plan(c, g1, 1, want);
 
     PackXParams px{};
     px.dst = h->pf_x; px.dst2 = two_orders ? h->pf_xs : nullptr; px.permute = c.routed_bits == 4 ? 1 : 0;
@@ -2552,6 +2560,14 @@ int nvmai_cuda_moe_read_route_log_rows(nvmai_cuda_moe *h, uint32_t *out_host, ui
 int nvmai_cuda_moe_debug_drop_prefill_copy(nvmai_cuda_moe *h) {
     if (!h) return NVMAI_CUDA_EINVAL;
     h->pf_debug_drop = true;
+    return NVMAI_CUDA_OK;
+}
+
+int nvmai_cuda_moe_debug_item_plan(const nvmai_cuda_moe *h, uint32_t tokens, int phase, uint32_t *out) {
+    if (!h || !out || tokens == 0 || phase < 0 || phase > 1 || !tc_shape_ok(h, true)) return NVMAI_CUDA_EINVAL;
+    EgParams g{};
+    const EgPlan plan = item_plan(h->cfg, g, phase, item_rows(tokens * h->cfg.top_k, h->cfg.num_experts, false));
+    out[0] = plan.cap; out[1] = g.acc_slots; out[2] = g.a_slots;
     return NVMAI_CUDA_OK;
 }
 

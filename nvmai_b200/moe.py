@@ -211,6 +211,12 @@ class MoE:
     def debug_drop_prefill_copy(self) -> None:
         check(self._lib.nvmai_cuda_moe_debug_drop_prefill_copy(self._h), "debug_drop_prefill_copy")
 
+    def debug_item_plan(self, tokens: int, phase: int) -> tuple[int, int, int]:
+        """Rows of the longest work item, sets of accumulators, slots of converted weights of a grouped GEMM (0 gate/up, 1 down)."""
+        out = (C.c_uint32 * 3)()
+        check(self._lib.nvmai_cuda_moe_debug_item_plan(self._h, tokens, phase, out), "debug_item_plan")
+        return tuple(out)
+
     def debug_drop_handover(self) -> None:
         check(self._lib.nvmai_cuda_moe_debug_drop_handover(self._h), "debug_drop_handover")
 

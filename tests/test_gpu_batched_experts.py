@@ -158,8 +158,8 @@ def test_stack_of_rows_equals_its_layers_one_by_one(rows, bits, out, d, f, exper
     assert torch.equal(y, y1)
 
 
-# Items whose accumulators leave other numbers of A slots than the above (8 experts see every row): 62 rows, items of 80, two sets
-# and three slots; 90 rows, items of 112, one set that all warps empty and four slots; 150 rows, items of 176, one set, two slots.
+# 8 experts see every row, 27 units of gate/up: 62 rows, items of 96, two sets of accumulators and two A slots; 90 rows, items of
+# 128, one set that all warps empty and four slots; 150 rows, items of 176, one set, two slots.
 @pytest.mark.parametrize("bits,meta,out,tokens", [(4, BF16, fmt.OUT_FP16, 62), (8, FP16, fmt.OUT_FP32, 62), (4, BF16, fmt.OUT_FP32, 90),
                                                   (8, FP16, fmt.OUT_FP16, 90), (4, FP16, fmt.OUT_FP16, 150), (8, BF16, fmt.OUT_FP16, 150)])
 @pytest.mark.parametrize("entry", ["decode", "prefill"])
@@ -169,6 +169,26 @@ def test_items_of_every_tensor_memory_plan_match_the_oracle(bits, meta, out, tok
     cfg = MoEConfig(d=768, f=384, shared_f=384, num_experts=8, top_k=8, routed_bits=bits, shared_bits=bits, meta_dtype=meta,
                     out_dtype=out, max_tokens=tokens)
     assert _worst_error(host, cfg, entry, tokens, sorted({0, 31, tokens // 2, tokens - 1})) < _tol(meta, out, entry)
+
+
+# Every plan by name, with more units than SMs, so that slots and parities go on from unit to unit, odd numbers of slots and of
+# stages among them (d = 768: 13 stages of a 4-bit unit, 25 of an 8-bit one).  plan: rows of the longest item, sets of accumulators,
+# A slots.  8192 / 384: the ring of rows leaves items of 80.
+@pytest.mark.parametrize("bits,out,tokens,d,f,experts,plan", [
+    (4, fmt.OUT_FP16, 64, 768, 384, 64, (48, 2, 5)), (8, fmt.OUT_FP32, 64, 768, 384, 64, (48, 2, 5)),
+    (4, fmt.OUT_FP32, 300, 768, 640, 64, (96, 2, 2)), (8, fmt.OUT_FP16, 300, 768, 640, 64, (96, 2, 2)),
+    (4, fmt.OUT_FP16, 300, 768, 768, 32, (128, 1, 4)), (8, fmt.OUT_FP32, 300, 768, 768, 32, (128, 1, 4)),
+    (4, fmt.OUT_FP32, 512, 768, 768, 32, (160, 1, 3)), (8, fmt.OUT_FP16, 512, 768, 768, 32, (160, 1, 3)),
+    (4, fmt.OUT_FP16, 640, 768, 768, 32, (192, 1, 2)),
+    (4, fmt.OUT_FP32, 300, 8192, 384, 64, (80, 2, 3)),
+])
+def test_units_walk_through_every_tensor_memory_plan(bits, out, tokens, d, f, experts, plan, monkeypatch):
+    monkeypatch.setenv("NVMAI_CUDA_STREAM_ROWS", "0")
+    cfg = MoEConfig(d=d, f=f, shared_f=f, num_experts=experts, top_k=8, routed_bits=bits, shared_bits=bits, meta_dtype=BF16,
+                    out_dtype=out, max_tokens=tokens)
+    assert MoE(cfg).debug_item_plan(tokens, 0) == plan
+    host = _host_layer(950 + tokens, bits, BF16, d, f, experts)
+    assert _worst_error(host, cfg, "prefill", tokens, sorted({0, 31, tokens // 2, tokens - 1})) < _tol(BF16, out, "prefill")
 
 
 # Routing in blocks of 8 tokens (up to 1024) and of 32, with a last block of one; the reduction walks more rows than its grid.
