@@ -277,10 +277,12 @@ __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
     if (tid == 0) *p.counter = 0u;
     uint32_t total = 0;
     if (tid < kMaxExperts) {
-        for (uint32_t i = tid; i < bp_route_segments(gridDim.x) * kMaxExperts; i += kMaxExperts) {
+        total = __ldcg(p.totals + tid);
+        p.totals[tid] = 0u;
+        for (uint32_t i = kMaxExperts + tid; i < bp_route_segments(gridDim.x) * kMaxExperts; i += kMaxExperts) {
             const uint32_t n = __ldcg(p.totals + i);
             p.totals[i] = 0u;
-            if (i >= (uint32_t)kMaxExperts) p.first[i] = total;
+            p.first[i] = total;
             total += n;
         }
     }
@@ -342,13 +344,16 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
     {
         constexpr uint32_t kBatch = kRouteSegment / 4u;
         const uint32_t part = tid >> 6, quad = tid & 63, b0 = segment * kRouteSegment + part;
-        uint2 c[kBatch], sum = make_uint2(0u, 0u);
+        uint2 sum = make_uint2(0u, 0u);
+        if (b0 < blockIdx.x) {
+            uint2 c[kBatch];
 #pragma unroll
-        for (uint32_t k = 0; k < kBatch; ++k)
-            c[k] = b0 + 4u * k < blockIdx.x
-                       ? __ldcg(reinterpret_cast<const uint2 *>(p.block_hist) + (size_t)(b0 + 4u * k) * (kMaxExperts / 4) + quad) : make_uint2(0u, 0u);
+            for (uint32_t k = 0; k < kBatch; ++k)
+                c[k] = b0 + 4u * k < blockIdx.x
+                           ? __ldcg(reinterpret_cast<const uint2 *>(p.block_hist) + (size_t)(b0 + 4u * k) * (kMaxExperts / 4) + quad) : make_uint2(0u, 0u);
 #pragma unroll
-        for (uint32_t k = 0; k < kBatch; ++k) { sum.x += c[k].x; sum.y += c[k].y; }      // (32 x 256 fits 16 bits)
+            for (uint32_t k = 0; k < kBatch; ++k) { sum.x += c[k].x; sum.y += c[k].y; }      // (32 x 256 fits 16 bits)
+        }
         *reinterpret_cast<uint4 *>(&before[part][4 * quad]) = make_uint4(sum.x & 0xFFFFu, sum.x >> 16, sum.y & 0xFFFFu, sum.y >> 16);
     }
     const bool live = e != kBpNotLocal;
