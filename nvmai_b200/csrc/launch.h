@@ -45,8 +45,8 @@ inline cudaError_t ensure_smem(Kern kern, size_t bytes) {
 //
 // whole_shared: an SM's split between L1 and shared memory is made for the kernel that runs and cannot change under its blocks, so a
 // kernel whose dependents are to fit beside it asks for all of the shared memory.  Asked for launch by launch: as an attribute of the
-// function it would also hold for the other handles whose layers the same function runs (six 8-bit layers of one row: 2048 / 768
-// 168 us, behind a handle of 2048 / 128 175; 1024 / 512 119, behind one of 2048 / 512 108).
+// function it would also hold for the other handles whose layers the same function runs (six 8-bit layers of one row, 2048 / 768:
+// 168 us, behind a handle of 2048 / 128 175).
 template <typename Kern, typename... Params>
 inline cudaError_t launch_granted(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, bool whole_shared,
                                   const Params &...p) {

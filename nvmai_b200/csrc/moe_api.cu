@@ -306,7 +306,7 @@ StageRoom decode_room(const nvmai_cuda_moe *h, uint32_t tokens, bool boxed, bool
     const uint32_t f = with_shared ? std::max(c.f, c.shared_f) : c.f, units = c.top_k + (c.shared_f ? 1 : 0);
     const uint32_t blocks = (f + kBlockFeatures - 1) / kBlockFeatures * (c.top_k + (with_shared ? 1 : 0)) * tokens;
     return stage_room(GateUpLayout(c.d, c.routed_bits, boxed).total, DownLayout(c.f, c.shared_f, c.routed_bits, c.shared_bits, units, boxed).total,
-                      blocks, (uint32_t)h->sm_count, units * kDownSplit, boxed);
+                      blocks, c.d / kTileRows * tokens, (uint32_t)h->sm_count, units * kDownSplit, boxed);
 }
 // A decode stage's launch.
 template <typename Kern, typename... Params>
@@ -684,8 +684,8 @@ Handover new_handover(nvmai_cuda_moe *h, uint32_t tokens, cudaStream_t st) {
     if (!h->room.early) {
         // One row's blocks of stage 2 all start at once; where stage 3's find no room beside two of them (8-bit tiles), there is
         // nothing to poll for (8 layers, fp16 / fp32 outputs: 189.6 / 199.6 us, 188.3 / 198.6 without; two rows 244 / 257, 255 / 261
-        // without).  Nor does it pay where the last 256 halves that a warp polls are not whole (6 layers, 4-bit: 2048 / 768 158 us,
-        // 152 without; two rows 195, 188 without; 2048 / 1024 149 us, 158 without).
+        // without).  Nor does it pay where the last 256 halves that a warp polls are not whole (6 layers, 4-bit: 2048 / 768 156 us,
+        // 150 without; two rows 193, 188 without; 2048 / 1024 146 us, 161 without).
         auto whole = [](uint32_t f) { return f <= 512u || f % 512u == 0; };
         if ((tokens == 1 && !h->room.beside_two) || !whole(c.f) || !whole(c.shared_f)) return Handover{};
     }
@@ -1802,8 +1802,8 @@ int nvmai_cuda_moe_layer_decode_prenorm(nvmai_cuda_moe *h, uint32_t layer, void 
 }
 
 // The same with the NEXT block's input norm folded into the last stage as well: the stage that writes the hidden
-// state also writes x_next = rmsnorm_bf16w(hidden, next_norm_weight) (single-token path: the down-stage block that
-// finishes a row last; batched paths: the combine block of the row).
+// state also writes x_next = rmsnorm_bf16w(hidden, next_norm_weight) (single-token path: a block of its own that polls the new
+// row, or, in calls that do not poll, the down-stage block that finishes the row last; batched paths: the combine block of the row).
 int nvmai_cuda_moe_layer_decode_fused_norms(nvmai_cuda_moe *h, uint32_t layer, void *hidden_inout, const void *attn_delta_f16,
                                             const void *norm_weight_bf16, float eps, uint32_t tokens,
                                             const void *next_norm_weight_bf16, float next_eps, void *x_next_out_f16,

@@ -726,7 +726,7 @@ struct Stage3Params {
     // ranges the next launch will read (the next layer's router and shared-expert
     // weights): each block asks the L2 for its share
     const void *next_ptr[6]; unsigned long long next_bytes[6];
-    NextNorm next;                      // optional: the block that finishes a row last also writes the next block's input
+    NextNorm next;                      // optional: the next block's input is written too, by the block that finishes a row last (or see hand)
     Handover hand;                      // with a tag: boxes, deferred selection; hand.hidden: a block past D / 16 makes the next norm
     uint32_t D, F, top_k;
     unsigned int *status;

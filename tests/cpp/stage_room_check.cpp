@@ -10,26 +10,28 @@ int main() {
     int bad = 0;
     auto expect = [&](const char *what, bool ok) { if (!ok) { std::printf("%s\n", what); ++bad; } };
     const uint32_t sms = 148;
-    // (shared memory of a block of stage 2 and 3, blocks of stage 2, warps of stage 3)
-    StageRoom r = stage_room(44864, 66816, 288, sms, 18, true);                 // 2048 / 512, 4-bit
+    // (shared memory of a block of stage 2 and 3, their blocks, warps of a block of stage 3)
+    StageRoom r = stage_room(44864, 66816, 288, 128, sms, 18, true);            // 2048 / 512, 4-bit
     expect("4-bit 2048 / 512", r.whole_shared && r.early && r.lean);
-    r = stage_room(40768, 103680, 288, sms, 18, true);                          // 1024 / 512, 8-bit: the same room, the same cap
+    r = stage_room(40768, 103680, 288, 64, sms, 18, true);                      // 1024 / 512, 8-bit: the same room, the same cap
     expect("8-bit 1024 / 512", r.whole_shared && r.early && r.lean);
-    r = stage_room(44864, 60416, 256, sms, 16, true);                           // top-7 and a shared expert: 16 warps fit at 64
+    r = stage_room(44864, 60416, 256, 128, sms, 16, true);                      // top-7 and a shared expert: 16 warps fit at 64
     expect("16 warps", r.early && !r.lean);
-    r = stage_room(44864, 122112, 576, sms, 18, true);                          // 2048 / 1024, 4-bit: four blocks an SM leave no room
+    r = stage_room(44864, 122112, 576, 128, sms, 18, true);                     // 2048 / 1024, 4-bit: four blocks an SM leave no room
     expect("4-bit 2048 / 1024", !r.whole_shared && !r.early && !r.lean && r.beside_two);
-    r = stage_room(85824, 122112, 576, sms, 18, true);                          // 4096 / 1024, 4-bit
+    r = stage_room(85824, 122112, 576, 256, sms, 18, true);                     // 4096 / 1024, 4-bit
     expect("4-bit 4096 / 1024", !r.whole_shared && !r.early && !r.lean && !r.beside_two);
-    r = stage_room(44864, 29952, 72, sms, 18, true);                            // a block an SM
+    r = stage_room(44864, 29952, 72, 128, sms, 18, true);                       // a block an SM
     expect("2048 / 128", r.early && !r.lean);
-    r = stage_room(44864, 66816, 0, 0, 18, true);                               // a device that was not asked
+    r = stage_room(44864, 39168, 288, 256, sms, 18, true);                      // two rows of 2048 / 256: half of stage 3 could be early
+    expect("two rows", r.early && !r.lean);
+    r = stage_room(44864, 66816, 0, 0, 0, 18, true);                            // a device that was not asked
     expect("no device", !r.whole_shared && !r.early && !r.lean);
     for (size_t gate_up = 8192; gate_up <= 160 * 1024; gate_up += 4096)
         for (size_t down = 8192; down <= 200 * 1024; down += 8192)
             for (uint32_t blocks = 1; blocks <= 1200; blocks += 29)
                 for (uint32_t warps = 2; warps <= 18; warps += 2) {
-                    r = stage_room(gate_up, down, blocks, sms, warps, true);
+                    r = stage_room(gate_up, down, blocks, 128, sms, warps, true);
                     const uint32_t most = (blocks + sms - 1) / sms, down_regs = (warps + 3) / 4 * 32 * 56;
                     // every SM that holds two blocks of stage 2 or fewer has room for one of stage 3
                     const uint32_t n = most < 2 ? most : 2;
@@ -39,8 +41,8 @@ int main() {
                     expect("cap without use", !r.lean || r.whole_shared);
                     expect("early only where it fits", !r.early || r.whole_shared);
                     // row copies never start early
-                    const StageRoom rows = stage_room(gate_up, down, blocks, sms, warps, false);
-                    expect("row copies", !rows.early && !rows.lean && (!rows.whole_shared || blocks > 2 * sms));
+                    const StageRoom rows = stage_room(gate_up, down, blocks, 128, sms, warps, false);
+                    expect("row copies", !rows.early && !rows.lean && (!rows.whole_shared || blocks > sms));
                 }
     std::printf(bad ? "FAILED %d\n" : "PASSED\n", bad);
     return bad != 0;
