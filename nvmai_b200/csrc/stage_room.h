@@ -44,8 +44,8 @@ inline StageRoom stage_room(size_t gate_up, size_t down, uint32_t blocks, uint32
     r.whole_shared = fits(per_sm);
     r.early = r.whole_shared && per_sm <= 2;
     const uint32_t down_regs = (down_warps + 3) / 4 * 32 * kDownRegs;
-    r.lean = r.whole_shared && (fullest > 2 || down_blocks <= sms) &&
-             fullest * (kGateUpWarps / 4) * 32 * kGateUpRegs + down_regs > kQuarterRegs;
+    const uint32_t held = std::min(fullest, (uint32_t)(kSmShared / (gate_up + kBlockReserve)));      // by the shared memory
+    r.lean = r.whole_shared && (held > 2 || down_blocks <= sms) && held * (kGateUpWarps / 4) * 32 * kGateUpRegs + down_regs > kQuarterRegs;
     return r;
 }
 

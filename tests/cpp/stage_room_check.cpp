@@ -25,6 +25,10 @@ int main() {
     expect("2048 / 128", r.early && !r.lean);
     r = stage_room(44864, 39168, 288, 256, sms, 18, true);                      // two rows of 2048 / 256: half of stage 3 could be early
     expect("two rows", r.early && !r.lean);
+    r = stage_room(77632, 58368, 320, 256, sms, 10, true);                      // 8-bit, top-4, two rows: an SM holds two blocks, not three
+    expect("two by shared memory", r.whole_shared && !r.lean);
+    r = stage_room(44864, 37888, 320, 256, sms, 10, true);                      // 4-bit: three
+    expect("three", r.whole_shared && r.lean);
     r = stage_room(44864, 66816, 0, 0, 0, 18, true);                            // a device that was not asked
     expect("no device", !r.whole_shared && !r.early && !r.lean);
     for (size_t gate_up = 8192; gate_up <= 160 * 1024; gate_up += 4096)
