@@ -157,10 +157,13 @@ uint32_t bp_route_blocks(uint32_t tokens) {
 cudaError_t bp_route(const RouteParams &p, cudaStream_t st) {
     if (p.tokens <= kSmallRoute) return launch_pdl(route_small_kernel, dim3(1), dim3(1024), 0, st, true, p);
     const dim3 grid(bp_route_blocks(p.tokens));
-    cudaError_t e = bp_tokens_per_block(p.tokens) == 8 ? launch_pdl(route_kernel<8>, grid, dim3(256), 0, st, true, p)
-                                                       : launch_pdl(route_kernel<32>, grid, dim3(1024), 0, st, true, p);
+    const bool eight = bp_tokens_per_block(p.tokens) == 8, one_segment = p.tokens <= kRouteShort;
+    cudaError_t e = one_segment ? launch_pdl(route_kernel<8, false>, grid, dim3(256), 0, st, true, p)
+                    : eight     ? launch_pdl(route_kernel<8, true>, grid, dim3(256), 0, st, true, p)
+                                : launch_pdl(route_kernel<32, true>, grid, dim3(1024), 0, st, true, p);
     if (e != cudaSuccess) return e;
-    return launch_pdl(route_scatter_kernel, grid, dim3(256), 0, st, true, p);
+    return one_segment ? launch_pdl(route_scatter_kernel<false>, grid, dim3(256), 0, st, true, p)
+                       : launch_pdl(route_scatter_kernel<true>, grid, dim3(256), 0, st, true, p);
 }
 
 cudaError_t bp_pack_acts(const PackActsParams &p, cudaStream_t st) {

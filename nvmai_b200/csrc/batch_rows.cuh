@@ -185,6 +185,8 @@ __global__ void __launch_bounds__(128) router_gemm_kernel(const __grid_constant_
 // ---- top-k and grouping -----------------------------------------------------------------------
 // Tokens (and warps) per block: 8 up to 1024 tokens, 32 above, so that a chunk of 4096 is one wave of 128 blocks.
 __host__ __device__ constexpr uint32_t bp_tokens_per_block(uint32_t tokens) { return tokens <= 1024u ? 8u : 32u; }
+constexpr uint32_t kRouteShort = 768;      // rows of calls that have one segment by their size (see route_kernel)
+static_assert(bp_tokens_per_block(kRouteShort) == 8u && kRouteShort <= 8u * kRouteSegment, "blocks of eight tokens, one segment");
 
 // Expert e's work items in list j: its rows split evenly over them (two items of 70 instead of 128 + 12).
 __device__ __forceinline__ void write_items(const RouteParams &p, int j, uint32_t e, uint32_t rows, uint32_t items, uint32_t first_row,
@@ -236,7 +238,9 @@ __device__ __forceinline__ void add_terms(float (&v)[kMaxExperts / 32], const Ro
 // it in its segment: one segment up to 4096 rows; counts of all blocks in front would grow with the square of the rows (256 /
 // 128 wide, 262,144 rows: 5519 us, 4940 with segments; 4096 rows 112 either way).  (With four tokens per warp and a last block that
 // scanned every block's counts, 4096 rows took 33 us from the router's end to this kernel's, 1531 rows 29, 256 rows 14.)
-template <int WARPS>
+// LONG: with segments; up to kRouteShort rows without, which their loop over the counts leaves at 32 registers instead of 80 (whole
+// call, 256 skewed rows 99.2 / 100.2 us without / with, 600 143.1 / 143.5; 1000 rows of 256 / 128 68.0 / 66.6, 1500 76.7 / 75.4).
+template <int WARPS, bool LONG>
 __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
     static_assert(WARPS * 32 >= kMaxExperts, "a thread per expert");
     __shared__ uint32_t hist[kMaxExperts];
@@ -263,7 +267,7 @@ __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
         }
     }
     __syncthreads();
-    if (tid < kMaxExperts && hist[tid] != 0u) atomicAdd(p.totals + blockIdx.x / kRouteSegment * kMaxExperts + tid, hist[tid]);
+    if (tid < kMaxExperts && hist[tid] != 0u) atomicAdd(p.totals + (LONG ? blockIdx.x / kRouteSegment * kMaxExperts : 0u) + tid, hist[tid]);
     if (tid < kMaxExperts / 4)      // at most 32 * kMaxTopK pairs of an expert (a caller's list may repeat one)
         reinterpret_cast<uint2 *>(p.block_hist)[(size_t)blockIdx.x * (kMaxExperts / 4) + tid] =
             make_uint2(hist[4 * tid] | hist[4 * tid + 1] << 16, hist[4 * tid + 2] | hist[4 * tid + 3] << 16);
@@ -279,12 +283,13 @@ __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
     if (tid < kMaxExperts) {
         total = __ldcg(p.totals + tid);
         p.totals[tid] = 0u;
-        for (uint32_t i = kMaxExperts + tid; i < bp_route_segments(gridDim.x) * kMaxExperts; i += kMaxExperts) {
-            const uint32_t n = __ldcg(p.totals + i);
-            p.totals[i] = 0u;
-            p.first[i] = total;
-            total += n;
-        }
+        if constexpr (LONG)
+            for (uint32_t i = kMaxExperts + tid; i < bp_route_segments(gridDim.x) * kMaxExperts; i += kMaxExperts) {
+                const uint32_t n = __ldcg(p.totals + i);
+                p.totals[i] = 0u;
+                p.first[i] = total;
+                total += n;
+            }
     }
     const uint32_t heavy = heavy_limit(p, total);
     uint32_t mine[4] = {}, pre[4];
@@ -323,6 +328,7 @@ __global__ void __launch_bounds__(WARPS * 32) route_kernel(RouteParams p) {
 }
 
 // stable scatter of a block's pairs
+template <bool LONG>
 __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
     __shared__ uint16_t cnt[8][kMaxExperts];
     __shared__ uint32_t before[4][kMaxExperts];
@@ -339,22 +345,29 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
         const uint32_t g = min(p.idx[i], p.E - 1u);
         e = p.expert_map != nullptr ? p.expert_map[g] : g;
     }
-    // the pairs of the segment's blocks in front: a quarter of the blocks a thread, four experts each, all counts in flight
-    const uint32_t segment = blockIdx.x / kRouteSegment;
+    // the pairs of the segment's blocks in front: a quarter of the blocks a thread, four experts each, 32 blocks' counts in flight
+    const uint32_t segment = LONG ? blockIdx.x / kRouteSegment : 0u;
     {
         constexpr uint32_t kBatch = kRouteSegment / 4u;
-        const uint32_t part = tid >> 6, quad = tid & 63, b0 = segment * kRouteSegment + part;
-        uint2 sum = make_uint2(0u, 0u);
-        if (b0 < blockIdx.x) {
-            uint2 c[kBatch];
+        const uint32_t part = tid >> 6, quad = tid & 63;
+        uint32_t n[4] = {};
+        auto add = [&](uint32_t b0) {
+            uint2 c[kBatch], sum = make_uint2(0u, 0u);
 #pragma unroll
             for (uint32_t k = 0; k < kBatch; ++k)
                 c[k] = b0 + 4u * k < blockIdx.x
                            ? __ldcg(reinterpret_cast<const uint2 *>(p.block_hist) + (size_t)(b0 + 4u * k) * (kMaxExperts / 4) + quad) : make_uint2(0u, 0u);
 #pragma unroll
             for (uint32_t k = 0; k < kBatch; ++k) { sum.x += c[k].x; sum.y += c[k].y; }      // (32 x 256 fits 16 bits)
+            n[0] += sum.x & 0xFFFFu; n[1] += sum.x >> 16; n[2] += sum.y & 0xFFFFu; n[3] += sum.y >> 16;
+        };
+        if constexpr (LONG) {
+            const uint32_t b0 = segment * kRouteSegment + part;
+            if (b0 < blockIdx.x) add(b0);
+        } else {
+            for (uint32_t b0 = part; b0 < blockIdx.x; b0 += 4u * kBatch) add(b0);
         }
-        *reinterpret_cast<uint4 *>(&before[part][4 * quad]) = make_uint4(sum.x & 0xFFFFu, sum.x >> 16, sum.y & 0xFFFFu, sum.y >> 16);
+        *reinterpret_cast<uint4 *>(&before[part][4 * quad]) = make_uint4(n[0], n[1], n[2], n[3]);
     }
     const bool live = e != kBpNotLocal;
     if (mine && !live) p.inv[i] = kBpNotLocal;
@@ -365,7 +378,7 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(RouteParams p) {
     __syncthreads();
     if (live) {
         uint32_t pos = __ldcg(p.first + e) + rank;
-        if (segment != 0u) pos += __ldcg(p.first + segment * kMaxExperts + e);
+        if (LONG && segment != 0u) pos += __ldcg(p.first + segment * kMaxExperts + e);
 #pragma unroll
         for (int q = 0; q < 4; ++q) pos += before[q][e];
         for (int w = 0; w < warp; ++w) pos += cnt[w][e];

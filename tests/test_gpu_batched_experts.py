@@ -202,13 +202,13 @@ def test_rows_at_the_borders_of_the_routing_blocks_match_the_oracle(tokens):
 
 
 # More than 128 routing blocks of 32 tokens: a block's first pair is found from the counts of its own segment of 128 blocks and the
-# totals of those in front (8225: three segments, the last of two blocks).
-@pytest.mark.parametrize("tokens", [4096, 4097, 8225])
+# totals of those in front (8225: three segments, the last of two blocks).  Up to 768 rows the kernels know of one segment only.
+@pytest.mark.parametrize("tokens", [768, 769, 4096, 4097, 8225])
 def test_rows_past_a_segment_of_routing_blocks_match_the_oracle(tokens):
     host = _host_layer(78, 4, BF16, 256, 128, 256)
     cfg = MoEConfig(d=256, f=128, shared_f=128, num_experts=256, top_k=8, routed_bits=4, shared_bits=4, meta_dtype=BF16,
                     out_dtype=fmt.OUT_FP32, max_tokens=tokens)
-    sample = sorted({t for t in (0, 4063, 4064, 4095, 4096, 8191, 8192, 8223, tokens - 1) if t < tokens})
+    sample = sorted({t for t in (0, 759, 760, 767, 4063, 4064, 4095, 4096, 8191, 8192, 8223, tokens - 1) if t < tokens})
     assert _worst_error(host, cfg, "prefill", tokens, sample) < _tol(BF16, fmt.OUT_FP32, "prefill")
 
 
